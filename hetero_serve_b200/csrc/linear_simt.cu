@@ -11,186 +11,201 @@
 // Every output element is one chain of fused multiply-adds over k = 0..K-1 in index order,
 // whatever M is and wherever the row sits in its tile: a row's result does not depend on
 // the batch it is computed in.  No tensor cores, no TF32, no split over K.
-#include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace hs {
 
-constexpr int LS_BM = 64, LS_BN = 64, LS_BK = 16, LS_THREADS = 256;
-
 // four consecutive elements of a row in one load (the rows are 16-byte / 8-byte aligned there)
-__device__ __forceinline__ void lb_load4(const float* p, float (&v)[4]) {
+__device__ __forceinline__ void ls_load4(const float* p, float (&v)[4]) {
   const float4 x = *(const float4*)p;
   v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
 }
-__device__ __forceinline__ void lb_load4(const __nv_bfloat16* p, float (&v)[4]) {
+__device__ __forceinline__ void ls_load4(const __nv_bfloat16* p, float (&v)[4]) {
   const uint2 x = *(const uint2*)p;
   v[0] = __uint_as_float(x.x << 16); v[1] = __uint_as_float(x.x & 0xffff0000u);
   v[2] = __uint_as_float(x.y << 16); v[3] = __uint_as_float(x.y & 0xffff0000u);
 }
 
+// Where lanes read 16 bytes each and share addresses, a warp's read takes two wavefronts of shared
+// memory when the lanes of a pair (2i, 2i + 1) or all but every eighth agree, and four otherwise
+// (counted: lane % 8 -> four, (lane >> 1) & 7 -> two).  So eight columns go to lane bits 1-3 and
+// four rows to bits 0 and 4.
+__device__ __forceinline__ int ls_col(int lane) { return (lane >> 1) & 7; }
+__device__ __forceinline__ int ls_row(int lane) { return (lane & 1) | ((lane >> 3) & 2); }
 
-// VEC: K is a multiple of 4 and both matrices start on a 16-byte boundary: a thread's four k
-// of a row come in one load.
-template <typename TI, typename TO, bool VEC>
-__global__ void __launch_bounds__(LS_THREADS)
-linear_simt_kernel(TO* out, const TI* __restrict__ a, const TI* __restrict__ w,
-                   const float* __restrict__ bias, const float* residual, int M, int N, int K,
-                   int act, float2 ab) {
-  __shared__ float As[LS_BK][LS_BM + 4];
-  __shared__ float Ws[LS_BK][LS_BN + 4];
-  const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;
-  const int m0 = blockIdx.y * LS_BM, n0 = blockIdx.x * LS_BN;
-  // loader mapping: thread -> (row 0..63, 4 consecutive k)
-  const int lr = tid >> 2, lk = (tid & 3) * 4;
-  float acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-
-  for (int k0 = 0; k0 < K; k0 += LS_BK) {
-    {
-      const int gm = m0 + lr, gn = n0 + lr;
-      if (VEC) {
-        float ra[4] = {0.f, 0.f, 0.f, 0.f}, rw[4] = {0.f, 0.f, 0.f, 0.f};
-        const int gk = k0 + lk;                           // K % 4 == 0: all four or none
-        if (gm < M && gk < K) lb_load4(a + (size_t)gm * K + gk, ra);
-        if (gn < N && gk < K) lb_load4(w + (size_t)gn * K + gk, rw);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          As[lk + j][lr] = ra[j];
-          Ws[lk + j][lr] = rw[j];
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int gk = k0 + lk + j;
-          As[lk + j][lr] = (gm < M && gk < K) ? to_f(a[(size_t)gm * K + gk]) : 0.f;
-          Ws[lk + j][lr] = (gn < N && gk < K) ? to_f(w[(size_t)gn * K + gk]) : 0.f;
-        }
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < LS_BK; ++kk) {
-      float av[4], wv[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) av[i] = As[kk][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) wv[j] = Ws[kk][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], wv[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int gm = m0 + ty * 4 + i;
-    if (gm >= M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int gn = n0 + tx * 4 + j;
-      if (gn >= N) continue;
-      float v = acc[i][j];
-      if (bias) v += bias[gn];
-      v = apply_act(v, act, ab);
-      if (residual) v += residual[(size_t)gm * N + gn];
-      out[(size_t)gm * N + gn] = from_f<TO>(v);
-    }
-  }
+// Two fused multiply-adds in one instruction, each rounded as fmaf rounds (fma.rn.f32x2): half as
+// many issue slots go to the products.
+__device__ __forceinline__ void fma2(uint64_t& acc, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ uint64_t twice(float a) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
+  return r;
 }
 
-// ---- many rows (prompts): 128 x 128 tiles, an 8 x 8 patch of outputs per thread ---------------
-// The same chains again (every output one fmaf chain over k = 0..K-1 in index order), with
-// twice the outputs per shared-memory word read: a thread's 64 outputs take 16 words per k.
-// Tiles of both operands arrive k-major ([k][row]) through registers, two buffers.
-constexpr int LB_BM = 128, LB_BN = 128, LB_BK = 8, LB_THREADS = 256;
+// ---- many rows (prompts): tiles of 64 x 64 outputs (H = 2) or 32 x 32 (H = 1) -----------------
+// A CTA is two warps, a thread owns a patch of 8 x 8 (4 x 4) outputs; several CTAs share an SM, so
+// the tiles of a layer spread evenly (1,024 x 1,024 outputs are 64 tiles of 128 x 128, which left
+// 84 of 148 SMs idle) and one CTA's products cover another's loads and barriers.  Both operands are kept k-major ([k][row]), a
+// row's column XORed with a multiple of four that depends on k, so that neither the 4-byte stores
+// nor the 16-byte reads meet a bank conflict.  32-bit operands are scattered there by 4-byte
+// cp.async copies through a ring of LT_STAGES stages of 8 k (fetched through registers, one stage
+// ahead, the L2's latency was exposed in every stage); bfloat16 ones go through registers.
+// Measured (float32, one B200, before -> now; the form before fetched 128 x 128 tiles through
+// registers and used single FMAs): 2,048 x 4,096 x 1,024 485 -> 384 us (44.8 TFLOP/s, FMA pipe 60 %
+// busy, shared-memory pipe 70 %), 1,024 x 1,024 x 4,096 632 -> 316 us, 256 x 1,024 x 4,096 660 -> 163.
+constexpr int LT_BK = 8, LT_THREADS = 64, LT_STAGES = 4;
 
-// VEC: K is a multiple of 4 and both matrices start on a 16-byte boundary, so a thread's four
-// k of a row come in one load (with one 4-byte load per element the load pipe, 16 sectors an
-// instruction, took as long as the products).
-template <typename TI, typename TO, bool VEC>
-__global__ void __launch_bounds__(LB_THREADS)
-linear_simt_big_kernel(TO* out, const TI* __restrict__ a, const TI* __restrict__ w,
-                       const float* __restrict__ bias, const float* residual, int M, int N, int K,
-                       int act, float2 ab) {
-  __shared__ __align__(16) float As[2][LB_BK][LB_BM];
-  __shared__ __align__(16) float Ws[2][LB_BK][LB_BN];
-  const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;                 // 16 x 16 threads, 8 x 8 outputs each
-  const int m0 = blockIdx.y * LB_BM, n0 = blockIdx.x * LB_BN;
-  // loader: thread -> (row 0..127, 4 consecutive k of the 8)
-  const int lr = tid >> 1, lk = (tid & 1) * 4;
-  float acc[8][8];
+__device__ __forceinline__ int lt_swizzle(int k) { return (k & 7) << 2; }
+
+// LOAD: 2 (32-bit operands): asynchronous copies; 1: K is a multiple of 4 and both matrices start on
+// an 8-byte (32-bit: 16-byte) boundary, so a thread's four k of a row come in one load; 0: any.
+template <typename TI, typename TO, int H, int LOAD>
+__global__ void __launch_bounds__(LT_THREADS)
+linear_simt_tile_kernel(TO* out, const TI* __restrict__ a, const TI* __restrict__ w,
+                        const float* __restrict__ bias, const float* residual, int M, int N, int K,
+                        int act, float2 ab) {
+  constexpr int LT_BM = 32 * H, LT_BN = 32 * H, P = 4 * H;
+  constexpr int BUFS = LOAD == 2 ? LT_STAGES : 2;
+  __shared__ __align__(16) float As[BUFS][LT_BK][LT_BM];
+  __shared__ __align__(16) float Ws[BUFS][LT_BK][LT_BN];
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int tx = ls_col(lane), ty = ls_row(lane) | ((tid >> 5) << 2);
+  const int m0 = blockIdx.y * LT_BM, n0 = blockIdx.x * LT_BN;
+  uint64_t acc[P][P / 2];
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < P; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-  float ra[4], rw[4];
-  auto fetch = [&](int k0) {
-    const int gm = m0 + lr, gn = n0 + lr;
-    if (VEC) {
-      const int gk = k0 + lk;                             // K % 4 == 0: all four or none
+    for (int j = 0; j < P / 2; ++j) acc[i][j] = 0;
+
+  auto products = [&](int buf) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) ra[j] = rw[j] = 0.f;
-      if (gm < M && gk < K) lb_load4(a + (size_t)gm * K + gk, ra);
-      if (gn < N && gk < K) lb_load4(w + (size_t)gn * K + gk, rw);
-    } else {
+    for (int kk = 0; kk < LT_BK; ++kk) {
+      // rows ty*4..+3 and columns tx*4..+3 of each half
+      const int sx = lt_swizzle(kk);
+      float av[P];
+      uint64_t wv[P / 2];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int gk = k0 + lk + j;
-        ra[j] = (gm < M && gk < K) ? to_f(a[(size_t)gm * K + gk]) : 0.f;
-        rw[j] = (gn < N && gk < K) ? to_f(w[(size_t)gn * K + gk]) : 0.f;
+      for (int u = 0; u < H; ++u) {
+        const float4 x = *(const float4*)&As[buf][kk][32 * u + ((ty * 4) ^ sx)];
+        const ulonglong2 y = *(const ulonglong2*)&Ws[buf][kk][32 * u + ((tx * 4) ^ sx)];
+        av[4 * u] = x.x; av[4 * u + 1] = x.y; av[4 * u + 2] = x.z; av[4 * u + 3] = x.w;
+        wv[2 * u] = y.x; wv[2 * u + 1] = y.y;
+      }
+#pragma unroll
+      for (int i = 0; i < P; ++i) {
+        const uint64_t a2 = twice(av[i]);
+#pragma unroll
+        for (int j = 0; j < P / 2; ++j) fma2(acc[i][j], a2, wv[j]);
       }
     }
   };
-  auto stash = [&](int buf) {
+  // rows past the last one repeat it (their outputs are never stored); k past the end is zero
+  if constexpr (LOAD == 2) {
+    // a warp copies the eight k of four rows at a time: thread -> k, rows lr + 8 i
+    const int lk = tid & 7, lr = tid >> 3;
+    const int n_kt = (K + LT_BK - 1) / LT_BK;
+    uint32_t sa[2];
+    sa[0] = (uint32_t)__cvta_generic_to_shared(&As[0][lk][0]);
+    sa[1] = (uint32_t)__cvta_generic_to_shared(&Ws[0][lk][0]);
+    int row_a[4 * H], row_w[4 * H];                       // offsets of the rows from the tile's first
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      As[buf][lk + j][lr] = ra[j];
-      Ws[buf][lk + j][lr] = rw[j];
+    for (int i = 0; i < 4 * H; ++i) {
+      row_a[i] = min(lr + 8 * i, M - 1 - m0) * K;
+      row_w[i] = min(lr + 8 * i, N - 1 - n0) * K;
     }
-  };
-  fetch(0);
-  stash(0);
-  __syncthreads();
-  int buf = 0;
-  for (int k0 = 0; k0 < K; k0 += LB_BK) {
-    const bool more = k0 + LB_BK < K;
-    if (more) fetch(k0 + LB_BK);                          // in flight during the products below
+    const TI* a_t = a + (size_t)m0 * K;
+    const TI* w_t = w + (size_t)n0 * K;
+    auto issue = [&](int kt) {
+      if (kt < n_kt) {
+        const int gk = kt * LT_BK + lk;
+        const int n = gk < K ? 4 : 0;
+        const int ck = gk < K ? gk : 0;
+        const uint32_t to = (uint32_t)((kt % LT_STAGES) * LT_BK * LT_BM * 4);
 #pragma unroll
-    for (int kk = 0; kk < LB_BK; ++kk) {
-      // rows ty*4..+3 and 64+ty*4..+3, columns tx*4..+3 and 64+tx*4..+3: 16-byte reads, no
-      // bank conflicts
-      const float4 a0 = *(const float4*)&As[buf][kk][ty * 4];
-      const float4 a1 = *(const float4*)&As[buf][kk][64 + ty * 4];
-      const float4 w0 = *(const float4*)&Ws[buf][kk][tx * 4];
-      const float4 w1 = *(const float4*)&Ws[buf][kk][64 + tx * 4];
-      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-      const float wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(av[i], wv[j], acc[i][j]);
+        for (int i = 0; i < 4 * H; ++i) {
+          const uint32_t col = (uint32_t)((((lr + 8 * i) & 31) ^ lt_swizzle(lk)) + (i >= 4 ? 32 : 0)) * 4;
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(sa[0] + to + col),
+                       "l"(a_t + row_a[i] + ck), "r"(n) : "memory");
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(sa[1] + to + col),
+                       "l"(w_t + row_w[i] + ck), "r"(n) : "memory");
+        }
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (int s = 0; s < LT_STAGES - 1; ++s) issue(s);
+#pragma unroll 1
+    for (int kt = 0; kt < n_kt; ++kt) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(LT_STAGES - 2) : "memory");
+      __syncthreads();               // stage kt has landed; stage kt - 1 is free for every thread
+      issue(kt + LT_STAGES - 1);
+      products(kt % LT_STAGES);
     }
-    if (more) {
-      stash(buf ^ 1);
-      __syncthreads();
-      buf ^= 1;
+  } else {
+    // thread -> row lr of each half, four consecutive k of the 8
+    const int lr = tid >> 1, lk = (tid & 1) * 4;
+    const TI *ap[H], *wp[H];
+    float ra[H][4], rw[H][4];
+#pragma unroll
+    for (int i = 0; i < H; ++i) {
+      ap[i] = a + (size_t)min(m0 + lr + 32 * i, M - 1) * K;
+      wp[i] = w + (size_t)min(n0 + lr + 32 * i, N - 1) * K;
+    }
+    auto fetch = [&](int k0) {
+      const int gk = k0 + lk;
+#pragma unroll
+      for (int i = 0; i < H; ++i) {
+        if (LOAD == 1) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) ra[i][j] = rw[i][j] = 0.f;
+          if (gk < K) {                                   // K % 4 == 0: all four or none
+            ls_load4(ap[i] + gk, ra[i]);
+            ls_load4(wp[i] + gk, rw[i]);
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            ra[i][j] = gk + j < K ? to_f(ap[i][gk + j]) : 0.f;
+            rw[i][j] = gk + j < K ? to_f(wp[i][gk + j]) : 0.f;
+          }
+        }
+      }
+    };
+    auto stash = [&](int buf) {
+#pragma unroll
+      for (int i = 0; i < H; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          As[buf][lk + j][(lr ^ lt_swizzle(lk + j)) + 32 * i] = ra[i][j];
+          Ws[buf][lk + j][(lr ^ lt_swizzle(lk + j)) + 32 * i] = rw[i][j];
+        }
+    };
+    fetch(0);
+    stash(0);
+    __syncthreads();
+    int buf = 0;
+#pragma unroll 1
+    for (int k0 = 0; k0 < K; k0 += LT_BK) {
+      const bool more = k0 + LT_BK < K;
+      if (more) fetch(k0 + LT_BK);                        // in flight during the products below
+      products(buf);
+      if (more) {
+        stash(buf ^ 1);
+        __syncthreads();
+        buf ^= 1;
+      }
     }
   }
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int gm = m0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + (i - 4));
+  for (int i = 0; i < P; ++i) {
+    const int gm = m0 + 32 * (i >> 2) + ty * 4 + (i & 3);
     if (gm >= M) continue;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int gn = n0 + (j < 4 ? tx * 4 + j : 64 + tx * 4 + (j - 4));
+    for (int j = 0; j < P; ++j) {
+      const int gn = n0 + 32 * (j >> 2) + tx * 4 + (j & 3);
       if (gn >= N) continue;
-      float v = acc[i][j];
+      float v = __uint_as_float((uint32_t)(acc[i][j >> 1] >> ((j & 1) * 32)));
       if (bias) v += bias[gn];
       v = apply_act(v, act, ab);
       if (residual) v += residual[(size_t)gm * N + gn];
@@ -200,104 +215,142 @@ linear_simt_big_kernel(TO* out, const TI* __restrict__ a, const TI* __restrict__
 }
 
 // ---- few rows (decode): the same chains, laid out for a weight stream -------------------------
-// With M <= 16 the tile kernel above leaves most of the machine idle (N / 64 CTAs, each walking
-// all of K behind two barriers per 16 columns).  Here a CTA owns 16 output features and all
-// rows; thread (feature f, row group g) runs the chains of rows g and g + 8 for feature f over
-// k = 0..K-1 in index order - the same chain of fused multiply-adds, so the same bits, as the
-// tile kernel gives that element.  The weight rows and the activation rows arrive through a
-// ring of four 128-column stages of 16-byte cp.async copies.  RPT rows per thread: 2 for up to
-// 16 rows, 8 for up to 64 (rows g, g + 8, ..., g + 56).
-constexpr int LF_BN = 16, LF_BK = 128, LF_THREADS = 128, LF_STAGES = 4;
-
-template <typename TI, int RPT>
+// An output is one chain of K dependent FMAs, so no layout is through before 4 K cycles (2.1 us
+// at K = 1,024); what a layout can do is to keep that chain fed.  A CTA owns F features.  Lane
+// (f, g) of a consumer warp runs the chains of RPT rows (g, g + G, ...) for feature f.  One more
+// warp fetches: weight and activation rows arrive in stages of BK k through a ring of 16-byte
+// cp.async copies that arrive on an mbarrier (the copies' addresses and issue slots, in the
+// consumers' own instruction stream, took longer than the chain).  Rows are padded by 16 bytes
+// against bank conflicts; the operands of the next 16 (8) k are read from shared memory while this
+// set's chains run.  Measured (float32, M x N x K, before -> now): 8 x 1,024 x 4,096 53.5 -> 19.3 us,
+// 8 x 3,072 x 1,024 17.9 -> 11.2, 64 x 4,096 x 1,024 45.9 -> 28.3, 8 x 50,257 x 1,024 146 -> 88.
+template <typename TI, int RPT, int F, int WARPS>
 struct LfShape {
-  static constexpr int MAX_M = 8 * RPT;
-  static constexpr int VEC = 16 / (int)sizeof(TI);           // elements per 16-byte copy
-  static constexpr int WS = LF_BK + VEC;                     // weight row stride: no bank conflicts
-  static constexpr int STAGE = LF_BN * WS + MAX_M * LF_BK;   // elements per stage
-  static constexpr size_t SMEM = (size_t)LF_STAGES * STAGE * sizeof(TI);
+  static constexpr int G = 32 / F * WARPS;                   // row groups
+  static constexpr int ROWS = G * RPT;
+  static constexpr int BK = ROWS <= 16 ? 128 : 64;           // k per stage
+  static constexpr int VEC = 16 / (int)sizeof(TI);           // elements per 16 bytes
+  static constexpr int LD = BK + VEC;                        // row stride in shared memory
+  static constexpr int STAGE = (F + ROWS) * LD;              // elements per stage
+  static constexpr int STAGES = sizeof(TI) * STAGE * 6 <= 56 * 1024 ? 6 : 4;
+  static constexpr size_t SMEM = (size_t)STAGES * STAGE * sizeof(TI);
 };
 
-__device__ __forceinline__ void lf_copy16(void* smem_dst, const void* src, bool valid) {
-  const int n = valid ? 16 : 0;                              // 0: the 16 bytes are zero-filled
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(smem_dst)), "l"(src),
-               "r"(n)
-               : "memory");
-}
-__device__ __forceinline__ void lf_load4(const float* p, float (&v)[4]) {
-  const float4 x = *(const float4*)p;
-  v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
-}
-__device__ __forceinline__ void lf_load4(const __nv_bfloat16* p, float (&v)[4]) {
-  const uint2 x = *(const uint2*)p;
-  v[0] = __uint_as_float(x.x << 16); v[1] = __uint_as_float(x.x & 0xffff0000u);
-  v[2] = __uint_as_float(x.y << 16); v[3] = __uint_as_float(x.y & 0xffff0000u);
-}
-
-template <typename TI, typename TO, int RPT>
-__global__ void __launch_bounds__(LF_THREADS)
+// K is a multiple of 16 bytes and both matrices start on a 16-byte boundary.
+template <typename TI, typename TO, int RPT, int F, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32 + 32)
 linear_simt_few_rows_kernel(TO* out, const TI* __restrict__ a, const TI* __restrict__ w,
                             const float* __restrict__ bias, const float* residual, int M, int N,
-                            int K, int act, float2 ab) {
-  using S = LfShape<TI, RPT>;
+                            int K, int act, float2 ab, int* status) {
+  using S = LfShape<TI, RPT, F, WARPS>;
+  constexpr int BK = S::BK;
   extern __shared__ __align__(16) uint8_t lf_smem[];
+  __shared__ uint64_t full[S::STAGES], empty[S::STAGES];
   TI* ring = (TI*)lf_smem;
-  const int tid = threadIdx.x;
-  const int f = tid & 15, grp = tid >> 4;                    // rows grp, grp + 8, ...
-  const int n0 = blockIdx.x * LF_BN;
-  const int num_kt = (K + LF_BK - 1) / LF_BK;
-  constexpr int CPR = LF_BK / S::VEC;                        // copies per row of a stage
-
-  auto issue = [&](int kt) {
-    if (kt < num_kt) {
-      TI* sw = ring + (size_t)(kt % LF_STAGES) * S::STAGE;
-      TI* sa = sw + LF_BN * S::WS;
-      for (int c = tid; c < LF_BN * CPR; c += LF_THREADS) {
-        const int row = c / CPR, kc = (c - row * CPR) * S::VEC;
-        const int gk = kt * LF_BK + kc, gn = n0 + row;
-        const bool ok = gn < N && gk < K;
-        lf_copy16(sw + row * S::WS + kc, ok ? w + (size_t)gn * K + gk : w, ok);
-      }
-      for (int c = tid; c < S::MAX_M * CPR; c += LF_THREADS) {
-        const int row = c / CPR, kc = (c - row * CPR) * S::VEC;
-        const int gk = kt * LF_BK + kc;
-        const bool ok = row < M && gk < K;
-        lf_copy16(sa + row * LF_BK + kc, ok ? a + (size_t)row * K + gk : a, ok);
-      }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n0 = blockIdx.x * F;
+  const int num_kt = (K + BK - 1) / BK;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < S::STAGES; ++s) {
+      mbar_init(&full[s], 32);
+      mbar_init(&empty[s], WARPS);
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");   // one group per call, empty or not
-  };
-
-  for (int s = 0; s < LF_STAGES - 1; ++s) issue(s);
+    fence_barrier_init();
+  }
+  __syncthreads();
+  if (warp == WARPS) {
+    // the copying warp: RPI rows a trip, a lane per 16-byte piece.  Rows past the last one repeat
+    // it (nothing is stored for them); pieces past the end of K are left out
+    constexpr int CPR = BK / S::VEC;                         // pieces per row of a stage
+    constexpr int RPI = 32 / CPR;
+    const int crow = lane / CPR, ck = (lane % CPR) * S::VEC;
+    const uint32_t ring_at = smem_u32(ring) + (uint32_t)(crow * S::LD + ck) * (uint32_t)sizeof(TI);
+    for (int kt = 0; kt < num_kt; ++kt) {
+      const int s = kt % S::STAGES;
+      if (kt >= S::STAGES && !mbar_wait(&empty[s], ((kt / S::STAGES) - 1) & 1, status)) break;
+      const int gk = kt * BK + ck;
+      if (gk < K) {
+        uint32_t to = ring_at + (uint32_t)(s * S::STAGE) * (uint32_t)sizeof(TI);
+#pragma unroll
+        for (int row = 0; row < F; row += RPI) {
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to),
+                       "l"(w + (size_t)min(n0 + row + crow, N - 1) * K + gk) : "memory");
+          to += RPI * S::LD * (uint32_t)sizeof(TI);
+        }
+#pragma unroll 8
+        for (int row = 0; row < S::ROWS; row += RPI) {
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to),
+                       "l"(a + (size_t)min(row + crow, M - 1) * K + gk) : "memory");
+          to += RPI * S::LD * (uint32_t)sizeof(TI);
+        }
+      }
+      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&full[s]))
+                   : "memory");
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    return;
+  }
+  const int f = F == 8 ? ls_col(lane) : lane >> 1;         // (F is 8 or 16)
+  const int g = warp * (32 / F) + (F == 8 ? ls_row(lane) : lane & 1);
   float acc[RPT];
 #pragma unroll
   for (int r = 0; r < RPT; ++r) acc[r] = 0.f;
+  constexpr int U = RPT > 2 ? 8 : 16;                        // k per register set
+  struct Set { float w[U], x[RPT][U]; };
   for (int kt = 0; kt < num_kt; ++kt) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(LF_STAGES - 2) : "memory");
-    __syncthreads();                 // stage kt has landed; stage kt - 1 is free for every thread
-    issue(kt + LF_STAGES - 1);
-    const TI* sw = ring + (size_t)(kt % LF_STAGES) * S::STAGE + f * S::WS;
-    const TI* sa = ring + (size_t)(kt % LF_STAGES) * S::STAGE + LF_BN * S::WS + grp * LF_BK;
-    const int kmax = min(LF_BK, K - kt * LF_BK);             // a multiple of 4
-#pragma unroll 4
-    for (int k = 0; k < kmax; k += 4) {
-      float wv[4];
-      lf_load4(sw + k, wv);
+    const int st = kt % S::STAGES;
+    if (!mbar_wait(&full[st], (kt / S::STAGES) & 1, status)) return;
+    const TI* sw = ring + (size_t)st * S::STAGE + f * S::LD;
+    const TI* sa = ring + (size_t)st * S::STAGE + (F + g) * S::LD;
+    auto read = [&](int k, Set& s) {
 #pragma unroll
-      for (int r = 0; r < RPT; ++r) {
-        float x[4];
-        lf_load4(sa + r * 8 * LF_BK + k, x);
+      for (int q = 0; q < U; q += 4) {
+        ls_load4(sw + k + q, *(float(*)[4])&s.w[q]);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) acc[r] = fmaf(x[i], wv[i], acc[r]);
+        for (int r = 0; r < RPT; ++r)
+          ls_load4(sa + r * S::G * S::LD + k + q, *(float(*)[4])&s.x[r][q]);
+      }
+    };
+    auto products = [&](const Set& s, int n) {
+      if (n >= U) {
+#pragma unroll
+        for (int q = 0; q < U; ++q)
+#pragma unroll
+          for (int r = 0; r < RPT; ++r) acc[r] = fmaf(s.x[r][q], s.w[q], acc[r]);
+      } else {                                               // the end of K: no product past it
+#pragma unroll
+        for (int q = 0; q < U; ++q)
+          if (q < n) {
+#pragma unroll
+            for (int r = 0; r < RPT; ++r) acc[r] = fmaf(s.x[r][q], s.w[q], acc[r]);
+          }
+      }
+    };
+    const int kmax = min(BK, K - kt * BK);                   // a multiple of 4
+    Set s0, s1;
+    read(0, s0);
+    if (kmax == BK) {
+#pragma unroll
+      for (int k = 0; k < BK; k += 2 * U) {
+        read(k + U, s1);
+        products(s0, U);
+        if (k + 2 * U < BK) read(k + 2 * U, s0);
+        products(s1, U);
+      }
+    } else {
+      for (int k = 0; k < kmax; k += U) {
+        products(s0, kmax - k);
+        if (k + U < kmax) read(k + U, s0);
       }
     }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&empty[st]);
   }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
   const int gn = n0 + f;
   if (gn >= N) return;
 #pragma unroll
   for (int r = 0; r < RPT; ++r) {
-    const int gm = grp + 8 * r;
+    const int gm = g + S::G * r;
     if (gm >= M) continue;
     float v = acc[r];
     if (bias) v += bias[gn];
@@ -307,95 +360,93 @@ linear_simt_few_rows_kernel(TO* out, const TI* __restrict__ a, const TI* __restr
   }
 }
 
-template <typename TI, typename TO, int RPT>
+template <typename TI, typename TO, int RPT, int F, int WARPS>
 static int launch_few_rows_as(void* out, const void* a, const void* w, const float* bias,
                               const float* residual, int M, int N, int K, int act, float2 ab,
-                              cudaStream_t st) {
-  auto* k = linear_simt_few_rows_kernel<TI, TO, RPT>;
+                              int* status, cudaStream_t st) {
+  using S = LfShape<TI, RPT, F, WARPS>;
+  auto* k = linear_simt_few_rows_kernel<TI, TO, RPT, F, WARPS>;
   static cudaError_t state = cudaErrorUnknown;
   if (state != cudaSuccess)
-    state = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)LfShape<TI, RPT>::SMEM);
+    state = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
   if (state != cudaSuccess) return (int)state;
-  k<<<(N + LF_BN - 1) / LF_BN, LF_THREADS, LfShape<TI, RPT>::SMEM, st>>>(
-      (TO*)out, (const TI*)a, (const TI*)w, bias, residual, M, N, K, act, ab);
+  k<<<(N + F - 1) / F, WARPS * 32 + 32, S::SMEM, st>>>(
+      (TO*)out, (const TI*)a, (const TI*)w, bias, residual, M, N, K, act, ab, status);
   return HS_OK;
 }
 
 template <typename TI, typename TO>
 static int launch_few_rows(void* out, const void* a, const void* w, const float* bias,
-                           const float* residual, int M, int N, int K, int act, float2 ab, cudaStream_t st) {
-  if (M <= 16) return launch_few_rows_as<TI, TO, 2>(out, a, w, bias, residual, M, N, K, act, ab, st);
-  return launch_few_rows_as<TI, TO, 8>(out, a, w, bias, residual, M, N, K, act, ab, st);
+                           const float* residual, int M, int N, int K, int act, float2 ab,
+                           int* status, cudaStream_t st) {
+  if (M <= 4) return launch_few_rows_as<TI, TO, 1, 8, 1>(out, a, w, bias, residual, M, N, K, act, ab, status, st);
+  if (M <= 8) return launch_few_rows_as<TI, TO, 2, 8, 1>(out, a, w, bias, residual, M, N, K, act, ab, status, st);
+  if (M <= 16) return launch_few_rows_as<TI, TO, 2, 8, 2>(out, a, w, bias, residual, M, N, K, act, ab, status, st);
+  // 16 features a CTA where that still gives every SM one, else 8 (64 rows of 1,024 features: 64
+  // CTAs took 62 us at k = 4,096)
+  const bool wide = (N + 15) / 16 >= hs_sm_count();
+  if (M <= 32) return wide ? launch_few_rows_as<TI, TO, 4, 16, 4>(out, a, w, bias, residual, M, N, K, act, ab, status, st)
+                           : launch_few_rows_as<TI, TO, 2, 8, 4>(out, a, w, bias, residual, M, N, K, act, ab, status, st);
+  return wide ? launch_few_rows_as<TI, TO, 8, 16, 4>(out, a, w, bias, residual, M, N, K, act, ab, status, st)
+              : launch_few_rows_as<TI, TO, 4, 8, 4>(out, a, w, bias, residual, M, N, K, act, ab, status, st);
 }
 
 }  // namespace hs
 
 HS_EXPORT int hs_linear_simt(void* out, const void* a, const void* w, const float* bias,
                              const float* residual, int M, int N, int K, int act, float act_a,
-                             float act_b, int in_dtype, int out_dtype, void* stream) {
+                             float act_b, int in_dtype, int out_dtype, int* status, void* stream) {
   const float2 ab = make_float2(act_a, act_b);
-  if (!out || !a || !w) return HS_ERR_ARGUMENT;
+  if (!out || !a || !w || !status) return HS_ERR_ARGUMENT;
   if (M <= 0 || N <= 0) return HS_OK;
   if (K <= 0) return HS_ERR_ARGUMENT;
   if (act < HS_ACT_NONE || act > HS_ACT_LAST) return HS_ERR_UNSUPPORTED;
-  dim3 grid((N + hs::LS_BN - 1) / hs::LS_BN, (M + hs::LS_BM - 1) / hs::LS_BM);
-  if (grid.y > 65535) return HS_ERR_UNSUPPORTED;
   cudaStream_t st = (cudaStream_t)stream;
   using bf16 = __nv_bfloat16;
   // few rows: the weight-stream kernel (rows and pointers that 16-byte copies can take)
   const int vec = in_dtype == HS_DT_F32 ? 4 : 8;
-  // (17-64 rows: while the layer's feature blocks are a few per SM; a wide layer such as the
-  // vocabulary head keeps more in flight with the tile kernel: 233 us against 599 at 64 rows)
-  const bool few = M <= 16 || (M <= 64 && (N + hs::LF_BN - 1) / hs::LF_BN <= 4 * hs_sm_count());
+  const bool few = M <= 16 || (M <= 64 && (N + 15) / 16 <= 4 * hs_sm_count());
   if (few && K % vec == 0 && !((uintptr_t)a & 15) && !((uintptr_t)w & 15)) {
     int rc = HS_ERR_UNSUPPORTED;
     if (in_dtype == HS_DT_F32 && out_dtype == HS_DT_F32)
-      rc = hs::launch_few_rows<float, float>(out, a, w, bias, residual, M, N, K, act, ab, st);
+      rc = hs::launch_few_rows<float, float>(out, a, w, bias, residual, M, N, K, act, ab, status, st);
     else if (in_dtype == HS_DT_BF16 && out_dtype == HS_DT_BF16)
-      rc = hs::launch_few_rows<bf16, bf16>(out, a, w, bias, residual, M, N, K, act, ab, st);
+      rc = hs::launch_few_rows<bf16, bf16>(out, a, w, bias, residual, M, N, K, act, ab, status, st);
     else if (in_dtype == HS_DT_BF16 && out_dtype == HS_DT_F32)
-      rc = hs::launch_few_rows<bf16, float>(out, a, w, bias, residual, M, N, K, act, ab, st);
+      rc = hs::launch_few_rows<bf16, float>(out, a, w, bias, residual, M, N, K, act, ab, status, st);
     if (rc != HS_OK) return rc;
     HS_LAUNCH_CHECK();
     return HS_OK;
   }
-  if (M >= 256) {                    // prompts: the larger tile
-    dim3 big((N + hs::LB_BN - 1) / hs::LB_BN, (M + hs::LB_BM - 1) / hs::LB_BM);
-    if (big.y > 65535) return HS_ERR_UNSUPPORTED;
-    const bool vec4 = K % 4 == 0 && !((uintptr_t)a & 15) && !((uintptr_t)w & 15);
-#define HS_LB_LAUNCH(TI, TO)                                                                   \
+  // the large tile where it gives every SM about four (below that an SM has too few warps to hide
+  // its own latencies)
+  const long long large = (long long)((N + 63) / 64) * ((M + 63) / 64);
+  const int side = large >= 4ll * hs_sm_count() ? 64 : 32;
+  const dim3 grid((N + side - 1) / side, (M + side - 1) / side);
+  if (grid.y > 65535) return HS_ERR_UNSUPPORTED;
+#define HS_LT_LAUNCH(TI, TO, LOAD)                                                             \
   do {                                                                                         \
-    if (vec4)                                                                                  \
-      hs::linear_simt_big_kernel<TI, TO, true><<<big, hs::LB_THREADS, 0, st>>>(                \
-          (TO*)out, (const TI*)a, (const TI*)w, bias, residual, M, N, K, act, ab);                 \
+    if (side == 64)                                                                            \
+      hs::linear_simt_tile_kernel<TI, TO, 2, LOAD><<<grid, hs::LT_THREADS, 0, st>>>(           \
+          (TO*)out, (const TI*)a, (const TI*)w, bias, residual, M, N, K, act, ab);             \
     else                                                                                       \
-      hs::linear_simt_big_kernel<TI, TO, false><<<big, hs::LB_THREADS, 0, st>>>(               \
-          (TO*)out, (const TI*)a, (const TI*)w, bias, residual, M, N, K, act, ab);                 \
+      hs::linear_simt_tile_kernel<TI, TO, 1, LOAD><<<grid, hs::LT_THREADS, 0, st>>>(           \
+          (TO*)out, (const TI*)a, (const TI*)w, bias, residual, M, N, K, act, ab);             \
   } while (0)
-    if (in_dtype == HS_DT_F32 && out_dtype == HS_DT_F32) HS_LB_LAUNCH(float, float);
-    else if (in_dtype == HS_DT_BF16 && out_dtype == HS_DT_BF16) HS_LB_LAUNCH(bf16, bf16);
-    else if (in_dtype == HS_DT_BF16 && out_dtype == HS_DT_F32) HS_LB_LAUNCH(bf16, float);
-    else return HS_ERR_UNSUPPORTED;
-#undef HS_LB_LAUNCH
-    HS_LAUNCH_CHECK();
-    return HS_OK;
+  const bool vec4 = K % 4 == 0 && !((uintptr_t)a & 7) && !((uintptr_t)w & 7);
+  if (in_dtype == HS_DT_F32 && out_dtype == HS_DT_F32) {
+    if (64ll * K < (1ll << 31)) HS_LT_LAUNCH(float, float, 2);      // (32-bit offsets in a tile)
+    else HS_LT_LAUNCH(float, float, 0);
+  } else if (in_dtype == HS_DT_BF16 && out_dtype == HS_DT_BF16) {
+    if (vec4) HS_LT_LAUNCH(bf16, bf16, 1);
+    else HS_LT_LAUNCH(bf16, bf16, 0);
+  } else if (in_dtype == HS_DT_BF16 && out_dtype == HS_DT_F32) {
+    if (vec4) HS_LT_LAUNCH(bf16, float, 1);
+    else HS_LT_LAUNCH(bf16, float, 0);
+  } else {
+    return HS_ERR_UNSUPPORTED;
   }
-  const bool ls_vec = K % 4 == 0 && !((uintptr_t)a & 15) && !((uintptr_t)w & 15);
-#define HS_LS_LAUNCH(TI, TO)                                                                  \
-  do {                                                                                        \
-    if (ls_vec)                                                                               \
-      hs::linear_simt_kernel<TI, TO, true><<<grid, hs::LS_THREADS, 0, st>>>(                  \
-          (TO*)out, (const TI*)a, (const TI*)w, bias, residual, M, N, K, act, ab);                \
-    else                                                                                      \
-      hs::linear_simt_kernel<TI, TO, false><<<grid, hs::LS_THREADS, 0, st>>>(                 \
-          (TO*)out, (const TI*)a, (const TI*)w, bias, residual, M, N, K, act, ab);                \
-  } while (0)
-  if (in_dtype == HS_DT_F32 && out_dtype == HS_DT_F32) HS_LS_LAUNCH(float, float);
-  else if (in_dtype == HS_DT_BF16 && out_dtype == HS_DT_BF16) HS_LS_LAUNCH(bf16, bf16);
-  else if (in_dtype == HS_DT_BF16 && out_dtype == HS_DT_F32) HS_LS_LAUNCH(bf16, float);
-  else return HS_ERR_UNSUPPORTED;
-#undef HS_LS_LAUNCH
+#undef HS_LT_LAUNCH
   HS_LAUNCH_CHECK();
   return HS_OK;
 }

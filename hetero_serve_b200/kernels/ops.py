@@ -181,7 +181,7 @@ def _declare(lib) -> None:
     sig = {
         "hs_embed": [P, P, P, P, P, P, I, I, I, I, I, P, I, F, P, P],
         "hs_layernorm": [P, P, P, P, P, I, I, F, I, P],
-        "hs_linear_simt": [P, P, P, P, P, I, I, I, I, F, F, I, I, P],
+        "hs_linear_simt": [P, P, P, P, P, I, I, I, I, F, F, I, I, P, P],
         "hs_linear_tcgen05": [P, P, P, P, P, I, I, I, I, F, F, I, I, I, P, P, P, P],
         "hs_linear_tcgen05_scratch": [I, I, I, I, I, P, P],
         "hs_linear_skinny": [P, P, P, P, P, F, P, P, P, I, I, I, I, F, F, I, P, P, I, P],
@@ -568,7 +568,7 @@ class CudaOps:
                 return
         _check(self.lib.hs_linear_simt(_ptr(out), _ptr(a), _ptr(w), _ptr(bias), _ptr(residual),
                                        M, N, K, act, act_a, act_b, _DT[a.dtype],
-                                       _DT[out.dtype], self._stream()),
+                                       _DT[out.dtype], _ptr(self.status), self._stream()),
                f"linear(M={M},N={N},K={K})")
 
     def _skinny_ok(self, M, N, K) -> bool:
