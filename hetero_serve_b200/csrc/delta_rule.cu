@@ -17,7 +17,7 @@
 // neighbouring threads read neighbouring weights.
 //
 // State of a slot: [heads x D x V | (taps-1) x channels] floats.
-#include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace hs {
 
@@ -302,6 +302,273 @@ delta_recurrence_kernel(float* __restrict__ o, float* __restrict__ state,
   }
 }
 
+// ---- portions: four tokens at a time ----------------------------------------------------------
+// Token after token, the chain above is bounded by its latencies: a token's dot product with the
+// state, the butterfly over a column's lanes, the update (0.4 us a token, one warp a scheduler).
+// Four tokens i = 0..3 that start from the state S need only S itself:
+//     a_i = S^T K'_i,   K'_i = k_i g_0 .. g_i                 (g: decays, per row)
+//     u_i = beta_i (v_i - a_i - sum_{j<i} c_ij u_j),           c_ij  = sum k_i k_j g_j+1 .. g_i
+//     o_i = S^T Q'_i + sum_{j<=i} e_ij u_j,  Q'_i = q_i g_0 .. g_i,  e_ij = sum q_i k_j g_j+1 .. g_i
+//     S <- g_0 .. g_3 S + sum_j K"_j u_j,                      K"_j  = k_j g_j+1 .. g_3
+// so four butterflies overlap and the chain is paid once in four tokens.  The decays enter as
+// products of at most four factors below one (no quotients, nothing can overflow).  What does not
+// depend on the state (K', Q', K", the decay of all four, c, e, beta) is formed beforehand for all
+// tokens in parallel; a head's blocks lie one behind the other, so that a stage of the recurrence
+// is one bulk copy.  All of it is float32, packed two rows an instruction.  Measured: 2 x 1,024
+// tokens, 8 heads of 128 x 128, see the launch below.
+constexpr int DB_TOK = 4, DB_COEF = 32;
+constexpr int DB_STAGE_BLOCKS = 2, DB_STAGES = 4;
+constexpr int DB_WARPS = 4;                       // that work; one more fetches
+__host__ __device__ constexpr int db_floats(int D) { return 13 * D + DB_COEF; }
+
+// blocks of four tokens of the requests before r
+__device__ __forceinline__ int db_first(const int* __restrict__ req_len, int r) {
+  int b = 0;
+  for (int i = 0; i < r; ++i) b += (max(req_len[i], 0) + DB_TOK - 1) / DB_TOK;
+  return b;
+}
+
+__global__ void __launch_bounds__(128)
+delta_blocks_prepare_kernel(float* __restrict__ blocks, const float* __restrict__ qn,
+                            const float* __restrict__ kn, const float* __restrict__ beta,
+                            const float* __restrict__ decay, const int* __restrict__ req_start,
+                            const int* __restrict__ req_len, int n_requests, int cap_blocks,
+                            DeltaShape s) {
+  __shared__ float red[4][16];
+  const int h = blockIdx.y;
+  // the request this block of tokens belongs to
+  int blk = blockIdx.x, r = 0;
+  for (; r < n_requests; ++r) {
+    const int nb = (max(req_len[r], 0) + DB_TOK - 1) / DB_TOK;
+    if (blk < nb) break;
+    blk -= nb;
+  }
+  if (r >= n_requests) return;
+  const int n = min(DB_TOK, req_len[r] - blk * DB_TOK);       // tokens that exist
+  const int t0 = req_start[r] + blk * DB_TOK;
+  const int kh = h / (s.heads / s.kv_heads);
+  const int QK = s.kv_heads * s.D, HD = s.heads * s.D, D = s.D;
+  float* out = blocks + ((size_t)h * cap_blocks + blockIdx.x) * db_floats(D);
+  float c[6] = {}, e[10] = {};
+  for (int d = threadIdx.x; d < D; d += 128) {
+    float k[4], q[4], g[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const bool on = i < n;
+      k[i] = on ? kn[(size_t)(t0 + i) * QK + kh * D + d] : 0.f;
+      q[i] = on ? qn[(size_t)(t0 + i) * QK + kh * D + d] : 0.f;
+      g[i] = on ? decay[(size_t)(t0 + i) * HD + h * D + d] : 1.f;
+    }
+    float all = 1.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      all *= g[i];
+      out[i * D + d] = k[i] * all;
+      out[(4 + i) * D + d] = q[i] * all;
+      float rest = 1.f;
+#pragma unroll
+      for (int m = i + 1; m < 4; ++m) rest *= g[m];
+      out[(8 + i) * D + d] = k[i] * rest;
+    }
+    out[12 * D + d] = all;
+    int ci = 0, ei = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j <= i; ++j) {
+        float f = k[j];
+#pragma unroll
+        for (int m = j + 1; m <= i; ++m) f *= g[m];
+        e[ei] = fmaf(q[i], f, e[ei]);
+        ++ei;
+        if (j < i) {
+          c[ci] = fmaf(k[i], f, c[ci]);
+          ++ci;
+        }
+      }
+  }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const float v = warp_sum(i < 6 ? c[i < 6 ? i : 0] : e[i < 6 ? 0 : i - 6]);
+    if (lane == 0) red[warp][i] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x < DB_COEF) {
+    const int i = threadIdx.x;
+    float v = 0.f;
+    if (i < 16) v = (red[0][i] + red[1][i]) + (red[2][i] + red[3][i]);
+    else if (i < 20 && i - 16 < n) v = beta[(size_t)(t0 + i - 16) * s.heads + h];
+    out[13 * D + i] = v;
+  }
+}
+
+__device__ __forceinline__ void db_fma(uint64_t& acc, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ uint64_t db_mul(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t db_pair(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float db_fold(uint64_t a) {
+  return __uint_as_float((uint32_t)a) + __uint_as_float((uint32_t)(a >> 32));
+}
+
+// KS = D / 16 lanes hold a column of S, 16 rows each (rows 4 part + 4 KS j .. + 3, j < 4, as
+// above).  The parts lie on lane bits 1 up, so that a 16-byte read of a row by a warp takes two
+// wavefronts of shared memory (on bits 0 up it took four).
+template <int KS>
+__global__ void __launch_bounds__(DB_WARPS * 32 + 32)
+delta_blocks_kernel(float* __restrict__ o, float* __restrict__ state,
+                    const float* __restrict__ blocks, const float* __restrict__ vv,
+                    const int* __restrict__ req_start, const int* __restrict__ req_len,
+                    const int* __restrict__ req_slot, int cap_blocks, DeltaShape s, int* status) {
+  constexpr int D = 16 * KS, SZ = db_floats(D);
+  constexpr int COLS = 32 / KS;                                // of a warp
+  extern __shared__ __align__(16) float sm[];                  // [stages][blocks of a stage][SZ]
+  __shared__ uint64_t full[DB_STAGES], empty[DB_STAGES];
+  const int r = blockIdx.x, h = blockIdx.y;
+  const int n = req_len[r];
+  if (n <= 0) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nb = (n + DB_TOK - 1) / DB_TOK, n_stages = (nb + DB_STAGE_BLOCKS - 1) / DB_STAGE_BLOCKS;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < DB_STAGES; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], DB_WARPS);
+    }
+    fence_barrier_init();
+  }
+  __syncthreads();
+  if (warp == DB_WARPS) {
+    if (lane == 0) {
+      const float* src = blocks + ((size_t)h * cap_blocks + db_first(req_len, r)) * SZ;
+      for (int i = 0; i < n_stages; ++i) {
+        const int st = i % DB_STAGES;
+        if (i >= DB_STAGES && !mbar_wait(&empty[st], ((i / DB_STAGES) - 1) & 1, status)) break;
+        const int here = min(DB_STAGE_BLOCKS, nb - i * DB_STAGE_BLOCKS);
+        const uint32_t bytes = (uint32_t)(here * SZ * 4);
+        mbar_expect_tx(&full[st], bytes);
+        asm volatile(
+            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                smem_u32(sm + (size_t)st * DB_STAGE_BLOCKS * SZ)),
+            "l"(src + (size_t)i * DB_STAGE_BLOCKS * SZ), "r"(bytes), "r"(smem_u32(&full[st]))
+            : "memory");
+      }
+    }
+    return;
+  }
+  const int part = (lane >> 1) & (KS - 1);
+  const int col = blockIdx.z * DB_WARPS * COLS + warp * COLS + ((lane & 1) | ((lane >> 1) / KS) << 1);
+  const bool col_ok = col < s.V;
+  const int first = req_start[r], HV = s.heads * s.V;
+  float* S = state + (size_t)req_slot[r] * s.state_stride + (size_t)h * D * s.V + col;
+  uint64_t st[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const int d = 4 * part + 4 * KS * (j >> 1) + 2 * (j & 1);
+    st[j] = col_ok ? db_pair(S[(size_t)d * s.V], S[(size_t)(d + 1) * s.V]) : 0;
+  }
+  const float* vcol = vv + (size_t)first * HV + h * s.V + (col_ok ? col : 0);
+  float* ocol = o + (size_t)first * HV + h * s.V + col;
+  float v[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v[i] = vcol[(size_t)min(i, n - 1) * HV];
+  for (int i = 0; i < n_stages; ++i) {
+    const int sg = i % DB_STAGES;
+    if (!mbar_wait(&full[sg], (i / DB_STAGES) & 1, status)) return;
+#pragma unroll
+    for (int b = 0; b < DB_STAGE_BLOCKS; ++b) {
+      const int blk = i * DB_STAGE_BLOCKS + b;
+      if (blk >= nb) break;
+      const float* x = sm + (size_t)(sg * DB_STAGE_BLOCKS + b) * SZ + 4 * part;
+      auto piece = [&](int vec, int j) { return *(const ulonglong2*)(x + vec * D + 4 * KS * j); };
+      float vn[4];                                 // the next block's values
+#pragma unroll
+      for (int t = 0; t < 4; ++t) vn[t] = vcol[(size_t)min(blk * 4 + 4 + t, n - 1) * HV];
+      uint64_t aw[4] = {0, 0, 0, 0}, ow[4] = {0, 0, 0, 0};
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const ulonglong2 p = piece(t, j);
+          db_fma(aw[t], st[2 * j], p.x);
+          db_fma(aw[t], st[2 * j + 1], p.y);
+        }
+      float a[4], ob[4];
+#pragma unroll
+      for (int t = 0; t < 4; ++t) a[t] = db_fold(aw[t]);
+#pragma unroll
+      for (int off = 2; off <= KS; off <<= 1)
+#pragma unroll
+        for (int t = 0; t < 4; ++t) a[t] += __shfl_xor_sync(0xffffffffu, a[t], off);
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const ulonglong2 p = piece(4 + t, j);
+          db_fma(ow[t], st[2 * j], p.x);
+          db_fma(ow[t], st[2 * j + 1], p.y);
+        }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const ulonglong2 p = piece(12, j);
+        st[2 * j] = db_mul(st[2 * j], p.x);
+        st[2 * j + 1] = db_mul(st[2 * j + 1], p.y);
+      }
+      const float4* cf = (const float4*)(x - 4 * part + 13 * D);
+      const float4 c0 = cf[0], c1 = cf[1], c2 = cf[2], c3 = cf[3], be = cf[4];
+      // c: 10 20 21 30 31 32   e: 00 10 11 20 21 22 30 31 32 33
+      float u[4];
+      u[0] = be.x * (v[0] - a[0]);
+      u[1] = be.y * ((v[1] - a[1]) - c0.x * u[0]);
+      u[2] = be.z * ((v[2] - a[2]) - c0.y * u[0] - c0.z * u[1]);
+      u[3] = be.w * ((v[3] - a[3]) - c0.w * u[0] - c1.x * u[1] - c1.y * u[2]);
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const uint64_t u2 = db_pair(u[t], u[t]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const ulonglong2 p = piece(8 + t, j);
+          db_fma(st[2 * j], p.x, u2);
+          db_fma(st[2 * j + 1], p.y, u2);
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < 4; ++t) ob[t] = db_fold(ow[t]);
+#pragma unroll
+      for (int off = 2; off <= KS; off <<= 1)
+#pragma unroll
+        for (int t = 0; t < 4; ++t) ob[t] += __shfl_xor_sync(0xffffffffu, ob[t], off);
+      ob[0] += c1.z * u[0];
+      ob[1] += c1.w * u[0] + c2.x * u[1];
+      ob[2] += c2.y * u[0] + c2.z * u[1] + c2.w * u[2];
+      ob[3] += c3.x * u[0] + c3.y * u[1] + c3.z * u[2] + c3.w * u[3];
+      // lane `part` of a column stores token `part` of the block
+      const float mine = part == 0 ? ob[0] : part == 1 ? ob[1] : part == 2 ? ob[2] : ob[3];
+      if (part < 4 && col_ok && blk * 4 + part < n) ocol[(size_t)(blk * 4 + part) * HV] = mine;
+#pragma unroll
+      for (int t = 0; t < 4; ++t) v[t] = vn[t];
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&empty[sg]);
+  }
+  if (col_ok) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int d = 4 * part + 4 * KS * (j >> 1) + 2 * (j & 1);
+      S[(size_t)d * s.V] = __uint_as_float((uint32_t)st[j]);
+      S[(size_t)(d + 1) * s.V] = __uint_as_float((uint32_t)(st[j] >> 32));
+    }
+  }
+}
+
 // One block per token and head: the head's root mean square by a block reduction, then one
 // thread per output forms its gate (a sum over the rg inputs, several loads in flight).
 template <typename TO>
@@ -390,16 +657,58 @@ HS_EXPORT int hs_delta_prepare(float* qn, float* kn, float* vv, float* beta, flo
   return HS_OK;
 }
 
+// Floats the blocks of n_tokens tokens of n_requests requests take, or 0 when the sizes are not
+// taken four tokens at a time.
+HS_EXPORT int hs_delta_blocks_scratch(int n_tokens, int n_requests, int heads, int D,
+                                      long long* floats) {
+  if (!floats) return HS_ERR_ARGUMENT;
+  *floats = D == 64 || D == 128 || D == 256
+                ? (long long)heads * (n_tokens / hs::DB_TOK + n_requests) * hs::db_floats(D)
+                : 0;
+  return HS_OK;
+}
+
+// `blocks` (hs_delta_blocks_scratch floats, 16-byte aligned; null: token after token): portions four
+// tokens at a time.
 HS_EXPORT int hs_delta_recurrence(float* o, float* state, const float* qn, const float* kn,
                                   const float* vv, const float* beta, const float* decay,
                                   const int* req_start, const int* req_len, const int* req_slot,
                                   int n_requests, int heads, int kv_heads, int D, int V, int taps,
-                                  int ra, int rg, void* stream) {
+                                  int ra, int rg, int n_tokens, float* blocks, int* status,
+                                  void* stream) {
   if (!o || !state || !qn || !kn || !vv || !beta || !decay || !req_start || !req_len || !req_slot)
     return HS_ERR_ARGUMENT;
   hs::DeltaShape s;
   int rc = delta_shape(&s, heads, kv_heads, D, V, taps, ra, rg);
   if (rc) return rc;
+  if (blocks && n_requests > 0 && n_tokens > 0) {
+    if ((D != 64 && D != 128 && D != 256) || ((uintptr_t)blocks & 15) || !status)
+      return HS_ERR_ARGUMENT;
+    const int cap = n_tokens / hs::DB_TOK + n_requests;
+    cudaStream_t st = (cudaStream_t)stream;
+    hs::delta_blocks_prepare_kernel<<<dim3(cap, heads), 128, 0, st>>>(
+        blocks, qn, kn, beta, decay, req_start, req_len, n_requests, cap, s);
+    HS_LAUNCH_CHECK();
+    const size_t smem = (size_t)hs::DB_STAGES * hs::DB_STAGE_BLOCKS * hs::db_floats(D) * sizeof(float);
+    cudaError_t e = cudaSuccess;
+#define HS_DB(KS)                                                                                 \
+  do {                                                                                            \
+    const int cols = hs::DB_WARPS * 32 / KS;                                                      \
+    e = cudaFuncSetAttribute(hs::delta_blocks_kernel<KS>,                                         \
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);             \
+    if (e == cudaSuccess)                                                                         \
+      hs::delta_blocks_kernel<KS><<<dim3(n_requests, heads, (V + cols - 1) / cols),               \
+                                    hs::DB_WARPS * 32 + 32, smem, st>>>(                          \
+          o, state, blocks, vv, req_start, req_len, req_slot, cap, s, status);                    \
+  } while (0)
+    if (D == 64) HS_DB(4);
+    else if (D == 128) HS_DB(8);
+    else HS_DB(16);
+#undef HS_DB
+    if (e != cudaSuccess) return (int)e;
+    HS_LAUNCH_CHECK();
+    return HS_OK;
+  }
   if (D > hs::DR_DP * 32) return HS_ERR_UNSUPPORTED;   // a column's parts are lanes of one warp
   if (n_requests <= 0) return HS_OK;
   int KS = 1;

@@ -217,7 +217,8 @@ def _declare(lib) -> None:
         "hs_latent_prefill_mma": [P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, I, I, I, P, P,
                                   I, I, P],
         "hs_delta_prepare": [P] * 15 + [I] * 9 + [P, P],
-        "hs_delta_recurrence": [P] * 10 + [I] * 8 + [P],
+        "hs_delta_recurrence": [P] * 10 + [I] * 9 + [P, P, P],
+        "hs_delta_blocks_scratch": [I, I, I, I, P],
         "hs_delta_finish": [P, P, P, P, P, P, I, F, I, I, I, I, I, I, I, I, P, P],
         "hs_moe_route": [P, P, P, P, P, I, I, I, I, I, I, I, P, P],
         "hs_moe_experts": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, F, I, I, P, P, I, I, P],
@@ -373,6 +374,7 @@ class CudaOps:
         self.folds_pooled_means = True   # pooled_prepare takes the companion pool (single tokens)
         self.lightning_bulk_rows = 64   # from this many tokens a step on, lightning attention
         #                                 activates its rows in a pass of their own
+        self.delta_blocks = True    # portions of the delta rule four tokens at a time
         self.latent_splits = None   # blocks a token's keys are split over in latent attention
         #                             (None: chosen from the number of tokens in the step)
         self.sorted_experts = True  # many (token, expert) pairs in bfloat16: sorted by expert and
@@ -1328,9 +1330,10 @@ class CudaOps:
             f"latent_gather(rank={rank},dim={dim})")
 
     def latent_prompt_attention(self, out, q, kv, rope, base, plan, *, n_heads, dim, rot_dim, vdim,
-                                rank, window, scale, status, gate=None, gate_offset=0):
+                                rank, window, scale, status, gate=None, gate_offset=0,
+                                sink=None):
         """Softmax attention of the plan's prompt portions over the last ``window`` positions (0:
-        over all), with ``gate`` (float32 [T, *]) times sigmoid(gate[t, gate_offset + column]):
+        over all), with ``sink`` (float32 [n_heads]) exp(sink[h]) in the denominator too, with ``gate`` (float32 [T, *]) times sigmoid(gate[t, gate_offset + column]):
         ``q`` as ``latent_gather`` left it, ``kv`` [rows, n_heads * (dim + vdim)] the expanded
         keys of all heads, then the values; ``out`` [T, n_heads * vdim] bfloat16 (rows of single-
         query tokens are left alone)."""
@@ -1342,6 +1345,10 @@ class CudaOps:
         if out.shape[1] != n_heads * vdim or tuple(q.shape) != (T, n_heads * (pad + 64)) or \
                 kv.shape[1] != n_heads * (dim + vdim) or tuple(rope.shape) != (rows, 64):
             raise KernelError("latent_prompt_attention: shapes do not fit")
+        if sink is not None:
+            _want(sink, "sink", torch.float32, 1)
+            if sink.shape[0] != n_heads:
+                raise KernelError("latent_prompt_attention: one sink a head")
         g_stride = 0
         if gate is not None:
             _want(gate, "gate", torch.float32, 2)
@@ -1353,7 +1360,7 @@ class CudaOps:
             _ptr(out), _ptr(q), _ptr(kv), _ptr(rope), _ptr(base), _ptr(plan.data),
             4 + plan_decode_ints(plan.n_rows), plan.tile_cap, T, rows, n_heads, dim, rot_dim, vdim,
             rank, int(window), float(scale), _ptr(gate), g_stride, int(gate_offset), n_heads, 0.0,
-            None, _ptr(status), self._stream()), f"latent_prompt_attention(dim={dim},rot_dim={rot_dim},vdim={vdim})")
+            _ptr(sink), _ptr(status), self._stream()), f"latent_prompt_attention(dim={dim},rot_dim={rot_dim},vdim={vdim})")
 
     # -- the gated delta rule ---------------------------------------------------------------
     @staticmethod
@@ -1389,18 +1396,29 @@ class CudaOps:
 
     def delta_recurrence(self, o, state, qn, kn, vv, beta, decay, req_start, req_len, req_slot,
                          shape):
-        """Per request and head, token after token on the float32 state S [dim, vdim]:
-        S <- decay * S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q."""
+        """Per request and head on the float32 state S [dim, vdim], token after token or (portions,
+        heads of 64, 128 or 256) four tokens at a time: S <- decay * S; u = beta (v - S^T k);
+        S <- S + k u^T; o = S^T q."""
         H, HK, D, V, taps, ra, rg = self._delta_sizes(shape)
         for t, nm in ((o, "o"), (qn, "qn"), (kn, "kn"), (vv, "vv"), (beta, "beta"),
                       (decay, "decay")):
             _want(t, nm, torch.float32, 2)
         _want(state, "state", torch.float32)
-        self.launches += 1
+        # four tokens at a time where requests bring some eight tokens each: two launches, of which
+        # the second pays its chain once in four tokens
+        T, R = o.shape[0], req_start.shape[0]
+        blocks = None
+        if self.delta_blocks and T >= 8 * R:
+            need = ctypes.c_longlong(0)
+            self.lib.hs_delta_blocks_scratch(T, R, H, D, ctypes.byref(need))
+            if need.value:
+                blocks = self._scratch_buffer("delta_blocks", need.value, torch.float32)
+        self.launches += 2 if blocks is not None else 1
         _check(self.lib.hs_delta_recurrence(
             _ptr(o), _ptr(state), _ptr(qn), _ptr(kn), _ptr(vv), _ptr(beta), _ptr(decay),
-            _ptr(req_start), _ptr(req_len), _ptr(req_slot), req_start.shape[0], H, HK, D, V,
-            taps, ra, rg, self._stream()), f"delta_recurrence(dim={D},vdim={V})")
+            _ptr(req_start), _ptr(req_len), _ptr(req_slot), R, H, HK, D, V,
+            taps, ra, rg, T, _ptr(blocks), _ptr(self.status), self._stream()),
+            f"delta_recurrence(dim={D},vdim={V})")
 
     def delta_finish(self, out, o, proj, g2, norm_w, tok_req, eps, shape, z_g=None):
         """out = o / sqrt(mean(o^2) + eps) per head * norm_w * sigmoid(g2^T g); ``g2`` is

@@ -68,7 +68,7 @@ class LatentAttention(Mixer):
                           g=gate)
         self.rot_pairing = rot_pairing
         # without a window, prompts in expanded form need a row for every position they see
-        self.counts_prompt_rows = self.window == 0 and sink is None
+        self.counts_prompt_rows = self.window == 0
         self.shares_cache = bool(shares_cache)
         self.q_width = self.H * (self.D + self.P)
         # columns of the input projection: the queries or their latent, then the key/value latent
@@ -139,7 +139,7 @@ class LatentAttention(Mixer):
             self.w_expand_nk = tensors[n["uv"]].view(self.H, self.V, self.R).contiguous()
         # both expansions as one matrix, for the dense rows of prompt portions
         self.w_kv = None
-        if wq.dtype == torch.bfloat16 and not n["sink"]:
+        if wq.dtype == torch.bfloat16:
             self.w_kv = torch.cat([tensors[n["uk"]], tensors[n["uv"]]]).contiguous()
         self.sink = tensors[n["sink"]] if n["sink"] else None
         self.w_out = tensors[n["o"]]
@@ -223,7 +223,7 @@ class LatentAttention(Mixer):
         ops.linear(kv, lat, self.w_kv)
         ops.latent_prompt_attention(att, qp, kv, rope, base, ctx.plan, n_heads=H, dim=D, rot_dim=P,
                                     vdim=V, rank=R, window=self.window, scale=self.scale,
-                                    status=ctx.status, **gate)
+                                    status=ctx.status, sink=self.sink, **gate)
 
 
 register_mixer("latent_attention", LatentAttention)
