@@ -314,8 +314,8 @@ delta_recurrence_kernel(float* __restrict__ o, float* __restrict__ state,
 // products of at most four factors below one (no quotients, nothing can overflow).  What does not
 // depend on the state (K', Q', K", the decay of all four, c, e, beta) is formed beforehand for all
 // tokens in parallel; a head's blocks lie one behind the other, so that a stage of the recurrence
-// is one bulk copy.  All of it is float32, packed two rows an instruction.  Measured: 2 x 1,024
-// tokens, 8 heads of 128 x 128, see the launch below.
+// is one bulk copy.  All of it is float32, packed two rows an instruction.  Measured (2 x 1,024
+// tokens, 8 heads of 128 x 128): 412 us token after token, 16 + 155 us so.
 constexpr int DB_TOK = 4, DB_COEF = 32;
 constexpr int DB_STAGE_BLOCKS = 2, DB_STAGES = 4;
 constexpr int DB_WARPS = 4;                       // that work; one more fetches
@@ -394,11 +394,18 @@ delta_blocks_prepare_kernel(float* __restrict__ blocks, const float* __restrict_
     if (lane == 0) red[warp][i] = v;
   }
   __syncthreads();
+  // [c: 10 20 21 30 31 32, - -][beta, - - - -][e: four rows of four, zero above the diagonal]
   if (threadIdx.x < DB_COEF) {
     const int i = threadIdx.x;
+    int from = -1;
+    if (i < 6) from = i;
+    else if (i >= 16 && (i & 3) <= ((i - 16) >> 2)) {
+      const int row = (i - 16) >> 2;
+      from = 6 + row * (row + 1) / 2 + (i & 3);
+    }
     float v = 0.f;
-    if (i < 16) v = (red[0][i] + red[1][i]) + (red[2][i] + red[3][i]);
-    else if (i < 20 && i - 16 < n) v = beta[(size_t)(t0 + i - 16) * s.heads + h];
+    if (from >= 0) v = (red[0][from] + red[1][from]) + (red[2][from] + red[3][from]);
+    else if (i >= 8 && i < 12 && i - 8 < n) v = beta[(size_t)(t0 + i - 8) * s.heads + h];
     out[13 * D + i] = v;
   }
 }
@@ -411,6 +418,11 @@ __device__ __forceinline__ uint64_t db_mul(uint64_t a, uint64_t b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
+__device__ __forceinline__ uint64_t db_add(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
 __device__ __forceinline__ uint64_t db_pair(float a, float b) {
   uint64_t r;
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
@@ -420,38 +432,46 @@ __device__ __forceinline__ float db_fold(uint64_t a) {
   return __uint_as_float((uint32_t)a) + __uint_as_float((uint32_t)(a >> 32));
 }
 
-// KS = D / 16 lanes hold a column of S, 16 rows each (rows 4 part + 4 KS j .. + 3, j < 4, as
-// above).  The parts lie on lane bits 1 up, so that a 16-byte read of a row by a warp takes two
-// wavefronts of shared memory (on bits 0 up it took four).
+// KS = D / 16 lanes hold a column of S, 16 rows each (rows 4 part + 4 KS j .. + 3, j < 4).  The
+// parts lie on lane bits 1 up, so that a 16-byte read of a row by a warp takes two wavefronts of
+// shared memory (on bits 0 up it took four).  There is about one warp a scheduler, so what a phase
+// reads from shared memory is read a phase ahead, into registers (225 -> 155 us; with 8 rows a lane
+// and twice the warps 170: shared memory, busy for half of the time, then serves every row twice as
+// often).
 template <int KS>
 __global__ void __launch_bounds__(DB_WARPS * 32 + 32)
 delta_blocks_kernel(float* __restrict__ o, float* __restrict__ state,
                     const float* __restrict__ blocks, const float* __restrict__ vv,
                     const int* __restrict__ req_start, const int* __restrict__ req_len,
                     const int* __restrict__ req_slot, int cap_blocks, DeltaShape s, int* status) {
-  constexpr int D = 16 * KS, SZ = db_floats(D);
-  constexpr int COLS = 32 / KS;                                // of a warp
+  constexpr int NJ = 4, D = 4 * NJ * KS, SZ = db_floats(D);
+  constexpr int COLS = 32 / KS, CTA_COLS = DB_WARPS * COLS;      // of a warp, of the block
+  constexpr int ST_TOK = DB_STAGE_BLOCKS * DB_TOK;             // tokens of a stage
   extern __shared__ __align__(16) float sm[];                  // [stages][blocks of a stage][SZ]
+  __shared__ float s_v[DB_STAGES][ST_TOK][CTA_COLS];
   __shared__ uint64_t full[DB_STAGES], empty[DB_STAGES];
   const int r = blockIdx.x, h = blockIdx.y;
   const int n = req_len[r];
   if (n <= 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nb = (n + DB_TOK - 1) / DB_TOK, n_stages = (nb + DB_STAGE_BLOCKS - 1) / DB_STAGE_BLOCKS;
+  const int first = req_start[r], HV = s.heads * s.V, col0 = blockIdx.z * CTA_COLS;
   if (threadIdx.x == 0) {
     for (int i = 0; i < DB_STAGES; ++i) {
-      mbar_init(&full[i], 1);
+      mbar_init(&full[i], 1 + 32);
       mbar_init(&empty[i], DB_WARPS);
     }
     fence_barrier_init();
   }
   __syncthreads();
   if (warp == DB_WARPS) {
-    if (lane == 0) {
-      const float* src = blocks + ((size_t)h * cap_blocks + db_first(req_len, r)) * SZ;
-      for (int i = 0; i < n_stages; ++i) {
-        const int st = i % DB_STAGES;
-        if (i >= DB_STAGES && !mbar_wait(&empty[st], ((i / DB_STAGES) - 1) & 1, status)) break;
+    // the fetching warp: lane 0 copies the blocks of a stage, all lanes the stage's values
+    const float* src = blocks + ((size_t)h * cap_blocks + db_first(req_len, r)) * SZ;
+    const float* vsrc = vv + (size_t)first * HV + h * s.V;
+    for (int i = 0; i < n_stages; ++i) {
+      const int st = i % DB_STAGES;
+      if (i >= DB_STAGES && !mbar_wait(&empty[st], ((i / DB_STAGES) - 1) & 1, status)) break;
+      if (lane == 0) {
         const int here = min(DB_STAGE_BLOCKS, nb - i * DB_STAGE_BLOCKS);
         const uint32_t bytes = (uint32_t)(here * SZ * 4);
         mbar_expect_tx(&full[st], bytes);
@@ -461,107 +481,122 @@ delta_blocks_kernel(float* __restrict__ o, float* __restrict__ state,
             "l"(src + (size_t)i * DB_STAGE_BLOCKS * SZ), "r"(bytes), "r"(smem_u32(&full[st]))
             : "memory");
       }
+      for (int e = lane; e < ST_TOK * CTA_COLS; e += 32) {
+        const int t = min(i * ST_TOK + e / CTA_COLS, n - 1), c = min(col0 + e % CTA_COLS, s.V - 1);
+        cp_async4(&s_v[st][0][0] + e, vsrc + (size_t)t * HV + c);
+      }
+      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&full[st]))
+                   : "memory");
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     return;
   }
   const int part = (lane >> 1) & (KS - 1);
-  const int col = blockIdx.z * DB_WARPS * COLS + warp * COLS + ((lane & 1) | ((lane >> 1) / KS) << 1);
+  const int lc = warp * COLS + ((lane & 1) | ((lane >> 1) / KS) << 1);
+  const int col = col0 + lc;
   const bool col_ok = col < s.V;
-  const int first = req_start[r], HV = s.heads * s.V;
+  const int tok = 2 * (part & 1) + ((part >> 1) & 1);          // the token of a block this lane stores
+  const bool stores = part < 4 && col_ok;
+  float* ocol = o + (size_t)(first + tok) * HV + h * s.V + col;
   float* S = state + (size_t)req_slot[r] * s.state_stride + (size_t)h * D * s.V + col;
-  uint64_t st[8];
+  uint64_t st[2 * NJ];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
+  for (int j = 0; j < 2 * NJ; ++j) {
     const int d = 4 * part + 4 * KS * (j >> 1) + 2 * (j & 1);
     st[j] = col_ok ? db_pair(S[(size_t)d * s.V], S[(size_t)(d + 1) * s.V]) : 0;
   }
-  const float* vcol = vv + (size_t)first * HV + h * s.V + (col_ok ? col : 0);
-  float* ocol = o + (size_t)first * HV + h * s.V + col;
-  float v[4];
+  struct Four { ulonglong2 p[4][NJ]; };            // this lane's rows of four vectors
+  auto read4 = [&](const float* x, int vec, Four& f) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) v[i] = vcol[(size_t)min(i, n - 1) * HV];
-  for (int i = 0; i < n_stages; ++i) {
-    const int sg = i % DB_STAGES;
-    if (!mbar_wait(&full[sg], (i / DB_STAGES) & 1, status)) return;
+    for (int t = 0; t < 4; ++t)
 #pragma unroll
-    for (int b = 0; b < DB_STAGE_BLOCKS; ++b) {
-      const int blk = i * DB_STAGE_BLOCKS + b;
-      if (blk >= nb) break;
-      const float* x = sm + (size_t)(sg * DB_STAGE_BLOCKS + b) * SZ + 4 * part;
-      auto piece = [&](int vec, int j) { return *(const ulonglong2*)(x + vec * D + 4 * KS * j); };
-      float vn[4];                                 // the next block's values
+      for (int j = 0; j < NJ; ++j)
+        f.p[t][j] = *(const ulonglong2*)(x + (vec + t) * D + 4 * part + 4 * KS * j);
+  };
+  Four fk, fq, fw;
+  if (!mbar_wait(&full[0], 0, status)) return;
+  read4(sm, 0, fk);
+  for (int blk = 0; blk < nb; ++blk) {
+    const int i = blk / DB_STAGE_BLOCKS, sg = i % DB_STAGES, in = blk % DB_STAGE_BLOCKS;
+    const float* x = sm + (size_t)(sg * DB_STAGE_BLOCKS + in) * SZ;
+    read4(x, 4, fq);
+    uint64_t aw[4][2] = {}, ow[4][2] = {};
 #pragma unroll
-      for (int t = 0; t < 4; ++t) vn[t] = vcol[(size_t)min(blk * 4 + 4 + t, n - 1) * HV];
-      uint64_t aw[4] = {0, 0, 0, 0}, ow[4] = {0, 0, 0, 0};
+    for (int j = 0; j < NJ; ++j) {
 #pragma unroll
-      for (int t = 0; t < 4; ++t)
+      for (int t = 0; t < 4; ++t) db_fma(aw[t][0], st[2 * j], fk.p[t][j].x);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const ulonglong2 p = piece(t, j);
-          db_fma(aw[t], st[2 * j], p.x);
-          db_fma(aw[t], st[2 * j + 1], p.y);
-        }
-      float a[4], ob[4];
-#pragma unroll
-      for (int t = 0; t < 4; ++t) a[t] = db_fold(aw[t]);
-#pragma unroll
-      for (int off = 2; off <= KS; off <<= 1)
-#pragma unroll
-        for (int t = 0; t < 4; ++t) a[t] += __shfl_xor_sync(0xffffffffu, a[t], off);
-#pragma unroll
-      for (int t = 0; t < 4; ++t)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const ulonglong2 p = piece(4 + t, j);
-          db_fma(ow[t], st[2 * j], p.x);
-          db_fma(ow[t], st[2 * j + 1], p.y);
-        }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const ulonglong2 p = piece(12, j);
-        st[2 * j] = db_mul(st[2 * j], p.x);
-        st[2 * j + 1] = db_mul(st[2 * j + 1], p.y);
-      }
-      const float4* cf = (const float4*)(x - 4 * part + 13 * D);
-      const float4 c0 = cf[0], c1 = cf[1], c2 = cf[2], c3 = cf[3], be = cf[4];
-      // c: 10 20 21 30 31 32   e: 00 10 11 20 21 22 30 31 32 33
-      float u[4];
-      u[0] = be.x * (v[0] - a[0]);
-      u[1] = be.y * ((v[1] - a[1]) - c0.x * u[0]);
-      u[2] = be.z * ((v[2] - a[2]) - c0.y * u[0] - c0.z * u[1]);
-      u[3] = be.w * ((v[3] - a[3]) - c0.w * u[0] - c1.x * u[1] - c1.y * u[2]);
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const uint64_t u2 = db_pair(u[t], u[t]);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const ulonglong2 p = piece(8 + t, j);
-          db_fma(st[2 * j], p.x, u2);
-          db_fma(st[2 * j + 1], p.y, u2);
-        }
-      }
-#pragma unroll
-      for (int t = 0; t < 4; ++t) ob[t] = db_fold(ow[t]);
-#pragma unroll
-      for (int off = 2; off <= KS; off <<= 1)
-#pragma unroll
-        for (int t = 0; t < 4; ++t) ob[t] += __shfl_xor_sync(0xffffffffu, ob[t], off);
-      ob[0] += c1.z * u[0];
-      ob[1] += c1.w * u[0] + c2.x * u[1];
-      ob[2] += c2.y * u[0] + c2.z * u[1] + c2.w * u[2];
-      ob[3] += c3.x * u[0] + c3.y * u[1] + c3.z * u[2] + c3.w * u[3];
-      // lane `part` of a column stores token `part` of the block
-      const float mine = part == 0 ? ob[0] : part == 1 ? ob[1] : part == 2 ? ob[2] : ob[3];
-      if (part < 4 && col_ok && blk * 4 + part < n) ocol[(size_t)(blk * 4 + part) * HV] = mine;
-#pragma unroll
-      for (int t = 0; t < 4; ++t) v[t] = vn[t];
+      for (int t = 0; t < 4; ++t) db_fma(aw[t][1], st[2 * j + 1], fk.p[t][j].y);
     }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&empty[sg]);
+    float a[4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) a[t] = db_fold(db_add(aw[t][0], aw[t][1]));
+    ulonglong2 g[NJ];
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) g[j] = *(const ulonglong2*)(x + 12 * D + 4 * part + 4 * KS * j);
+    const float4* cf = (const float4*)(x + 13 * D);
+    const float4 c0 = cf[0], c1 = cf[1], be = cf[2], ev = cf[4 + tok];
+    const float* vt = &s_v[sg][in * DB_TOK][lc];
+    const float v0 = vt[0], v1 = vt[CTA_COLS], v2 = vt[2 * CTA_COLS], v3 = vt[3 * CTA_COLS];
+    // the sums over a column's lanes of what the u need, between the products for the outputs
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if ((2 << j) <= KS) {
+#pragma unroll
+        for (int t = 0; t < 4; ++t) a[t] += __shfl_xor_sync(0xffffffffu, a[t], 2 << j);
+      }
+#pragma unroll
+      for (int t = 0; t < 4; ++t) db_fma(ow[t][0], st[2 * j], fq.p[t][j].x);
+#pragma unroll
+      for (int t = 0; t < 4; ++t) db_fma(ow[t][1], st[2 * j + 1], fq.p[t][j].y);
+    }
+    read4(x, 8, fw);
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      st[2 * j] = db_mul(st[2 * j], g[j].x);
+      st[2 * j + 1] = db_mul(st[2 * j + 1], g[j].y);
+    }
+    if (blk + 1 < nb) {                            // the next block's K'
+      const int i2 = (blk + 1) / DB_STAGE_BLOCKS, sg2 = i2 % DB_STAGES;
+      if (i2 != i && !mbar_wait(&full[sg2], (i2 / DB_STAGES) & 1, status)) return;
+      read4(sm + (size_t)(sg2 * DB_STAGE_BLOCKS + (blk + 1) % DB_STAGE_BLOCKS) * SZ, 0, fk);
+    }
+    float u[4];
+    u[0] = be.x * (v0 - a[0]);
+    u[1] = be.y * ((v1 - a[1]) - c0.x * u[0]);
+    u[2] = be.z * ((v2 - a[2]) - c0.y * u[0] - c0.z * u[1]);
+    u[3] = be.w * ((v3 - a[3]) - c0.w * u[0] - c1.x * u[1] - c1.y * u[2]);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const uint64_t u2 = db_pair(u[t], u[t]);
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) {
+        db_fma(st[2 * j], fw.p[t][j].x, u2);
+        db_fma(st[2 * j + 1], fw.p[t][j].y, u2);
+      }
+    }
+    // the four outputs' sums: two exchanges leave every lane one token's share, then they add up
+    float ob[4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) ob[t] = db_fold(db_add(ow[t][0], ow[t][1]));
+    const bool hi = part & 1, hi2 = part & 2;
+    float w0 = hi ? ob[2] : ob[0], w1 = hi ? ob[3] : ob[1];
+    w0 += __shfl_xor_sync(0xffffffffu, hi ? ob[0] : ob[2], 2);
+    w1 += __shfl_xor_sync(0xffffffffu, hi ? ob[1] : ob[3], 2);
+    float out = hi2 ? w1 : w0;
+    out += __shfl_xor_sync(0xffffffffu, hi2 ? w0 : w1, 4);
+#pragma unroll
+    for (int off = 8; off <= KS; off <<= 1) out += __shfl_xor_sync(0xffffffffu, out, off);
+    out += ev.x * u[0] + ev.y * u[1] + ev.z * u[2] + ev.w * u[3];
+    if (stores && blk * DB_TOK + tok < n) ocol[(size_t)blk * DB_TOK * HV] = out;
+    if (in == DB_STAGE_BLOCKS - 1) {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[sg]);
+    }
   }
   if (col_ok) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < 2 * NJ; ++j) {
       const int d = 4 * part + 4 * KS * (j >> 1) + 2 * (j & 1);
       S[(size_t)d * s.V] = __uint_as_float((uint32_t)st[j]);
       S[(size_t)(d + 1) * s.V] = __uint_as_float((uint32_t)(st[j] >> 32));
@@ -693,12 +728,12 @@ HS_EXPORT int hs_delta_recurrence(float* o, float* state, const float* qn, const
     cudaError_t e = cudaSuccess;
 #define HS_DB(KS)                                                                                 \
   do {                                                                                            \
-    const int cols = hs::DB_WARPS * 32 / KS;                                                      \
-    e = cudaFuncSetAttribute(hs::delta_blocks_kernel<KS>,                                         \
+    const int cols = hs::DB_WARPS * (32 / KS);                                                    \
+    e = cudaFuncSetAttribute(hs::delta_blocks_kernel<KS>,                                     \
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);             \
     if (e == cudaSuccess)                                                                         \
-      hs::delta_blocks_kernel<KS><<<dim3(n_requests, heads, (V + cols - 1) / cols),               \
-                                    hs::DB_WARPS * 32 + 32, smem, st>>>(                          \
+      hs::delta_blocks_kernel<KS><<<dim3(n_requests, heads, (V + cols - 1) / cols),           \
+                                        hs::DB_WARPS * 32 + 32, smem, st>>>(                           \
           o, state, blocks, vv, req_start, req_len, req_slot, cap, s, status);                    \
   } while (0)
     if (D == 64) HS_DB(4);
