@@ -120,7 +120,10 @@ __global__ void __launch_bounds__(AS_STREAMS * 32)
 attention_simt_kernel(T* __restrict__ out, const T* __restrict__ qkv, const T* __restrict__ pool,
                       const int* __restrict__ table, const int* __restrict__ tok_pos,
                       const int* __restrict__ tok_req, int n_tokens, AttnGeom g, float scale,
-                      int both, int* status) {
+                      int both, const int* __restrict__ listed,
+                      const int* __restrict__ n_listed, int* status) {
+  // a list of tokens (their numbers in every third int; G is 1): the others are served elsewhere
+  if (G == 1 && listed != nullptr && (int)blockIdx.x >= *n_listed) return;
   extern __shared__ __align__(16) uint8_t as_smem[];
   constexpr int VEC = 16 / (int)sizeof(T);             // elements per 16-byte piece
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -148,8 +151,8 @@ attention_simt_kernel(T* __restrict__ out, const T* __restrict__ qkv, const T* _
   const int dkey = 32 / pieces, dpc = 32 - dkey * pieces;
 
   // the CTA's tokens: one run of consecutive positions of a request, or one by one
-  const int t_first = blockIdx.x * G;
-  const int n_here = min(G, n_tokens - t_first);
+  const int t_first = G == 1 && listed != nullptr ? listed[3 * blockIdx.x] : blockIdx.x * G;
+  const int n_here = G == 1 ? 1 : min(G, n_tokens - t_first);
   bool run = G > 1 && n_here > 1 && g.window == 0;
   if (run) {
     const int r0 = tok_req[t_first], p0 = tok_pos[t_first];
@@ -421,8 +424,8 @@ HS_EXPORT int hs_kv_append(void* pool, const void* qkv, const int* table, const 
 template <typename T, int G>
 static int launch_attention_simt(void* out, const void* qkv, const void* pool, const int* table,
                                  const int* tok_pos, const int* tok_req, int n_tokens,
-                                 const hs::AttnGeom& g, float scale, size_t esz, int* status,
-                                 cudaStream_t st) {
+                                 const hs::AttnGeom& g, float scale, size_t esz, const int* listed,
+                                 const int* n_listed, int* status, cudaStream_t st) {
   // keys and values side by side in shared memory while four warps of them fit in 160 KB
   const size_t rows_bytes = (size_t)hs::AS_CHUNK * g.head_dim * esz;
   const size_t q_bytes = (size_t)G * g.head_dim * 4;
@@ -435,18 +438,21 @@ static int launch_attention_simt(void* out, const void* qkv, const void* pool, c
     state = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 164 * 1024);
   if (state != cudaSuccess) return (int)state;
   k<<<grid, hs::AS_STREAMS * 32, smem, st>>>((T*)out, (const T*)qkv, (const T*)pool, table,
-                                              tok_pos, tok_req, n_tokens, g, scale, both, status);
+                                              tok_pos, tok_req, n_tokens, g, scale, both, listed,
+                                              n_listed, status);
   HS_LAUNCH_CHECK();
   return HS_OK;
 }
 
+// `listed` (or null; group 1): every third int names a token, the first *n_listed are served and
+// n_tokens is the grid.
 HS_EXPORT int hs_attention_simt_grouped(void* out, const void* qkv, const void* pool,
                                         const int* table, const int* tok_pos, const int* tok_req,
                                         int n_tokens, int n_heads, int n_kv_heads, int head_dim,
                                         int page_size, int num_pages, int max_pages, int q_off,
                                         int k_off, int v_off, int qkv_stride, int window,
-                                        float scale, int dtype, int group, int* status,
-                                        void* stream) {
+                                        float scale, int dtype, int group, const int* listed,
+                                        const int* n_listed, int* status, void* stream) {
   if (!out || !pool || !qkv || !table || !tok_pos || !tok_req || !status) return HS_ERR_ARGUMENT;
   hs::AttnGeom g{n_heads, n_kv_heads, head_dim, page_size, num_pages, max_pages,
                  q_off,   k_off,      v_off,    qkv_stride, window};
@@ -456,17 +462,18 @@ HS_EXPORT int hs_attention_simt_grouped(void* out, const void* qkv, const void* 
   if ((uintptr_t)pool & 15) return HS_ERR_UNSUPPORTED;   // rows are copied 16 bytes at a time
   if (n_heads > 65535) return HS_ERR_UNSUPPORTED;
   if (group != 1 && group != 4) return HS_ERR_ARGUMENT;
+  if (listed && (group != 1 || !n_listed)) return HS_ERR_ARGUMENT;
   using bf16 = __nv_bfloat16;
   if (dtype == HS_DT_F32)
     return group == 4 ? launch_attention_simt<float, 4>(out, qkv, pool, table, tok_pos, tok_req,
-                                                         n_tokens, g, scale, 4, status, st)
+                                                         n_tokens, g, scale, 4, listed, n_listed, status, st)
                       : launch_attention_simt<float, 1>(out, qkv, pool, table, tok_pos, tok_req,
-                                                         n_tokens, g, scale, 4, status, st);
+                                                         n_tokens, g, scale, 4, listed, n_listed, status, st);
   if (dtype == HS_DT_BF16)
     return group == 4 ? launch_attention_simt<bf16, 4>(out, qkv, pool, table, tok_pos, tok_req,
-                                                        n_tokens, g, scale, 2, status, st)
+                                                        n_tokens, g, scale, 2, listed, n_listed, status, st)
                       : launch_attention_simt<bf16, 1>(out, qkv, pool, table, tok_pos, tok_req,
-                                                        n_tokens, g, scale, 2, status, st);
+                                                        n_tokens, g, scale, 2, listed, n_listed, status, st);
   return HS_ERR_UNSUPPORTED;
 }
 
@@ -477,6 +484,6 @@ HS_EXPORT int hs_attention_simt(void* out, const void* qkv, const void* pool, co
                                 int window, float scale, int dtype, int* status, void* stream) {
   return hs_attention_simt_grouped(out, qkv, pool, table, tok_pos, tok_req, n_tokens, n_heads,
                                    n_kv_heads, head_dim, page_size, num_pages, max_pages, q_off,
-                                   k_off, v_off, qkv_stride, window, scale, dtype, 1, status,
-                                   stream);
+                                   k_off, v_off, qkv_stride, window, scale, dtype, 1, nullptr,
+                                   nullptr, status, stream);
 }

@@ -1,0 +1,69 @@
+"""Float32 prompt portions as tiles of queries: the same bits as the kernel that takes up to four
+tokens a block, at lengths around its tiles and chunks, behind earlier positions, with heads that share
+keys, beside single tokens, and with an infinite value behind a query's own position."""
+
+import pytest
+import torch
+
+from hetero_serve_b200.kernels.ops import AttentionGeometry, CudaOps
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.mark.parametrize("heads,kv_heads,page", [(2, 2, 16), (4, 2, 32)])
+@pytest.mark.parametrize("batch", [[(0, 5)], [(0, 64), (31, 65)], [(7, 1), (0, 33), (200, 3), (96, 128)],
+                                   [(100, 300)], [(0, 129), (511, 1), (33, 31)]])
+def test_same_bits_as_token_by_token(heads, kv_heads, page, batch):
+    ops, D = CudaOps(DEV), 64
+    g = torch.Generator(device=DEV).manual_seed(len(batch) + heads)
+    T, R = sum(n for _, n in batch), len(batch)
+    need = [-(-(p + n) // page) for p, n in batch]
+    pages, width = sum(need) + 1, max(need) + 1
+    order = torch.randperm(pages, generator=torch.Generator().manual_seed(1)).tolist()
+    table = torch.full((R, width), -1, dtype=torch.int32)
+    for r, k in enumerate(need):
+        table[r, :k] = torch.tensor([order.pop() for _ in range(k)], dtype=torch.int32)
+    qkv_w = (heads + 2 * kv_heads) * D
+    qkv = torch.randn(T, qkv_w, device=DEV, generator=g)
+    pool = torch.randn(pages, 2, kv_heads, page, D, device=DEV, generator=g)
+    pos, req = [], []
+    for r, (p, n) in enumerate(batch):
+        pos += range(p, p + n)
+        req += [r] * n
+    # a value no earlier query may see: the last position of the first request
+    p, n = batch[0]
+    last = p + n - 1
+    pool[table[0, last // page], 1, :, last % page] = float("inf")
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    geo = AttentionGeometry(heads, kv_heads, D, page, pages, width, 0, heads * D,
+                            (heads + kv_heads) * D, qkv_w)
+    plan = ops.make_plan([(r, r, p, n) for r, (p, n) in enumerate(batch)], T, page)
+    outs = []
+    for tiles in (True, False):
+        ops.f32_tiles = tiles
+        out = torch.zeros(T, heads * D, device=DEV)
+        ops.attention(out, qkv, pool, table.to(DEV), i32(pos), i32(req), geo, 0.13, ops.status, plan)
+        outs.append(out)
+    assert torch.equal(torch.nan_to_num(outs[0], nan=-77.0), torch.nan_to_num(outs[1], nan=-77.0))
+    assert torch.isfinite(outs[0][:n - 1]).all() and not torch.isfinite(outs[0][n - 1]).any()
+    assert ops.status.item() == 0
+
+
+def test_refused_page_is_reported():
+    ops, D = CudaOps(DEV), 64
+    table = torch.tensor([[0, 9]], dtype=torch.int32, device=DEV)
+    geo = AttentionGeometry(1, 1, D, 16, 2, 2, 0, D, 2 * D, 3 * D)
+    qkv, pool = torch.randn(20, 3 * D, device=DEV), torch.randn(2, 2, 1, 16, D, device=DEV)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    plan = ops.make_plan([(0, 0, 0, 20)], 20, 16)
+    outs = []
+    for tiles in (True, False):
+        ops.f32_tiles = tiles
+        ops.status.zero_()
+        out = torch.zeros(20, D, device=DEV)
+        ops.attention(out, qkv, pool, table, i32(list(range(20))), i32([0] * 20), geo, 0.1, ops.status,
+                      plan)
+        assert ops.status.item() == 4
+        outs.append(out)
+    assert torch.equal(*outs)
