@@ -1,5 +1,6 @@
-// Causal attention of prompt portions over the paged cache in float32 on the CUDA cores, head size
-// 64: the arithmetic of attention_simt.cu, operation for operation, laid out for tiles of queries.
+// Causal attention over the paged cache in float32 on the CUDA cores, head size 64: the arithmetic
+// of attention_simt.cu, operation for operation, laid out for tiles of queries (prompt portions) and,
+// further down, for single tokens.
 //
 // A token's keys are taken 32 at a time; chunk c belongs to stream c mod 4.  A score is one chain of
 // fused multiply-adds over d, times the scale; a stream keeps a running maximum, a running sum (the
@@ -330,6 +331,188 @@ attention_f32_tile_kernel(const AfParams p) {
   for (int c = 0; c < 16; ++c) orow[16 * (c >> 2) + (c & 3)] = o[c] * inv;
 }
 
+// ---- single tokens --------------------------------------------------------------------------------
+// One block per token and head, a warp per stream, as in attention_simt.cu and with its arithmetic.
+// That kernel looks a chunk's pages up, copies it, waits and computes, chunk after chunk: every chunk
+// costs two trips to the L2 or beyond.  Here NB chunks of a stream are on their way while one is
+// worked on: a chunk's place in the ring is refilled as soon as its keys, and then its values, have
+// been used, and the page of the chunk to fetch is read before the scores.  A whole chunk takes
+// straight-line code: a score per lane (keys swizzled against bank conflicts), two dimensions of the
+// values per lane.  Measured (8 tokens, 350-1,050 keys, 16 heads): 56 us in attention_simt.cu, 17 here.
+template <int NB>
+struct AfSingle {
+  static constexpr int WARP_FLOATS = NB * 2 * AF_CHUNK * AF_D + AF_D + AF_CHUNK;
+  static constexpr size_t SMEM = (size_t)AF_STREAMS * WARP_FLOATS * sizeof(float);
+};
+
+template <int NB>
+__global__ void __launch_bounds__(AF_STREAMS * 32)
+attention_f32_single_kernel(const AfParams p, const int* __restrict__ tok_pos,
+                            const int* __restrict__ tok_req, const int* __restrict__ listed,
+                            const int* __restrict__ n_listed) {
+  extern __shared__ __align__(16) float af_smem[];
+  if (listed != nullptr && (int)blockIdx.x >= *n_listed) return;
+  const int tok = listed != nullptr ? listed[3 * blockIdx.x] : blockIdx.x;
+  const int h = blockIdx.y, hk = h / (p.n_heads / p.n_kv_heads);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int r = tok_req[tok], pos = tok_pos[tok];
+  float* orow = p.out + ((size_t)tok * p.n_heads + h) * AF_D;
+  if (r < 0 || pos < 0 || pos / p.page_size >= p.max_pages) {
+    if (threadIdx.x < AF_D) orow[threadIdx.x] = 0.f;
+    return;
+  }
+  float* sk = af_smem + warp * AfSingle<NB>::WARP_FLOATS;      // [NB][32 keys][64]
+  float* sv = sk + NB * AF_CHUNK * AF_D;
+  float* sq = sv + NB * AF_CHUNK * AF_D;
+  float* sp = sq + AF_D;
+  const int* trow = p.table + (size_t)r * p.max_pages;
+  const size_t tile = (size_t)p.page_size * AF_D, page_stride = 2 * (size_t)p.n_kv_heads * tile;
+  const size_t v_off = (size_t)p.n_kv_heads * tile;
+  constexpr int STEP = AF_STREAMS * AF_CHUNK;
+
+  auto page_of = [&](int j0) { return j0 + lane <= pos ? trow[(j0 + lane) / p.page_size] : -1; };
+  auto row_of = [&](int j0, int page) -> long long {
+    const int j = j0 + lane;
+    if (j > pos) return -1;
+    if (page < 0 || page >= p.num_pages) {
+      atomicOr(p.status, HS_STATUS_BAD_PAGE);
+      return -1;
+    }
+    return (long long)(page * page_stride + hk * tile + (size_t)(j % p.page_size) * AF_D);
+  };
+  // a warp copies two rows at a time, 16 pieces of 16 bytes each
+  auto fetch = [&](float* dst, long long rows, size_t extra, bool swizzled) {
+#pragma unroll
+    for (int i = 0; i < AF_CHUNK / 2; ++i) {
+      const int key = 2 * i + (lane >> 4), pc = lane & 15;
+      const long long ko = __shfl_sync(0xffffffffu, rows, key);
+      if (ko >= 0)
+        af_copy16(dst + key * AF_D + (swizzled ? pc ^ (key & 7) : pc) * 4, p.pool + ko + extra + pc * 4);
+    }
+  };
+
+  const int first = warp * AF_CHUNK;
+  unsigned live[NB];
+#pragma unroll
+  for (int b = 0; b < NB; ++b) {
+    const int j0 = first + b * STEP;
+    live[b] = 0;
+    if (j0 <= pos) {
+      const long long rows = row_of(j0, page_of(j0));
+      live[b] = __ballot_sync(0xffffffffu, rows >= 0);
+      fetch(sk + b * AF_CHUNK * AF_D, rows, 0, true);
+      af_commit();
+      fetch(sv + b * AF_CHUNK * AF_D, rows, v_off, false);
+      af_commit();
+    } else {
+      af_commit();
+      af_commit();
+    }
+  }
+  const float* qrow = p.qkv + (size_t)tok * p.qkv_stride + p.q_off + h * AF_D;
+  sq[lane] = qrow[lane];
+  sq[lane + 32] = qrow[lane + 32];
+
+  float m = -INFINITY, l = 0.f, o0 = 0.f, o1 = 0.f;            // dimensions 2 lane, 2 lane + 1
+  for (int j00 = first; j00 <= pos; j00 += NB * STEP) {
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      const int j0 = j00 + b * STEP;
+      if (j0 > pos) break;                                     // (the same for the whole warp)
+      const int nxt = j0 + NB * STEP;
+      const bool more = nxt <= pos;
+      const int page = more ? page_of(nxt) : -1;
+      float* kb = sk + b * AF_CHUNK * AF_D;
+      float* vb = sv + b * AF_CHUNK * AF_D;
+      asm volatile("cp.async.wait_group %0;" ::"n"(2 * NB - 1) : "memory");
+      __syncwarp();
+      const unsigned here = live[b];
+      float s = -INFINITY;
+      {
+        float dot = 0.f;
+        const float4* krow = (const float4*)(kb + lane * AF_D);
+        const float4* q4 = (const float4*)sq;
+#pragma unroll
+        for (int c = 0; c < AF_D / 4; ++c) {
+          const float4 k = krow[c ^ (lane & 7)], q = q4[c];
+          dot = fmaf(q.x, k.x, dot);
+          dot = fmaf(q.y, k.y, dot);
+          dot = fmaf(q.z, k.z, dot);
+          dot = fmaf(q.w, k.w, dot);
+        }
+        if ((here >> lane) & 1u) s = dot * p.scale;
+      }
+      __syncwarp();                                            // the keys' place is free
+      long long rows = -1;
+      if (more) {
+        rows = row_of(nxt, page);
+        live[b] = __ballot_sync(0xffffffffu, rows >= 0);
+        fetch(kb, rows, 0, true);
+      }
+      af_commit();
+      const float m_new = fmaxf(m, warp_max(s));
+      asm volatile("cp.async.wait_group %0;" ::"n"(2 * NB - 1) : "memory");
+      // a chunk whose pages were all refused leaves m_new at -inf: skip it
+      if (m_new != -INFINITY) {
+        const float w = (s == -INFINITY) ? 0.f : expf(s - m_new);
+        const float corr = expf(m - m_new);
+        sp[lane] = w;
+        l = l * corr + warp_sum(w);
+        o0 *= corr;
+        o1 *= corr;
+        m = m_new;
+        __syncwarp();
+        if (here == 0xffffffffu) {
+#pragma unroll
+          for (int k4 = 0; k4 < AF_CHUNK / 4; ++k4) {
+            const float4 w4 = ((const float4*)sp)[k4];
+            const float wk[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float2 v = *(const float2*)(vb + (4 * k4 + i) * AF_D + 2 * lane);
+              o0 = fmaf(wk[i], v.x, o0);
+              o1 = fmaf(wk[i], v.y, o1);
+            }
+          }
+        } else {
+          for (int k = 0; k < AF_CHUNK; ++k) {
+            if (!((here >> k) & 1u)) continue;
+            const float2 v = *(const float2*)(vb + k * AF_D + 2 * lane);
+            o0 = fmaf(sp[k], v.x, o0);
+            o1 = fmaf(sp[k], v.y, o1);
+          }
+        }
+      }
+      __syncwarp();                                            // the values' place is free
+      if (more) fetch(vb, rows, v_off, false);
+      af_commit();
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  // fold the streams in stream order
+  __shared__ float s_fold[AF_STREAMS][AF_D + 2];
+  s_fold[warp][2 * lane] = o0;
+  s_fold[warp][2 * lane + 1] = o1;
+  if (lane == 0) {
+    s_fold[warp][AF_D] = m;
+    s_fold[warp][AF_D + 1] = l;
+  }
+  __syncthreads();
+  if (threadIdx.x >= AF_D) return;
+  float M = -INFINITY, L = 0.f, o = 0.f;
+  for (int i = 0; i < AF_STREAMS; ++i) {
+    const float ms = s_fold[i][AF_D];
+    if (ms == -INFINITY) continue;                             // a stream without keys
+    const float m_new = fmaxf(M, ms);
+    const float c0 = expf(M - m_new), c1 = expf(ms - m_new);
+    L = L * c0 + s_fold[i][AF_D + 1] * c1;
+    o = fmaf(s_fold[i][threadIdx.x], c1, o * c0);
+    M = m_new;
+  }
+  const float inv = L > 0.f ? 1.0f / L : 0.f;
+  orow[threadIdx.x] = o * inv;
+}
+
 }  // namespace hs
 
 static_assert(hs::AF_STREAMS * hs::AF_Q * (hs::AF_D + 4) * sizeof(float) <= hs::AF_SMEM,
@@ -356,6 +539,44 @@ HS_EXPORT int hs_attention_f32_tiles(float* out, const float* qkv, const float* 
              num_pages, max_pages, q_off, qkv_stride, scale};
   attention_f32_tile_kernel<<<dim3(2 * tile_cap, n_heads), AF_THREADS, AF_SMEM,
                               (cudaStream_t)stream>>>(p);
+  HS_LAUNCH_CHECK();
+  return HS_OK;
+}
+
+// Single tokens: all n_tokens of the batch, or (listed: every third int names a token) the first
+// *n_listed, n_tokens being the grid.
+HS_EXPORT int hs_attention_f32_single(float* out, const float* qkv, const float* pool,
+                                      const int* table, const int* tok_pos, const int* tok_req,
+                                      const int* listed, const int* n_listed, int n_tokens,
+                                      int n_heads, int n_kv_heads, int head_dim, int page_size,
+                                      int num_pages, int max_pages, int q_off, int qkv_stride,
+                                      float scale, int* status, void* stream) {
+  using namespace hs;
+  if (!out || !qkv || !pool || !table || !tok_pos || !tok_req || !status || (listed && !n_listed))
+    return HS_ERR_ARGUMENT;
+  if (head_dim != AF_D || n_heads <= 0 || n_kv_heads <= 0 || n_heads % n_kv_heads ||
+      n_heads > 65535 || page_size <= 0 || num_pages <= 0 || max_pages <= 0 || ((uintptr_t)pool & 15))
+    return HS_ERR_UNSUPPORTED;
+  if (n_tokens <= 0) return HS_OK;
+  AfParams p{out, qkv, pool, table, nullptr, nullptr, status, n_heads, n_kv_heads, page_size,
+             num_pages, max_pages, q_off, qkv_stride, scale};
+  // up to a block an SM: the deepest ring; more blocks: three share an SM instead
+  const bool deep = (long long)n_tokens * n_heads <= hs_sm_count();
+  cudaError_t e;
+#define HS_AF(NB)                                                                                 \
+  do {                                                                                            \
+    e = cudaFuncSetAttribute(attention_f32_single_kernel<NB>,                                     \
+                             cudaFuncAttributeMaxDynamicSharedMemorySize,                         \
+                             (int)AfSingle<NB>::SMEM);                                            \
+    if (e == cudaSuccess)                                                                         \
+      attention_f32_single_kernel<NB><<<dim3(n_tokens, n_heads), AF_STREAMS * 32,                 \
+                                        AfSingle<NB>::SMEM, (cudaStream_t)stream>>>(              \
+          p, tok_pos, tok_req, listed, n_listed);                                                 \
+  } while (0)
+  if (deep) HS_AF(3);
+  else HS_AF(1);
+#undef HS_AF
+  if (e != cudaSuccess) return (int)e;
   HS_LAUNCH_CHECK();
   return HS_OK;
 }

@@ -193,6 +193,7 @@ def _declare(lib) -> None:
         "hs_attention_simt_grouped": [P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, I, F, I, I,
                                       P, P, P, P],
         "hs_attention_f32_tiles": [P] * 6 + [I] * 9 + [F, P, P],
+        "hs_attention_f32_single": [P] * 8 + [I] * 9 + [F, P, P],
         "hs_attention_decode_append": [P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, I,
                                        F, I, I, I, I, P, P, P, P, P],
         "hs_attention_decode_mma": [P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, F, I, I, I,
@@ -376,6 +377,7 @@ class CudaOps:
         self.lightning_bulk_rows = 64   # from this many tokens a step on, lightning attention
         #                                 activates its rows in a pass of their own
         self.f32_tiles = True       # float32 prompt portions of heads of 64 as tiles of queries
+        self.f32_single = True      # ... and their single tokens with chunks fetched ahead
         self.delta_blocks = True    # portions of the delta rule four tokens at a time
         self.latent_splits = None   # blocks a token's keys are split over in latent attention
         #                             (None: chosen from the number of tokens in the step)
@@ -869,11 +871,22 @@ class CudaOps:
         # (with a work list: the step has prompt portions; the counts may be padded ones)
         group = 4 if (plan.tile_cap > 0 if plan is not None else n >= 4 * table.shape[0]) else 1
         group = 1 if listed is not None else group
+        n_listed = None if listed is None else _ptr(plan.data)
+        if group == 1 and self.f32_single and qkv.dtype == torch.float32 and g.window == 0 \
+                and g.head_dim == 64:
+            code = self.lib.hs_attention_f32_single(
+                _ptr(out), _ptr(qkv), _ptr(pool), _ptr(table), _ptr(tok_pos), _ptr(tok_req),
+                _ptr(listed), n_listed, n, g.n_heads, g.n_kv_heads, g.head_dim, g.page_size,
+                g.num_pages, g.max_pages, g.q_off, g.qkv_stride, scale, _ptr(status),
+                self._stream())
+            if code != -1:
+                _check(code, "attention_f32_single")
+                return
         _check(self.lib.hs_attention_simt_grouped(
             _ptr(out), _ptr(qkv), _ptr(pool), _ptr(table), _ptr(tok_pos), _ptr(tok_req), n,
             g.n_heads, g.n_kv_heads, g.head_dim, g.page_size, g.num_pages, g.max_pages, g.q_off,
             g.k_off, g.v_off, g.qkv_stride, g.window, scale, _DT[qkv.dtype], group, _ptr(listed),
-            None if listed is None else _ptr(plan.data), _ptr(status),
+            n_listed, _ptr(status),
             self._stream()), f"attention(head_dim={g.head_dim}, heads={g.n_heads})")
 
     def _attention_fast(self, out, qkv, pool, table, tok_pos, tok_req, g, scale, status, plan,

@@ -1,5 +1,5 @@
-"""Float32 prompt portions as tiles of queries: the same bits as the kernel that takes up to four
-tokens a block, at lengths around its tiles and chunks, behind earlier positions, with heads that share
+"""Float32 prompt portions as tiles of queries and single tokens with chunks fetched ahead: the same
+bits as the kernel that takes up to four tokens a block, at lengths around its tiles and chunks, behind earlier positions, with heads that share
 keys, beside single tokens, and with an infinite value behind a query's own position."""
 
 import pytest
@@ -13,7 +13,9 @@ DEV = "cuda"
 
 @pytest.mark.parametrize("heads,kv_heads,page", [(2, 2, 16), (4, 2, 32)])
 @pytest.mark.parametrize("batch", [[(0, 5)], [(0, 64), (31, 65)], [(7, 1), (0, 33), (200, 3), (96, 128)],
-                                   [(100, 300)], [(0, 129), (511, 1), (33, 31)]])
+                                   [(100, 300)], [(0, 129), (511, 1), (33, 31)], [(0, 1)],
+                                   [(p, 1) for p in (31, 32, 127, 128, 160, 511, 900, 1500)],
+                                   [(5 * i, 1) for i in range(90)]])
 def test_same_bits_as_token_by_token(heads, kv_heads, page, batch):
     ops, D = CudaOps(DEV), 64
     g = torch.Generator(device=DEV).manual_seed(len(batch) + heads)
@@ -41,7 +43,7 @@ def test_same_bits_as_token_by_token(heads, kv_heads, page, batch):
     plan = ops.make_plan([(r, r, p, n) for r, (p, n) in enumerate(batch)], T, page)
     outs = []
     for tiles in (True, False):
-        ops.f32_tiles = tiles
+        ops.f32_tiles = ops.f32_single = tiles
         out = torch.zeros(T, heads * D, device=DEV)
         ops.attention(out, qkv, pool, table.to(DEV), i32(pos), i32(req), geo, 0.13, ops.status, plan)
         outs.append(out)
@@ -50,20 +52,22 @@ def test_same_bits_as_token_by_token(heads, kv_heads, page, batch):
     assert ops.status.item() == 0
 
 
-def test_refused_page_is_reported():
+@pytest.mark.parametrize("tokens", [20, 3])
+def test_refused_page_is_reported(tokens):
     ops, D = CudaOps(DEV), 64
     table = torch.tensor([[0, 9]], dtype=torch.int32, device=DEV)
     geo = AttentionGeometry(1, 1, D, 16, 2, 2, 0, D, 2 * D, 3 * D)
     qkv, pool = torch.randn(20, 3 * D, device=DEV), torch.randn(2, 2, 1, 16, D, device=DEV)
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
-    plan = ops.make_plan([(0, 0, 0, 20)], 20, 16)
+    start = 20 - tokens
+    plan = ops.make_plan([(0, 0, start, tokens)], tokens, 16)
     outs = []
     for tiles in (True, False):
-        ops.f32_tiles = tiles
+        ops.f32_tiles = ops.f32_single = tiles
         ops.status.zero_()
-        out = torch.zeros(20, D, device=DEV)
-        ops.attention(out, qkv, pool, table, i32(list(range(20))), i32([0] * 20), geo, 0.1, ops.status,
-                      plan)
+        out = torch.zeros(tokens, D, device=DEV)
+        ops.attention(out, qkv[:tokens].contiguous(), pool, table, i32(list(range(start, 20))),
+                      i32([0] * tokens), geo, 0.1, ops.status, plan)
         assert ops.status.item() == 4
         outs.append(out)
     assert torch.equal(*outs)
