@@ -18,8 +18,8 @@
 // rot_dims numbers (number i pairs with i + rot_dims/2) and k scaled: with a table of
 // frequencies the rows are turned where they are activated (in the pass of its own, or while
 // they are staged), by the same expression in both places.
-#include "common.cuh"
 #include "rotary.cuh"
+#include "tcgen05.cuh"
 
 namespace hs {
 
@@ -230,19 +230,253 @@ lightning_kernel(float* __restrict__ o, float* __restrict__ state, const float* 
   }
 }
 
+// ---- steps of many tokens, heads of 64, 128 or 256 --------------------------------------------
+// The same chain of operations per token (the same bits), laid out for a stream of tokens.  The
+// kernel above spends 108 instructions a token and warp and waits for shared memory in front of most
+// of them (0.24 us a token at one warp a scheduler).  Here
+//   * the rows pass through `lightning_rows_kernel`, which activates, turns and scales them (an angle
+//     is formed once per token, not once per head and entry) and leaves them in the order in which
+//     they are used: per head and token, 16-byte piece j of every part side by side, and inside a part
+//     entries i and i + 4 neighbours, so that a part's four partial sums are two packed pairs;
+//     values per head and group of columns;
+//   * a warp of the recurrence only fetches: a stage of LS_TOK tokens is two bulk copies;
+//   * state, products and sums are packed two an instruction (fma.rn.f32x2, each half rounded as
+//     fmaf rounds), four tokens at a time, the rows of the next four read ahead; the parts lie on
+//     lane bits 1 up (a 16-byte read by a warp: two wavefronts of shared memory, four on bits 0 up);
+//   * the four tokens' sums over the parts are exchanged so that a lane finishes one of them (the
+//     butterfly's tree, a third of its shuffles).
+// Measured (2 x 1,024 tokens, 8 heads of 128 x 128): the recurrence 249 -> 70-99 us; shared-memory
+// reads bound it (eight 16-byte reads a token and warp).
+constexpr int LS_TOK = 8, LS_STAGES = 4, LS_WARPS = 4;
+
+__host__ __device__ constexpr int ls_cols(int D) { return LS_WARPS * 32 * LA_ROWS / D; }
+
+// q | k of token t and head h: rows + ((h * n_tokens + t) * 2 D); value column c of head h: group
+// c / cols: vals + (((h * groups + c / cols) * n_tokens + t) * cols + c % cols), columns past V zero
+__global__ void __launch_bounds__(256)
+lightning_rows_kernel(float* __restrict__ rows, float* __restrict__ vals,
+                      const float* __restrict__ proj, int n_tokens, int stride, int q_off, int k_off,
+                      int v_off, int H, int D, int V, int act, const int* __restrict__ tok_pos,
+                      const float* __restrict__ freq, int rot_dims, float k_scale) {
+  pdl_trigger();
+  pdl_wait();
+  __shared__ float s_c[128], s_s[128];
+  const int t = blockIdx.x, half = rot_dims >> 1;
+  const int pos = rot_dims > 0 ? tok_pos[t] : 0;
+  for (int i = threadIdx.x; i < half; i += blockDim.x) pair_angle(pos, freq[i], &s_c[i], &s_s[i]);
+  __syncthreads();
+  const float* row = proj + (size_t)t * stride;
+  const int P4 = D / 4;                                   // floats of a piece over all parts
+  for (int x = threadIdx.x; x < 2 * H * D; x += blockDim.x) {
+    const int h = x / (2 * D), y = x - h * 2 * D;
+    const bool is_q = y < D;
+    const int z = is_q ? y : y - D;
+    const int j = z / P4, part = (z - j * P4) >> 2, e = z & 3;
+    const int at = 4 * j + e;                             // place inside the part
+    const int i = (at & 8) + ((at & 7) >> 1) + ((at & 1) << 2);
+    const int d = part * LA_ROWS + i;
+    const float* vec = row + (is_q ? q_off : k_off) + h * D;
+    float own = la_act(vec[d], act);
+    if (d < rot_dims) {                                   // as la_entry
+      const bool low = d < half;
+      const float partner = la_act(vec[low ? d + half : d - half], act);
+      const int f = low ? d : d - half;
+      const float cross = __fmul_rn(partner, s_s[f]);
+      own = fmaf(own, s_c[f], low ? -cross : cross);
+    }
+    rows[((size_t)h * n_tokens + t) * 2 * D + y] = __fmul_rn(own, is_q ? 1.0f : k_scale);
+  }
+  const int cols = ls_cols(D), groups = (V + cols - 1) / cols;
+  for (int x = threadIdx.x; x < H * groups * cols; x += blockDim.x) {
+    const int h = x / (groups * cols), c = x - h * groups * cols, g = c / cols;
+    vals[(((size_t)h * groups + g) * n_tokens + t) * cols + (c - g * cols)] =
+        c < V ? la_act(row[v_off + h * V + c], act) : 0.f;
+  }
+}
+
+__device__ __forceinline__ uint64_t ls_fma(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t ls_mul(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t ls_pair(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float ls_lo(uint64_t a) { return __uint_as_float((uint32_t)a); }
+__device__ __forceinline__ float ls_hi(uint64_t a) { return __uint_as_float((uint32_t)(a >> 32)); }
+
+template <int P>                                          // parts of a column: D / 16
+__global__ void __launch_bounds__(LS_WARPS * 32 + 32, 1)
+lightning_stream_kernel(float* __restrict__ o, float* __restrict__ state,
+                        const float* __restrict__ rows, const float* __restrict__ vals,
+                        const float* __restrict__ decay, const int* __restrict__ req_start,
+                        const int* __restrict__ req_len, const int* __restrict__ req_slot,
+                        int n_tokens, int H, int V, int* status) {
+  constexpr int D = P * LA_ROWS, COLS = 32 / P, CTA_COLS = LS_WARPS * COLS;
+  extern __shared__ __align__(16) float smem[];           // [stages][LS_TOK][q | k], then the values
+  __shared__ uint64_t full[LS_STAGES], empty[LS_STAGES];
+  float* s_v = smem + LS_STAGES * LS_TOK * 2 * D;         // [stages][LS_TOK][CTA_COLS]
+  const int r = blockIdx.z, h = blockIdx.y;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < LS_STAGES; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], LS_WARPS);
+    }
+    fence_barrier_init();
+  }
+  __syncthreads();
+  pdl_trigger();
+  pdl_wait();
+  const int n = req_len[r];
+  if (n <= 0) return;
+  const int t0 = req_start[r], n_stages = (n + LS_TOK - 1) / LS_TOK;
+  if (warp == LS_WARPS) {
+    if (lane == 0) {
+      const float* src = rows + ((size_t)h * n_tokens + t0) * 2 * D;
+      const float* vsrc = vals + (((size_t)h * gridDim.x + blockIdx.x) * n_tokens + t0) * CTA_COLS;
+      for (int i = 0; i < n_stages; ++i) {
+        const int st = i % LS_STAGES;
+        if (i >= LS_STAGES && !mbar_wait(&empty[st], ((i / LS_STAGES) - 1) & 1, status)) break;
+        const int here = min(LS_TOK, n - i * LS_TOK);
+        const uint32_t rb = (uint32_t)(here * 2 * D * 4), vb = (uint32_t)(here * CTA_COLS * 4);
+        mbar_expect_tx(&full[st], rb + vb);
+        asm volatile(
+            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                smem_u32(smem + (size_t)st * LS_TOK * 2 * D)),
+            "l"(src + (size_t)i * LS_TOK * 2 * D), "r"(rb), "r"(smem_u32(&full[st]))
+            : "memory");
+        asm volatile(
+            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                smem_u32(s_v + (size_t)st * LS_TOK * CTA_COLS)),
+            "l"(vsrc + (size_t)i * LS_TOK * CTA_COLS), "r"(vb), "r"(smem_u32(&full[st]))
+            : "memory");
+      }
+    }
+    return;
+  }
+  const int part = (lane >> 1) & (P - 1);
+  const int lc = warp * COLS + ((lane & 1) | ((lane >> 1) / P) << 1);
+  const int v = blockIdx.x * CTA_COLS + lc;
+  const bool col_ok = v < V;
+  const int tok = 2 * (part & 1) + ((part >> 1) & 1);     // the token of four this lane finishes
+  const bool stores = part < 4 && col_ok;
+  const uint64_t dh = ls_pair(decay[h], decay[h]);
+  float* S = state + (((size_t)req_slot[r] * H + h) * D + part * LA_ROWS) * V + v;
+  uint64_t s[8];                                          // rows (i, i + 4), then (8 + i, 12 + i)
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int d = (i & 4) * 2 + (i & 3);
+    s[i] = col_ok ? ls_pair(S[(size_t)d * V], S[(size_t)(d + 4) * V]) : 0;
+  }
+  float* ocol = o + (size_t)(t0 + tok) * H * V + (size_t)h * V + v;
+
+  struct Rows { ulonglong2 q[4], k[4]; float v; };
+  auto read = [&](const float* x, const float* xv, int tt, Rows& f) {
+    const float* at = x + (size_t)tt * 2 * D + 4 * part;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      f.q[j] = *(const ulonglong2*)(at + 4 * P * j);
+      f.k[j] = *(const ulonglong2*)(at + D + 4 * P * j);
+    }
+    f.v = xv[tt * CTA_COLS + lc];
+  };
+  auto token = [&](const Rows& f) {
+    const uint64_t vt = ls_pair(f.v, f.v);
+    uint64_t sum[2];
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {                         // quads 0 and 1, quads 2 and 3
+      const uint64_t k[4] = {f.k[2 * g].x, f.k[2 * g].y, f.k[2 * g + 1].x, f.k[2 * g + 1].y};
+      const uint64_t q[4] = {f.q[2 * g].x, f.q[2 * g].y, f.q[2 * g + 1].x, f.q[2 * g + 1].y};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) s[4 * g + e] = ls_fma(k[e], vt, ls_mul(dh, s[4 * g + e]));
+      uint64_t a = ls_mul(s[4 * g], q[0]);
+#pragma unroll
+      for (int e = 1; e < 4; ++e) a = ls_fma(s[4 * g + e], q[e], a);
+      sum[g] = a;
+    }
+    return (ls_lo(sum[0]) + ls_hi(sum[0])) + (ls_lo(sum[1]) + ls_hi(sum[1]));
+  };
+  const bool hi = part & 1, hi2 = part & 2;
+  for (int i = 0; i < n_stages; ++i) {
+    const int st = i % LS_STAGES;
+    if (!mbar_wait(&full[st], (i / LS_STAGES) & 1, status)) return;
+    const float* x = smem + (size_t)st * LS_TOK * 2 * D;
+    const float* xv = s_v + st * LS_TOK * CTA_COLS;
+    const int here = min(LS_TOK, n - i * LS_TOK);
+    int tt = 0;
+#pragma unroll
+    for (int b = 0; b < LS_TOK; b += 4) {
+      if (b + 4 > here) break;
+      Rows f[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) read(x, xv, b + u, f[u]);
+      float a[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) a[u] = token(f[u]);
+      float w0 = hi ? a[2] : a[0], w1 = hi ? a[3] : a[1];
+      w0 += __shfl_xor_sync(0xffffffffu, hi ? a[0] : a[2], 2);
+      w1 += __shfl_xor_sync(0xffffffffu, hi ? a[1] : a[3], 2);
+      float out = hi2 ? w1 : w0;
+      out += __shfl_xor_sync(0xffffffffu, hi2 ? w0 : w1, 4);
+#pragma unroll
+      for (int off = 8; off <= P; off <<= 1) out += __shfl_xor_sync(0xffffffffu, out, off);
+      if (stores) ocol[(size_t)(i * LS_TOK + b) * H * V] = out;
+      tt = b + 4;
+    }
+    for (; tt < here; ++tt) {
+      Rows f;
+      read(x, xv, tt, f);
+      float a = token(f);
+#pragma unroll
+      for (int off = 2; off <= P; off <<= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
+      if (part == 0 && col_ok) o[(size_t)(t0 + i * LS_TOK + tt) * H * V + (size_t)h * V + v] = a;
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&empty[st]);
+  }
+  if (col_ok) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int d = (i & 4) * 2 + (i & 3);
+      S[(size_t)d * V] = ls_lo(s[i]);
+      S[(size_t)(d + 4) * V] = ls_hi(s[i]);
+    }
+  }
+}
+
 }  // namespace hs
+
+// Floats of scratch with which hs_lightning_recurrence takes many tokens a step.
+HS_EXPORT int hs_lightning_scratch(int n_tokens, int H, int D, int V, long long* floats) {
+  if (!floats || n_tokens < 0 || H <= 0 || D <= 0 || V <= 0) return HS_ERR_ARGUMENT;
+  if (D == 64 || D == 128 || D == 256) {
+    const int cols = hs::ls_cols(D);
+    *floats = (long long)n_tokens * H * (2 * D + (V + cols - 1) / cols * cols);
+  } else {
+    *floats = D % 4 == 0 && V % 4 == 0 ? (long long)n_tokens * H * (2 * D + V) : 0;
+  }
+  return HS_OK;
+}
 
 // proj: float32 rows of `stride` columns holding q (H*D at q_off), k (H*D at k_off) and v (H*V at
 // v_off), head by head; o: float32 [tokens, H*V]; state: [slots, H*D*V] float32.  `scratch`
-// (n_tokens * (2 H D + H V) floats, or null): with it the activations are applied in a pass of
-// their own and the recurrence streams the activated rows; the results are the same bits.
+// (hs_lightning_scratch floats, or null): with it the activations are applied in a pass of their own
+// and the recurrence streams the activated rows; the results are the same bits.
 HS_EXPORT int hs_lightning_recurrence(float* o, float* state, const float* proj,
                                       const float* decay, const int* req_start,
                                       const int* req_len, const int* req_slot, int n_requests,
                                       int n_tokens, int stride, int q_off, int k_off, int v_off,
                                       int H, int D, int V, int act, float* scratch,
                                       const int* tok_pos, const float* freq, int rot_dims,
-                                      float k_scale, void* stream) {
+                                      float k_scale, int* status, void* stream) {
   if (!o || !state || !proj || !decay || !req_start || !req_len || !req_slot)
     return HS_ERR_ARGUMENT;
   if (rot_dims < 0 || rot_dims % 2 || rot_dims > D || (rot_dims > 0 && (!freq || !tok_pos)))
@@ -251,6 +485,32 @@ HS_EXPORT int hs_lightning_recurrence(float* o, float* state, const float* proj,
     return HS_ERR_UNSUPPORTED;
   if (n_requests <= 0 || n_tokens <= 0) return HS_OK;
   cudaStream_t st = (cudaStream_t)stream;
+  if (scratch && status && (D == 64 || D == 128 || D == 256) && !((uintptr_t)scratch & 15)) {
+    // (measured, 2 x 1,024 tokens, 8 heads of 128 x 128: retention's mixer takes 176 us this way, 395
+    // with the two kernels below)
+    const int cols = hs::ls_cols(D), groups = (V + cols - 1) / cols;
+    float* vals = scratch + (size_t)n_tokens * H * 2 * D;
+    cudaError_t e = hs_launch(hs::lightning_rows_kernel, dim3(n_tokens), dim3(256), 0, st,
+                              hs_pdl_enabled(), scratch, vals, proj, n_tokens, stride, q_off, k_off,
+                              v_off, H, D, V, act, tok_pos, freq, rot_dims, k_scale);
+    if (e != cudaSuccess) return (int)e;
+    const size_t smem = (size_t)hs::LS_STAGES * hs::LS_TOK * (2 * D + cols) * sizeof(float);
+#define HS_LS(P)                                                                                 \
+  do {                                                                                           \
+    e = cudaFuncSetAttribute(hs::lightning_stream_kernel<P>,                                     \
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);            \
+    if (e == cudaSuccess)                                                                        \
+      e = hs_launch(hs::lightning_stream_kernel<P>, dim3(groups, H, n_requests),                 \
+                    dim3(hs::LS_WARPS * 32 + 32), smem, st, hs_pdl_enabled(), o, state,          \
+                    (const float*)scratch, (const float*)vals, decay, req_start, req_len,        \
+                    req_slot, n_tokens, H, V, status);                                           \
+  } while (0)
+    if (D == 64) HS_LS(4);
+    else if (D == 128) HS_LS(8);
+    else HS_LS(16);
+#undef HS_LS
+    return (int)e;
+  }
   int P = 1;
   while (P * hs::LA_ROWS < D) P *= 2;
   const int cols = hs::LA_THREADS / P;

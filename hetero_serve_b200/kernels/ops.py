@@ -236,7 +236,8 @@ def _declare(lib) -> None:
         "hs_biased_attention_prefill": [P, P, P, P, P, P, I, P, P, I, P, I, I, I, I, I, I, I, I,
                                         F, F, I, I, P, P],
         "hs_lightning_recurrence": [P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, P, P, P, I,
-                                    F, P],
+                                    F, P, P],
+        "hs_lightning_scratch": [I, I, I, I, P],
         "hs_token_shift_mix": [P, P, P, P, I, I, P, P, P, P, I, I, I, I, P],
         "hs_timemix_decay": [P, P, P, P, I, I, I, P],
         "hs_timemix_recurrence": [P, P, I, P, P, P, P, P, P, P, P, I, I, I, I, P],
@@ -1885,16 +1886,18 @@ class CudaOps:
         # the recurrence then streams 16 bytes at a time (the same bits either way)
         T = o.shape[0]
         scratch = None
-        if T >= self.lightning_bulk_rows and dim % 4 == 0 and vdim % 4 == 0:
-            scratch = self._scratch_buffer("lightning_rows", T * (2 * heads * dim + heads * vdim),
-                                           torch.float32)
+        if T >= self.lightning_bulk_rows:
+            need = ctypes.c_longlong(0)
+            self.lib.hs_lightning_scratch(T, heads, dim, vdim, ctypes.byref(need))
+            if need.value:
+                scratch = self._scratch_buffer("lightning_rows", need.value, torch.float32)
         self.launches += 2 if scratch is not None else 1
         _check(self.lib.hs_lightning_recurrence(
             _ptr(o), _ptr(state), _ptr(proj), _ptr(decay), _ptr(req_start), _ptr(req_len),
             _ptr(req_slot), req_start.shape[0], T, proj.shape[1], int(q_off), int(k_off),
             int(v_off), heads, dim, vdim, ACTIVATIONS[act], _ptr(scratch),
             _ptr(tok_pos) if rot_dims else None, _ptr(freq) if rot_dims else None, int(rot_dims),
-            float(k_scale), self._stream()),
+            float(k_scale), _ptr(self.status), self._stream()),
             f"lightning_recurrence(dim={dim},vdim={vdim})")
 
     # -- norms behind a sublayer, a learned activation, capped logits -----------------------
