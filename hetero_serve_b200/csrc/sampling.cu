@@ -268,13 +268,14 @@ sample_kernel(int* __restrict__ out, const float* __restrict__ logits,
 // A row of up to ~55k logits fits a CTA's shared memory.  It is read from global memory once;
 // thread t owns the positions [t*C, (t+1)*C) (C odd: its walks are free of bank conflicts), so
 // sums over threads in thread order are sums in index order.  The k-th largest logit is found
-// by a radix select of four 8-bit digits over a 256-bin histogram (not 32 one-bit passes over
-// the row), the kept entries' weights exp(x/T - max/T) replace the logits in place, one scan
+// by a radix select of four 8-bit digits over a 256-bin histogram, among the few entries that the
+// threads' maxima leave in question, the kept entries' weights exp(x/T - max/T) replace the logits in place, one scan
 // over the threads gives every thread the weight before its range, and the thread that holds
 // the crossing of u * total finds the token.  Streaming the row from global memory for every
 // pass (the kernel above, which stays for longer rows) took 90 us without top-k and 240-270 us
 // with it at 50,257 logits.
 constexpr int SS_THREADS = 1024;
+constexpr int SS_CAND = 1024;       // entries that may be among the k largest
 
 __device__ float block_max_f(float v) {
   __shared__ float sh[SS_THREADS / 32];
@@ -356,7 +357,8 @@ sample_smem_kernel(int* __restrict__ out, const float* __restrict__ logits,
                    const int* __restrict__ feedback_slot, const int* __restrict__ status_word) {
   extern __shared__ float s_row[];                  // [vocab]: logits, then weights (-1: dropped)
   __shared__ int hist[256];
-  __shared__ int s_digit, s_above, s_found, s_last;
+  __shared__ int s_digit, s_above, s_same, s_found, s_last, s_n;
+  __shared__ uint32_t s_cand[SS_CAND];
   const int rowi = blockIdx.x;
   const float* row = logits + (size_t)rowi * vocab;
   const float temp = temperature[rowi];
@@ -372,7 +374,7 @@ sample_smem_kernel(int* __restrict__ out, const float* __restrict__ logits,
     return;
   }
   float m = -INFINITY;                              // the maximum needs no order: taken on the way in
-#pragma unroll 8
+#pragma unroll 16
   for (int i = threadIdx.x; i < vocab; i += blockDim.x) {
     const float v = row[i];
     s_row[i] = v;
@@ -381,6 +383,7 @@ sample_smem_kernel(int* __restrict__ out, const float* __restrict__ logits,
   if (threadIdx.x == 0) {
     s_found = 0x7fffffff;
     s_last = 0;
+    s_n = 0;
   }
   const float mx = block_max_f(m) / temp;           // (its barriers also publish the row)
   int C = (vocab + blockDim.x - 1) / blockDim.x;
@@ -391,74 +394,116 @@ sample_smem_kernel(int* __restrict__ out, const float* __restrict__ logits,
   const bool use_k = k > 0 && k < vocab;
   uint32_t thr = 0;     // order key of the k-th largest logit; 0 keeps everything
   int need_eq = 0;      // how many entries equal to the threshold are kept (lowest indices)
+  bool all_eq = true;   // ... which is all of them
   if (use_k) {
-    uint32_t prefix = 0;
-    int remaining = k;  // the k-th largest is the remaining-th largest among keys with the prefix
-    for (int shift = 24; shift >= 0; shift -= 8) {
-      if (threadIdx.x < 256) hist[threadIdx.x] = 0;
-      __syncthreads();
-      const uint32_t above_mask = shift == 24 ? 0u : (0xffffffffu << (shift + 8));
-      // (one atomic per entry: shared-memory atomics to the few digits most logits share
-      // measured 4 us a pass; adding once per warp and digit through __match_any_sync 9 us)
-      for (int i = lo; i < hi; ++i) {
-        const uint32_t key = order_key(s_row[i]);
-        if ((key & above_mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1);
-      }
-      __syncthreads();
-      if (threadIdx.x < 32) {
-        // lane l owns digits 8l .. 8l+7; digits are taken from the largest down
-        const int lane = threadIdx.x;
-        int c[8], grp = 0;
+    // the want-th largest of the keys that `walk` hands on, and among the keys equal to it: s_above
+    // (of the last digit) lie above, s_same are equal
+    int remaining = 0;
+    auto select = [&](int want, auto walk) {
+      uint32_t prefix = 0;
+      remaining = want; // the want-th largest is the remaining-th largest among keys with the prefix
+      for (int shift = 24; shift >= 0; shift -= 8) {
+        if (threadIdx.x < 256) hist[threadIdx.x] = 0;
+        __syncthreads();
+        const uint32_t above_mask = shift == 24 ? 0u : (0xffffffffu << (shift + 8));
+        // (one atomic per entry: adding once per warp and digit through __match_any_sync took
+        // twice as long)
+        walk([&](uint32_t key) {
+          if ((key & above_mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1);
+        });
+        __syncthreads();
+        if (threadIdx.x < 32) {
+          // lane l owns digits 8l .. 8l+7; digits are taken from the largest down
+          const int lane = threadIdx.x;
+          int c[8], grp = 0;
 #pragma unroll
-        for (int b = 0; b < 8; ++b) {
-          c[b] = hist[8 * lane + b];
-          grp += c[b];
-        }
-        int incl = grp;             // inclusive sum over lanes lane .. 31
+          for (int b = 0; b < 8; ++b) {
+            c[b] = hist[8 * lane + b];
+            grp += c[b];
+          }
+          int incl = grp;             // inclusive sum over lanes lane .. 31
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int u = __shfl_down_sync(0xffffffffu, incl, o);
-          if (lane + o < 32) incl += u;
-        }
-        int run = incl - grp;       // keys with a digit above this lane's
-        if (run < remaining && remaining <= incl) {
+          for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_down_sync(0xffffffffu, incl, o);
+            if (lane + o < 32) incl += u;
+          }
+          int run = incl - grp;       // keys with a digit above this lane's
+          if (run < remaining && remaining <= incl) {
 #pragma unroll
-          for (int b = 7; b >= 0; --b) {
-            if (run < remaining && remaining <= run + c[b]) {
-              s_digit = 8 * lane + b;
-              s_above = run;
+            for (int b = 7; b >= 0; --b) {
+              if (run < remaining && remaining <= run + c[b]) {
+                s_digit = 8 * lane + b;
+                s_above = run;
+                s_same = c[b];
+              }
+              run += c[b];
             }
-            run += c[b];
           }
         }
+        __syncthreads();
+        prefix |= (uint32_t)s_digit << shift;
+        remaining -= s_above;
+      }
+      return prefix;
+    };
+    auto whole_row = [&](auto take) {
+      for (int i = lo; i < hi; ++i) take(order_key(s_row[i]));
+    };
+    // Few of the row's entries can be among the k largest: k of the threads' maxima, so k entries,
+    // are no smaller than the k-th largest maximum.  The entries from there up (k and a few more)
+    // are listed in one walk and the threshold is found among them; walking the row once per digit
+    // took 4 us a digit at 50,257 logits (32 rows, a third with top-k 40: 56 us, 42 this way).  More of them than the list holds (many equal logits), or
+    // more wanted than there are threads: the digits walk the row.
+    bool listed = k <= (int)blockDim.x && k <= SS_CAND;
+    if (listed) {
+      const uint32_t own = order_key(m);
+      const uint32_t bound = select(k, [&](auto take) { take(own); });
+      for (int i = lo; i < hi; ++i) {
+        const uint32_t key = order_key(s_row[i]);
+        if (key >= bound) {
+          const int at = atomicAdd(&s_n, 1);
+          if (at < SS_CAND) s_cand[at] = key;
+        }
       }
       __syncthreads();
-      prefix |= (uint32_t)s_digit << shift;
-      remaining -= s_above;
+      listed = s_n >= k && s_n <= SS_CAND;
     }
-    thr = prefix;
+    if (listed) {
+      const int n = s_n;
+      thr = select(k, [&](auto take) {
+        for (int i = threadIdx.x; i < n; i += blockDim.x) take(s_cand[i]);
+      });
+    } else {
+      thr = select(k, whole_row);
+    }
     need_eq = remaining;
+    all_eq = s_same == remaining;
   }
 
   // entries equal to the threshold are kept in index order until k are reached
   int eq = 0;
-  if (use_k) {                                      // the same for the whole CTA
+  if (use_k && !all_eq) {                           // the same for the whole CTA
     for (int i = lo; i < hi; ++i) eq += order_key(s_row[i]) == thr;
     float unused = 0.f, tf;
     int tn;
     block_exclusive_scan(unused, eq, tf, tn);       // eq: equal entries before this range
   }
   float sum = 0.f;
+  bool any = false;                                 // of this range's entries is kept
+#pragma unroll 4
   for (int i = lo; i < hi; ++i) {
     const float v = s_row[i];
     bool kept = true;
     if (use_k) {
       const uint32_t key = order_key(v);
-      kept = key > thr || (key == thr && eq++ < need_eq);
+      kept = key > thr || (key == thr && (all_eq || eq++ < need_eq));
     }
     const float e = kept ? expf(v / temp - mx) : -1.f;
     s_row[i] = e;
-    if (kept) sum += e;
+    if (kept) {
+      sum += e;
+      any = true;
+    }
   }
   float before = sum, total;
   int nz = 0, tnz;
@@ -468,7 +513,7 @@ sample_smem_kernel(int* __restrict__ out, const float* __restrict__ logits,
   const float target = u * total;
   int cand = 0x7fffffff, last_kept = -1;
   float run = before;
-  for (int i = lo; i < hi; ++i) {
+  for (int i = any ? lo : hi; i < hi; ++i) {
     const float e = s_row[i];
     if (e >= 0.f) {
       run += e;
