@@ -11,7 +11,8 @@
 // A persistent CTA (one per SM) walks over 128 x BN output tiles (n fastest, so that CTAs running
 // together share rows of `a`):
 //   warp 0       TMA producer: cp.async.bulk.tensor loads of a [128 x 64] tile of `a` and a
-//                [BN x 64] tile of `w` per stage, 128-byte swizzle, completion on an mbarrier;
+//                [BN x 64] tile of `w` per k block, 128-byte swizzle, completion on an mbarrier (two
+//                k blocks share one for tiles up to 128 wide);
 //   warp 1       allocates TMEM (two accumulators), then one elected thread issues tcgen05.mma
 //                (M=128, N=BN, K=16, kind::f16, bf16 inputs, f32 accumulate), four per stage, and
 //                commits each stage's completion to the stage's "empty" barrier and each tile's
@@ -369,6 +370,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                       const __grid_constant__ CUtensorMap map_w, const TcParams p) {
   using S = TcSmem<BN, STAGES>;
+  // k blocks that share a barrier round, and rounds the ring holds.  Waiting for a stage, announcing
+  // it and committing it costs the issuing threads about 90 ns whatever the width, while the MMAs of a
+  // 64- or 128-wide k block take 70-140 ns: two k blocks a round there (2,048 x 1,024 x 4,096: 25.8 ->
+  // 22.7 us, 512 x 1,280 x 5,120: 27.3 -> 23.2).  Wider tiles hold too few stages to pair them, and
+  // their MMAs (325 ns for 256 columns) cover the round.
+  constexpr int PER = BN <= 128 ? 2 : 1, RING = STAGES / PER;
   extern __shared__ uint8_t smem_raw[];
   // 128-byte swizzled tiles need 1024-byte alignment
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -388,7 +395,7 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
 
   pdl_trigger();       // the next kernel may set itself up while this one runs
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < RING; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
     }
@@ -416,11 +423,14 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
     const int tile = blockIdx.x / p.splits, split = blockIdx.x - tile * p.splits;
     const int n0 = (tile % p.tiles_n) * BN;
     const int kb0 = split * p.kb_per_split;
-    pre = min(STAGES, min(kb0 + p.kb_per_split, num_kb) - kb0);
+    const int blocks = min(kb0 + p.kb_per_split, num_kb) - kb0;
+    pre = min(RING, (blocks + PER - 1) / PER);
     for (int i = 0; i < pre; ++i) {
-      mbar_expect_tx(&full_bar[i], S::STAGE_BYTES);
-      tma_load_2d(smem + i * S::STAGE_BYTES + S::A_BYTES, &map_w, &full_bar[i],
-                  (kb0 + i) * TC_BK, n0);
+      const int here = min(PER, blocks - i * PER);
+      mbar_expect_tx(&full_bar[i], here * S::STAGE_BYTES);
+      for (int j = 0; j < here; ++j)
+        tma_load_2d(smem + (i * PER + j) * S::STAGE_BYTES + S::A_BYTES, &map_w, &full_bar[i],
+                    (kb0 + i * PER + j) * TC_BK, n0);
     }
   }
   pdl_wait();
@@ -428,25 +438,30 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
   if (warp == 0) {
     if (lane == 0) {
       // ---------------- TMA producer
-      uint32_t it = 0;                          // k blocks issued so far (over all work items)
+      uint32_t it = 0;                          // rounds issued so far (over all work items)
       bool ok = true;
       for (int w = blockIdx.x; w < n_items && ok; w += gridDim.x) {
         const int tile = w / p.splits, split = w - tile * p.splits;
         const int m0 = (tile / p.tiles_n) * TC_BM, n0 = (tile % p.tiles_n) * BN;
         const int kb0 = split * p.kb_per_split;
         const int kb1 = min(kb0 + p.kb_per_split, num_kb);
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t round = it / STAGES;
+        for (int kb = kb0; kb < kb1; kb += PER, ++it) {
+          const int s = it % RING;
+          const uint32_t round = it / RING;
+          const int here = PER == 1 ? 1 : min(PER, kb1 - kb);
           if (round > 0) ok = mbar_wait(&empty_bar[s], (round - 1) & 1, p.status);
           if (!ok) break;
-          uint8_t* a_dst = smem + s * S::STAGE_BYTES;
-          uint8_t* b_dst = a_dst + S::A_BYTES;
-          if ((int)it >= pre) {
-            mbar_expect_tx(&full_bar[s], S::STAGE_BYTES);
-            tma_load_2d(b_dst, &map_w, &full_bar[s], kb * TC_BK, n0);
-          }
-          tma_load_2d(a_dst, &map_a, &full_bar[s], kb * TC_BK, m0);
+          uint8_t* dst = smem + s * PER * S::STAGE_BYTES;
+          const bool fresh = (int)it >= pre;
+          if (fresh) mbar_expect_tx(&full_bar[s], here * S::STAGE_BYTES);
+#pragma unroll
+          for (int j = 0; j < PER; ++j)
+            if (j < here) {
+              if (fresh)
+                tma_load_2d(dst + j * S::STAGE_BYTES + S::A_BYTES, &map_w, &full_bar[s],
+                            (kb + j) * TC_BK, n0);
+              tma_load_2d(dst + j * S::STAGE_BYTES, &map_a, &full_bar[s], (kb + j) * TC_BK, m0);
+            }
         }
       }
     }
@@ -465,22 +480,28 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
         if (!ok) break;
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + acc * ACC_COLS;
-        for (int kb = kb0; kb < kb1 && ok; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t round = it / STAGES;
+        for (int kb = kb0; kb < kb1 && ok; kb += PER, ++it) {
+          const int s = it % RING;
+          const uint32_t round = it / RING;
+          const int here = PER == 1 ? 1 : min(PER, kb1 - kb);
           ok = mbar_wait(&full_bar[s], round & 1, p.status);
           if (!ok) break;
           tc_fence_after();
-          const uint32_t a_addr = smem_u32(smem + s * S::STAGE_BYTES);
-          const uint32_t b_addr = a_addr + S::A_BYTES;
+          const uint32_t a_addr = smem_u32(smem + s * PER * S::STAGE_BYTES);
           const uint64_t adesc = make_smem_desc(a_addr);
-          const uint64_t bdesc = make_smem_desc(b_addr);
+          const uint64_t bdesc = make_smem_desc(a_addr + S::A_BYTES);
 #pragma unroll
-          for (int k = 0; k < TC_BK / TC_UMMA_K; ++k) {
-            // advance 16 elements = 32 bytes along K inside the swizzled row: +2 in 16-byte units
-            umma_bf16(tmem_d, adesc + (uint64_t)(k * 2), bdesc + (uint64_t)(k * 2), idesc,
-                      (kb > kb0 || k > 0) ? 1u : 0u);
-          }
+          for (int j = 0; j < PER; ++j)
+            if (j < here) {
+              const uint64_t next = (uint64_t)(j * (S::STAGE_BYTES >> 4));
+#pragma unroll
+              for (int k = 0; k < TC_BK / TC_UMMA_K; ++k) {
+                // advance 16 elements = 32 bytes along K inside the swizzled row: +2 in 16-byte
+                // units
+                umma_bf16(tmem_d, adesc + next + (uint64_t)(k * 2), bdesc + next + (uint64_t)(k * 2),
+                          idesc, (kb > kb0 || j > 0 || k > 0) ? 1u : 0u);
+              }
+            }
           umma_commit(&empty_bar[s]);     // the stage may be refilled once these MMAs are done
         }
         umma_commit(&acc_full[acc]);      // this accumulator is complete (or the pipeline gave up)
