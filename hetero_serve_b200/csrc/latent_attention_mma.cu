@@ -229,8 +229,18 @@ latent_prefill_mma_kernel(float* __restrict__ out, const float* __restrict__ qa,
 
 }  // namespace hs
 
+static size_t latent_prefill_smem(int R, int P) {
+  const int W16 = (R + P + 15) & ~15;
+  return (size_t)(hs::LM_ROWS + hs::LM_KEYS) * (W16 + 8) * sizeof(__nv_bfloat16);
+}
+
+// Whether the kernel takes these sizes: R a multiple of 16 up to 512, the shared tiles within 200 KB.
+HS_EXPORT int hs_latent_prefill_mma_takes(int R, int P) {
+  return R > 0 && R % 16 == 0 && R <= 512 && P >= 0 && latent_prefill_smem(R, P) <= 200 * 1024 ? 1 : 0;
+}
+
 // Returns HS_ERR_UNSUPPORTED for sizes the kernel does not take (the caller then uses the
-// CUDA-core kernel): R a multiple of 16 up to 512, the shared tiles within 200 KB.
+// CUDA-core kernel).
 HS_EXPORT int hs_latent_prefill_mma(float* out, const float* qa, const float* qr,
                                     const void* pool, const int* table, const float* sink,
                                     const int* plan, int tiles_off, int tile_cap, int n_heads,
@@ -241,11 +251,9 @@ HS_EXPORT int hs_latent_prefill_mma(float* out, const float* qa, const float* qr
   if (!out || !qa || !qr || !pool || !table || !plan || !status || window < 0)
     return HS_ERR_ARGUMENT;
   if (rot_dims < 0 || rot_dims % 2 || rot_dims > P || (rot_dims && !freq)) return HS_ERR_ARGUMENT;
-  if (R <= 0 || R % 16 || R > 512 || P < 0 || n_heads <= 0 || page_size <= 0)
+  if (!hs_latent_prefill_mma_takes(R, P) || n_heads <= 0 || page_size <= 0)
     return HS_ERR_UNSUPPORTED;
-  const int W16 = (R + P + 15) & ~15;
-  const size_t smem = (size_t)(hs::LM_ROWS + hs::LM_KEYS) * (W16 + 8) * sizeof(__nv_bfloat16);
-  if (smem > 200 * 1024) return HS_ERR_UNSUPPORTED;
+  const size_t smem = latent_prefill_smem(R, P);
   if (tile_cap <= 0) return HS_OK;
   const int halves = R > 256 ? 2 : 1;
   const int per = R / halves;

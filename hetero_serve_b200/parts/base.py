@@ -79,6 +79,8 @@ class Part:
     # True for a part that sizes buffers by ``plan.prompt_rows``, which the runner then counts
     # (and captures a graph per class of it).
     counts_prompt_rows: bool = False
+    # ... in steps of at least this many tokens
+    prompt_rows_from: int = 1
 
     def tensor_requests(self) -> dict[str, TensorRequest]:
         return {}

@@ -35,6 +35,7 @@ from __future__ import annotations
 
 import torch
 
+from ..kernels.ops import CudaOps
 from .base import CacheRequest, Mixer, TensorRequest, register_mixer
 
 
@@ -69,6 +70,8 @@ class LatentAttention(Mixer):
         self.rot_pairing = rot_pairing
         # without a window, prompts in expanded form need a row for every position they see
         self.counts_prompt_rows = self.window == 0
+        if sink is not None:        # (smaller steps keep to the latent: _prompt_rows)
+            self.prompt_rows_from = CudaOps.GROUPED_MMA_TOKENS
         self.shares_cache = bool(shares_cache)
         self.q_width = self.H * (self.D + self.P)
         # columns of the input projection: the queries or their latent, then the key/value latent
@@ -141,6 +144,7 @@ class LatentAttention(Mixer):
         self.w_kv = None
         if wq.dtype == torch.bfloat16:
             self.w_kv = torch.cat([tensors[n["uk"]], tensors[n["uv"]]]).contiguous()
+        self.counts_prompt_rows = self.window == 0 and self.w_kv is not None
         self.sink = tensors[n["sink"]] if n["sink"] else None
         self.w_out = tensors[n["o"]]
         i = torch.arange(self.rot_dims // 2, dtype=torch.float64)
@@ -178,7 +182,7 @@ class LatentAttention(Mixer):
         att = ctx.buffer("latent_heads", (T, H * V), ctx.dtype)
         gate = dict(gate=proj, gate_offset=self.gate_off) if self.names["g"] else {}
         only = {}
-        rows = self._prompt_rows(ctx)
+        rows = self._prompt_rows(ctx, T)
         if rows:
             self._prompt_portions(ctx, att, q, cache, rows, rot, gate)
             if ctx.plan.decode_cap == 0:         # no single-query token in this step
@@ -200,13 +204,19 @@ class LatentAttention(Mixer):
         ops.grouped_linear(att, lat, self.w_expand, w_nk=self.w_expand_nk, parts=8, **only, **gate)
         ops.linear(x, att, self.w_out, None, residual=None if fresh else x)
 
-    def _prompt_rows(self, ctx) -> int:
-        """Dense rows the step's prompt portions need in expanded form; 0: not in that form."""
+    def _prompt_rows(self, ctx, T) -> int:
+        """Dense rows the step's prompt portions need in expanded form; 0: not in that form.
+        Where both forms round alike the expanded one is the faster: portions of 5 to 1,024 tokens
+        behind 0 to 8,000 positions, 64 tokens a step or more, take 2 to 21 times as long on the
+        latent (1,024 tokens from position 0, 8 heads: 422 us against 59; 2 x 64 tokens behind
+        500 and 64 single tokens: 311 against 131).  A layer with a sink, which had the form on
+        the latent first, keeps it in smaller steps, where that one rounds less."""
         takes = getattr(ctx.ops, "latent_prompt_rows", None)
         if self.w_kv is None or takes is None:
             return 0
         return takes(ctx.plan, ctx.n_requests, n_heads=self.H, dim=self.D, rot_dim=self.P,
-                     vdim=self.V, rank=self.R, window=self.window, scale=self.scale)
+                     vdim=self.V, rank=self.R, window=self.window, scale=self.scale,
+                     absorbed_tokens=None if self.sink is None else T)
 
     def _prompt_portions(self, ctx, att, q, cache, rows, rot, gate):
         ops, T = ctx.ops, q.shape[0]

@@ -388,12 +388,17 @@ class Model:
         self.schedule: tuple[LayerCall, ...] = spec.resolved_schedule()
         self.keeps_embedding = any(call.adds_embedding for call in self.schedule)
         self.capturable = all(part.capturable for part in self.parts())
-        self.counts_prompt_rows = any(part.counts_prompt_rows for part in self.parts())
+        self._derive_prompt_rows()
         self._derive_cache()
         self.dtype = None
         self.device = None
 
     # -- structure ----------------------------------------------------------
+    def _derive_prompt_rows(self):
+        counting = [part for part in self.parts() if part.counts_prompt_rows]
+        self.counts_prompt_rows = bool(counting)
+        self.prompt_rows_from = min((part.prompt_rows_from for part in counting), default=1)
+
     def parts(self):
         yield self.embedding
         yield self.position
@@ -480,6 +485,7 @@ class Model:
             converted[name] = t.contiguous()
         for part in self.parts():
             part.bind({n: converted[n] for n in part.tensor_requests()})
+        self._derive_prompt_rows()           # (bound in float32 a part may not need them)
         self.dtype, self.device = dtype, device
         self.tensors = converted
 
