@@ -594,11 +594,14 @@ delta_blocks_kernel(float* __restrict__ o, float* __restrict__ state,
       if (i2 != i && !mbar_wait(&full[sg2], (i2 / DB_STAGES) & 1, status)) return;
       read4(sm + (size_t)(sg2 * DB_STAGE_BLOCKS + (blk + 1) % DB_STAGE_BLOCKS) * SZ, 0, fk);
     }
+    // (a token past the end leaves the state alone: its zero beta and key would make NaN of an
+    // infinity)
+    const int here = n - blk * DB_TOK;
     float u[4];
     u[0] = be.x * (v0 - a[0]);
-    u[1] = be.y * ((v1 - a[1]) - c0.x * u[0]);
-    u[2] = be.z * ((v2 - a[2]) - c0.y * u[0] - c0.z * u[1]);
-    u[3] = be.w * ((v3 - a[3]) - c0.w * u[0] - c1.x * u[1] - c1.y * u[2]);
+    u[1] = here > 1 ? be.y * ((v1 - a[1]) - c0.x * u[0]) : 0.f;
+    u[2] = here > 2 ? be.z * ((v2 - a[2]) - c0.y * u[0] - c0.z * u[1]) : 0.f;
+    u[3] = here > 3 ? be.w * ((v3 - a[3]) - c0.w * u[0] - c1.x * u[1] - c1.y * u[2]) : 0.f;
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
       const uint64_t u2 = db_pair(u[t], u[t]);
@@ -620,8 +623,11 @@ delta_blocks_kernel(float* __restrict__ o, float* __restrict__ state,
     out += __shfl_xor_sync(0xffffffffu, hi2 ? w0 : w1, 4);
 #pragma unroll
     for (int off = 8; off <= KS; off <<= 1) out += __shfl_xor_sync(0xffffffffu, out, off);
-    out += ev.x * u[0] + ev.y * u[1] + ev.z * u[2] + ev.w * u[3];
-    if (stores && blk * DB_TOK + tok < n) ocol[(size_t)blk * DB_TOK * HV] = out;
+    // (a later token's u is left out, not multiplied by the zero above the diagonal: it may be an
+    // infinity or a NaN that the token must not see)
+    out += ev.x * u[0] + ev.y * (tok > 0 ? u[1] : 0.f) + ev.z * (tok > 1 ? u[2] : 0.f) +
+           ev.w * (tok > 2 ? u[3] : 0.f);
+    if (stores && tok < here) ocol[(size_t)blk * DB_TOK * HV] = out;
     if (in == DB_STAGE_BLOCKS - 1) {
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty[sg]);

@@ -61,6 +61,60 @@ def test_blocks_of_four(dim, vdim, heads, kv_heads, lens):
     assert ops.status.item() == 0
 
 
+@pytest.mark.parametrize("dim", [64, 128, 256])
+@pytest.mark.parametrize("n", [64, 65, 66, 67])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_values_that_are_not_finite_stay_behind_their_token(dim, n, bad):
+    """A token that brings an infinity or a NaN in one value column, or in its key or query: the
+    outputs in front of it, the other columns and, behind the last token, the infinities of the state
+    are those of the kernel that goes token after token."""
+    ops, vdim = CudaOps(DEV), 24
+    g = torch.Generator(device=DEV).manual_seed(dim + n)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g)  # noqa: E731
+    unit = lambda x: x / x.norm(dim=-1, keepdim=True)  # noqa: E731
+    shape = dict(heads=1, kv_heads=1, dim=dim, vdim=vdim, taps=1, a_rank=4, g_rank=4)
+    qn, kn, vv = unit(rnd(n, dim)) * dim ** -0.5, unit(rnd(n, dim)), rnd(n, vdim)
+    beta, decay = torch.sigmoid(rnd(n, 1)), torch.sigmoid(rnd(n, dim) + 2.0)
+    state0 = rnd(1, dim * vdim) * 0.3
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    bound = 4.0 * (dim ** 0.5 + 2.0) * 2.0 ** -24          # of either kernel off the exact result
+
+    def both(q, k, v, s0):
+        got = []
+        for blocks in (True, False):
+            ops.delta_blocks = blocks
+            o, state = torch.zeros(n, vdim, device=DEV), s0.clone()
+            before = ops.launches
+            ops.delta_recurrence(o, state, q, k, v, beta, decay, i32([0]), i32([n]), i32([0]), shape)
+            assert (ops.launches - before > 1) == blocks
+            got.append((o, state.view(dim, vdim)))
+        return got
+
+    def close(a, b):
+        assert torch.isfinite(b).all() and float((a - b).norm()) <= bound * float(b.norm())
+    for at in range(n - 7, n):                             # every place of a block, and its end
+        v = vv.clone()
+        v[at, 3] = bad
+        (o, s), (o1, s1) = both(qn, kn, v, state0)
+        close(o[:at], o1[:at])
+        others = [c for c in range(vdim) if c != 3]
+        close(o[:, others], o1[:, others])
+        close(s[:, others], s1[:, others])
+        assert not torch.isfinite(o[at, 3])
+        if at == n - 1 and bad == float("inf"):            # nothing behind it: infinities of k's signs
+            assert torch.isinf(s1[:, 3]).all() and torch.equal(s[:, 3], s1[:, 3])
+        else:
+            assert not torch.isfinite(s[:, 3]).any()
+        for name in ("q", "k"):
+            x = (qn if name == "q" else kn).clone()
+            x[at, 5] = bad
+            (o, s), (o1, s1) = both(x if name == "q" else qn, x if name == "k" else kn, vv, state0)
+            close(o[:at], o1[:at])
+            if name == "q":                                # only this token's output reads it
+                close(o[at + 1:], o1[at + 1:])
+                close(s, s1)
+
+
 def test_few_tokens_a_request_go_token_after_token():
     ops = CudaOps(DEV)
     shape = dict(heads=1, kv_heads=1, dim=64, vdim=8, taps=1, a_rank=4, g_rank=4)
