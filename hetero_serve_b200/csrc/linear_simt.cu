@@ -261,8 +261,8 @@ linear_simt_few_rows_kernel(TO* out, const TI* __restrict__ a, const TI* __restr
   if (warp == WARPS) {
     // the copying warp: RPI rows a trip, a lane per 16-byte piece.  Rows past the last one and
     // pieces past the end of K are left out: what their places hold reaches no output.  (Copies of
-    // the last row in their stead went to one line of the L2 from every block: 9 x 20,000 x 256 took
-    // 66 us, 16 rows 25.)
+    // the last row in their stead went to one line of the L2 from every block: float32, 9 x
+    // 20,000 x 256 took 66 us and takes 18, 33 x 4,096 x 1,024 66 and 31.)
     constexpr int CPR = BK / S::VEC;                         // pieces per row of a stage
     constexpr int RPI = 32 / CPR;
     const int crow = lane / CPR, ck = (lane % CPR) * S::VEC;
