@@ -188,11 +188,11 @@ delta_recurrence_kernel(float* __restrict__ o, float* __restrict__ state,
                         const float* __restrict__ vv, const float* __restrict__ beta,
                         const float* __restrict__ decay, const int* __restrict__ req_start,
                         const int* __restrict__ req_len, const int* __restrict__ req_slot,
-                        DeltaShape s, int KS, int CH, int vec) {
+                        DeltaShape s, int KS, int CH, int vec, int long_from) {
   extern __shared__ __align__(16) float sm[];
   const int r = blockIdx.x, h = blockIdx.y;
   const int n = req_len[r];
-  if (n <= 0) return;
+  if (n <= 0 || n >= long_from) return;            // long portions: delta_blocks_kernel
   const int Dp = KS * DR_DP;
   const int cols = DR_THREADS / KS;
   const int per_buf = (3 * CH * Dp + CH * cols + CH + 3) & ~3;      // buffers 16-byte aligned
@@ -349,16 +349,47 @@ delta_recurrence_kernel(float* __restrict__ o, float* __restrict__ state,
 // tokens in parallel; a head's blocks lie one behind the other, so that a stage of the recurrence
 // is one bulk copy.  All of it is float32, packed two rows an instruction.  Measured (2 x 1,024
 // tokens, 8 heads of 128 x 128): 412 us token after token, 16 + 155 us so.
+//
+// The form is chosen per request, from its own number of tokens, so that its sums do not depend on
+// its neighbours: each kernel leaves the other's requests alone.
 constexpr int DB_TOK = 4, DB_COEF = 32;
 constexpr int DB_STAGE_BLOCKS = 2, DB_STAGES = 4;
 constexpr int DB_WARPS = 4;                       // that work; one more fetches
 __host__ __device__ constexpr int db_floats(int D) { return 13 * D + DB_COEF; }
 
-// blocks of four tokens of the requests before r
-__device__ __forceinline__ int db_first(const int* __restrict__ req_len, int r) {
-  int b = 0;
-  for (int i = 0; i < r; ++i) b += (max(req_len[i], 0) + DB_TOK - 1) / DB_TOK;
-  return b;
+// blocks of four tokens of a request of n tokens (long_from > 0)
+__device__ __forceinline__ int db_blocks(int n, int long_from) {
+  return n >= long_from ? (n + DB_TOK - 1) / DB_TOK : 0;
+}
+// The long request of number i, or (by_block) the one that block number i belongs to: its row, or -1
+// where there are fewer; `before`: blocks of the long requests before it.  By a whole warp, 32
+// requests at a time (one after the other, a block of a step of 64 requests spent 8 us on this).
+__device__ __forceinline__ int db_request(const int* __restrict__ req_len, int n_requests,
+                                          int long_from, int i, bool by_block, int* before) {
+  const int lane = threadIdx.x & 31;
+  int seen = 0;                                    // long requests, or blocks, before these 32
+  *before = 0;
+  for (int r0 = 0; r0 < n_requests; r0 += 32) {
+    const int nb = r0 + lane < n_requests ? db_blocks(req_len[r0 + lane], long_from) : 0;
+    int incl = nb;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += u;
+    }
+    const unsigned many = __ballot_sync(0xffffffffu, nb > 0);
+    const int at = seen + (by_block ? incl - nb : __popc(many & ((1u << lane) - 1u)));
+    const unsigned hit = __ballot_sync(0xffffffffu, nb > 0 && i >= at && i < at + (by_block ? nb : 1));
+    const int total = __shfl_sync(0xffffffffu, incl, 31);
+    if (hit) {
+      const int who = __ffs(hit) - 1;
+      *before += __shfl_sync(0xffffffffu, incl - nb, who);
+      return r0 + who;
+    }
+    seen += by_block ? total : __popc(many);
+    *before += total;
+  }
+  return -1;
 }
 
 __global__ void __launch_bounds__(128)
@@ -366,17 +397,13 @@ delta_blocks_prepare_kernel(float* __restrict__ blocks, const float* __restrict_
                             const float* __restrict__ kn, const float* __restrict__ beta,
                             const float* __restrict__ decay, const int* __restrict__ req_start,
                             const int* __restrict__ req_len, int n_requests, int cap_blocks,
-                            DeltaShape s) {
+                            DeltaShape s, int long_from) {
   __shared__ float red[4][16];
   const int h = blockIdx.y;
-  // the request this block of tokens belongs to
-  int blk = blockIdx.x, r = 0;
-  for (; r < n_requests; ++r) {
-    const int nb = (max(req_len[r], 0) + DB_TOK - 1) / DB_TOK;
-    if (blk < nb) break;
-    blk -= nb;
-  }
-  if (r >= n_requests) return;
+  int before;                                      // the request this block of tokens belongs to
+  const int r = db_request(req_len, n_requests, long_from, blockIdx.x, true, &before);
+  if (r < 0) return;
+  const int blk = blockIdx.x - before;
   const int n = min(DB_TOK, req_len[r] - blk * DB_TOK);       // tokens that exist
   const int t0 = req_start[r] + blk * DB_TOK;
   const int kh = h / (s.heads / s.kv_heads);
@@ -476,16 +503,19 @@ __global__ void __launch_bounds__(DB_WARPS * 32 + 32)
 delta_blocks_kernel(float* __restrict__ o, float* __restrict__ state,
                     const float* __restrict__ blocks, const float* __restrict__ vv,
                     const int* __restrict__ req_start, const int* __restrict__ req_len,
-                    const int* __restrict__ req_slot, int cap_blocks, DeltaShape s, int* status) {
+                    const int* __restrict__ req_slot, int n_requests, int cap_blocks, DeltaShape s,
+                    int long_from, int* status) {
   constexpr int NJ = 4, D = 4 * NJ * KS, SZ = db_floats(D);
   constexpr int COLS = 32 / KS, CTA_COLS = DB_WARPS * COLS;      // of a warp, of the block
   constexpr int ST_TOK = DB_STAGE_BLOCKS * DB_TOK;             // tokens of a stage
   extern __shared__ __align__(16) float sm[];                  // [stages][blocks of a stage][SZ]
   __shared__ float s_v[DB_STAGES][ST_TOK][CTA_COLS];
   __shared__ uint64_t full[DB_STAGES], empty[DB_STAGES];
-  const int r = blockIdx.x, h = blockIdx.y;
+  const int h = blockIdx.y;
+  int before;                                      // (there may be fewer long requests than blocks)
+  const int r = db_request(req_len, n_requests, long_from, blockIdx.x, false, &before);
+  if (r < 0) return;
   const int n = req_len[r];
-  if (n <= 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nb = (n + DB_TOK - 1) / DB_TOK, n_stages = (nb + DB_STAGE_BLOCKS - 1) / DB_STAGE_BLOCKS;
   const int first = req_start[r], HV = s.heads * s.V, col0 = blockIdx.z * CTA_COLS;
@@ -499,7 +529,7 @@ delta_blocks_kernel(float* __restrict__ o, float* __restrict__ state,
   __syncthreads();
   if (warp == DB_WARPS) {
     // the fetching warp: lane 0 copies the blocks of a stage, all lanes the stage's values
-    const float* src = blocks + ((size_t)h * cap_blocks + db_first(req_len, r)) * SZ;
+    const float* src = blocks + ((size_t)h * cap_blocks + before) * SZ;
     const float* vsrc = vv + (size_t)first * HV + h * s.V;
     for (int i = 0; i < n_stages; ++i) {
       const int st = i % DB_STAGES;
@@ -731,58 +761,41 @@ HS_EXPORT int hs_delta_prepare(float* qn, float* kn, float* vv, float* beta, flo
   return HS_OK;
 }
 
-// Floats the blocks of n_tokens tokens of n_requests requests take, or 0 when the sizes are not
-// taken four tokens at a time.
-HS_EXPORT int hs_delta_blocks_scratch(int n_tokens, int n_requests, int heads, int D,
+// requests of long_from tokens or more that n_tokens tokens of n_requests requests can hold, and the
+// blocks of four tokens these can bring
+static int delta_most_long(int n_tokens, int n_requests, int long_from) {
+  const int most = n_tokens / long_from;
+  return n_requests < most ? n_requests : most;
+}
+static int delta_blocks_cap(int n_tokens, int n_requests, int long_from) {
+  return n_tokens / hs::DB_TOK + delta_most_long(n_tokens, n_requests, long_from);
+}
+
+// Floats the blocks of n_tokens tokens of n_requests requests take when those of long_from tokens or
+// more go four tokens at a time, or 0 when none can, by their number or by their size.
+HS_EXPORT int hs_delta_blocks_scratch(int n_tokens, int n_requests, int heads, int D, int long_from,
                                       long long* floats) {
-  if (!floats) return HS_ERR_ARGUMENT;
-  *floats = D == 64 || D == 128 || D == 256
-                ? (long long)heads * (n_tokens / hs::DB_TOK + n_requests) * hs::db_floats(D)
+  if (!floats || long_from <= 0) return HS_ERR_ARGUMENT;
+  *floats = (D == 64 || D == 128 || D == 256) && n_tokens >= long_from
+                ? (long long)heads * delta_blocks_cap(n_tokens, n_requests, long_from) *
+                      hs::db_floats(D)
                 : 0;
   return HS_OK;
 }
 
-// `blocks` (hs_delta_blocks_scratch floats, 16-byte aligned; null: token after token): portions four
-// tokens at a time.
+// `blocks` (hs_delta_blocks_scratch floats, 16-byte aligned; null: token after token): requests of
+// long_from tokens or more go four tokens at a time.  `has_short` 0: there are no others.
 HS_EXPORT int hs_delta_recurrence(float* o, float* state, const float* qn, const float* kn,
                                   const float* vv, const float* beta, const float* decay,
                                   const int* req_start, const int* req_len, const int* req_slot,
                                   int n_requests, int heads, int kv_heads, int D, int V, int taps,
-                                  int ra, int rg, int n_tokens, float* blocks, int* status,
-                                  void* stream) {
+                                  int ra, int rg, int n_tokens, int long_from, int has_short,
+                                  float* blocks, int* status, void* stream) {
   if (!o || !state || !qn || !kn || !vv || !beta || !decay || !req_start || !req_len || !req_slot)
     return HS_ERR_ARGUMENT;
   hs::DeltaShape s;
   int rc = delta_shape(&s, heads, kv_heads, D, V, taps, ra, rg);
   if (rc) return rc;
-  if (blocks && n_requests > 0 && n_tokens > 0) {
-    if ((D != 64 && D != 128 && D != 256) || ((uintptr_t)blocks & 15) || !status)
-      return HS_ERR_ARGUMENT;
-    const int cap = n_tokens / hs::DB_TOK + n_requests;
-    cudaStream_t st = (cudaStream_t)stream;
-    hs::delta_blocks_prepare_kernel<<<dim3(cap, heads), 128, 0, st>>>(
-        blocks, qn, kn, beta, decay, req_start, req_len, n_requests, cap, s);
-    HS_LAUNCH_CHECK();
-    const size_t smem = (size_t)hs::DB_STAGES * hs::DB_STAGE_BLOCKS * hs::db_floats(D) * sizeof(float);
-    cudaError_t e = cudaSuccess;
-#define HS_DB(KS)                                                                                 \
-  do {                                                                                            \
-    const int cols = hs::DB_WARPS * (32 / KS);                                                    \
-    e = cudaFuncSetAttribute(hs::delta_blocks_kernel<KS>,                                     \
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);             \
-    if (e == cudaSuccess)                                                                         \
-      hs::delta_blocks_kernel<KS><<<dim3(n_requests, heads, (V + cols - 1) / cols),           \
-                                        hs::DB_WARPS * 32 + 32, smem, st>>>(                           \
-          o, state, blocks, vv, req_start, req_len, req_slot, cap, s, status);                    \
-  } while (0)
-    if (D == 64) HS_DB(4);
-    else if (D == 128) HS_DB(8);
-    else HS_DB(16);
-#undef HS_DB
-    if (e != cudaSuccess) return (int)e;
-    HS_LAUNCH_CHECK();
-    return HS_OK;
-  }
   if (D > hs::DR_DP * 32) return HS_ERR_UNSUPPORTED;   // a column's parts are lanes of one warp
   if (n_requests <= 0) return HS_OK;
   int KS = 1;
@@ -796,8 +809,42 @@ HS_EXPORT int hs_delta_recurrence(float* o, float* state, const float* qn, const
   const int vec = D % 4 == 0 && !((uintptr_t)qn & 15) && !((uintptr_t)kn & 15) &&
                   !((uintptr_t)decay & 15);
   dim3 grid(n_requests, heads, (V + cols - 1) / cols);
-  hs::delta_recurrence_kernel<<<grid, hs::DR_THREADS, smem, (cudaStream_t)stream>>>(
-      o, state, qn, kn, vv, beta, decay, req_start, req_len, req_slot, s, KS, CH, vec);
+  cudaStream_t st = (cudaStream_t)stream;
+  const bool with_blocks = blocks && n_tokens >= long_from;
+  if (with_blocks && ((D != 64 && D != 128 && D != 256) || ((uintptr_t)blocks & 15) || !status ||
+                      long_from <= 0))
+    return HS_ERR_ARGUMENT;
+  if (has_short || !with_blocks) {
+    hs::delta_recurrence_kernel<<<grid, hs::DR_THREADS, smem, st>>>(
+        o, state, qn, kn, vv, beta, decay, req_start, req_len, req_slot, s, KS, CH, vec,
+        with_blocks ? long_from : 0x7fffffff);
+    HS_LAUNCH_CHECK();
+  }
+  if (!with_blocks) return HS_OK;
+  const int most = delta_most_long(n_tokens, n_requests, long_from);
+  const int cap = delta_blocks_cap(n_tokens, n_requests, long_from);
+  hs::delta_blocks_prepare_kernel<<<dim3(cap, heads), 128, 0, st>>>(
+      blocks, qn, kn, beta, decay, req_start, req_len, n_requests, cap, s, long_from);
+  HS_LAUNCH_CHECK();
+  cudaError_t e = cudaSuccess;
+  const size_t block_smem =
+      (size_t)hs::DB_STAGES * hs::DB_STAGE_BLOCKS * hs::db_floats(D) * sizeof(float);
+#define HS_DB(KS)                                                                                 \
+  do {                                                                                            \
+    const int block_cols = hs::DB_WARPS * (32 / KS);                                              \
+    e = cudaFuncSetAttribute(hs::delta_blocks_kernel<KS>,                                         \
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)block_smem);       \
+    if (e == cudaSuccess)                                                                         \
+      hs::delta_blocks_kernel<KS><<<dim3(most, heads, (V + block_cols - 1) / block_cols),         \
+                                    hs::DB_WARPS * 32 + 32, block_smem, st>>>(                    \
+          o, state, blocks, vv, req_start, req_len, req_slot, n_requests, cap, s, long_from,      \
+          status);                                                                                \
+  } while (0)
+  if (D == 64) HS_DB(4);
+  else if (D == 128) HS_DB(8);
+  else HS_DB(16);
+#undef HS_DB
+  if (e != cudaSuccess) return (int)e;
   HS_LAUNCH_CHECK();
   return HS_OK;
 }

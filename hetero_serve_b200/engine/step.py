@@ -495,9 +495,13 @@ class Runner:
             if self.model.counts_prompt_rows and T >= self.model.prompt_rows_from:
                 plan_shape += (self.ops.plan_prompt_rows(host_batch, self.use_graphs),)
 
+        sides = ()
+        if plan_shape is not None and self.model.portion_limits:
+            sides = self.ops.plan_sides(host_batch, self.model.portion_limits)
+
         # ---- device side -------------------------------------------------------------
         greedy = all(e.temperature <= 0.0 for e in entries)
-        key = (T, R, W, bool(sample), plan_shape, greedy, parity)
+        key = (T, R, W, bool(sample), plan_shape, sides, greedy, parity)
         dev = self._dev_meta.get((T, R, W, parity))
         fresh = dev is None
         if fresh:
@@ -551,6 +555,7 @@ class Runner:
             if plan_shape is not None:
                 from ..kernels.ops import AttentionPlan
                 ctx.plan = AttentionPlan(dev[lay.plan:lay.plan + lay.plan_ints], T, *plan_shape)
+                ctx.plan.sides = sides
             if self.use_graphs and self.model.capturable:
                 # run once eagerly (loads kernels, sizes buffers), then capture and replay.  The
                 # replay must see the same inputs as the eager run: all of them come from the

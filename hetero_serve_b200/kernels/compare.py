@@ -64,7 +64,7 @@ class TimedOps:
 
 _UNTIMED = {"stream", "register_kernel", "load_extension", "attention_plan_ints",
             "plan_attention", "make_plan", "decode_wide", "decode_splits",
-            "latent_prompt_rows", "plan_prompt_rows", "ssm_rows_dtype"}
+            "latent_prompt_rows", "plan_prompt_rows", "plan_sides", "ssm_rows_dtype"}
 
 
 def _contexts(batch):

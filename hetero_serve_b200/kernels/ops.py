@@ -81,6 +81,14 @@ class AttentionPlan:
     single_new: bool = False     # every single-query token is the only new token of its request
     prompt_rows: int = 0         # at least the positions up to the last token of every request that
     #                              brings tiles (0: not counted; only some models' parts ask for it)
+    sides: tuple = ()            # for some limits (``plan_sides``): which requests there are
+
+    def side(self, limit: int) -> tuple[bool, bool]:
+        """Whether some request may bring ``limit`` new tokens or more, and some fewer."""
+        for known, above, below in self.sides:
+            if known == limit:
+                return above, below
+        return True, True
 
     @property
     def tile_slots(self) -> int:
@@ -220,8 +228,8 @@ def _declare(lib) -> None:
                                   I, I, P],
         "hs_latent_prefill_mma_takes": [I, I],
         "hs_delta_prepare": [P] * 15 + [I] * 9 + [P, P],
-        "hs_delta_recurrence": [P] * 10 + [I] * 9 + [P, P, P],
-        "hs_delta_blocks_scratch": [I, I, I, I, P],
+        "hs_delta_recurrence": [P] * 10 + [I] * 11 + [P, P, P],
+        "hs_delta_blocks_scratch": [I, I, I, I, I, P],
         "hs_delta_finish": [P, P, P, P, P, P, I, F, I, I, I, I, I, I, I, I, P, P],
         "hs_moe_route": [P, P, P, P, P, I, I, I, I, I, I, I, P, P],
         "hs_moe_experts": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, F, I, I, P, P, I, I, P],
@@ -783,6 +791,14 @@ class CudaOps:
         rows = sum(start + n for _req, _slot, start, n in host_batch if n > DECODE_MAX_NEW)
         return size_class(rows) if rows and bucketed else rows
 
+    @staticmethod
+    def plan_sides(host_batch, limits) -> tuple[tuple[int, bool, bool], ...]:
+        """``AttentionPlan.sides`` of a batch: per limit whether some request brings as many new
+        tokens, and whether some brings fewer."""
+        new = [n for _req, _slot, _start, n in host_batch if n > 0]
+        return tuple((limit, any(n >= limit for n in new), any(n < limit for n in new))
+                     for limit in limits)
+
     def make_plan(self, host_batch, n_rows: int, page_size: int) -> AttentionPlan:
         """A plan built and uploaded on the spot (the runner packs it into the step's single
         upload instead)."""
@@ -791,7 +807,8 @@ class CudaOps:
         dec, tiles, single = self.plan_attention(view, host_batch, n_rows, len(host_batch),
                                                  page_size, False)
         return AttentionPlan(torch.from_numpy(view).to(self.device), n_rows, dec, tiles, single,
-                             self.plan_prompt_rows(host_batch, False))
+                             self.plan_prompt_rows(host_batch, False),
+                             self.plan_sides(host_batch, sorted(set(self.DELTA_LONG.values()))))
 
     def _scratch_buffer(self, name, numel, dtype):
         key = (name, dtype)
@@ -1441,30 +1458,38 @@ class CudaOps:
             _ptr(req_len), _ptr(req_slot), proj.shape[0], req_start.shape[0], H, HK, D, V, taps,
             ra, rg, _ptr(z_a), self._stream()), "delta_prepare")
 
+    # Tokens from which on a request goes four tokens at a time, by head size.  us, token after token
+    # against blocks of four: 8 heads of 64, 16 portions of 32 tokens 18.5 and 19.5, 8 of 64 25.6 and
+    # 17.3; 8 heads of 128, 16 of 32 78 and 52; 2 heads of 128 with 20 value columns, 64 of 16 12 and
+    # 17, 16 of 32 15 and 12; 4 heads of 256, 16 of 32 185 and 104.
+    DELTA_LONG = {64: 64, 128: 32, 256: 32}
+
     def delta_recurrence(self, o, state, qn, kn, vv, beta, decay, req_start, req_len, req_slot,
-                         shape):
-        """Per request and head on the float32 state S [dim, vdim], token after token or (portions,
-        heads of 64, 128 or 256) four tokens at a time: S <- decay * S; u = beta (v - S^T k);
-        S <- S + k u^T; o = S^T q."""
+                         shape, plan=None):
+        """Per request and head on the float32 state S [dim, vdim]: S <- decay * S;
+        u = beta (v - S^T k); S <- S + k u^T; o = S^T q.  Token after token, or four tokens at a
+        time for a request that brings ``DELTA_LONG[dim]`` tokens or more: the number of its own
+        tokens alone decides, so its sums do not depend on its neighbours.  ``plan``, the step's
+        attention plan, may know that the step has no request of one kind, whose kernels are then
+        not launched."""
         H, HK, D, V, taps, ra, rg = self._delta_sizes(shape)
         for t, nm in ((o, "o"), (qn, "qn"), (kn, "kn"), (vv, "vv"), (beta, "beta"),
                       (decay, "decay")):
             _want(t, nm, torch.float32, 2)
         _want(state, "state", torch.float32)
-        # four tokens at a time where requests bring some eight tokens each: two launches, of which
-        # the second pays its chain once in four tokens
         T, R = o.shape[0], req_start.shape[0]
-        blocks = None
-        if self.delta_blocks and T >= 8 * R:
+        blocks, long_from = None, self.DELTA_LONG.get(D, 0)
+        above, below = (True, True) if plan is None else plan.side(long_from)
+        if self.delta_blocks and long_from and above:
             need = ctypes.c_longlong(0)
-            self.lib.hs_delta_blocks_scratch(T, R, H, D, ctypes.byref(need))
+            self.lib.hs_delta_blocks_scratch(T, R, H, D, long_from, ctypes.byref(need))
             if need.value:
                 blocks = self._scratch_buffer("delta_blocks", need.value, torch.float32)
-        self.launches += 2 if blocks is not None else 1
+        self.launches += 1 if blocks is None else 2 + below
         _check(self.lib.hs_delta_recurrence(
             _ptr(o), _ptr(state), _ptr(qn), _ptr(kn), _ptr(vv), _ptr(beta), _ptr(decay),
             _ptr(req_start), _ptr(req_len), _ptr(req_slot), R, H, HK, D, V,
-            taps, ra, rg, T, _ptr(blocks), _ptr(self.status), self._stream()),
+            taps, ra, rg, T, long_from, int(below), _ptr(blocks), _ptr(self.status), self._stream()),
             f"delta_recurrence(dim={D},vdim={V})")
 
     def delta_finish(self, out, o, proj, g2, norm_w, tok_req, eps, shape, z_g=None):

@@ -81,6 +81,9 @@ class Part:
     counts_prompt_rows: bool = False
     # ... in steps of at least this many tokens
     prompt_rows_from: int = 1
+    # Numbers of new tokens on which the part's route depends, request by request: the runner tells it
+    # through ``plan.sides`` (and captures a graph per answer).
+    portion_limits: tuple = ()
 
     def tensor_requests(self) -> dict[str, TensorRequest]:
         return {}

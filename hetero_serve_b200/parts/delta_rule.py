@@ -20,6 +20,7 @@ from __future__ import annotations
 
 import torch
 
+from ..kernels.ops import CudaOps
 from .base import Mixer, TensorRequest, register_mixer
 
 
@@ -34,6 +35,8 @@ class ChannelDeltaRule(Mixer):
         self.taps, self.eps, self.p = int(taps), float(eps), prefix
         self.channels = 2 * self.HK * self.D + self.H * self.V
         self.shape = None
+        limit = CudaOps.DELTA_LONG.get(dim)
+        self.portion_limits = () if limit is None else (limit,)
 
     def tensor_requests(self):
         p, W = self.p, self.width
@@ -106,8 +109,10 @@ class ChannelDeltaRule(Mixer):
                           self.a_log, state, ctx.tok_req, ctx.req_start, ctx.req_len,
                           ctx.req_slot, self.shape, z_a=z_a)
         o = ctx.buffer("delta_o", (T, self.H * self.V), f32)
+        plan = getattr(ctx, "plan", None)
+        plan = {} if plan is None else {"plan": plan}
         ops.delta_recurrence(o, state, qn, kn, vv, beta, decay, ctx.req_start, ctx.req_len,
-                             ctx.req_slot, self.shape)
+                             ctx.req_slot, self.shape, **plan)
         gated = ctx.buffer("delta_gated", (T, self.H * self.V), ctx.dtype)
         ops.delta_finish(gated, o, proj, self.g2, self.norm_w, ctx.tok_req, self.eps, self.shape,
                          z_g=z_g)

@@ -389,6 +389,7 @@ class Model:
         self.keeps_embedding = any(call.adds_embedding for call in self.schedule)
         self.capturable = all(part.capturable for part in self.parts())
         self._derive_prompt_rows()
+        self.portion_limits = sorted({n for part in self.parts() for n in part.portion_limits})
         self._derive_cache()
         self.dtype = None
         self.device = None
