@@ -18,7 +18,9 @@
 // The keys of the next chunk are on their way from the end of the scores on, the values from the end
 // of the values on.  112 KB of shared memory, so two blocks an SM.  Keys arrive by 4-byte cp.async
 // copies into d-major rows whose columns are XORed against bank conflicts.  Chunks that some query of
-// the block does not see, or whose pages were refused, take a path that adds visible keys only.
+// the block does not see, or whose pages were refused, take a path that adds visible keys only, and so
+// do chunks in which some query has no score above minus infinity: it leaves such a chunk out, as the
+// one-token kernel does (its weights would be zeros, which make NaN of an infinite value).
 // Bounded by the FMA pipe and by shared-memory reads.  Measured (2 x 512 tokens, 16 heads): 340 us in
 // attention_simt.cu, 84 us here (13 TFLOP/s of causal work).
 #include "common.cuh"
@@ -68,6 +70,16 @@ __device__ __forceinline__ void af_commit() { asm volatile("cp.async.commit_grou
 // the 64 threads of a stream
 __device__ __forceinline__ void af_sync(int stream) {
   asm volatile("bar.sync %0, 64;" ::"r"(1 + stream) : "memory");
+}
+
+// ... and whether any of them says so
+__device__ __forceinline__ bool af_sync_any(int stream, bool mine) {
+  unsigned any;
+  asm volatile(
+      "{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n barrier.cta.red.or.pred q, %2, 64, p;\n"
+      " selp.u32 %0, 1, 0, q;\n}"
+      : "=r"(any) : "r"((unsigned)mine), "r"(1 + stream) : "memory");
+  return any != 0;
 }
 
 __global__ void __launch_bounds__(AF_THREADS, 2)
@@ -206,8 +218,9 @@ attention_f32_tile_kernel(const AfParams p) {
       af_commit();
     }
     // every query sees every key of the chunk
-    const bool whole = here == 0xffffffffu && j0 + AF_CHUNK - 1 <= pos0;
+    bool whole = here == 0xffffffffu && j0 + AF_CHUNK - 1 <= pos0;
     // ---- softmax: query t
+    bool left_out = false;
     {
       float x[AF_CHUNK];
       float* col = sS + (t & 32);
@@ -221,6 +234,7 @@ attention_f32_tile_kernel(const AfParams p) {
       for (int k = 1; k < AF_CHUNK; ++k) cm = fmaxf(cm, x[k]);
       const float m_new = fmaxf(m, cm);
       float corr = 1.f;
+      left_out = m_new == -INFINITY && j0 <= pos_t;          // (no corr below is negative)
       if (m_new == -INFINITY || j0 > pos_t) {                // nothing of the chunk is this query's
 #pragma unroll
         for (int k = 0; k < AF_CHUNK; ++k) x[k] = 0.f;
@@ -239,10 +253,10 @@ attention_f32_tile_kernel(const AfParams p) {
         l = l * corr + x[0];
         m = m_new;
       }
-      s_corr[stream][t] = corr;
+      s_corr[stream][t] = left_out ? -1.f : corr;
     }
     asm volatile("cp.async.wait_group 1;" ::: "memory");     // this chunk's values
-    af_sync(stream);
+    if (af_sync_any(stream, left_out)) whole = false;
     // ---- values
     {
       const float4 c0 = *(const float4*)&s_corr[stream][qg * 4];
@@ -250,7 +264,7 @@ attention_f32_tile_kernel(const AfParams p) {
       const float cr[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        const uint64_t c2 = af_twice(cr[i]);
+        const uint64_t c2 = af_twice(cr[i] < 0.f ? 1.f : cr[i]);
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = af_mul2(acc[i][j], c2);
       }
@@ -274,7 +288,7 @@ attention_f32_tile_kernel(const AfParams p) {
           const int first = j0 + k - pos0;                   // the first query that sees the key
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
-            if ((i < 4 ? qg * 4 + i : 28 + qg * 4 + i) < first) continue;
+            if ((i < 4 ? qg * 4 + i : 28 + qg * 4 + i) < first || cr[i] < 0.f) continue;
             const uint64_t p2 = af_twice(pv[i]);
             af_fma2(acc[i][0], p2, v0.x);
             af_fma2(acc[i][1], p2, v0.y);

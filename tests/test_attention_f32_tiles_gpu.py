@@ -52,6 +52,42 @@ def test_same_bits_as_token_by_token(heads, kv_heads, page, batch):
     assert ops.status.item() == 0
 
 
+@pytest.mark.parametrize("start,tokens", [(0, 200), (130, 70), (40, 1), (64, 33)])
+@pytest.mark.parametrize("scale", [0.125, -0.125])
+def test_chunks_in_which_no_score_is_above_minus_infinity(start, tokens, scale):
+    """Keys of whole chunks whose scores overflow to minus infinity, for some queries or for all, with
+    values that are infinite or NaN there: a query leaves such a chunk out."""
+    ops, D, page = CudaOps(DEV), 64, 16
+    g = torch.Generator(device=DEV).manual_seed(start + tokens)
+    end = start + tokens
+    n_pages = -(-end // page)
+    pool = torch.randn(n_pages, 2, 1, page, D, device=DEV, generator=g)
+    qkv = torch.randn(tokens, 3 * D, device=DEV, generator=g)
+    keys = lambda a, b: (slice(a // page, b // page), 0, 0)  # noqa: E731
+    vals = lambda a, b: (slice(a // page, b // page), 1, 0)  # noqa: E731
+    sign = 1.0 if scale > 0 else -1.0
+    qkv[:, 0] = 2.0 * sign * torch.where(torch.arange(tokens, device=DEV) % 3 == 0, -1.0, 1.0)
+    for a, bad in ((0, float("inf")), (96, float("nan"))):   # one chunk of two streams
+        if a + 32 <= end:
+            pool[keys(a, a + 32)][..., 0] = -3e38            # every third query: + infinity
+            pool[vals(a, a + 32)][..., 5] = bad
+    table = torch.arange(n_pages, dtype=torch.int32, device=DEV).view(1, -1)
+    geo = AttentionGeometry(1, 1, D, page, n_pages, n_pages, 0, D, 2 * D, 3 * D)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    plan = ops.make_plan([(0, 0, start, tokens)], tokens, page)
+    outs = []
+    for tiles in (True, False):
+        ops.f32_tiles = ops.f32_single = tiles
+        out = torch.zeros(tokens, D, device=DEV)
+        ops.attention(out, qkv, pool, table, i32(list(range(start, end))), i32([0] * tokens), geo,
+                      scale, ops.status, plan)
+        outs.append(torch.nan_to_num(out, nan=-77.0, posinf=-78.0, neginf=-79.0))
+    assert torch.equal(*outs)
+    rest = outs[0][torch.arange(tokens, device=DEV) % 3 != 0]
+    if end > 160 and start > 31:                             # those that skip both chunks are finite
+        assert (rest > -70.0).all()
+
+
 @pytest.mark.parametrize("tokens", [20, 3])
 def test_refused_page_is_reported(tokens):
     ops, D = CudaOps(DEV), 64
