@@ -37,8 +37,9 @@ constexpr size_t AF_SMEM = (AF_Q_FLOATS + AF_STREAMS * AF_STREAM_FLOATS) * sizeo
 struct AfParams {
   float* out;
   const float *qkv, *pool;
-  const int *table, *tile_info, *plan_head;
+  const int *table, *tile_info, *plan_head, *tok_req;
   int* status;
+  int n_tokens;
   int n_heads, n_kv_heads, page_size, num_pages, max_pages, q_off, qkv_stride;
   float scale;
 };
@@ -86,6 +87,12 @@ __global__ void __launch_bounds__(AF_THREADS, 2)
 attention_f32_tile_kernel(const AfParams p) {
   extern __shared__ __align__(16) float af_smem[];
   __shared__ float s_m[AF_STREAMS][AF_Q], s_l[AF_STREAMS][AF_Q], s_corr[AF_STREAMS][AF_Q];
+  // rows of no request (a captured step's padding): zeros
+  for (int i = blockIdx.x * AF_THREADS + threadIdx.x; i < p.n_tokens; i += gridDim.x * AF_THREADS)
+    if (p.tok_req[i] < 0) {
+      float* row = p.out + ((size_t)i * p.n_heads + blockIdx.y) * AF_D;
+      for (int d = 0; d < AF_D; ++d) row[d] = 0.f;
+    }
   if ((int)(blockIdx.x >> 1) >= p.plan_head[1]) return;
   const int4 ti = *(const int4*)(p.tile_info + 4 * (blockIdx.x >> 1));
   const int q0 = (blockIdx.x & 1) * AF_Q;
@@ -533,14 +540,17 @@ static_assert(hs::AF_STREAMS * hs::AF_Q * (hs::AF_D + 4) * sizeof(float) <= hs::
               "the folded accumulators fit where queries, keys, values and scores were");
 
 // The plan's tiles (prompt portions): float32, head size 64, no window; `tile_info` entries of up to
-// 128 queries (first token, queries, request row, first position).
+// 128 queries (first token, queries, request row, first position).  Rows of tokens without a request
+// (tok_req below zero) become zeros.
 HS_EXPORT int hs_attention_f32_tiles(float* out, const float* qkv, const float* pool,
-                                     const int* table, const int* tile_info, const int* plan_head,
-                                     int tile_cap, int n_heads, int n_kv_heads, int head_dim,
+                                     const int* table, const int* tok_req, int n_tokens,
+                                     const int* tile_info, const int* plan_head, int tile_cap,
+                                     int n_heads, int n_kv_heads, int head_dim,
                                      int page_size, int num_pages, int max_pages, int q_off,
                                      int qkv_stride, float scale, int* status, void* stream) {
   using namespace hs;
-  if (!out || !qkv || !pool || !table || !tile_info || !plan_head || !status) return HS_ERR_ARGUMENT;
+  if (!out || !qkv || !pool || !table || !tok_req || !tile_info || !plan_head || !status)
+    return HS_ERR_ARGUMENT;
   if (head_dim != AF_D || n_heads <= 0 || n_kv_heads <= 0 || n_heads % n_kv_heads ||
       n_heads > 65535 || page_size <= 0 || num_pages <= 0 || max_pages <= 0 ||
       ((uintptr_t)pool & 15) || ((uintptr_t)tile_info & 15) || tile_cap > (1 << 28))
@@ -549,8 +559,8 @@ HS_EXPORT int hs_attention_f32_tiles(float* out, const float* qkv, const float* 
   cudaError_t e = cudaFuncSetAttribute(attention_f32_tile_kernel,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AF_SMEM);
   if (e != cudaSuccess) return (int)e;
-  AfParams p{out, qkv, pool, table, tile_info, plan_head, status, n_heads, n_kv_heads, page_size,
-             num_pages, max_pages, q_off, qkv_stride, scale};
+  AfParams p{out, qkv, pool, table, tile_info, plan_head, tok_req, status, n_tokens, n_heads,
+             n_kv_heads, page_size, num_pages, max_pages, q_off, qkv_stride, scale};
   attention_f32_tile_kernel<<<dim3(2 * tile_cap, n_heads), AF_THREADS, AF_SMEM,
                               (cudaStream_t)stream>>>(p);
   HS_LAUNCH_CHECK();
@@ -572,8 +582,8 @@ HS_EXPORT int hs_attention_f32_single(float* out, const float* qkv, const float*
       n_heads > 65535 || page_size <= 0 || num_pages <= 0 || max_pages <= 0 || ((uintptr_t)pool & 15))
     return HS_ERR_UNSUPPORTED;
   if (n_tokens <= 0) return HS_OK;
-  AfParams p{out, qkv, pool, table, nullptr, nullptr, status, n_heads, n_kv_heads, page_size,
-             num_pages, max_pages, q_off, qkv_stride, scale};
+  AfParams p{out, qkv, pool, table, nullptr, nullptr, tok_req, status, n_tokens, n_heads,
+             n_kv_heads, page_size, num_pages, max_pages, q_off, qkv_stride, scale};
   // up to a block an SM: the deepest ring; more blocks: three share an SM instead
   const bool deep = (long long)n_tokens * n_heads <= hs_sm_count();
   cudaError_t e;

@@ -200,7 +200,7 @@ def _declare(lib) -> None:
         "hs_attention_simt": [P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, I, F, I, P, P],
         "hs_attention_simt_grouped": [P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, I, F, I, I,
                                       P, P, P, P],
-        "hs_attention_f32_tiles": [P] * 6 + [I] * 9 + [F, P, P],
+        "hs_attention_f32_tiles": [P] * 5 + [I, P, P] + [I] * 9 + [F, P, P],
         "hs_attention_f32_single": [P] * 8 + [I] * 9 + [F, P, P],
         "hs_attention_decode_append": [P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, I,
                                        F, I, I, I, I, P, P, P, P, P],
@@ -874,7 +874,7 @@ class CudaOps:
                 and qkv.dtype == torch.float32 and g.window == 0 and g.head_dim == 64):
             # prompt portions as tiles of queries (the same bits); the single tokens stay behind
             code = self.lib.hs_attention_f32_tiles(
-                _ptr(out), _ptr(qkv), _ptr(pool), _ptr(table),
+                _ptr(out), _ptr(qkv), _ptr(pool), _ptr(table), _ptr(tok_req), n,
                 _ptr(plan.data[4 + plan_decode_ints(plan.n_rows):]), _ptr(plan.data),
                 plan.tile_cap, g.n_heads, g.n_kv_heads, g.head_dim, g.page_size, g.num_pages,
                 g.max_pages, g.q_off, g.qkv_stride, scale, _ptr(status), self._stream())

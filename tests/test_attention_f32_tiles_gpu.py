@@ -88,6 +88,30 @@ def test_chunks_in_which_no_score_is_above_minus_infinity(start, tokens, scale):
         assert (rest > -70.0).all()
 
 
+@pytest.mark.parametrize("batch", [[(0, 40)], [(0, 40), (9, 1)], [(0, 9), (100, 140), (3, 1), (50, 3)]])
+def test_rows_of_no_request_become_zeros(batch):
+    """Padding behind the tokens of a step, as captured steps have it, beside portions and singles."""
+    ops, D, H, page = CudaOps(DEV), 64, 2, 16
+    T, R, pad = sum(n for _, n in batch), len(batch), 700
+    width = max(-(-(p + n) // page) for p, n in batch)
+    table = torch.arange(R * width, dtype=torch.int32, device=DEV).view(R, width)
+    geo = AttentionGeometry(H, H, D, page, R * width, width, 0, H * D, 2 * H * D, 3 * H * D)
+    g = torch.Generator(device=DEV).manual_seed(T)
+    qkv = torch.randn(T + pad, 3 * H * D, device=DEV, generator=g)
+    pool = torch.randn(R * width, 2, H, page, D, device=DEV, generator=g)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    pos = i32([p + i for p, n in batch for i in range(n)] + [0] * pad)
+    req = i32([r for r, (_, n) in enumerate(batch) for _ in range(n)] + [-1] * pad)
+    plan = ops.make_plan([(r, r, p, n) for r, (p, n) in enumerate(batch)], T + pad, page)
+    outs = []
+    for tiles in (True, False):
+        ops.f32_tiles = ops.f32_single = tiles
+        out = torch.full((T + pad, H * D), float("nan"), device=DEV)
+        ops.attention(out, qkv, pool, table, pos, req, geo, 0.125, ops.status, plan)
+        outs.append(out)
+    assert torch.equal(*outs) and not outs[0][T:].any() and ops.status.item() == 0
+
+
 @pytest.mark.parametrize("tokens", [20, 3])
 def test_refused_page_is_reported(tokens):
     ops, D = CudaOps(DEV), 64
