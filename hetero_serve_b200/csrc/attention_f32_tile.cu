@@ -16,7 +16,7 @@
 //     softmax  a thread per query: its 32 scores from shared memory, the weights back to their place;
 //     values   8 queries x 8 dimensions a thread, packed two dimensions an FMA.
 // The keys of the next chunk are on their way from the end of the scores on, the values from the end
-// of the values on.  112 KB of shared memory, so two blocks an SM.  Keys arrive by 4-byte cp.async
+// of the values on.  113 KB of shared memory: two blocks can share an SM.  Keys arrive by 4-byte cp.async
 // copies into d-major rows whose columns are XORed against bank conflicts.  Chunks that some query of
 // the block does not see, or whose pages were refused, take a path that adds visible keys only, and so
 // do chunks in which some query has no score above minus infinity: it leaves such a chunk out, as the
@@ -83,10 +83,15 @@ __device__ __forceinline__ bool af_sync_any(int stream, bool mine) {
   return any != 0;
 }
 
-__global__ void __launch_bounds__(AF_THREADS, 2)
+// BLOCKS an SM: two (128 registers a thread, some of them spilled) where there are more than two blocks
+// an SM, else one (no such limit).  us, one block an SM against two, 12 heads: 64 portions of 16 tokens
+// 59 and 45, 16 of 200 behind 300 positions 231 and 218; but one of 1,000 behind 3,000 507 and 567, 16
+// of 8 tokens and 2 heads behind 3,000 218 and 287.
+template <int BLOCKS>
+__global__ void __launch_bounds__(AF_THREADS, BLOCKS)
 attention_f32_tile_kernel(const AfParams p) {
   extern __shared__ __align__(16) float af_smem[];
-  __shared__ float s_m[AF_STREAMS][AF_Q], s_l[AF_STREAMS][AF_Q], s_corr[AF_STREAMS][AF_Q];
+  __shared__ float s_corr[AF_STREAMS][AF_Q];
   // rows of no request (a captured step's padding): zeros
   for (int i = blockIdx.x * AF_THREADS + threadIdx.x; i < p.n_tokens; i += gridDim.x * AF_THREADS)
     if (p.tok_req[i] < 0) {
@@ -314,6 +319,8 @@ attention_f32_tile_kernel(const AfParams p) {
   __syncthreads();
   float* fold = af_smem;                                     // [stream][query][d], 68 floats a row
   constexpr int LD = AF_D + 4;
+  float(*s_m)[AF_Q] = (float(*)[AF_Q])(fold + AF_STREAMS * AF_Q * LD);      // behind the rows
+  float(*s_l)[AF_Q] = s_m + AF_STREAMS;
   s_m[stream][t] = m;
   s_l[stream][t] = l;
 #pragma unroll
@@ -536,8 +543,11 @@ attention_f32_single_kernel(const AfParams p, const int* __restrict__ tok_pos,
 
 }  // namespace hs
 
-static_assert(hs::AF_STREAMS * hs::AF_Q * (hs::AF_D + 4) * sizeof(float) <= hs::AF_SMEM,
-              "the folded accumulators fit where queries, keys, values and scores were");
+static_assert(hs::AF_STREAMS * hs::AF_Q * (hs::AF_D + 4 + 2) * sizeof(float) <= hs::AF_SMEM,
+              "the folded accumulators, maxima and sums fit where queries, keys, values and scores were");
+// (an SM has 228 KB; a block is charged its static array and 1 KB of the system's beside them)
+static_assert(2 * (hs::AF_SMEM + hs::AF_STREAMS * hs::AF_Q * sizeof(float) + 1024) <= 228 * 1024,
+              "two blocks share an SM");
 
 // The plan's tiles (prompt portions): float32, head size 64, no window; `tile_info` entries of up to
 // 128 queries (first token, queries, request row, first position).  Rows of tokens without a request
@@ -556,13 +566,13 @@ HS_EXPORT int hs_attention_f32_tiles(float* out, const float* qkv, const float* 
       ((uintptr_t)pool & 15) || ((uintptr_t)tile_info & 15) || tile_cap > (1 << 28))
     return HS_ERR_UNSUPPORTED;
   if (tile_cap <= 0) return HS_OK;
-  cudaError_t e = cudaFuncSetAttribute(attention_f32_tile_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AF_SMEM);
-  if (e != cudaSuccess) return (int)e;
   AfParams p{out, qkv, pool, table, tile_info, plan_head, tok_req, status, n_tokens, n_heads,
              n_kv_heads, page_size, num_pages, max_pages, q_off, qkv_stride, scale};
-  attention_f32_tile_kernel<<<dim3(2 * tile_cap, n_heads), AF_THREADS, AF_SMEM,
-                              (cudaStream_t)stream>>>(p);
+  const bool two = 2ll * tile_cap * n_heads > 2ll * hs_sm_count();
+  auto* kernel = two ? attention_f32_tile_kernel<2> : attention_f32_tile_kernel<1>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AF_SMEM);
+  if (e != cudaSuccess) return (int)e;
+  kernel<<<dim3(2 * tile_cap, n_heads), AF_THREADS, AF_SMEM, (cudaStream_t)stream>>>(p);
   HS_LAUNCH_CHECK();
   return HS_OK;
 }
