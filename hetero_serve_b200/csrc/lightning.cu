@@ -252,23 +252,27 @@ constexpr int LS_TOK = 8, LS_STAGES = 4, LS_WARPS = 4;
 __host__ __device__ constexpr int ls_cols(int D) { return LS_WARPS * 32 * LA_ROWS / D; }
 
 // q | k of token t and head h: rows + ((h * n_tokens + t) * 2 D); value column c of head h: group
-// c / cols: vals + (((h * groups + c / cols) * n_tokens + t) * cols + c % cols), columns past V zero
+// c / cols: vals + (((h * groups + c / cols) * n_tokens + t) * cols + c % cols), columns past V zero.
+// A block takes one token and `per` heads: all of them where there are tokens enough, fewer where the
+// blocks would leave SMs idle (the whole operation, 128 tokens of 32 heads of 128: 71 us with one
+// block a token, 28 so).
 __global__ void __launch_bounds__(256)
 lightning_rows_kernel(float* __restrict__ rows, float* __restrict__ vals,
                       const float* __restrict__ proj, int n_tokens, int stride, int q_off, int k_off,
                       int v_off, int H, int D, int V, int act, const int* __restrict__ tok_pos,
-                      const float* __restrict__ freq, int rot_dims, float k_scale) {
+                      const float* __restrict__ freq, int rot_dims, float k_scale, int per) {
   pdl_trigger();
   pdl_wait();
   __shared__ float s_c[128], s_s[128];
+  const int h0 = blockIdx.y * per, nh = min(per, H - h0);
   const int t = blockIdx.x, half = rot_dims >> 1;
   const int pos = rot_dims > 0 ? tok_pos[t] : 0;
   for (int i = threadIdx.x; i < half; i += blockDim.x) pair_angle(pos, freq[i], &s_c[i], &s_s[i]);
   __syncthreads();
   const float* row = proj + (size_t)t * stride;
   const int P4 = D / 4;                                   // floats of a piece over all parts
-  for (int x = threadIdx.x; x < 2 * H * D; x += blockDim.x) {
-    const int h = x / (2 * D), y = x - h * 2 * D;
+  for (int x = threadIdx.x; x < 2 * nh * D; x += blockDim.x) {
+    const int hh = x / (2 * D), y = x - hh * 2 * D, h = h0 + hh;
     const bool is_q = y < D;
     const int z = is_q ? y : y - D;
     const int j = z / P4, part = (z - j * P4) >> 2, e = z & 3;
@@ -287,8 +291,8 @@ lightning_rows_kernel(float* __restrict__ rows, float* __restrict__ vals,
     rows[((size_t)h * n_tokens + t) * 2 * D + y] = __fmul_rn(own, is_q ? 1.0f : k_scale);
   }
   const int cols = ls_cols(D), groups = (V + cols - 1) / cols;
-  for (int x = threadIdx.x; x < H * groups * cols; x += blockDim.x) {
-    const int h = x / (groups * cols), c = x - h * groups * cols, g = c / cols;
+  for (int x = threadIdx.x; x < nh * groups * cols; x += blockDim.x) {
+    const int hh = x / (groups * cols), c = x - hh * groups * cols, g = c / cols, h = h0 + hh;
     vals[(((size_t)h * groups + g) * n_tokens + t) * cols + (c - g * cols)] =
         c < V ? la_act(row[v_off + h * V + c], act) : 0.f;
   }
@@ -454,10 +458,19 @@ lightning_stream_kernel(float* __restrict__ o, float* __restrict__ state,
 
 }  // namespace hs
 
+// Whether a step goes as a stream: sizes it is written for, and four tokens a request or more on
+// average.  With fewer the blocks' set-up outweighs what a token saves (256 single
+// tokens, 8 heads of 128: 145 us as a stream, 131 otherwise); the bits are the same
+// either way.
+static bool lightning_streams(int n_tokens, int n_requests, int D) {
+  return (D == 64 || D == 128 || D == 256) && n_tokens >= 4ll * n_requests;
+}
+
 // Floats of scratch with which hs_lightning_recurrence takes many tokens a step.
-HS_EXPORT int hs_lightning_scratch(int n_tokens, int H, int D, int V, long long* floats) {
+HS_EXPORT int hs_lightning_scratch(int n_tokens, int n_requests, int H, int D, int V,
+                                   long long* floats) {
   if (!floats || n_tokens < 0 || H <= 0 || D <= 0 || V <= 0) return HS_ERR_ARGUMENT;
-  if (D == 64 || D == 128 || D == 256) {
+  if (lightning_streams(n_tokens, n_requests, D)) {
     const int cols = hs::ls_cols(D);
     *floats = (long long)n_tokens * H * (2 * D + (V + cols - 1) / cols * cols);
   } else {
@@ -485,14 +498,17 @@ HS_EXPORT int hs_lightning_recurrence(float* o, float* state, const float* proj,
     return HS_ERR_UNSUPPORTED;
   if (n_requests <= 0 || n_tokens <= 0) return HS_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  if (scratch && status && (D == 64 || D == 128 || D == 256) && !((uintptr_t)scratch & 15)) {
+  if (scratch && status && lightning_streams(n_tokens, n_requests, D) && !((uintptr_t)scratch & 15)) {
     // (measured, 2 x 1,024 tokens, 8 heads of 128 x 128: retention's mixer takes 176 us this way, 395
     // with the two kernels below)
     const int cols = hs::ls_cols(D), groups = (V + cols - 1) / cols;
     float* vals = scratch + (size_t)n_tokens * H * 2 * D;
-    cudaError_t e = hs_launch(hs::lightning_rows_kernel, dim3(n_tokens), dim3(256), 0, st,
+    const int want = (8 * hs_sm_count() + n_tokens - 1) / n_tokens;     // blocks a token
+    const int per = want >= H ? 1 : (H + want - 1) / want;
+    cudaError_t e = hs_launch(hs::lightning_rows_kernel, dim3(n_tokens, (H + per - 1) / per),
+                              dim3(256), 0, st,
                               hs_pdl_enabled(), scratch, vals, proj, n_tokens, stride, q_off, k_off,
-                              v_off, H, D, V, act, tok_pos, freq, rot_dims, k_scale);
+                              v_off, H, D, V, act, tok_pos, freq, rot_dims, k_scale, per);
     if (e != cudaSuccess) return (int)e;
     const size_t smem = (size_t)hs::LS_STAGES * hs::LS_TOK * (2 * D + cols) * sizeof(float);
 #define HS_LS(P)                                                                                 \

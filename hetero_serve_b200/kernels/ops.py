@@ -246,7 +246,7 @@ def _declare(lib) -> None:
                                         F, F, I, I, P, P],
         "hs_lightning_recurrence": [P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, P, P, P, I,
                                     F, P, P],
-        "hs_lightning_scratch": [I, I, I, I, P],
+        "hs_lightning_scratch": [I, I, I, I, I, P],
         "hs_token_shift_mix": [P, P, P, P, I, I, P, P, P, P, I, I, I, I, P],
         "hs_timemix_decay": [P, P, P, P, I, I, I, P],
         "hs_timemix_recurrence": [P, P, I, P, P, P, P, P, P, P, P, I, I, I, I, P],
@@ -1927,7 +1927,8 @@ class CudaOps:
         scratch = None
         if T >= self.lightning_bulk_rows:
             need = ctypes.c_longlong(0)
-            self.lib.hs_lightning_scratch(T, heads, dim, vdim, ctypes.byref(need))
+            self.lib.hs_lightning_scratch(T, req_start.shape[0], heads, dim, vdim,
+                                          ctypes.byref(need))
             if need.value:
                 scratch = self._scratch_buffer("lightning_rows", need.value, torch.float32)
         self.launches += 2 if scratch is not None else 1

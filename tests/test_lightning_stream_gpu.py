@@ -40,3 +40,35 @@ def test_same_bits_as_few_tokens(dim, vdim, rot, act, lens):
     assert torch.isfinite(got[0][0]).all()
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
     assert ops.status.item() == 0
+
+
+@pytest.mark.parametrize("dim,vdim", [(64, 64), (128, 30), (256, 12)])
+@pytest.mark.parametrize("heads", [1, 5])
+def test_steps_of_few_tokens_a_request_do_not_stream(dim, vdim, heads):
+    """Single tokens beside each other: the kernel for few tokens, and the bits of the stream that the
+    same tokens take as parts of longer portions."""
+    ops = CudaOps(DEV)
+    g = torch.Generator(device=DEV).manual_seed(dim + heads)
+    T = 70
+    proj = torch.randn(T, heads * (2 * dim + vdim), device=DEV, generator=g)
+    decay = torch.rand(heads, device=DEV, generator=g)
+    state0 = torch.randn(T, heads * dim * vdim, device=DEV, generator=g)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+
+    def run(lens, rows):
+        o, state = torch.zeros(len(rows), heads * vdim, device=DEV), state0.clone()
+        before = ops.launches
+        ops.lightning_recurrence(o, state, proj[rows].contiguous(), decay,
+                                 i32([sum(lens[:r]) for r in range(len(lens))]), i32(lens),
+                                 i32(list(range(len(lens)))), q_off=0, k_off=heads * dim,
+                                 v_off=2 * heads * dim, heads=heads, dim=dim, vdim=vdim, act="silu")
+        return o, state, ops.launches - before
+    o, state, launches = run([1] * T, list(range(T)))
+    assert launches == (2 if vdim % 4 == 0 else 1)
+    # each of the first eight tokens at the head of a portion of its own
+    rows = [r if i == 0 else (r + 9 * i) % T for r in range(8) for i in range(9)]
+    want, _, launches = run([9] * 8, rows)
+    assert launches == 2
+    for r in range(8):
+        assert torch.equal(o[r], want[9 * r])
+    assert ops.status.item() == 0
