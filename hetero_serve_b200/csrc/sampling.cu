@@ -276,6 +276,9 @@ sample_kernel(int* __restrict__ out, const float* __restrict__ logits,
 // with it at 50,257 logits.
 constexpr int SS_THREADS = 1024;
 constexpr int SS_CAND = 1024;       // entries that may be among the k largest
+constexpr int SS_LIST_K = 512;      // the largest k for which they are listed ...
+constexpr int SS_LIST_VOCAB = 12000;    // ... the shortest row ...
+constexpr int SS_LIST_MAXIMA = 600;     // ... and the most maxima from the bound up (903 entries)
 
 __device__ float block_max_f(float v) {
   __shared__ float sh[SS_THREADS / 32];
@@ -385,7 +388,8 @@ sample_smem_kernel(int* __restrict__ out, const float* __restrict__ logits,
     s_last = 0;
     s_n = 0;
   }
-  const float mx = block_max_f(m) / temp;           // (its barriers also publish the row)
+  const float top = block_max_f(m);                 // (its barriers also publish the row)
+  const float mx = top / temp;
   int C = (vocab + blockDim.x - 1) / blockDim.x;
   C |= 1;                                           // odd
   const int lo = min(vocab, (int)threadIdx.x * C), hi = min(vocab, lo + C);
@@ -450,15 +454,20 @@ sample_smem_kernel(int* __restrict__ out, const float* __restrict__ logits,
       for (int i = lo; i < hi; ++i) take(order_key(s_row[i]));
     };
     // Few of the row's entries can be among the k largest: k of the threads' maxima, so k entries,
-    // are no smaller than the k-th largest maximum.  The entries from there up (k and a few more)
-    // are listed in one walk and the threshold is found among them; walking the row once per digit
-    // took 4 us a digit at 50,257 logits (32 rows, a third with top-k 40: 56 us, 42 this way).  More of them than the list holds (many equal logits), or
-    // more wanted than there are threads: the digits walk the row.
-    bool listed = k <= (int)blockDim.x && k <= SS_CAND;
-    if (listed) {
-      const uint32_t own = order_key(m);
+    // are no smaller than the k-th largest maximum.  In a row in no order about 1,024 ln(1024 / (1024
+    // - k)) entries lie from there up (41 for k = 40, 710 for 512, the list's 1,024 at 647); they are
+    // listed in one walk and the threshold is found among them.  A walk of the row per digit takes 4
+    // us at 50,257 logits, the selection among the maxima 3 (32 rows, digits against list: k = 40 41.9
+    // and 28.7 us, k = 512 44.2 and 33.3; 12,000 logits, k = 40 16.1 and 14.4, k = 512
+    // 17.2 and 16.7; 5,000 logits, k = 40 10.7 and 11.4).  So the digits walk the row where k is larger or the row is short, where the maxima are mostly
+    // equal (then the entries are too), and where the list overflows after all.
+    bool listed = k <= SS_LIST_K && vocab >= SS_LIST_VOCAB;
+    const uint32_t own = order_key(m);
+    if (listed && !__syncthreads_and(own == order_key(top))) {
       const uint32_t bound = select(k, [&](auto take) { take(own); });
-      for (int i = lo; i < hi; ++i) {
+      // maxima from the bound up: k, and those equal to it that k leaves out
+      listed = k - remaining + s_same <= SS_LIST_MAXIMA;
+      for (int i = listed ? lo : hi; i < hi; ++i) {
         const uint32_t key = order_key(s_row[i]);
         if (key >= bound) {
           const int at = atomicAdd(&s_n, 1);
@@ -466,7 +475,9 @@ sample_smem_kernel(int* __restrict__ out, const float* __restrict__ logits,
         }
       }
       __syncthreads();
-      listed = s_n >= k && s_n <= SS_CAND;
+      listed = listed && s_n >= k && s_n <= SS_CAND;
+    } else {
+      listed = false;
     }
     if (listed) {
       const int n = s_n;

@@ -13,8 +13,8 @@ DEV = "cuda"
 
 
 @pytest.mark.parametrize("vocab,step", [(50257, 0.25), (50257, 2.0), (50257, 0.0), (5000, 1.0),
-                                        (56320, 0.5)])
-@pytest.mark.parametrize("top_k", [1, 40, 1023, 1024, 1025])
+                                        (56320, 0.5), (12000, 1.0), (11999, 0.05)])
+@pytest.mark.parametrize("top_k", [1, 40, 511, 512, 513, 1023, 1024, 1025])
 def test_threshold_among_equal_logits(vocab, step, top_k):
     ops, plain = CudaOps(DEV), plain_ops.PlainOps()
     g = torch.Generator(device=DEV).manual_seed(vocab + top_k)
