@@ -37,6 +37,7 @@ __device__ __forceinline__ int channels(const DeltaShape& s) {
 
 // Three blocks a token (blockIdx.y): 0 convolves q and k and makes them unit vectors, 1 convolves
 // v and forms beta, 2 forms the decay.  They share nothing.
+template <bool FOUR>
 __global__ void __launch_bounds__(256)
 delta_prepare_kernel(float* __restrict__ qn, float* __restrict__ kn, float* __restrict__ vv,
                      float* __restrict__ beta, float* __restrict__ decay,
@@ -72,24 +73,27 @@ delta_prepare_kernel(float* __restrict__ qn, float* __restrict__ kn, float* __re
   const int l = t - first;
   const float* cst = state + (size_t)req_slot[r] * s.state_stride + (size_t)s.heads * s.D * s.V;
   const int hist = s.taps - 1;
-  // four channels c, c + 256, ... of this thread at a time: the loads of all are on their way before
-  // the first sum (channel by channel the kernel waited for every row in turn: 49 us for 2 x 1,024
-  // tokens of 3,072 channels, 38 this way)
+  // FOUR (prompts through four taps with more than two channels a thread): four channels c, c + 256, ...
+  // at a time where every input is of this portion; the loads of all are on their way before the first
+  // sum.  Everything else channel by channel: the other form's registers cost more than it gives.  us,
+  // channel by channel against four: 1,024 tokens of 3,072 channels and 4 taps 30.7 and 25.8, of 512
+  // channels 11.3 and 13.1; 64 single tokens of 3,072 10.7 and 11.7.
   auto conv = [&](int c0, int end, auto put) {
-    constexpr int U = 4;
-    for (int c = c0; c < end; c += U * blockDim.x) {
-      float acc[U];
-      if (s.taps == 4 && l >= 3) {                 // every input is of this portion
+    if (FOUR && l >= 3) {
+      constexpr int U = 4;
+      const int step = blockDim.x;
+      for (int c = c0; c < end; c += U * step) {
         float in[U][4];
         float4 w[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-          const int cc = min(c + u * (int)blockDim.x, end - 1);
+          const int cc = min(c + u * step, end - 1);
 #pragma unroll
           for (int j = 0; j < 4; ++j) in[u][j] = proj[(size_t)(t - 3 + j) * s.stride + cc];
           w[u] = make_float4(conv_w[4 * (size_t)cc], conv_w[4 * (size_t)cc + 1],
                              conv_w[4 * (size_t)cc + 2], conv_w[4 * (size_t)cc + 3]);
         }
+        float acc[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
           acc[u] = fmaf(w[u].x, in[u][0], 0.f);
@@ -97,22 +101,22 @@ delta_prepare_kernel(float* __restrict__ qn, float* __restrict__ kn, float* __re
           acc[u] = fmaf(w[u].z, in[u][2], acc[u]);
           acc[u] = fmaf(w[u].w, in[u][3], acc[u]);
         }
-      } else {
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const int cc = min(c + u * (int)blockDim.x, end - 1);
-          acc[u] = 0.f;
-          for (int j = 0; j < s.taps; ++j) {
-            const int local = l - (hist - j);
-            const float in = local >= 0 ? proj[(size_t)(first + local) * s.stride + cc]
-                                        : cst[(size_t)(local + hist) * C + cc];
-            acc[u] = fmaf(conv_w[(size_t)cc * s.taps + j], in, acc[u]);
-          }
-        }
+        for (int u = 0; u < U; ++u)
+          if (c + u * step < end) put(c + u * step, acc[u] * sigmoidf_(acc[u]));
       }
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (c + u * (int)blockDim.x < end) put(c + u * blockDim.x, acc[u] * sigmoidf_(acc[u]));
+      return;
+    }
+    for (int c = c0; c < end; c += blockDim.x) {
+      float acc = 0.f;
+#pragma unroll 4
+      for (int j = 0; j < s.taps; ++j) {
+        const int local = l - (hist - j);
+        const float in = local >= 0 ? proj[(size_t)(first + local) * s.stride + c]
+                                    : cst[(size_t)(local + hist) * C + c];
+        acc = fmaf(conv_w[(size_t)c * s.taps + j], in, acc);
+      }
+      put(c, acc * sigmoidf_(acc));
     }
   };
   if (blockIdx.y == 1) {
@@ -746,12 +750,13 @@ HS_EXPORT int hs_delta_prepare(float* qn, float* kn, float* vv, float* beta, flo
   const size_t smem = (size_t)2 * kv_heads * D * sizeof(float);
   if (smem > 200 * 1024) return HS_ERR_UNSUPPORTED;
   cudaStream_t st = (cudaStream_t)stream;
+  const int widest = 2 * kv_heads * D > heads * V ? 2 * kv_heads * D : heads * V;
+  const bool four = taps == 4 && widest > 512 && n_tokens >= 512 && n_tokens >= 8 * n_requests;
+  auto* prepare = four ? hs::delta_prepare_kernel<true> : hs::delta_prepare_kernel<false>;
   if (smem > 48 * 1024)
-    cudaFuncSetAttribute(hs::delta_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem);
-  hs::delta_prepare_kernel<<<dim3(n_tokens, 3), 256, smem, st>>>(qn, kn, vv, beta, decay, proj, conv_w, a2,
-                                                        dt_bias, A_log, state, tok_req, req_start,
-                                                        req_slot, s, z_a);
+    cudaFuncSetAttribute(prepare, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  prepare<<<dim3(n_tokens, 3), 256, smem, st>>>(qn, kn, vv, beta, decay, proj, conv_w, a2, dt_bias, A_log,
+                                                state, tok_req, req_start, req_slot, s, z_a);
   HS_LAUNCH_CHECK();
   if (taps > 1) {
     dim3 grid((C + 127) / 128, n_requests);
