@@ -535,7 +535,8 @@ delta_blocks_kernel(float* __restrict__ o, float* __restrict__ state,
     // the fetching warp: lane 0 copies the blocks of a stage, all lanes the stage's values
     const float* src = blocks + ((size_t)h * cap_blocks + before) * SZ;
     const float* vsrc = vv + (size_t)first * HV + h * s.V;
-    for (int i = 0; i < n_stages; ++i) {
+    int i = 0;
+    for (; i < n_stages; ++i) {
       const int st = i % DB_STAGES;
       if (i >= DB_STAGES && !mbar_wait(&empty[st], ((i / DB_STAGES) - 1) & 1, status)) break;
       if (lane == 0) {
@@ -556,6 +557,9 @@ delta_blocks_kernel(float* __restrict__ o, float* __restrict__ state,
                    : "memory");
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
+    // the block stays until what it fetched has landed, also where the working warps gave up
+    for (int k = max(0, i - DB_STAGES); k < i; ++k)
+      mbar_wait(&full[k % DB_STAGES], (k / DB_STAGES) & 1, status);
     return;
   }
   const int part = (lane >> 1) & (KS - 1);

@@ -346,7 +346,8 @@ lightning_stream_kernel(float* __restrict__ o, float* __restrict__ state,
     if (lane == 0) {
       const float* src = rows + ((size_t)h * n_tokens + t0) * 2 * D;
       const float* vsrc = vals + (((size_t)h * gridDim.x + blockIdx.x) * n_tokens + t0) * CTA_COLS;
-      for (int i = 0; i < n_stages; ++i) {
+      int i = 0;
+      for (; i < n_stages; ++i) {
         const int st = i % LS_STAGES;
         if (i >= LS_STAGES && !mbar_wait(&empty[st], ((i / LS_STAGES) - 1) & 1, status)) break;
         const int here = min(LS_TOK, n - i * LS_TOK);
@@ -363,6 +364,9 @@ lightning_stream_kernel(float* __restrict__ o, float* __restrict__ state,
             "l"(vsrc + (size_t)i * LS_TOK * CTA_COLS), "r"(vb), "r"(smem_u32(&full[st]))
             : "memory");
       }
+      // the block stays until what it fetched has landed, also where the working warps gave up
+      for (int k = max(0, i - LS_STAGES); k < i; ++k)
+        mbar_wait(&full[k % LS_STAGES], (k / LS_STAGES) & 1, status);
     }
     return;
   }
