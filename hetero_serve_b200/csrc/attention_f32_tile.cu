@@ -21,8 +21,9 @@
 // the block does not see, or whose pages were refused, take a path that adds visible keys only, and so
 // do chunks in which some query has no score above minus infinity: it leaves such a chunk out, as the
 // one-token kernel does (its weights would be zeros, which make NaN of an infinite value).
-// Bounded by the FMA pipe and by shared-memory reads.  Measured (2 x 512 tokens, 16 heads): 340 us in
-// attention_simt.cu, 84 us here (13 TFLOP/s of causal work).
+// Bounded by each stream's chain of scores, softmax and values (FMA pipe 52 % busy, shared-memory pipe
+// 40 %, with two blocks an SM).  Measured (2 x 512 tokens, 16 heads): 340 us in attention_simt.cu, 75 us
+// here (14 TFLOP/s of causal work).
 #include "common.cuh"
 
 namespace hs {

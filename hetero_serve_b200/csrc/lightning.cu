@@ -245,8 +245,9 @@ lightning_kernel(float* __restrict__ o, float* __restrict__ state, const float* 
 //     lane bits 1 up (a 16-byte read by a warp: two wavefronts of shared memory, four on bits 0 up);
 //   * the four tokens' sums over the parts are exchanged so that a lane finishes one of them (the
 //     butterfly's tree, a third of its shuffles).
-// Measured (2 x 1,024 tokens, 8 heads of 128 x 128): the recurrence 249 -> 70-99 us; shared-memory
-// reads bound it (eight 16-byte reads a token and warp).
+// Measured (2 x 1,024 tokens, 8 heads of 128 x 128): the recurrence 249 -> 70-99 us; about one working
+// warp a scheduler waits on its chain (shared-memory pipe 38 % busy: eight 16-byte reads a token and
+// warp).
 constexpr int LS_TOK = 8, LS_STAGES = 4, LS_WARPS = 4;
 
 __host__ __device__ constexpr int ls_cols(int D) { return LS_WARPS * 32 * LA_ROWS / D; }
