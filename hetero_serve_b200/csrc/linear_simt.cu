@@ -259,10 +259,12 @@ linear_simt_few_rows_kernel(TO* out, const TI* __restrict__ a, const TI* __restr
   }
   __syncthreads();
   if (warp == WARPS) {
-    // the copying warp: RPI rows a trip, a lane per 16-byte piece.  Rows past the last one and
-    // pieces past the end of K are left out: what their places hold reaches no output.  (Copies of
-    // the last row in their stead went to one line of the L2 from every block: float32, 9 x
-    // 20,000 x 256 took 66 us and takes 18, 33 x 4,096 x 1,024 66 and 31.)
+    // the copying warp: RPI rows a trip, a lane per 16-byte piece.  Trips past the last row and pieces
+    // past the end of K are left out: what their places hold reaches no output.  (Copies of the last
+    // row in their stead went to one line of the L2 from every block: float32, 9 x 20,000 x 256 took
+    // 66 us and takes 18, 33 x 4,096 x 1,024 82 and 27.  Asking per row instead of per trip: 48 x
+    // 1,024 x 4,096 55 us with the copies, 69 with the questions, 43 so.)  A trip's last row may
+    // stand in for the next ones.
     constexpr int CPR = BK / S::VEC;                         // pieces per row of a stage
     constexpr int RPI = 32 / CPR;
     const int crow = lane / CPR, ck = (lane % CPR) * S::VEC;
@@ -275,17 +277,24 @@ linear_simt_few_rows_kernel(TO* out, const TI* __restrict__ a, const TI* __restr
         uint32_t to = ring_at + (uint32_t)(s * S::STAGE) * (uint32_t)sizeof(TI);
 #pragma unroll
         for (int row = 0; row < F; row += RPI) {
-          if (n0 + row + crow < N)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to),
-                         "l"(w + (size_t)(n0 + row + crow) * K + gk) : "memory");
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to),
+                       "l"(w + (size_t)min(n0 + row + crow, N - 1) * K + gk) : "memory");
           to += RPI * S::LD * (uint32_t)sizeof(TI);
         }
+        if (M >= S::ROWS) {
 #pragma unroll 8
-        for (int row = 0; row < S::ROWS; row += RPI) {
-          if (row + crow < M)
+          for (int row = 0; row < S::ROWS; row += RPI) {
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to),
                          "l"(a + (size_t)(row + crow) * K + gk) : "memory");
-          to += RPI * S::LD * (uint32_t)sizeof(TI);
+            to += RPI * S::LD * (uint32_t)sizeof(TI);
+          }
+        } else {
+#pragma unroll 8
+          for (int row = 0; row < M; row += RPI) {
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to),
+                         "l"(a + (size_t)min(row + crow, M - 1) * K + gk) : "memory");
+            to += RPI * S::LD * (uint32_t)sizeof(TI);
+          }
         }
       }
       asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&full[s]))
