@@ -26,6 +26,14 @@ __device__ __forceinline__ void ls_load4(const __nv_bfloat16* p, float (&v)[4]) 
   v[2] = __uint_as_float(x.y << 16); v[3] = __uint_as_float(x.y & 0xffff0000u);
 }
 
+__device__ __forceinline__ void ls_store4(float* p, const float (&v)[4]) {
+  *(float4*)p = make_float4(v[0], v[1], v[2], v[3]);
+}
+__device__ __forceinline__ void ls_store4(__nv_bfloat16* p, const float (&v)[4]) {
+  const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
+  *(uint2*)p = make_uint2(*(const uint32_t*)&a, *(const uint32_t*)&b);
+}
+
 // Where lanes read 16 bytes each and share addresses, a warp's read takes two wavefronts of shared
 // memory when the lanes of a pair (2i, 2i + 1) or all but every eighth agree, and four otherwise
 // (counted: lane % 8 -> four, (lane >> 1) & 7 -> two).  So eight columns go to lane bits 1-3 and
@@ -197,10 +205,33 @@ linear_simt_tile_kernel(TO* out, const TI* __restrict__ a, const TI* __restrict_
       }
     }
   }
+  // four neighbouring columns a store where every row of the outputs allows it
+  const bool wide = N % 4 == 0 && !((uintptr_t)out & (4 * sizeof(TO) - 1)) && !((uintptr_t)residual & 15);
 #pragma unroll
   for (int i = 0; i < P; ++i) {
     const int gm = m0 + 32 * (i >> 2) + ty * 4 + (i & 3);
     if (gm >= M) continue;
+    if (wide) {
+#pragma unroll
+      for (int u = 0; u < H; ++u) {
+        const int gn = n0 + 32 * u + tx * 4;
+        if (gn >= N) continue;
+        const size_t at = (size_t)gm * N + gn;
+        float v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          v[j] = __uint_as_float((uint32_t)(acc[i][2 * u + (j >> 1)] >> ((j & 1) * 32)));
+          if (bias) v[j] += bias[gn + j];
+          v[j] = apply_act(v[j], act, ab);
+        }
+        if (residual) {
+          const float4 r = *(const float4*)(residual + at);
+          v[0] += r.x; v[1] += r.y; v[2] += r.z; v[3] += r.w;
+        }
+        ls_store4(out + at, v);
+      }
+      continue;
+    }
 #pragma unroll
     for (int j = 0; j < P; ++j) {
       const int gn = n0 + 32 * (j >> 2) + tx * 4 + (j & 3);

@@ -37,6 +37,37 @@ def test_rows_keep_their_bits(n, k):
     assert ops.status.item() == 0
 
 
+@pytest.mark.parametrize("dtype,m,n,k", [(torch.float32, 1601, 1537, 70), (torch.float32, 1601, 1540, 33),
+                                         (torch.bfloat16, 1601, 1537, 70), (torch.bfloat16, 1601, 1540, 100),
+                                         (torch.bfloat16, 1601, 1537, 97), (torch.bfloat16, 200, 9477, 70),
+                                         (torch.bfloat16, 200, 9480, 100)])
+def test_rows_keep_their_bits_in_the_large_tiles(dtype, m, n, k):
+    """Enough 64 x 64 tiles that the large ones are taken, with remainders in every direction: a row's
+    bits are those it has in the small tiles and among few rows."""
+    ops = CudaOps("cuda")
+    ops.tensor_cores = False
+    assert -(-m // 64) * -(-n // 64) >= 4 * ops.sm_count
+    g = torch.Generator(device="cuda").manual_seed(n + k)
+    a = torch.randn(m, k, device="cuda", generator=g).to(dtype)
+    w = torch.randn(n, k, device="cuda", generator=g).to(dtype)
+    bias, res = (torch.randn(*s, device="cuda", generator=g) for s in ((n,), (m, n)))
+    exact = a.double() @ w.double().T + bias.double() + res.double()
+    bound = (k + 2) * 2.0 ** -24 * (a.abs().double() @ w.abs().double().T + bias.abs() + res.abs())
+    whole = torch.full((m, n), float("nan"), device="cuda")
+    ops.linear(whole, a, w, bias, residual=res)
+    assert bool(((whole.double() - exact).abs() <= bound).all())
+    for rows in (r for r in (1, 33, 65, 257) if r <= m):
+        for first in (0, m - rows):
+            part = torch.full((rows, n), float("nan"), device="cuda")
+            ops.linear(part, a[first:first + rows].clone(), w, bias, residual=res[first:first + rows].clone())
+            assert torch.equal(part, whole[first:first + rows]), (rows, first)
+    if dtype == torch.bfloat16:                              # outputs rounded once, from the same sums
+        out = torch.empty(m, n, device="cuda", dtype=dtype)
+        ops.linear(out, a, w, bias, residual=res)
+        assert torch.equal(out, whole.bfloat16())
+    assert ops.status.item() == 0
+
+
 def test_bfloat16_rows_on_the_cuda_cores():
     ops = CudaOps("cuda")
     ops.tensor_cores = False
