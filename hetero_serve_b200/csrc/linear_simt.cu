@@ -61,8 +61,8 @@ __device__ __forceinline__ uint64_t twice(float a) {
 // cp.async copies through a ring of LT_STAGES stages of 8 k (fetched through registers, one stage
 // ahead, the L2's latency was exposed in every stage); bfloat16 ones go through registers.
 // Measured (float32, one B200, before -> now; the form before fetched 128 x 128 tiles through
-// registers and used single FMAs): 2,048 x 4,096 x 1,024 485 -> 384 us (44.8 TFLOP/s, FMA pipe 60 %
-// busy, shared-memory pipe 70 %), 1,024 x 1,024 x 4,096 632 -> 316 us, 256 x 1,024 x 4,096 660 -> 163.
+// registers and used single FMAs): 2,048 x 4,096 x 1,024 485 -> 384 us (44.8 TFLOP/s, FMA pipe 62 %
+// busy, shared-memory pipe 62 %), 1,024 x 1,024 x 4,096 632 -> 316 us, 256 x 1,024 x 4,096 660 -> 163.
 constexpr int LT_BK = 8, LT_THREADS = 64, LT_STAGES = 4;
 
 __device__ __forceinline__ int lt_swizzle(int k) { return (k & 7) << 2; }
@@ -237,6 +237,102 @@ linear_simt_tile_kernel(TO* out, const TI* __restrict__ a, const TI* __restrict_
       const int gn = n0 + 32 * (j >> 2) + tx * 4 + (j & 3);
       if (gn >= N) continue;
       float v = __uint_as_float((uint32_t)(acc[i][j >> 1] >> ((j & 1) * 32)));
+      if (bias) v += bias[gn];
+      v = apply_act(v, act, ab);
+      if (residual) v += residual[(size_t)gm * N + gn];
+      out[(size_t)gm * N + gn] = from_f<TO>(v);
+    }
+  }
+}
+
+// ---- bfloat16, many large tiles: 128 x 128 outputs, an 8 x 8 patch per thread ------------------
+// The same chains again.  bfloat16 operands reach the tiles above through registers, one stage of 8 k
+// ahead, and their two warps wait for the L2 in every stage; eight warps on a tile twice as wide share
+// one such wait, two tiles an SM.  The wider tile pays where it fills the device (see the launch).
+constexpr int LB_BM = 128, LB_BN = 128, LB_BK = 8, LB_THREADS = 256;
+
+// VEC: K is a multiple of 4 and both matrices start on a 16-byte boundary, so a thread's four
+// k of a row come in one load (with one 4-byte load per element the load pipe, 16 sectors an
+// instruction, took as long as the products).
+template <typename TI, typename TO, bool VEC>
+__global__ void __launch_bounds__(LB_THREADS)
+linear_simt_big_kernel(TO* out, const TI* __restrict__ a, const TI* __restrict__ w,
+                       const float* __restrict__ bias, const float* residual, int M, int N, int K,
+                       int act, float2 ab) {
+  __shared__ __align__(16) float As[2][LB_BK][LB_BM];
+  __shared__ __align__(16) float Ws[2][LB_BK][LB_BN];
+  const int tid = threadIdx.x;
+  const int tx = tid & 15, ty = tid >> 4;                 // 16 x 16 threads, 8 x 8 outputs each
+  const int m0 = blockIdx.y * LB_BM, n0 = blockIdx.x * LB_BN;
+  // loader: thread -> (row 0..127, 4 consecutive k of the 8)
+  const int lr = tid >> 1, lk = (tid & 1) * 4;
+  float acc[8][8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+  float ra[4], rw[4];
+  auto fetch = [&](int k0) {
+    const int gm = m0 + lr, gn = n0 + lr;
+    if (VEC) {
+      const int gk = k0 + lk;                             // K % 4 == 0: all four or none
+#pragma unroll
+      for (int j = 0; j < 4; ++j) ra[j] = rw[j] = 0.f;
+      if (gm < M && gk < K) ls_load4(a + (size_t)gm * K + gk, ra);
+      if (gn < N && gk < K) ls_load4(w + (size_t)gn * K + gk, rw);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int gk = k0 + lk + j;
+        ra[j] = (gm < M && gk < K) ? to_f(a[(size_t)gm * K + gk]) : 0.f;
+        rw[j] = (gn < N && gk < K) ? to_f(w[(size_t)gn * K + gk]) : 0.f;
+      }
+    }
+  };
+  auto stash = [&](int buf) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      As[buf][lk + j][lr] = ra[j];
+      Ws[buf][lk + j][lr] = rw[j];
+    }
+  };
+  fetch(0);
+  stash(0);
+  __syncthreads();
+  int buf = 0;
+  for (int k0 = 0; k0 < K; k0 += LB_BK) {
+    const bool more = k0 + LB_BK < K;
+    if (more) fetch(k0 + LB_BK);                          // in flight during the products below
+#pragma unroll
+    for (int kk = 0; kk < LB_BK; ++kk) {
+      // rows ty*4..+3 and 64+ty*4..+3, columns tx*4..+3 and 64+tx*4..+3: 16-byte reads, no
+      // bank conflicts
+      const float4 a0 = *(const float4*)&As[buf][kk][ty * 4];
+      const float4 a1 = *(const float4*)&As[buf][kk][64 + ty * 4];
+      const float4 w0 = *(const float4*)&Ws[buf][kk][tx * 4];
+      const float4 w1 = *(const float4*)&Ws[buf][kk][64 + tx * 4];
+      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+      const float wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(av[i], wv[j], acc[i][j]);
+    }
+    if (more) {
+      stash(buf ^ 1);
+      __syncthreads();
+      buf ^= 1;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int gm = m0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + (i - 4));
+    if (gm >= M) continue;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int gn = n0 + (j < 4 ? tx * 4 + j : 64 + tx * 4 + (j - 4));
+      if (gn >= N) continue;
+      float v = acc[i][j];
       if (bias) v += bias[gn];
       v = apply_act(v, act, ab);
       if (residual) v += residual[(size_t)gm * N + gn];
@@ -449,7 +545,10 @@ HS_EXPORT int hs_linear_simt(void* out, const void* a, const void* w, const floa
   using bf16 = __nv_bfloat16;
   // few rows: the weight-stream kernel (rows and pointers that 16-byte copies can take)
   const int vec = in_dtype == HS_DT_F32 ? 4 : 8;
-  const bool few = M <= 16 || (M <= 64 && (N + 15) / 16 <= 4 * hs_sm_count());
+  // (float32, us, few-rows kernel against tiles: 32 x 4,096 x 1,024 20 and 44, 32 x
+  // 50,257 x 768 114 and 141, 64 x 4,096 x 1,024 34 and 46; but 64 x 6,400 x 768 50 and 40, 64 x 50,257
+  // x 768 287 and 153)
+  const bool few = M <= 32 || (M <= 64 && (N + 15) / 16 <= 2 * hs_sm_count());
   if (few && K % vec == 0 && !((uintptr_t)a & 15) && !((uintptr_t)w & 15)) {
     int rc = HS_ERR_UNSUPPORTED;
     if (in_dtype == HS_DT_F32 && out_dtype == HS_DT_F32)
@@ -459,6 +558,30 @@ HS_EXPORT int hs_linear_simt(void* out, const void* a, const void* w, const floa
     else if (in_dtype == HS_DT_BF16 && out_dtype == HS_DT_F32)
       rc = hs::launch_few_rows<bf16, float>(out, a, w, bias, residual, M, N, K, act, ab, status, st);
     if (rc != HS_OK) return rc;
+    HS_LAUNCH_CHECK();
+    return HS_OK;
+  }
+  const long long big = (long long)((N + 127) / 128) * ((M + 127) / 128);
+  const bool vec4 = K % 4 == 0 && !((uintptr_t)a & 7) && !((uintptr_t)w & 7);
+  // bfloat16, us, 64 x 64 against 128 x 128 tiles.  Loads of four: the last round of two tiles an SM is
+  // mostly full (1,024 x 4,096 x 1,028, 256 tiles, 263 and 229; 1,024 x 8,192 x 1,028, 512, 546 and 459;
+  // but 300 x 8,192 x 1,028, 192, 209 and 226; 300 x 16,384 x 516, 384, 185 and 235).  Single loads: one
+  // round of a tile an SM, mostly full (2,048 x 1,024 x 1,023, 128 tiles, 233 and 186; but 2,048 x 4,096
+  // x 1,022, 512, 470 and 547)
+  const long long sms = hs_sm_count();
+  const bool fills = vec4 ? big > sms && (big % (2 * sms) == 0 || 10 * (big % (2 * sms)) >= 14 * sms)
+                          : 4 * big >= 3 * sms && big <= sms;
+  if (in_dtype == HS_DT_BF16 && M >= 256 && fills && (M + 127) / 128 <= 65535) {
+    const dim3 grid((N + 127) / 128, (M + 127) / 128);
+#define HS_LB_LAUNCH(TO, VEC)                                                                  \
+  hs::linear_simt_big_kernel<bf16, TO, VEC><<<grid, hs::LB_THREADS, 0, st>>>(                  \
+      (TO*)out, (const bf16*)a, (const bf16*)w, bias, residual, M, N, K, act, ab)
+    if (out_dtype == HS_DT_F32 && vec4) HS_LB_LAUNCH(float, true);
+    else if (out_dtype == HS_DT_F32) HS_LB_LAUNCH(float, false);
+    else if (out_dtype == HS_DT_BF16 && vec4) HS_LB_LAUNCH(bf16, true);
+    else if (out_dtype == HS_DT_BF16) HS_LB_LAUNCH(bf16, false);
+    else return HS_ERR_UNSUPPORTED;
+#undef HS_LB_LAUNCH
     HS_LAUNCH_CHECK();
     return HS_OK;
   }
@@ -477,7 +600,6 @@ HS_EXPORT int hs_linear_simt(void* out, const void* a, const void* w, const floa
       hs::linear_simt_tile_kernel<TI, TO, 1, LOAD><<<grid, hs::LT_THREADS, 0, st>>>(           \
           (TO*)out, (const TI*)a, (const TI*)w, bias, residual, M, N, K, act, ab);             \
   } while (0)
-  const bool vec4 = K % 4 == 0 && !((uintptr_t)a & 7) && !((uintptr_t)w & 7);
   if (in_dtype == HS_DT_F32 && out_dtype == HS_DT_F32) {
     if (64ll * K < (1ll << 31)) HS_LT_LAUNCH(float, float, 2);      // (32-bit offsets in a tile)
     else HS_LT_LAUNCH(float, float, 0);
