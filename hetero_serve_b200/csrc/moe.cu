@@ -24,12 +24,12 @@
 // (the summed index runs fastest).  Two paths:
 //   * few (token, expert) pairs, and all of float32: every pair streams its expert's rows, one
 //     warp per output row with 16-byte loads (a matrix-vector product per pair);
-//   * many pairs in bfloat16: the pairs are sorted by expert on the device (no host round
-//     trip), and tiles of 64 pairs x 64 outputs of one expert go through mma.sync m16n8k16 with
-//     float32 accumulators (two stages of cp.async copies, fragments by ldmatrix); the down projection's rows are added into the stream per token in
-//     the order the experts were chosen, so a token's result does not depend on its neighbours.
+//   * many pairs in bfloat16: the pairs are sorted by expert on the device (no host round trip) and
+//     go through tcgen05 in tiles of one expert's rows (moe_tiles_tc.cu); the down projection's rows
+//     are added into the stream per token in the order the experts were chosen, so a token's result
+//     does not depend on its neighbours.
 #include "common.cuh"
-#include "mma_tiles.cuh"
+#include "moe_tiles_tc.cuh"
 
 namespace hs {
 
@@ -82,23 +82,33 @@ __device__ __forceinline__ float row_dot(const __nv_bfloat16* __restrict__ w, co
 
 constexpr int ROUTE_THREADS = 256;
 
-// One block per token: the warps share the experts' dot products, warp 0 then chooses.
+// z handed in (the logits formed as one matrix product over the step): a warp chooses for a token,
+// `blockDim.x / 32` tokens a block (2,048 tokens, 32 experts: 6.3 us, against 11.2 with a block a token of
+// which one warp chooses).  Else one block per token: the warps share the experts' dot products, warp 0 chooses.
 template <typename TH>
 __global__ void __launch_bounds__(ROUTE_THREADS)
 moe_route_kernel(int* __restrict__ sel_idx, float* __restrict__ sel_w, const TH* __restrict__ h,
-                 const float* __restrict__ w_router, const int* __restrict__ tok_req, int width,
-                 int E, int top, int n_groups, int keep, const float* __restrict__ z_in) {
+                 const float* __restrict__ w_router, const int* __restrict__ tok_req, int n_tokens,
+                 int width, int E, int top, int n_groups, int keep, const float* __restrict__ z_in) {
   extern __shared__ float smem[];
-  float* s_h = smem;                // [width]
-  float* s_s = smem + width;        // [E] scores (-1 once taken)
-  float* s_g = s_s + E;             // [n_groups] (-2 marks a kept group)
-  const int t = blockIdx.x;
-  if (tok_req[t] < 0) return;
+  pdl_trigger();
+  pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (z_in) {                        // the logits were formed as one matrix product over the step
-    for (int e = threadIdx.x; e < E; e += ROUTE_THREADS)
-      s_s[e] = 1.0f / (1.0f + expf(-z_in[(size_t)t * E + e]));
+  float *s_s, *s_g;                 // [E] scores (-1 once taken), [n_groups] (-2 marks a kept group)
+  int t;
+  if (z_in) {
+    t = blockIdx.x * (blockDim.x >> 5) + warp;
+    if (t >= n_tokens || tok_req[t] < 0) return;
+    s_s = smem + (size_t)warp * (E + n_groups);
+    s_g = s_s + E;
+    for (int e = lane; e < E; e += 32) s_s[e] = 1.0f / (1.0f + expf(-z_in[(size_t)t * E + e]));
+    __syncwarp();
   } else {
+    t = blockIdx.x;
+    if (tok_req[t] < 0) return;
+    float* s_h = smem;              // [width]
+    s_s = smem + width;
+    s_g = s_s + E;
     for (int k = threadIdx.x; k < width; k += ROUTE_THREADS) s_h[k] = to_f(h[(size_t)t * width + k]);
     __syncthreads();
     for (int e = warp; e < E; e += ROUTE_THREADS / 32) {
@@ -106,9 +116,9 @@ moe_route_kernel(int* __restrict__ sel_idx, float* __restrict__ sel_w, const TH*
       const float z = row_dot(wr, s_h, width, lane);
       if (lane == 0) s_s[e] = 1.0f / (1.0f + expf(-z));
     }
+    __syncthreads();
+    if (warp != 0) return;
   }
-  __syncthreads();
-  if (warp != 0) return;
   const int per = E / n_groups;
   for (int g = lane; g < n_groups; g += 32) {
     float a = -1.f, b = -1.f;                          // the two largest of the group
@@ -272,16 +282,6 @@ moe_route_softmax_kernel(int* __restrict__ sel_idx, float* __restrict__ sel_w,
     }
     __syncwarp();
   }
-}
-
-// act 0: the clamped form above; act 1: silu(g) * u; act 2: relu(u)^2 (an expert without a gate
-// matrix)
-__device__ __forceinline__ float expert_act(float g, float u, float limit, int act) {
-  if (act == 1) return g / (1.0f + expf(-g)) * u;
-  if (act == 2) { const float r = fmaxf(u, 0.f); return r * r; }
-  g = fminf(g, limit);
-  u = fminf(fmaxf(u, -limit), limit);
-  return g * (1.0f / (1.0f + expf(-1.702f * g))) * (u + 1.0f);
 }
 
 // a matrix-vector product per pair: rows of the expert, one warp each
@@ -457,160 +457,97 @@ moe_down_rows_kernel(float* __restrict__ x, const float* __restrict__ y,
 // -- path 2: pairs sorted by expert, tiles on the tensor cores --------------------------------
 constexpr int SORT_THREADS = 1024;
 
-// work: [0] number of tiles; then per expert E counts, E segment starts; then per tile its
-// expert and its first row.  pair_pos[pair] = row of the pair in expert order (-1: not there),
-// row_token[row] = the token of that row.
-__global__ void __launch_bounds__(SORT_THREADS)
-moe_sort_kernel(int* __restrict__ work, int* __restrict__ pair_pos, int* __restrict__ row_token,
-                const int* __restrict__ sel_idx, const int* __restrict__ tok_req, int n_tokens,
-                int top, int E, int max_tiles) {
-  extern __shared__ int s_cnt[];             // [E] counts, then [E] cursors
-  pdl_trigger();
-  pdl_wait();
-  int* s_cur = s_cnt + E;
-  for (int e = threadIdx.x; e < E; e += SORT_THREADS) s_cnt[e] = 0;
-  __syncthreads();
-  const int pairs = n_tokens * top;
-  for (int p = threadIdx.x; p < pairs; p += SORT_THREADS) {
-    const int e = sel_idx[p];
-    if (tok_req[p / top] >= 0 && e >= 0 && e < E) atomicAdd(&s_cnt[e], 1);
+// inclusive sums over the block of two numbers a thread
+__device__ __forceinline__ int2 block_sums(int2 v, int2* s_warp) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int x = __shfl_up_sync(0xffffffffu, v.x, o), y = __shfl_up_sync(0xffffffffu, v.y, o);
+    if (lane >= o) { v.x += x; v.y += y; }
   }
+  if (lane == 31) s_warp[warp] = v;
   __syncthreads();
-  int* counts = work + 1;
-  int* starts = work + 1 + E;
-  int* tile_e = work + 1 + 2 * E;
-  int* tile_r = tile_e + max_tiles;
-  if (threadIdx.x == 0) {
-    int at = 0, tiles = 0;
-    for (int e = 0; e < E; ++e) {
-      counts[e] = s_cnt[e];
-      starts[e] = at;
-      s_cur[e] = at;
-      for (int r = 0; r < s_cnt[e] && tiles < max_tiles; r += TM) {
-        tile_e[tiles] = e;
-        tile_r[tiles] = at + r;
-        ++tiles;
-      }
-      at += s_cnt[e];
-    }
-    work[0] = tiles;
+  int2 w = s_warp[lane];            // 32 warps
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int x = __shfl_up_sync(0xffffffffu, w.x, o), y = __shfl_up_sync(0xffffffffu, w.y, o);
+    if (lane >= o) { w.x += x; w.y += y; }
   }
+  const int from = max(warp - 1, 0);
+  const int x = __shfl_sync(0xffffffffu, w.x, from), y = __shfl_sync(0xffffffffu, w.y, from);
+  if (warp > 0) { v.x += x; v.y += y; }
   __syncthreads();
-  for (int p = threadIdx.x; p < pairs; p += SORT_THREADS) {
-    const int e = sel_idx[p];
-    int pos = -1;
-    if (tok_req[p / top] >= 0 && e >= 0 && e < E) {
-      pos = atomicAdd(&s_cur[e], 1);
-      row_token[pos] = p / top;
-    }
-    pair_pos[p] = pos;
+  return v;
+}
+
+// the tiles of an expert with `count` rows from `start` on: as few as MT_PAIRS rows each allow, of one
+// size (a multiple of 16), the last takes what is left
+__device__ __forceinline__ void list_tiles(int* tiles, int* widest, int at, int e, int start, int count) {
+  const int n = (count + MT_PAIRS - 1) / MT_PAIRS;
+  if (n == 0) return;
+  const int size = ((count + n - 1) / n + 15) & ~15;
+  atomicMax(widest, size);
+  for (int i = 0; i < n; ++i) {
+    int* t = tiles + 2 + 3 * (at + i);
+    t[0] = e;
+    t[1] = start + i * size;
+    t[2] = min(size, count - i * size);
   }
 }
 
-// One block: 64 rows of one expert's segment x 64 outputs.  NB = 2: gate and up together with
-// the activation as epilogue (out: bfloat16 rows); NB = 1: the down projection (out: float32).
-// A rows: `a` indexed through row_token when GATHER (the normed rows of the tokens), else the
-// sorted rows themselves.  4 warps, each 32 x 32 of the tile.  Two stages of tiles in shared
-// memory (the next one is copied while this one is used); fragments come through ldmatrix.
-// ACT (with NB = 1): the rows leave activated in bfloat16 as with NB = 2 (an expert without a gate).
-template <int NB, bool GATHER, bool ACT = (NB == 2)>
-__global__ void __launch_bounds__(128)
-moe_tiles_kernel(void* __restrict__ out, const __nv_bfloat16* __restrict__ a,
-                 const __nv_bfloat16* __restrict__ w0, const __nv_bfloat16* __restrict__ w1,
-                 const int* __restrict__ work, const int* __restrict__ row_token, int E,
-                 int max_tiles, int N, int K, float limit, int act) {
-  __shared__ __align__(16) __nv_bfloat16 s_a[2][TM * TS];
-  __shared__ __align__(16) __nv_bfloat16 s_b[NB][2][TN * TS];
+// pair_pos[pair] = row of the pair in expert order (-1: not there), row_token[row] = the token of that
+// row, tiles: see moe_tiles_tc.cuh.  One block: a pass that counts and numbers the pairs of each expert,
+// sums over the experts, a pass that places the pairs (8,192 pairs of 32 experts: 9.6 us; 12.8 with a
+// thread that walked the experts and a second round of atomics).
+__global__ void __launch_bounds__(SORT_THREADS)
+moe_sort_kernel(int* __restrict__ tiles, int* __restrict__ pair_pos, int* __restrict__ row_token,
+                const int* __restrict__ sel_idx,
+                const int* __restrict__ tok_req, int n_tokens, int top, int E) {
+  extern __shared__ int s_cnt[];             // [E] counts, then starts
+  __shared__ int2 s_warp[32];
+  __shared__ int s_most;                     // rows of the widest tile
   pdl_trigger();
+  if (threadIdx.x == 0) s_most = 16;
+  for (int e = threadIdx.x; e < E; e += SORT_THREADS) s_cnt[e] = 0;
   pdl_wait();
-  const int tile = blockIdx.x;
-  if (tile >= work[0]) return;
-  const int e = work[1 + 2 * E + tile];
-  const int row0 = work[1 + 2 * E + max_tiles + tile];
-  const int seg_end = work[1 + E + e] + work[1 + e];
-  const int rows = min(TM, seg_end - row0);
-  const int n0 = blockIdx.y * TN;
-  const int ncols = min(TN, N - n0);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
-  const int g = lane >> 2, tq = lane & 3;
-  auto a_row = [&](int r) {
-    const int src = GATHER ? row_token[row0 + r] : row0 + r;
-    return a + (size_t)src * K;
-  };
-  const __nv_bfloat16* b0 = w0 + ((size_t)e * N + n0) * K;
-  const __nv_bfloat16* b1 = NB == 2 ? w1 + ((size_t)e * N + n0) * K : nullptr;
-  auto b0_row = [&](int r) { return b0 + (size_t)r * K; };
-  auto b1_row = [&](int r) { return b1 + (size_t)r * K; };
-  float acc[NB][2][4][4];
-#pragma unroll
-  for (int x = 0; x < NB; ++x)
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) acc[x][i][j][c] = 0.f;
-  auto copy = [&](int buf, int k0) {
-    tile_copy(s_a[buf], a_row, rows, k0, a);
-    tile_copy(s_b[0][buf], b0_row, ncols, k0, w0);
-    if (NB == 2) tile_copy(s_b[NB - 1][buf], b1_row, ncols, k0, w0);
-    asm volatile("cp.async.commit_group;");
-  };
-  copy(0, 0);
-  int buf = 0;
-  // lane's row and column offsets inside a 16 x 16 (A) or two 8 x 16 (B) block for ldmatrix
-  const int a_r = lane & 15, a_c = (lane >> 4) * 8;
-  const int b_r = (lane & 7) + (lane >> 4) * 8, b_c = ((lane >> 3) & 1) * 8;
-  for (int k0 = 0; k0 < K; k0 += TK, buf ^= 1) {
-    if (k0 + TK < K) {
-      copy(buf ^ 1, k0 + TK);
-      asm volatile("cp.async.wait_group 1;");
-    } else {
-      asm volatile("cp.async.wait_group 0;");
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < TK; kk += 16) {
-      uint32_t fa[2][4];
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-        ldmatrix_x4(fa[i], s_a[buf] + (wm + 16 * i + a_r) * TS + kk + a_c);
-#pragma unroll
-      for (int x = 0; x < NB; ++x)
-#pragma unroll
-        for (int j = 0; j < 4; j += 2) {
-          uint32_t fb[4];                         // b0, b1 of column block j, then of j + 1
-          ldmatrix_x4(fb, s_b[x][buf] + (wn + 8 * j + b_r) * TS + kk + b_c);
-#pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            mma_bf16(acc[x][i][j], fa[i], fb);
-            mma_bf16(acc[x][i][j + 1], fa[i], fb + 2);
-          }
-        }
-    }
-    __syncthreads();                              // this stage is copied into again next turn
+  __syncthreads();
+  const int pairs = n_tokens * top;
+#pragma unroll 4
+  for (int p = threadIdx.x; p < pairs; p += SORT_THREADS) {
+    const int e = sel_idx[p];
+    int nth = -1;
+    if (tok_req[p / top] >= 0 && e >= 0 && e < E) nth = atomicAdd(&s_cnt[e], 1);
+    pair_pos[p] = nth;
   }
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const int r = wm + 16 * i + g + 8 * half;
-        const int c = wn + 8 * j + 2 * tq;
-        if (r >= rows) continue;
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          if (c + q >= ncols) continue;
-          const size_t at = (size_t)(row0 + r) * N + n0 + c + q;
-          if (ACT)
-            ((__nv_bfloat16*)out)[at] = __float2bfloat16_rn(
-                expert_act(acc[0][i][j][2 * half + q], acc[NB - 1][i][j][2 * half + q], limit, act));
-          else
-            ((float*)out)[at] = acc[0][i][j][2 * half + q];
-        }
-      }
+  __syncthreads();
+  int2 done = make_int2(0, 0);               // rows and tiles of the experts so far
+  for (int e0 = 0; e0 < E; e0 += SORT_THREADS) {
+    const int e = e0 + threadIdx.x, c = e < E ? s_cnt[e] : 0;
+    const int n = (c + MT_PAIRS - 1) / MT_PAIRS;
+    const int2 v = block_sums(make_int2(c, n), s_warp);
+    if (e < E) {
+      const int start = done.x + v.x - c;
+      s_cnt[e] = start;
+      list_tiles(tiles, &s_most, done.y + v.y - n, e, start, c);
+    }
+    if (threadIdx.x == SORT_THREADS - 1) s_warp[0] = v;
+    __syncthreads();
+    done.x += s_warp[0].x; done.y += s_warp[0].y;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    tiles[0] = done.y;
+    tiles[1] = s_most;
+  }
+#pragma unroll 4
+  for (int p = threadIdx.x; p < pairs; p += SORT_THREADS) {
+    const int nth = pair_pos[p];
+    if (nth >= 0) {
+      const int pos = s_cnt[sel_idx[p]] + nth;
+      pair_pos[p] = pos;
+      row_token[pos] = p / top;
+    }
+  }
 }
 
 // x[t] (+)= sum_k weight_k * rows[pair_pos[t, k]], experts in the order they were chosen
@@ -697,17 +634,26 @@ HS_EXPORT int hs_moe_route(int* sel_idx, float* sel_w, const void* h, const floa
   const size_t smem = (size_t)(width + E + n_groups) * sizeof(float);
   if (smem > 48 * 1024) return HS_ERR_UNSUPPORTED;
   cudaStream_t st = (cudaStream_t)stream;
+  // a warp a token where the logits are there, as many as their scores fit beside the limit above
+  int warps = hs::ROUTE_THREADS / 32;
+  size_t bytes = smem;
+  if (z_in) {
+    warps = 4;
+    while (warps > 1 && (size_t)warps * (E + n_groups) * sizeof(float) > 48 * 1024) warps /= 2;
+    bytes = (size_t)warps * (E + n_groups) * sizeof(float);
+  }
+  const dim3 grid(z_in ? (n_tokens + warps - 1) / warps : n_tokens);
+  cudaError_t e;
   if (h_dtype == HS_DT_F32)
-    hs::moe_route_kernel<float><<<n_tokens, hs::ROUTE_THREADS, smem, st>>>(
-        sel_idx, sel_w, (const float*)h, w_router, tok_req, width, E, top, n_groups, keep, z_in);
+    e = hs_launch(hs::moe_route_kernel<float>, grid, dim3(32 * warps), bytes, st, hs_pdl_enabled(), sel_idx,
+                  sel_w, (const float*)h, w_router, tok_req, n_tokens, width, E, top, n_groups, keep, z_in);
   else if (h_dtype == HS_DT_BF16)
-    hs::moe_route_kernel<__nv_bfloat16><<<n_tokens, hs::ROUTE_THREADS, smem, st>>>(
-        sel_idx, sel_w, (const __nv_bfloat16*)h, w_router, tok_req, width, E, top, n_groups,
-        keep, z_in);
+    e = hs_launch(hs::moe_route_kernel<__nv_bfloat16>, grid, dim3(32 * warps), bytes, st, hs_pdl_enabled(),
+                  sel_idx, sel_w, (const __nv_bfloat16*)h, w_router, tok_req, n_tokens, width, E, top,
+                  n_groups, keep, z_in);
   else
     return HS_ERR_UNSUPPORTED;
-  HS_LAUNCH_CHECK();
-  return HS_OK;
+  return e == cudaSuccess ? HS_OK : (int)e;
 }
 
 HS_EXPORT int hs_moe_route_top(int* sel_idx, float* sel_w, const void* h, const float* w_router,
@@ -808,10 +754,8 @@ HS_EXPORT int hs_moe_sorted_scratch(int n_tokens, int width, int ff, int top, in
   *ints = 0;
   *bytes = 0;
   const long long pairs = (long long)n_tokens * top;
-  if (dtype != HS_DT_BF16 || width % hs::TK || ff % hs::TK || pairs < 256 || E > 4096)
-    return HS_OK;
-  const long long max_tiles = pairs / hs::TM + E;
-  *ints = 1 + 2LL * E + 2 * max_tiles + 2 * pairs;
+  if (dtype != HS_DT_BF16 || width % 32 || ff % 32 || pairs < 256 || E > 4096) return HS_OK;
+  *ints = 2 + 3 * (pairs / hs::MT_PAIRS + E) + 2 * pairs;
   *bytes = ((pairs * ff * 2 + 255) / 256) * 256 + pairs * width * 4;
   return HS_OK;
 }
@@ -822,7 +766,8 @@ HS_EXPORT int hs_moe_experts(float* x, float* y, const void* h, const void* w_ga
                              const void* w_up, const void* w_down, const int* sel_idx,
                              const float* sel_w, const int* tok_req, int n_tokens, int width,
                              int ff, int top, int E, float limit, int act_kind, int dtype, int* ints,
-                             void* rows, int n_identity, int accumulate, void* stream) {
+                             void* rows, int n_identity, int accumulate, int* status,
+                             void* stream) {
   if (!x || !h || !w_up || !w_down || !sel_idx || !sel_w || !tok_req || (!w_gate && act_kind != 2))
     return HS_ERR_ARGUMENT;
   if (width <= 0 || ff <= 0 || top <= 0 || E <= 0 || act_kind < 0 || act_kind > 2 || n_identity < 0)
@@ -836,32 +781,21 @@ HS_EXPORT int hs_moe_experts(float* x, float* y, const void* h, const void* w_ga
     hs_moe_sorted_scratch(n_tokens, width, ff, top, E, dtype, &need_i, &need_b);
     if (need_i == 0) return HS_ERR_UNSUPPORTED;
     const int pairs = n_tokens * top;
-    const int max_tiles = pairs / hs::TM + E;
-    int* work = ints;
-    int* pair_pos = ints + 1 + 2 * E + 2 * max_tiles;
+    if (!status) return HS_ERR_ARGUMENT;
+    const int max_tiles = pairs / hs::MT_PAIRS + E;
+    int* tiles = ints;
+    int* pair_pos = tiles + 2 + 3 * max_tiles;
     int* row_token = pair_pos + pairs;
     __nv_bfloat16* act = (__nv_bfloat16*)rows;
     float* down = (float*)((char*)rows + (((size_t)pairs * ff * 2 + 255) / 256) * 256);
-    e = hs_launch(hs::moe_sort_kernel, dim3(1), dim3(hs::SORT_THREADS), 2 * E * sizeof(int), st,
-                  pdl, work, pair_pos, row_token, sel_idx, tok_req, n_tokens, top, E, max_tiles);
+    e = hs_launch(hs::moe_sort_kernel, dim3(1), dim3(hs::SORT_THREADS), E * sizeof(int), st, pdl,
+                  tiles, pair_pos, row_token, sel_idx, tok_req, n_tokens, top, E);
     if (e != cudaSuccess) return (int)e;
     const __nv_bfloat16* hb = (const __nv_bfloat16*)h;
-    const __nv_bfloat16* none = nullptr;
-    const dim3 g1(max_tiles, (ff + hs::TN - 1) / hs::TN);
-    if (w_gate)
-      e = hs_launch(hs::moe_tiles_kernel<2, true>, g1, dim3(128), 0, st, pdl, (void*)act, hb,
-                    (const __nv_bfloat16*)w_gate, (const __nv_bfloat16*)w_up, (const int*)work,
-                    (const int*)row_token, E, max_tiles, ff, width, limit, act_kind);
-    else
-      e = hs_launch(hs::moe_tiles_kernel<1, true, true>, g1, dim3(128), 0, st, pdl, (void*)act, hb,
-                    (const __nv_bfloat16*)w_up, none, (const int*)work, (const int*)row_token, E,
-                    max_tiles, ff, width, limit, act_kind);
-    if (e != cudaSuccess) return (int)e;
-    e = hs_launch(hs::moe_tiles_kernel<1, false>, dim3(max_tiles, (width + hs::TN - 1) / hs::TN),
-                  dim3(128), 0, st, pdl, (void*)down, (const __nv_bfloat16*)act,
-                  (const __nv_bfloat16*)w_down, none, (const int*)work, (const int*)row_token, E,
-                  max_tiles, width, ff, limit, act_kind);
-    if (e != cudaSuccess) return (int)e;
+    if (int rc = hs::moe_tiles_tc(act, down, hb, (const __nv_bfloat16*)w_gate, (const __nv_bfloat16*)w_up,
+                                  (const __nv_bfloat16*)w_down, tiles, max_tiles, row_token, pairs,
+                                  width, ff, E, limit, act_kind, status, st))
+      return rc;
     e = hs_launch(hs::moe_combine_kernel, dim3(n_tokens), dim3(256), 0, st, pdl, x,
                   (const float*)down, (const int*)pair_pos, sel_w, tok_req, width, top, sel_idx, hb,
                   E, n_identity, accumulate);

@@ -232,7 +232,7 @@ def _declare(lib) -> None:
         "hs_delta_blocks_scratch": [I, I, I, I, I, P],
         "hs_delta_finish": [P, P, P, P, P, P, I, F, I, I, I, I, I, I, I, I, P, P],
         "hs_moe_route": [P, P, P, P, P, I, I, I, I, I, I, I, P, P],
-        "hs_moe_experts": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, F, I, I, P, P, I, I, P],
+        "hs_moe_experts": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, F, I, I, P, P, I, I, P, P],
         "hs_moe_route_softmax": [P, P, P, P, P, P, I, I, I, I, F, I, P, P],
         "hs_moe_route_top": [P, P, P, P, P, P, I, I, I, I, I, P, P],
         "hs_rms_norm": [P, P, P, P, I, I, F, I, P, I, I, I, P],
@@ -1568,7 +1568,7 @@ class CudaOps:
                                        T, width, ff, top, E, float(limit),
                                        EXPERT_ACTIVATIONS[act], _DT[h.dtype],
                                        _ptr(ints), _ptr(rows), int(identity), int(not fresh),
-                                       self._stream()),
+                                       _ptr(self.status), self._stream()),
                f"moe_experts(ff={ff})")
 
     def moe_route_top(self, sel_idx, sel_w, h, w_router, bias, tok_req, *, top, z=None):
