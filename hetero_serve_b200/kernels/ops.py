@@ -192,6 +192,8 @@ def _declare(lib) -> None:
         "hs_linear_simt": [P, P, P, P, P, I, I, I, I, F, F, I, I, P, P],
         "hs_linear_tcgen05": [P, P, P, P, P, I, I, I, I, F, F, I, I, I, P, P, P, P],
         "hs_linear_tcgen05_scratch": [I, I, I, I, I, P, P],
+        "hs_linear_f32_tc": [P, P, P, P, P, I, I, I, I, F, F, I, P, P, P],
+        "hs_linear_f32_tc_scratch": [I, I, I, I, P],
         "hs_linear_skinny": [P, P, P, P, P, F, P, P, P, I, I, I, I, F, F, I, P, P, I, P],
         "hs_linear_skinny_scratch": [I, I, I, I, P, P],
         "hs_linear_skinny_argmax": [P, P, P, I, I, I, P, P, P, P, P, P, P, I, P],
@@ -369,6 +371,8 @@ class CudaOps:
         self.fuse_append = True    # key/value append fused into the decode attention
         self.pdl = True            # programmatic dependent launch (see the property below)
         self._skinny_need: dict = {}
+        self._f32_need: dict = {}
+        self.f32_rows = 0          # rows a tile of the float32 tensor-core linear takes (0: its choice)
         self._moe_need: dict = {}
         # windowed latent attention of prompt portions in expanded form, on tcgen05 tensor cores
         self.latent_expanded = True
@@ -582,10 +586,34 @@ class CudaOps:
             if code != -1:
                 _check(code, f"linear_tcgen05(M={M},N={N},K={K})")
                 return
+        if a.dtype == torch.float32 and self.tensor_cores and self._f32_tc(
+                out, a, w, bias, (act, act_a, act_b), residual, M, N, K):
+            return
         _check(self.lib.hs_linear_simt(_ptr(out), _ptr(a), _ptr(w), _ptr(bias), _ptr(residual),
                                        M, N, K, act, act_a, act_b, _DT[a.dtype],
                                        _DT[out.dtype], _ptr(self.status), self._stream()),
                f"linear(M={M},N={N},K={K})")
+
+    def _f32_tc(self, out, a, w, bias, act, residual, M, N, K) -> bool:
+        """float32 as sums of bfloat16 terms on the tensor cores; False (by N, K and alignment alone)
+        when the kernel does not take the shape."""
+        key = (M, N, K, self.f32_rows)
+        need = self._f32_need.get(key)
+        if need is None:
+            floats = ctypes.c_longlong(0)
+            rc = self.lib.hs_linear_f32_tc_scratch(M, N, K, self.f32_rows, ctypes.byref(floats))
+            need = self._f32_need[key] = floats.value if rc == 0 else False
+        if need is False:
+            return False
+        scratch = self._scratch_buffer("f32_partial", need, torch.float32) if need else None
+        code = self.lib.hs_linear_f32_tc(
+            _ptr(out), _ptr(a), _ptr(w), _ptr(bias), _ptr(residual), M, N, K, *act, self.f32_rows,
+            _ptr(scratch), _ptr(self.status), self._stream())
+        if code == -1:
+            return False
+        _check(code, f"linear_f32_tc(M={M},N={N},K={K})")
+        self.launches += int(need > 0)
+        return True
 
     def _skinny_ok(self, M, N, K) -> bool:
         return self.tensor_cores and M <= self.skinny_max_rows
