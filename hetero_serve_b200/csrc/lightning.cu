@@ -18,7 +18,7 @@
 // rot_dims numbers (number i pairs with i + rot_dims/2) and k scaled: with a table of
 // frequencies the rows are turned where they are activated (in the pass of its own, or while
 // they are staged), by the same expression in both places.
-#include "rotary.cuh"
+#include "lightning.cuh"
 #include "tcgen05.cuh"
 
 namespace hs {
@@ -29,26 +29,6 @@ constexpr int LA_PART = LA_ROWS + 4; // floats between two parts' rows of a toke
                                      // the parts of a column read 16-byte pieces from distinct banks
 constexpr int LA_TOK = 16;           // tokens staged at a time (8 when dim is above 128)
 
-__device__ __forceinline__ float la_act(float z, int act) {
-  return act == HS_ACT_SILU ? z / (1.0f + expf(-z)) : z;
-}
-// entry d of a head's q or k vector `vec`: activated, turned by position `pos` when d lies in the
-// first rot_dims numbers (rot_dims 0: never), times `mul`
-__device__ __forceinline__ float la_entry(const float* __restrict__ vec, int d, int act,
-                                          int rot_dims, const float* __restrict__ freq, int pos,
-                                          float mul) {
-  float own = la_act(vec[d], act);
-  if (d < rot_dims) {
-    const int half = rot_dims >> 1;
-    const bool low = d < half;
-    const float partner = la_act(vec[low ? d + half : d - half], act);
-    float c, sn;
-    pair_angle(pos, freq[low ? d : d - half], &c, &sn);
-    const float cross = __fmul_rn(partner, sn);
-    own = fmaf(own, c, low ? -cross : cross);
-  }
-  return __fmul_rn(own, mul);
-}
 __device__ __forceinline__ void la_cp16(void* smem_dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem_dst)), "l"(src)
                : "memory");
@@ -153,7 +133,7 @@ lightning_kernel(float* __restrict__ o, float* __restrict__ state, const float* 
                  const int* __restrict__ req_len, const int* __restrict__ req_slot, int stride,
                  int q_off, int k_off, int v_off, int H, int D, int V, int P, int act, int ntok,
                  int bulk, const int* __restrict__ tok_pos, const float* __restrict__ freq,
-                 int rot_dims, float k_scale) {
+                 int rot_dims, float k_scale, int most) {
   extern __shared__ __align__(16) float smem[];
   pdl_trigger();
   pdl_wait();
@@ -162,7 +142,7 @@ lightning_kernel(float* __restrict__ o, float* __restrict__ state, const float* 
   const int per_buf = ntok * (2 * Dp + cols);       // a buffer: q [ntok][Dp], k [ntok][Dp], v [ntok][cols]
   const int r = blockIdx.z, h = blockIdx.y;
   const int n = req_len[r];
-  if (n <= 0) return;
+  if (n <= 0 || n > most) return;
   const int t0 = req_start[r];
   const int slot = req_slot[r];
   const int part = threadIdx.x % P, col = threadIdx.x / P;
@@ -261,12 +241,20 @@ __global__ void __launch_bounds__(256)
 lightning_rows_kernel(float* __restrict__ rows, float* __restrict__ vals,
                       const float* __restrict__ proj, int n_tokens, int stride, int q_off, int k_off,
                       int v_off, int H, int D, int V, int act, const int* __restrict__ tok_pos,
-                      const float* __restrict__ freq, int rot_dims, float k_scale, int per) {
+                      const float* __restrict__ freq, int rot_dims, float k_scale, int per,
+                      const int* __restrict__ req_start, const int* __restrict__ req_len,
+                      int n_requests, int most) {
   pdl_trigger();
   pdl_wait();
   __shared__ float s_c[128], s_s[128];
   const int h0 = blockIdx.y * per, nh = min(per, H - h0);
   const int t = blockIdx.x, half = rot_dims >> 1;
+  if (most < n_tokens) {                                  // rows of a request that goes in chunks
+    bool left_out = false;
+    for (int r = threadIdx.x; r < n_requests; r += blockDim.x)
+      left_out = left_out || (req_len[r] > most && t >= req_start[r] && t < req_start[r] + req_len[r]);
+    if (__syncthreads_or(left_out)) return;
+  }
   const int pos = rot_dims > 0 ? tok_pos[t] : 0;
   for (int i = threadIdx.x; i < half; i += blockDim.x) pair_angle(pos, freq[i], &s_c[i], &s_s[i]);
   __syncthreads();
@@ -323,7 +311,7 @@ lightning_stream_kernel(float* __restrict__ o, float* __restrict__ state,
                         const float* __restrict__ rows, const float* __restrict__ vals,
                         const float* __restrict__ decay, const int* __restrict__ req_start,
                         const int* __restrict__ req_len, const int* __restrict__ req_slot,
-                        int n_tokens, int H, int V, int* status) {
+                        int n_tokens, int H, int V, int most, int* status) {
   constexpr int D = P * LA_ROWS, COLS = 32 / P, CTA_COLS = LS_WARPS * COLS;
   extern __shared__ __align__(16) float smem[];           // [stages][LS_TOK][q | k], then the values
   __shared__ uint64_t full[LS_STAGES], empty[LS_STAGES];
@@ -341,7 +329,7 @@ lightning_stream_kernel(float* __restrict__ o, float* __restrict__ state,
   pdl_trigger();
   pdl_wait();
   const int n = req_len[r];
-  if (n <= 0) return;
+  if (n <= 0 || n > most) return;
   const int t0 = req_start[r], n_stages = (n + LS_TOK - 1) / LS_TOK;
   if (warp == LS_WARPS) {
     if (lane == 0) {
@@ -484,17 +472,28 @@ HS_EXPORT int hs_lightning_scratch(int n_tokens, int n_requests, int H, int D, i
   return HS_OK;
 }
 
+// Floats of scratch with which requests of many tokens go in chunks (0: none can).
+HS_EXPORT int hs_lightning_chunk_scratch(int n_tokens, int n_requests, int H, int D, int V, int rot_dims,
+                                         long long* floats) {
+  if (!floats || n_tokens < 0 || n_requests < 0 || H <= 0 || D <= 0 || V <= 0) return HS_ERR_ARGUMENT;
+  *floats = hs::lightning_takes_chunks(D, V, rot_dims)
+                ? hs::lightning_chunk_floats(n_tokens, n_requests, H, D, V, rot_dims) : 0;
+  return HS_OK;
+}
+
 // proj: float32 rows of `stride` columns holding q (H*D at q_off), k (H*D at k_off) and v (H*V at
 // v_off), head by head; o: float32 [tokens, H*V]; state: [slots, H*D*V] float32.  `scratch`
 // (hs_lightning_scratch floats, or null): with it the activations are applied in a pass of their own
-// and the recurrence streams the activated rows; the results are the same bits.
+// and the recurrence streams the activated rows; the results are the same bits.  `chunks`
+// (hs_lightning_chunk_scratch floats, or null): with it requests of hs::LC_MIN tokens and more go in chunks
+// on the tensor cores (lightning_chunk.cu: sums in another order), each by its own length.
 HS_EXPORT int hs_lightning_recurrence(float* o, float* state, const float* proj,
                                       const float* decay, const int* req_start,
                                       const int* req_len, const int* req_slot, int n_requests,
                                       int n_tokens, int stride, int q_off, int k_off, int v_off,
                                       int H, int D, int V, int act, float* scratch,
                                       const int* tok_pos, const float* freq, int rot_dims,
-                                      float k_scale, int* status, void* stream) {
+                                      float k_scale, float* chunks, int* status, void* stream) {
   if (!o || !state || !proj || !decay || !req_start || !req_len || !req_slot)
     return HS_ERR_ARGUMENT;
   if (rot_dims < 0 || rot_dims % 2 || rot_dims > D || (rot_dims > 0 && (!freq || !tok_pos)))
@@ -503,6 +502,16 @@ HS_EXPORT int hs_lightning_recurrence(float* o, float* state, const float* proj,
     return HS_ERR_UNSUPPORTED;
   if (n_requests <= 0 || n_tokens <= 0) return HS_OK;
   cudaStream_t st = (cudaStream_t)stream;
+  int most = 0x7fffffff;                // tokens of the requests that are walked here
+  if (chunks && hs::lightning_chunk_slots(n_tokens, n_requests) > 0 &&
+      hs::lightning_takes_chunks(D, V, rot_dims) &&
+      !(((uintptr_t)chunks | (uintptr_t)state) & 15) && !((uintptr_t)o & 7)) {
+    if (int e = hs::lightning_chunks(o, state, proj, decay, req_start, req_len, req_slot, n_requests, n_tokens,
+                                     stride, q_off, k_off, v_off, H, D, V, act, chunks, tok_pos, freq, rot_dims,
+                                     k_scale, st))
+      return e;
+    most = hs::LC_MIN - 1;
+  }
   if (scratch && status && lightning_streams(n_tokens, n_requests, D) && !((uintptr_t)scratch & 15)) {
     // (measured, 2 x 1,024 tokens, 8 heads of 128 x 128: retention's mixer takes 176 us this way, 395
     // with the two kernels below)
@@ -513,7 +522,8 @@ HS_EXPORT int hs_lightning_recurrence(float* o, float* state, const float* proj,
     cudaError_t e = hs_launch(hs::lightning_rows_kernel, dim3(n_tokens, (H + per - 1) / per),
                               dim3(256), 0, st,
                               hs_pdl_enabled(), scratch, vals, proj, n_tokens, stride, q_off, k_off,
-                              v_off, H, D, V, act, tok_pos, freq, rot_dims, k_scale, per);
+                              v_off, H, D, V, act, tok_pos, freq, rot_dims, k_scale, per, req_start,
+                              req_len, n_requests, most);
     if (e != cudaSuccess) return (int)e;
     const size_t smem = (size_t)hs::LS_STAGES * hs::LS_TOK * (2 * D + cols) * sizeof(float);
 #define HS_LS(P)                                                                                 \
@@ -524,7 +534,7 @@ HS_EXPORT int hs_lightning_recurrence(float* o, float* state, const float* proj,
       e = hs_launch(hs::lightning_stream_kernel<P>, dim3(groups, H, n_requests),                 \
                     dim3(hs::LS_WARPS * 32 + 32), smem, st, hs_pdl_enabled(), o, state,          \
                     (const float*)scratch, (const float*)vals, decay, req_start, req_len,        \
-                    req_slot, n_tokens, H, V, status);                                           \
+                    req_slot, n_tokens, H, V, most, status);                                           \
   } while (0)
     if (D == 64) HS_LS(4);
     else if (D == 128) HS_LS(8);
@@ -557,7 +567,7 @@ HS_EXPORT int hs_lightning_recurrence(float* o, float* state, const float* proj,
   cudaError_t e = hs_launch(hs::lightning_kernel, grid, dim3(hs::LA_THREADS), smem, st,
                             hs_pdl_enabled(), o, state, proj, decay, req_start, req_len, req_slot,
                             stride, q_off, k_off, v_off, H, D, V, P, act, ntok, bulk, tok_pos, freq,
-                            rot_dims, k_scale);
+                            rot_dims, k_scale, most);
   if (e != cudaSuccess) return (int)e;
   return HS_OK;
 }

@@ -247,8 +247,9 @@ def _declare(lib) -> None:
         "hs_biased_attention_prefill": [P, P, P, P, P, P, I, P, P, I, P, I, I, I, I, I, I, I, I,
                                         F, F, I, I, P, P],
         "hs_lightning_recurrence": [P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, P, P, P, I,
-                                    F, P, P],
+                                    F, P, P, P],
         "hs_lightning_scratch": [I, I, I, I, I, P],
+        "hs_lightning_chunk_scratch": [I, I, I, I, I, I, P],
         "hs_token_shift_mix": [P, P, P, P, I, I, P, P, P, P, I, I, I, I, P],
         "hs_timemix_decay": [P, P, P, P, I, I, I, P],
         "hs_timemix_recurrence": [P, P, I, P, P, P, P, P, P, P, P, I, I, I, I, P],
@@ -1922,13 +1923,15 @@ class CudaOps:
     # -- linear attention with a decay per head ---------------------------------------------
     def lightning_recurrence(self, o, state, proj, decay, req_start, req_len, req_slot, *, q_off,
                              k_off, v_off, heads, dim, vdim, act="silu", tok_pos=None, freq=None,
-                             rot_dims=0, k_scale=1.0):
+                             rot_dims=0, k_scale=1.0, chunks=False):
         """Per request and head, token after token on the float32 state S [dim, vdim] of the
         request's slot: S <- decay[h] S + k v^T; o = S^T q, with q, k, v = act(columns of the
         float32 projection rows ``proj``), laid out head by head from ``q_off``, ``k_off``,
         ``v_off``.  ``o`` is float32 [T, heads * vdim].  With ``freq`` (float32 [rot_dims / 2])
         q and k are turned by ``tok_pos`` on their first ``rot_dims`` numbers (number i pairs
-        with i + rot_dims / 2) before they are used; k is multiplied by ``k_scale``."""
+        with i + rot_dims / 2) before they are used; k is multiplied by ``k_scale``.
+        ``chunks``: requests that bring many tokens may go in chunks on the tensor cores (float32 terms
+        and sums, in another order than token after token; each request by its own length)."""
         _want(o, "o", torch.float32, 2)
         _want(proj, "proj", torch.float32, 2)
         _want(state, "state", torch.float32)
@@ -1960,12 +1963,20 @@ class CudaOps:
             if need.value:
                 scratch = self._scratch_buffer("lightning_rows", need.value, torch.float32)
         self.launches += 2 if scratch is not None else 1
+        parts = None
+        if chunks:
+            need = ctypes.c_longlong(0)
+            self.lib.hs_lightning_chunk_scratch(T, req_start.shape[0], heads, dim, vdim, int(rot_dims),
+                                                ctypes.byref(need))
+            if need.value:
+                parts = self._scratch_buffer("lightning_chunks", need.value, torch.float32)
+                self.launches += 4 if rot_dims else 3
         _check(self.lib.hs_lightning_recurrence(
             _ptr(o), _ptr(state), _ptr(proj), _ptr(decay), _ptr(req_start), _ptr(req_len),
             _ptr(req_slot), req_start.shape[0], T, proj.shape[1], int(q_off), int(k_off),
             int(v_off), heads, dim, vdim, ACTIVATIONS[act], _ptr(scratch),
             _ptr(tok_pos) if rot_dims else None, _ptr(freq) if rot_dims else None, int(rot_dims),
-            float(k_scale), _ptr(self.status), self._stream()),
+            float(k_scale), _ptr(parts), _ptr(self.status), self._stream()),
             f"lightning_recurrence(dim={dim},vdim={vdim})")
 
     # -- norms behind a sublayer, a learned activation, capped logits -----------------------

@@ -58,10 +58,12 @@ class LightningAttention(Mixer):
         ops, T = ctx.ops, h.shape[0]
         hd, hv = self.H * self.D, self.H * self.V
         o = ctx.buffer("lightning_o", (T, hv), torch.float32)
+        # rows leave in bfloat16: long portions in chunks (float32 engines keep one order of the sums)
+        more = {"chunks": True} if ctx.dtype == torch.bfloat16 else {}
         ops.lightning_recurrence(o, ctx.state(), proj, self.decay, ctx.req_start, ctx.req_len,
                                  ctx.req_slot, q_off=offset, k_off=offset + hd,
                                  v_off=offset + 2 * hd, heads=self.H, dim=self.D, vdim=self.V,
-                                 act="silu")
+                                 act="silu", **more)
         gated = ctx.buffer("lightning_gated", (T, hv), ctx.dtype)
         ops.rms_norm(gated, o, self.norm_w, self.eps, gate=proj, gate_offset=offset + 2 * hd + hv)
         ops.linear(out, gated, self.w_out, None, residual=out if accumulate else None)

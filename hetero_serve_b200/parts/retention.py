@@ -68,10 +68,12 @@ class Retention(Mixer):
         proj = ctx.buffer("retention_proj", (T, self.w_in.shape[0]), torch.float32)
         ops.linear(proj, h, self.w_in)
         o = ctx.buffer("retention_o", (T, hv), torch.float32)
+        # rows leave in bfloat16: long portions in chunks (float32 engines keep one order of the sums)
+        more = {"chunks": True} if ctx.dtype == torch.bfloat16 else {}
         ops.lightning_recurrence(o, ctx.state(), proj, self.decay, ctx.req_start, ctx.req_len,
                                  ctx.req_slot, q_off=0, k_off=hd, v_off=2 * hd, heads=self.H,
                                  dim=self.D, vdim=self.V, act="none", tok_pos=ctx.tok_pos,
-                                 freq=self.freq, rot_dims=self.rot_dims, k_scale=self.k_scale)
+                                 freq=self.freq, rot_dims=self.rot_dims, k_scale=self.k_scale, **more)
         gated = ctx.buffer("retention_gated", (T, hv), ctx.dtype)
         ops.head_norm_gate(gated, o, None, proj, gate_offset=2 * hd + hv, heads=self.H,
                            dim=self.V, eps=self.eps, gate_act=self.gate_act)

@@ -1,0 +1,118 @@
+"""Lightning attention and retention in chunks: closer to float64 than the walk token by token, each
+request by its own length, and numbers that are not finite stay behind their token."""
+
+import pytest
+import torch
+
+from hetero_serve_b200.kernels.ops import CudaOps
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def inputs(lens, H, D, V, rot, seed):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    T, R = sum(lens), len(lens)
+    proj = torch.randn(T, 2 + H * (2 * D + V), device=DEV, generator=g)
+    state = torch.randn(R + 1, H * D * V, device=DEV, generator=g)
+    pos = [100 * r + t for r, n in enumerate(lens) for t in range(n)]
+    freq = 10000.0 ** (-torch.arange(max(rot // 2, 1), device=DEV) * 2.0 / max(rot, 1))
+    return proj, state, pos, freq.float()
+
+
+def walk(lens, proj, state, pos, freq, decay, H, D, V, rot, act, scale):
+    """The recurrence in float64; angles from the float32 frequencies."""
+    x = proj.double()
+    x = torch.nn.functional.silu(x) if act == "silu" else x
+    q, k, v = x[:, 2:2 + H * D], x[:, 2 + H * D:2 + 2 * H * D], x[:, 2 + 2 * H * D:]
+    q, k, v = q.view(-1, H, D).clone(), k.view(-1, H, D).clone(), v.view(-1, H, V)
+    if rot:
+        angle = torch.tensor(pos, device=DEV).double()[:, None] * freq.double()[:rot // 2]
+        c, s = torch.cos(angle)[:, None], torch.sin(angle)[:, None]
+        for u in (q, k):
+            a, b = u[..., :rot // 2].clone(), u[..., rot // 2:rot].clone()
+            u[..., :rot // 2], u[..., rot // 2:rot] = a * c - b * s, b * c + a * s
+        k = k * scale
+    o, S, at = torch.zeros_like(v), state.double().view(-1, H, D, V).clone(), 0
+    for r, n in enumerate(lens):
+        slot = len(lens) - r
+        for t in range(at, at + n):
+            S[slot] = S[slot] * decay.double()[:, None, None] + k[t, :, :, None] * v[t, :, None]
+            o[t] = torch.einsum("hdv,hd->hv", S[slot], q[t])
+        at += n
+    return o.flatten(1), S.flatten(1)
+
+
+def run(ops, lens, proj, state, pos, freq, decay, H, D, V, rot, act, scale, chunks):
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    o, S, R = torch.full((sum(lens), H * V), float("nan"), device=DEV), state.clone(), len(lens)
+    more = dict(tok_pos=i32(pos), freq=freq, rot_dims=rot, k_scale=scale) if rot else {}
+    ops.lightning_recurrence(o, S, proj, decay, i32([sum(lens[:r]) for r in range(R)]), i32(lens),
+                             i32(list(range(R, 0, -1))), q_off=2, k_off=2 + H * D, v_off=2 + 2 * H * D, heads=H,
+                             dim=D, vdim=V, act=act, chunks=chunks, **more)
+    return o, S
+
+
+@pytest.mark.parametrize("rot, act", [(128, "none"), (0, "silu"), (64, "silu"), (4, "none")])
+@pytest.mark.parametrize("lens", [(512,), (513, 3, 0, 511), (64, 575, 576), (600, 1, 1025)])
+def test_against_float64(rot, act, lens):
+    D, V = 128, 128
+    H, decay = 3, torch.tensor([0.9961, 0.55, 0.93], device=DEV)
+    ops = CudaOps(DEV)
+    proj, state, pos, freq = inputs(lens, H, D, V, rot, D + V + sum(lens))
+    args = (lens, proj, state, pos, freq, decay, H, D, V, rot, act, 0.125)
+    want_o, want_S = walk(*args)
+    (o, S), (po, pS) = run(ops, *args, chunks=True), run(ops, *args, chunks=False)
+    err = lambda a, b: float((a.double() - b).norm() / b.norm())  # noqa: E731
+    # sequential sums round every token: the chunks are to be no further off (a few roundings of 2^-24 where
+    # a portion has only a handful of chunks)
+    assert err(o, want_o) <= err(po, want_o) * 1.02 + 2e-8 and err(S, want_S) <= err(pS, want_S) * 1.02 + 2e-8
+    assert err(o, want_o) < 1e-6 and err(S, want_S) < 1e-6
+    at = 0
+    for r, n in enumerate(lens):               # short portions and their states: the same bits
+        if n < 512:
+            assert torch.equal(o[at:at + n], po[at:at + n])
+            assert torch.equal(S[len(lens) - r], pS[len(lens) - r])
+        at += n
+    assert torch.equal(S[0], state[0])         # nobody's slot
+    # a request's chunks do not depend on its neighbours
+    n = max(lens)
+    at = sum(lens[:lens.index(n)])
+    alone = (proj[at:at + n].clone(), state[[0, len(lens) - lens.index(n)]].clone(), pos[at:at + n])
+    ao, aS = run(ops, (n,), *alone, freq, decay, H, D, V, rot, act, 0.125, chunks=True)
+    assert torch.equal(ao, o[at:at + n]) and torch.equal(aS[1], S[len(lens) - lens.index(n)])
+    assert ops.status.item() == 0
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), 3.3e38])
+@pytest.mark.parametrize("where", ["q", "k", "v", "state"])
+def test_numbers_that_are_not_finite_stay_behind_their_token(bad, where):
+    H, D, V, lens, t = 2, 128, 128, (576,), 100
+    ops, decay = CudaOps(DEV), torch.tensor([0.99, 0.5], device=DEV)
+    proj, state, pos, freq = inputs(lens, H, D, V, 0, 7)
+    args = lambda p, s: (lens, p, s, pos, freq, decay, H, D, V, 0, "none", 1.0)  # noqa: E731
+    clean, _ = run(ops, *args(proj, state), chunks=True)
+    p, s = proj.clone(), state.clone()
+    if where == "state":
+        s[1, 5 * V + 3] = bad
+    else:
+        p[t, 2 + {"q": 0, "k": H * D, "v": 2 * H * D}[where] + 3] = bad
+    (o, S), (po, pS) = run(ops, *args(p, s), chunks=True), run(ops, *args(p, s), chunks=False)
+    if where != "state":
+        assert torch.equal(o[:64], clean[:64])             # the chunk before keeps its bits
+        assert o[:t].isfinite().all()
+    assert torch.equal(o.isnan(), po.isnan()) and torch.equal(S.isnan(), pS.isnan())
+    assert torch.equal(o.isfinite(), po.isfinite()) and torch.equal(S.isfinite(), pS.isfinite())
+    fine = po.isfinite() & (po.abs() < 1e30)
+    assert bool(((o - po)[fine].abs() <= 1e-3 + 1e-4 * po[fine].abs()).all())
+
+
+def test_decays_at_the_ends():
+    H, D, V, lens = 3, 128, 128, (550,)
+    ops, decay = CudaOps(DEV), torch.tensor([0.0, 1.0, 1e-3], device=DEV)
+    proj, state, pos, freq = inputs(lens, H, D, V, 0, 8)
+    args = (lens, proj, state, pos, freq, decay, H, D, V, 0, "none", 1.0)
+    want_o, want_S = walk(*args)
+    o, S = run(ops, *args, chunks=True)
+    assert float((o.double() - want_o).norm() / want_o.norm()) < 1e-6
+    assert float((S.double() - want_S).norm() / want_S.norm()) < 1e-6
