@@ -288,6 +288,34 @@ __device__ __forceinline__ void store_chunk_staged(const TcParams& p, const floa
   }
 }
 
+// The same for rows that do not start on 16 bytes (N not a multiple of 8, the vocabulary's logits among
+// them): the patch is read back a number a lane, 64 contiguous bytes a row.  (32 x 50,257 x 1,024, a lane
+// storing its own row number by number: 32 us in tiles of 128, so 29.)
+template <typename TO>
+__device__ __forceinline__ void store_chunk_ragged(const TcParams& p, const float (&f)[32], uint8_t* patch,
+                                                   int lane, int row0, int nbase) {
+  constexpr int PER = 64 / (int)sizeof(TO), ROWS = 32 / PER;     // rows an instruction covers
+  TO* out = (TO*)p.out;
+  const int sw_w = (lane >> 1) & 3;
+  const int c = lane % PER, rows = min(32, p.M - row0);
+#pragma unroll
+  for (int h = 0; h < 32 / PER; ++h) {
+#pragma unroll
+    for (int pc = 0; pc < 4; ++pc) {
+      alignas(16) TO v[PER / 4];
+#pragma unroll
+      for (int j = 0; j < PER / 4; ++j) v[j] = from_f<TO>(f[h * PER + pc * (PER / 4) + j]);
+      *(uint4*)(patch + lane * 64 + ((pc ^ sw_w) << 4)) = *(const uint4*)v;
+    }
+    __syncwarp();
+    const int pc = c / (PER / 4), at = (c % (PER / 4)) * (int)sizeof(TO);
+    for (int r = lane / PER; r < rows; r += ROWS)
+      out[(size_t)(row0 + r) * p.N + nbase + h * PER + c] =
+          *(const TO*)(patch + r * 64 + ((pc ^ ((r >> 1) & 3)) << 4) + at);
+    __syncwarp();
+  }
+}
+
 // One epilogue warp's share of a tile: NCHUNK chunks of 32 columns from c_begin on, of the 32
 // rows it owns in tensor memory.  Before it waits for the accumulator it has the residual of
 // its first two chunks on the way (the main loop hides the loads); afterwards the tcgen05.ld of
@@ -321,6 +349,13 @@ __device__ __forceinline__ bool epilogue_columns(const TcParams& p, uint64_t* ac
     tmem_ld_wait();
     const int nbase = n0 + c0;
     const int nvalid = min(32, p.N - nbase);
+    if (!SPLIT && !vec && p.residual == nullptr && nvalid == 32) {
+      float f[32];
+      bias_act32(p, v, bias_s ? bias_s + c0 : nullptr, f);
+      if (c + 1 < NCHUNK) tmem_ld32(t_addr + (uint32_t)(c0 + 32), v);
+      store_chunk_ragged<TO>(p, f, patch, lane, row0, nbase);
+      continue;
+    }
     if (!SPLIT && staged_ok && nvalid == 32) {
       float f[32];
       bias_act32(p, v, bias_s ? bias_s + c0 : nullptr, f);
@@ -1271,8 +1306,10 @@ static bool plan_tc(int M, int N, int K, int tile_n, int pair, TcPlan& pl) {
       }
     }
     // few rows: narrow tiles (more CTAs stream the weights) and splits; a very wide layer (the
-    // vocabulary) has tiles enough and reads the activations less often with 128 columns
-    if (mt == 1) bn = ((N + 63) / 64 >= 2 * sms) ? 128 : 64;
+    // vocabulary) has tiles enough, and wide ones keep more of the weights on their way (50,257 columns,
+    // us at 64, 128, 192 and 256 wide: 32 x 1,024 37, 29, 26, 30; 17 x 1,600 65, 48, 36, 37; 64 x 768 28, 22,
+    // 21, 27)
+    if (mt == 1) bn = ((N + 63) / 64 >= 2 * sms) ? 192 : 64;
   }
   if (bn != 64 && bn != 128 && bn != 192 && bn != 256) return false;
   pl.bn = bn;
