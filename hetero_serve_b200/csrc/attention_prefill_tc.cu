@@ -131,6 +131,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
   uint32_t n_item = 0;        // items processed by this CTA
   uint32_t n_tile = 0;        // key tiles processed by this CTA (over all items)
   bool ok = true;
+  uint32_t limit = HS_SPIN_LIMIT;      // of the issuing warp's waits
 
   // Items are listed heaviest first; CTA b takes b, 2G-1-b, 2G+b, 4G-1-b, ... (G CTAs): a
   // snake over the sorted list, so heavy and light items alternate per CTA.  Every role walks
@@ -203,22 +204,21 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
                       &bars[B_KV_FULL + st], 0, src_row);
       }
     } else if (warp == 1) {
-      if (lane == 0) {
-        // ---------------- MMA issuer
-        constexpr uint32_t idesc_s = make_idesc(TA_BQ, TA_BKV, false);
-        constexpr uint32_t idesc_o = make_idesc(TA_BQ, TA_D, true);
-        const int qb = n_item & 1;
-        const uint32_t q_addr = smem_u32(sQ + qb * TA_Q_BYTES);
-        ok = mbar_wait(&bars[B_Q_FULL + qb], (n_item >> 1) & 1, p.status);
-        auto issue_s = [&](int kt) -> bool {
-          const uint32_t it = n_tile + kt;
-          const int st = it % TA_KV_STAGES, sb = it & 1;
-          if (!mbar_wait(&bars[B_KV_FULL + st], (it / TA_KV_STAGES) & 1, p.status)) return false;
-          if (it >= 2 && !mbar_wait(&bars[B_S_EMPTY + sb], ((it >> 1) - 1) & 1, p.status))
-            return false;
-          tc_fence_after();
-          const uint64_t qd = make_smem_desc(q_addr);
-          const uint64_t kd = make_smem_desc(smem_u32(sK + st * TA_KV_BYTES));
+      // ---------------- MMA issuer
+      constexpr uint32_t idesc_s = make_idesc(TA_BQ, TA_BKV, false);
+      constexpr uint32_t idesc_o = make_idesc(TA_BQ, TA_D, true);
+      const int qb = n_item & 1;
+      const uint32_t q_addr = smem_u32(sQ + qb * TA_Q_BYTES);
+      mbar_wait_warp(&bars[B_Q_FULL + qb], (n_item >> 1) & 1, p.status, limit);
+      auto issue_s = [&](int kt) {
+        const uint32_t it = n_tile + kt;
+        const int st = it % TA_KV_STAGES, sb = it & 1;
+        mbar_wait_warp(&bars[B_KV_FULL + st], (it / TA_KV_STAGES) & 1, p.status, limit);
+        if (it >= 2) mbar_wait_warp(&bars[B_S_EMPTY + sb], ((it >> 1) - 1) & 1, p.status, limit);
+        tc_fence_after();
+        const uint64_t qd = make_smem_desc(q_addr);
+        const uint64_t kd = make_smem_desc(smem_u32(sK + st * TA_KV_BYTES));
+        if (elect_one()) {
 #pragma unroll
           for (int k = 0; k < TA_D / 16; ++k)
             umma_bf16(tmem_base + sb * S_COLS, qd + (uint64_t)(k * 2), kd + (uint64_t)(k * 2),
@@ -226,20 +226,20 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
           umma_commit(&bars[B_S_FULL + sb]);
           // the item's last S: once it has completed, Q may be replaced by the next item's
           if (kt == n_kv - 1) umma_commit(&bars[B_Q_EMPTY + qb]);
-          return true;
-        };
-        if (ok) ok = issue_s(0);
-        for (int kt = 0; kt < n_kv && ok; ++kt) {
-          const uint32_t it = n_tile + kt;
-          const int st = it % TA_KV_STAGES;
-          if (kt + 1 < n_kv) ok = issue_s(kt + 1);      // overlaps the softmax of tile kt
-          if (!ok) break;
-          ok = mbar_wait(&bars[B_P_FULL], it & 1, p.status);
-          if (ok && it >= 1) ok = mbar_wait(&bars[B_O_EMPTY], (it - 1) & 1, p.status);
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t p_addr = smem_u32(sP);
-          const uint32_t v_addr = smem_u32(sV + st * TA_KV_BYTES);
+        }
+        __syncwarp();
+      };
+      issue_s(0);
+      for (int kt = 0; kt < n_kv; ++kt) {
+        const uint32_t it = n_tile + kt;
+        const int st = it % TA_KV_STAGES;
+        if (kt + 1 < n_kv) issue_s(kt + 1);      // overlaps the softmax of tile kt
+        mbar_wait_warp(&bars[B_P_FULL], it & 1, p.status, limit);
+        if (it >= 1) mbar_wait_warp(&bars[B_O_EMPTY], (it - 1) & 1, p.status, limit);
+        tc_fence_after();
+        const uint32_t p_addr = smem_u32(sP);
+        const uint32_t v_addr = smem_u32(sV + st * TA_KV_BYTES);
+        if (elect_one()) {
 #pragma unroll
           for (int k = 0; k < TA_BKV / 16; ++k) {
             // P: k-block (k / 4) of 64 keys, 32 bytes per k-step inside its 128-byte rows;
@@ -252,6 +252,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
           umma_commit(&bars[B_P_EMPTY]);
           umma_commit(&bars[B_KV_EMPTY + st]);
         }
+        __syncwarp();
       }
     } else {
       // ---------------- softmax and output: two threads per query row, one per half of the

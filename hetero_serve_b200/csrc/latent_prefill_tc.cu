@@ -329,16 +329,16 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = make_idesc(LP_BQ, LP_BKV, false);
-      constexpr uint32_t idesc_o = make_idesc(LP_BQ, NV * 64, true);
-      ok = mbar_wait(&bars[LB_Q], 0, p.status);
-      auto issue_s = [&](int kt) -> bool {
-        const int st = kt & 1;
-        if (!mbar_wait(&bars[LB_K_FULL + st], (kt >> 1) & 1, p.status)) return false;
-        if (kt >= 2 && !mbar_wait(&bars[LB_S_EMPTY + st], ((kt >> 1) - 1) & 1, p.status))
-          return false;
-        tc_fence_after();
+    constexpr uint32_t idesc_s = make_idesc(LP_BQ, LP_BKV, false);
+    constexpr uint32_t idesc_o = make_idesc(LP_BQ, NV * 64, true);
+    uint32_t limit = HS_SPIN_LIMIT;
+    mbar_wait_warp(&bars[LB_Q], 0, p.status, limit);
+    auto issue_s = [&](int kt) {
+      const int st = kt & 1;
+      mbar_wait_warp(&bars[LB_K_FULL + st], (kt >> 1) & 1, p.status, limit);
+      if (kt >= 2) mbar_wait_warp(&bars[LB_S_EMPTY + st], ((kt >> 1) - 1) & 1, p.status, limit);
+      tc_fence_after();
+      if (elect_one()) {
 #pragma unroll
         for (int c = 0; c < NK; ++c) {
           const uint64_t qd = make_smem_desc(smem_u32(sQ + c * LP_CHUNK));
@@ -350,16 +350,17 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
         }
         umma_commit(&bars[LB_S_FULL + st]);
         umma_commit(&bars[LB_K_EMPTY + st]);
-        return true;
-      };
-      if (ok) ok = issue_s(0);
-      for (int kt = 0; kt < n_kv && ok; ++kt) {
-        if (kt + 1 < n_kv) ok = issue_s(kt + 1);         // overlaps the softmax of tile kt
-        if (ok) ok = mbar_wait(&bars[LB_P_FULL], kt & 1, p.status);
-        if (ok) ok = mbar_wait(&bars[LB_V_FULL], kt & 1, p.status);
-        if (ok && kt >= 1) ok = mbar_wait(&bars[LB_O_EMPTY], (kt - 1) & 1, p.status);
-        if (!ok) break;
-        tc_fence_after();
+      }
+      __syncwarp();
+    };
+    issue_s(0);
+    for (int kt = 0; kt < n_kv; ++kt) {
+      if (kt + 1 < n_kv) issue_s(kt + 1);         // overlaps the softmax of tile kt
+      mbar_wait_warp(&bars[LB_P_FULL], kt & 1, p.status, limit);
+      mbar_wait_warp(&bars[LB_V_FULL], kt & 1, p.status, limit);
+      if (kt >= 1) mbar_wait_warp(&bars[LB_O_EMPTY], (kt - 1) & 1, p.status, limit);
+      tc_fence_after();
+      if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < LP_BKV / 16; ++k) {
           const uint64_t pd =
@@ -370,6 +371,7 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
         umma_commit(&bars[LB_PV_DONE]);
         umma_commit(&bars[LB_V_EMPTY]);
       }
+      __syncwarp();
     }
   } else {
     const int qtr = warp & 3;                              // TMEM lane quarter of this warp

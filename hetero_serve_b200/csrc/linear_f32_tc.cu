@@ -199,23 +199,22 @@ __global__ void __launch_bounds__(LF_THREADS, 1) linear_f32_tc_kernel(const LfPa
   const uint32_t tmem = tmem_slot;
 
   if (warp == LF_CONV + LF_SUM) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc(LF_BM, NR);
-      constexpr uint64_t TA = LF_A_TERM >> 4, TB = S::B_TERM >> 4;
-      bool ok = true;
-      int s = 0, round = 0, cc = 0;
-      for (int w = blockIdx.x; w < p.items && ok; w += gridDim.x) {
-        const LfItem it = lf_item<NR>(p, w);
-        for (int kb = it.kb0; kb < it.kb1; ++kb, ++cc) {
-          const int b = cc & 1;
-          if (cc > 1) ok = mbar_wait(&acc_empty[b], ((cc >> 1) - 1) & 1, p.status);
-          ok = ok && mbar_wait(&full_bar[s], round & 1, p.status);
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t acc = tmem + b * NR, base = smem_u32(smem + s * S::STAGE);
-          const uint64_t da = make_smem_desc(base), db = make_smem_desc(base + 3 * LF_A_TERM);
+    constexpr uint32_t idesc = make_idesc(LF_BM, NR);
+    constexpr uint64_t TA = LF_A_TERM >> 4, TB = S::B_TERM >> 4;
+    uint32_t limit = HS_SPIN_LIMIT;
+    int s = 0, round = 0, cc = 0;
+    for (int w = blockIdx.x; w < p.items; w += gridDim.x) {
+      const LfItem it = lf_item<NR>(p, w);
+      for (int kb = it.kb0; kb < it.kb1; ++kb, ++cc) {
+        const int b = cc & 1;
+        if (cc > 1) mbar_wait_warp(&acc_empty[b], ((cc >> 1) - 1) & 1, p.status, limit);
+        mbar_wait_warp(&full_bar[s], round & 1, p.status, limit);
+        tc_fence_after();
+        const uint32_t acc = tmem + b * NR, base = smem_u32(smem + s * S::STAGE);
+        const uint64_t da = make_smem_desc(base), db = make_smem_desc(base + 3 * LF_A_TERM);
+        if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < LF_BK / 16; ++k) {           // small products
+          for (int k = 0; k < LF_BK / 16; ++k) {         // small products
             umma_bf16(acc, da + 2 * k, db + 2 * k + 2 * TB, idesc, k > 0 ? 1u : 0u);
             umma_bf16(acc, da + 2 * k + 2 * TA, db + 2 * k, idesc, 1u);
             umma_bf16(acc, da + 2 * k + TA, db + 2 * k + TB, idesc, 1u);
@@ -226,8 +225,9 @@ __global__ void __launch_bounds__(LF_THREADS, 1) linear_f32_tc_kernel(const LfPa
           for (int k = 0; k < LF_BK / 16; ++k) umma_bf16(acc, da + 2 * k, db + 2 * k, idesc, 1u);
           umma_commit(&empty_bar[s]);
           umma_commit(&acc_full[b]);
-          if (++s == S::STAGES) { s = 0; ++round; }
         }
+        __syncwarp();
+        if (++s == S::STAGES) { s = 0; ++round; }
       }
     }
   } else if (warp < LF_CONV) {

@@ -501,30 +501,28 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ---------------- MMA issuer
-      constexpr uint32_t idesc = make_idesc(TC_BM, BN);
-      uint32_t it = 0, wi = 0;
-      bool ok = true;
-      for (int w = blockIdx.x; w < n_items && ok; w += gridDim.x, ++wi) {
-        const int split = w % p.splits;
-        const int kb0 = split * p.kb_per_split;
-        const int kb1 = min(kb0 + p.kb_per_split, num_kb);
-        const uint32_t acc = wi & 1, acc_round = wi >> 1;
-        if (acc_round > 0) ok = mbar_wait(&acc_empty[acc], (acc_round - 1) & 1, p.status);
-        if (!ok) break;
+    // ---------------- MMA issuer (a whole warp, one elected lane: tcgen05.cuh)
+    constexpr uint32_t idesc = make_idesc(TC_BM, BN);
+    uint32_t it = 0, wi = 0;
+    uint32_t limit = HS_SPIN_LIMIT;
+    for (int w = blockIdx.x; w < n_items; w += gridDim.x, ++wi) {
+      const int split = w % p.splits;
+      const int kb0 = split * p.kb_per_split;
+      const int kb1 = min(kb0 + p.kb_per_split, num_kb);
+      const uint32_t acc = wi & 1, acc_round = wi >> 1;
+      if (acc_round > 0) mbar_wait_warp(&acc_empty[acc], (acc_round - 1) & 1, p.status, limit);
+      tc_fence_after();
+      const uint32_t tmem_d = tmem_base + acc * ACC_COLS;
+      for (int kb = kb0; kb < kb1; kb += PER, ++it) {
+        const int s = it % RING;
+        const uint32_t round = it / RING;
+        const int here = PER == 1 ? 1 : min(PER, kb1 - kb);
+        mbar_wait_warp(&full_bar[s], round & 1, p.status, limit);
         tc_fence_after();
-        const uint32_t tmem_d = tmem_base + acc * ACC_COLS;
-        for (int kb = kb0; kb < kb1 && ok; kb += PER, ++it) {
-          const int s = it % RING;
-          const uint32_t round = it / RING;
-          const int here = PER == 1 ? 1 : min(PER, kb1 - kb);
-          ok = mbar_wait(&full_bar[s], round & 1, p.status);
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t a_addr = smem_u32(smem + s * PER * S::STAGE_BYTES);
-          const uint64_t adesc = make_smem_desc(a_addr);
-          const uint64_t bdesc = make_smem_desc(a_addr + S::A_BYTES);
+        const uint32_t a_addr = smem_u32(smem + s * PER * S::STAGE_BYTES);
+        const uint64_t adesc = make_smem_desc(a_addr);
+        const uint64_t bdesc = make_smem_desc(a_addr + S::A_BYTES);
+        if (elect_one()) {
 #pragma unroll
           for (int j = 0; j < PER; ++j)
             if (j < here) {
@@ -539,8 +537,10 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
             }
           umma_commit(&empty_bar[s]);     // the stage may be refilled once these MMAs are done
         }
-        umma_commit(&acc_full[acc]);      // this accumulator is complete (or the pipeline gave up)
+        __syncwarp();
       }
+      if (elect_one()) umma_commit(&acc_full[acc]);      // this accumulator is complete (or the pipeline gave up)
+      __syncwarp();
     }
   } else if (warp >= 4) {
     // ---------------- epilogue: 8 warps; warp (w % 4) owns TMEM lanes 32*(w%4) .. +31, the two
@@ -775,34 +775,36 @@ linear_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
       // ---------------- MMA issuer (the even CTA only)
       constexpr uint32_t idesc = make_idesc(2 * TC_BM, BN);
       uint32_t it = 0, wi = 0;
-      bool ok = true;
-      for (int w = pair; w < n_items && ok; w += n_pairs, ++wi) {
+      uint32_t limit = HS_SPIN_LIMIT;
+      for (int w = pair; w < n_items; w += n_pairs, ++wi) {
         const uint32_t acc = wi & 1, acc_round = wi >> 1;
-        if (acc_round > 0) ok = mbar_wait(&acc_empty[acc], (acc_round - 1) & 1, p.status);
-        if (!ok) break;
+        if (acc_round > 0) mbar_wait_warp(&acc_empty[acc], (acc_round - 1) & 1, p.status, limit);
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + acc * ACC_COLS;
-        for (int kb = 0; kb < num_kb && ok; ++kb, ++it) {
+        for (int kb = 0; kb < num_kb; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t round = it / STAGES;
-          ok = mbar_wait(&full_bar[s], round & 1, p.status);
-          if (!ok) break;
+          mbar_wait_warp(&full_bar[s], round & 1, p.status, limit);
           tc_fence_after();
           const uint32_t a_addr = smem_u32(smem + s * S::STAGE_BYTES);
           const uint32_t b_addr = a_addr + S::A_BYTES;
           const uint64_t adesc = make_smem_desc(a_addr);
           const uint64_t bdesc = make_smem_desc(b_addr);
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < TC_BK / TC_UMMA_K; ++k)
-            umma_bf16_pair(tmem_d, adesc + (uint64_t)(k * 2), bdesc + (uint64_t)(k * 2), idesc,
-                           (kb > 0 || k > 0) ? 1u : 0u);
-          umma_commit_pair(&empty_bar[s], 3);       // both CTAs may refill the stage
+            for (int k = 0; k < TC_BK / TC_UMMA_K; ++k)
+              umma_bf16_pair(tmem_d, adesc + (uint64_t)(k * 2), bdesc + (uint64_t)(k * 2), idesc,
+                             (kb > 0 || k > 0) ? 1u : 0u);
+            umma_commit_pair(&empty_bar[s], 3);     // both CTAs may refill the stage
+          }
+          __syncwarp();
         }
-        umma_commit_pair(&acc_full[acc], 3);        // both CTAs' epilogues may read
+        if (elect_one()) umma_commit_pair(&acc_full[acc], 3);      // both CTAs' epilogues may read
+        __syncwarp();
       }
     }
   } else if (warp >= 4) {
@@ -949,26 +951,27 @@ linear_tcgen05_cluster_kernel(const __grid_constant__ CUtensorMap map_a,
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ---------------- MMA issuer
-      constexpr uint32_t idesc = make_idesc(TC_BM, CL_BN);
-      bool ok = true;
-      for (int kb = kb0, it = 0; kb < kb1 && ok; ++kb, ++it) {
-        const int s = it % CL_STAGES;
-        ok = mbar_wait(&full_bar[s], (it / CL_STAGES) & 1, p.status);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t a_addr = smem_u32(smem + s * S::STAGE_BYTES);
-        const uint64_t adesc = make_smem_desc(a_addr);
-        const uint64_t bdesc = make_smem_desc(a_addr + S::A_BYTES);
+    // ---------------- MMA issuer
+    constexpr uint32_t idesc = make_idesc(TC_BM, CL_BN);
+    uint32_t limit = HS_SPIN_LIMIT;
+    for (int kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
+      const int s = it % CL_STAGES;
+      mbar_wait_warp(&full_bar[s], (it / CL_STAGES) & 1, p.status, limit);
+      tc_fence_after();
+      const uint32_t a_addr = smem_u32(smem + s * S::STAGE_BYTES);
+      const uint64_t adesc = make_smem_desc(a_addr);
+      const uint64_t bdesc = make_smem_desc(a_addr + S::A_BYTES);
+      if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < TC_BK / TC_UMMA_K; ++k)
           umma_bf16(tmem_base, adesc + (uint64_t)(k * 2), bdesc + (uint64_t)(k * 2), idesc,
                     (kb > kb0 || k > 0) ? 1u : 0u);
         umma_commit(&empty_bar[s]);
       }
-      umma_commit(acc_full);            // the partial tile is complete (or the pipeline gave up)
+      __syncwarp();
     }
+    if (elect_one()) umma_commit(acc_full);   // the partial tile is complete (or the pipeline gave up)
+    __syncwarp();
   }
 
   // rows of the tile that exist, dealt to the CTAs of the cluster in blocks of `rpo`

@@ -136,24 +136,22 @@ moe_tiles_tc_kernel(const __grid_constant__ CUtensorMap map_w0,
       }
     }
   } else if (warp == MMA_WARP) {
-    if (lane == 0) {
-      bool ok = true;
-      int s = 0, round = 0, wi = 0;
-      for (int w = blockIdx.x; w < n_items && ok; w += gridDim.x, ++wi) {
-        const int rows = p.tiles[4 + 3 * (w / p.f_tiles)];
-        const uint32_t idesc = make_idesc(MT_BM, (rows + 15) & ~15);
-        const int acc = wi % NACC, acc_round = wi / NACC;
-        if (acc_round > 0) ok = mbar_wait(&acc_empty[acc], (acc_round - 1) & 1, p.status);
-        if (!ok) break;
+    uint32_t limit = HS_SPIN_LIMIT;
+    int s = 0, round = 0, wi = 0;
+    for (int w = blockIdx.x; w < n_items; w += gridDim.x, ++wi) {
+      const int rows = p.tiles[4 + 3 * (w / p.f_tiles)];
+      const uint32_t idesc = make_idesc(MT_BM, (rows + 15) & ~15);
+      const int acc = wi % NACC, acc_round = wi / NACC;
+      if (acc_round > 0) mbar_wait_warp(&acc_empty[acc], (acc_round - 1) & 1, p.status, limit);
+      tc_fence_after();
+      const uint32_t d = tmem + acc * 256;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        mbar_wait_warp(&full_bar[s], round & 1, p.status, limit);
+        if (GATHER) fence_proxy_async();     // rows the loading threads' copies wrote
         tc_fence_after();
-        const uint32_t d = tmem + acc * 256;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          ok = mbar_wait(&full_bar[s], round & 1, p.status);
-          if (!ok) break;
-          if (GATHER) fence_proxy_async();     // rows the loading threads' copies wrote
-          tc_fence_after();
-          const uint32_t base = smem_u32(smem + s * stage_bytes);
-          const uint64_t wdesc = make_smem_desc(base), bdesc = make_smem_desc(base + NB * W_BYTES);
+        const uint32_t base = smem_u32(smem + s * stage_bytes);
+        const uint64_t wdesc = make_smem_desc(base), bdesc = make_smem_desc(base + NB * W_BYTES);
+        if (elect_one()) {
 #pragma unroll
           for (int k = 0; k < MT_BK / 16; ++k) {
             const uint32_t more = (kb > 0 || k > 0) ? 1u : 0u;
@@ -161,10 +159,12 @@ moe_tiles_tc_kernel(const __grid_constant__ CUtensorMap map_w0,
             if (NB == 2) umma_bf16(d + 256, wdesc + (W_BYTES >> 4) + 2 * k, bdesc + 2 * k, idesc, more);
           }
           umma_commit(&empty_bar[s]);
-          if (++s == stages) { s = 0; ++round; }
         }
-        umma_commit(&acc_full[acc]);
+        __syncwarp();
+        if (++s == stages) { s = 0; ++round; }
       }
+      if (elect_one()) umma_commit(&acc_full[acc]);
+      __syncwarp();
     }
   } else if (GATHER && warp >= MT_EPI_WARPS) {
     // a piece of 16 bytes is column c of its row, rows r0, r0 + 16, ..; a row beyond the segment, and

@@ -89,6 +89,27 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint6
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// The same wait by a whole warp whose loop goes on either way (the lanes could differ in who saw the limit):
+// `limit` starts at HS_SPIN_LIMIT and is 1 once a wait has run out.  The status bit says that no result is
+// to be trusted.
+__device__ __forceinline__ void mbar_wait_warp(uint64_t* bar, uint32_t parity, int* status, uint32_t& limit) {
+  if (!mbar_wait(bar, parity, status, limit)) limit = 1;
+}
+// True in one lane of a whole warp, the same at every call.  A warp that issues MMAs walks its loop with all
+// lanes and elects one around the instructions alone: descriptors are then formed in uniform registers.
+// With a loop for a single lane they are moved there for every instruction, 66 cycles an MMA whatever its
+// width (2,048 x 1,024 x 4,096 in 128 x 128 tiles: 22.4 us so, 20.3 with the elected lane; a vote on the wait 21.3, one lane waiting for the others 21.9).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "elect.sync _|p, 0xffffffff;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(p));
+  return p != 0;
+}
 // Arrives on the mbarrier once every MMA issued so far by this thread has completed.
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
