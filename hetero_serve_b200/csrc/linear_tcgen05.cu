@@ -713,6 +713,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 linear_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a,
                            const __grid_constant__ CUtensorMap map_w, const TcParams p) {
   using S = PairSmem<BN, STAGES>;
+  constexpr int PER = 2, RING = STAGES / PER;           // k blocks a barrier round, as above
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* full_bar = (uint64_t*)(smem + S::BAR_OFFSET);
@@ -731,7 +732,7 @@ linear_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a,
 
   pdl_trigger();
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < RING; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
     }
@@ -750,6 +751,20 @@ linear_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a,
   cluster_sync();          // both CTAs' barriers exist before either signals the other's
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // as above: the weights of the first rounds are on their way before the kernel before has ended
+  int pre = 0;
+  if (threadIdx.x == 0 && pair < n_items) {
+    const int n0 = (pair % p.tiles_n) * BN + (int)rank * (BN / 2);
+    pre = min(RING, (num_kb + PER - 1) / PER);
+    for (int i = 0; i < pre; ++i) {
+      const int here = min(PER, num_kb - i * PER);
+      if (rank == 0) mbar_expect_tx(&full_bar[i], here * 2 * S::STAGE_BYTES);
+      const uint32_t bar = cluster_map(&full_bar[i], 0);
+      for (int j = 0; j < here; ++j)
+        tma_load_2d_pair(smem + (i * PER + j) * S::STAGE_BYTES + S::A_BYTES, &map_w, bar, (i * PER + j) * TC_BK,
+                         n0);
+    }
+  }
   pdl_wait();
 
   if (warp == 0) {
@@ -760,17 +775,22 @@ linear_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       for (int w = pair; w < n_items && ok; w += n_pairs) {
         const int m0 = (w / p.tiles_n) * (2 * TC_BM) + (int)rank * TC_BM;
         const int n0 = (w % p.tiles_n) * BN + (int)rank * (BN / 2);
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t round = it / STAGES;
+        for (int kb = 0; kb < num_kb; kb += PER, ++it) {
+          const int s = it % RING;
+          const uint32_t round = it / RING;
+          const int here = min(PER, num_kb - kb);
           if (round > 0) ok = mbar_wait(&empty_bar[s], (round - 1) & 1, p.status);
           if (!ok) break;
-          uint8_t* a_dst = smem + s * S::STAGE_BYTES;
-          uint8_t* b_dst = a_dst + S::A_BYTES;
-          if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * S::STAGE_BYTES);
+          const bool fresh = (int)it >= pre;
+          if (rank == 0 && fresh) mbar_expect_tx(&full_bar[s], here * 2 * S::STAGE_BYTES);
           const uint32_t bar = cluster_map(&full_bar[s], 0);
-          tma_load_2d_pair(a_dst, &map_a, bar, kb * TC_BK, m0);
-          tma_load_2d_pair(b_dst, &map_w, bar, kb * TC_BK, n0);
+#pragma unroll
+          for (int j = 0; j < PER; ++j)
+            if (j < here) {
+              uint8_t* a_dst = smem + (s * PER + j) * S::STAGE_BYTES;
+              if (fresh) tma_load_2d_pair(a_dst + S::A_BYTES, &map_w, bar, (kb + j) * TC_BK, n0);
+              tma_load_2d_pair(a_dst, &map_a, bar, (kb + j) * TC_BK, m0);
+            }
         }
       }
     }
@@ -785,20 +805,25 @@ linear_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a,
         if (acc_round > 0) mbar_wait_warp(&acc_empty[acc], (acc_round - 1) & 1, p.status, limit);
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + acc * ACC_COLS;
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t round = it / STAGES;
+        for (int kb = 0; kb < num_kb; kb += PER, ++it) {
+          const int s = it % RING;
+          const uint32_t round = it / RING;
+          const int here = min(PER, num_kb - kb);
           mbar_wait_warp(&full_bar[s], round & 1, p.status, limit);
           tc_fence_after();
-          const uint32_t a_addr = smem_u32(smem + s * S::STAGE_BYTES);
-          const uint32_t b_addr = a_addr + S::A_BYTES;
+          const uint32_t a_addr = smem_u32(smem + s * PER * S::STAGE_BYTES);
           const uint64_t adesc = make_smem_desc(a_addr);
-          const uint64_t bdesc = make_smem_desc(b_addr);
+          const uint64_t bdesc = make_smem_desc(a_addr + S::A_BYTES);
           if (elect_one()) {
 #pragma unroll
-            for (int k = 0; k < TC_BK / TC_UMMA_K; ++k)
-              umma_bf16_pair(tmem_d, adesc + (uint64_t)(k * 2), bdesc + (uint64_t)(k * 2), idesc,
-                             (kb > 0 || k > 0) ? 1u : 0u);
+            for (int j = 0; j < PER; ++j)
+              if (j < here) {
+                const uint64_t next = (uint64_t)(j * (S::STAGE_BYTES >> 4));
+#pragma unroll
+                for (int k = 0; k < TC_BK / TC_UMMA_K; ++k)
+                  umma_bf16_pair(tmem_d, adesc + next + (uint64_t)(k * 2), bdesc + next + (uint64_t)(k * 2),
+                                 idesc, (kb > 0 || j > 0 || k > 0) ? 1u : 0u);
+              }
             umma_commit_pair(&empty_bar[s], 3);     // both CTAs may refill the stage
           }
           __syncwarp();
@@ -1258,61 +1283,93 @@ static int cluster_capacity(int size) {
   return n;
 }
 
+// The most splits over k of `tiles` 64-column tiles that form clusters the device holds at once (0:
+// none).  A cluster that has to wait for the next round costs more than its splits save: of this kernel 74
+// clusters of two fit, 45 of three, 33 of four, 22 of six, 15 of eight, so 48 tiles take two splits and 16
+// tiles six.  Measured in a decode step of GPT-2 medium at batch 32: 1.23 ms, against 1.53 ms with the shares
+// going through scratch memory (3, 8, 2 and 8 splits).
+static int cluster_splits(int tiles, int num_kb, int sms) {
+  if (tiles * 2 > sms) return 0;
+  int most = sms / tiles, pick = 0;
+  if (most > num_kb / 2) most = num_kb / 2;
+  if (most > CL_MAX_SPLITS) most = CL_MAX_SPLITS;
+  for (int cand = 2; cand <= most; ++cand)
+    if (cluster_capacity(cand) >= tiles) pick = cand;
+  return pick;
+}
+
+// The tile of a layer of more than 128 rows: us a launch takes by rounds of tiles over the device and k
+// blocks, fitted to 70 shapes (512 to 4,096 rows, the layers of GPT-2 small to XL; off by 8 % rms, the choice
+// within 0.4 % of the best on average and 11 % at worst).  Pairs of CTAs load half a weight tile each; with two
+// k blocks a barrier round their 128-wide tiles are the cheapest per k block, alone (2,048 x 1,024 x 4,096: 19.0
+// us, 20.7 as single CTAs).  Behind another kernel a cluster starts later than single CTAs, which take each SM as
+// it falls free: a prompt layer with that shape takes 6 us more with pairs (109 and 102.5; 1,024 rows of width
+// 1,280 104.5 and 97.8), so 6 us are in their launch.
+struct TcShape {
+  int bn;
+  bool pair;
+  double launch, round, kb;
+};
+static const TcShape TC_SHAPES[] = {{64, false, 3.83, 0.363, 0.190},  {128, false, 5.32, 0.376, 0.229},
+                                    {192, false, 4.79, 0.234, 0.346}, {256, false, 5.84, 0.191, 0.371},
+                                    {128, true, 12.1, 0.626, 0.178},  {256, true, 13.7, 0.246, 0.309}};
+static TcShape pick_shape(int M, int N, int num_kb, int pair, int sms) {
+  TcShape best = TC_SHAPES[pair == 1 ? 4 : 0];
+  double least = -1.0;
+  for (const TcShape& s : TC_SHAPES) {
+    if (pair >= 0 && s.pair != (pair == 1)) continue;
+    if (s.bn > 64 && s.bn / 2 >= N && !(s.pair && s.bn == 128)) continue;
+    const int rows = s.pair ? 2 * TC_BM : TC_BM, units = s.pair ? (sms / 2 > 0 ? sms / 2 : 1) : sms;
+    const long long tiles = (long long)((M + rows - 1) / rows) * ((N + s.bn - 1) / s.bn);
+    double cost;
+    if (!s.pair && tiles * 2 <= sms) {
+      // a device left half empty is shared out over k: by clusters (64 columns), never better by scratch
+      if (s.bn != CL_BN) continue;
+      const int splits = g_split_clusters ? cluster_splits((int)tiles, num_kb, sms) : 0;
+      cost = s.launch + s.round + s.kb * (splits ? (num_kb + splits - 1) / splits : num_kb) + (splits ? 2.5 : 0.0);
+    } else {
+      cost = s.launch + (double)((tiles + units - 1) / units) * (s.round + s.kb * num_kb);
+    }
+    if (least < 0 || cost < least) {
+      least = cost;
+      best = s;
+    }
+  }
+  return best;
+}
+
 // pair: -1 = decide here, 0 = single CTAs, 1 = pairs of CTAs (256-row tiles)
 static bool plan_tc(int M, int N, int K, int tile_n, int pair, TcPlan& pl) {
   int sms = 148;
   sms = hs_sm_count();
   const int mt = (M + TC_BM - 1) / TC_BM;
   const int num_kb = (K + TC_BK - 1) / TC_BK;
-  // measured on B200: pairs gain 5-9 % from 4,096 rows on (4096^3, 8192^3) and nothing at 2,048
-  pl.pair = pair == 1 || (pair < 0 && M >= 4096);
   pl.cluster = false;
+  int bn = tile_n;
+  pl.pair = pair == 1 || (pair < 0 && tile_n != 0 && M >= 4096);
+  if (bn == 0 && (mt > 1 || pl.pair)) {
+    const TcShape shape = pick_shape(M, N, num_kb, pair, sms);
+    bn = shape.bn;
+    pl.pair = shape.pair;
+  } else if (bn == 0) {
+    // few rows: narrow tiles (more CTAs stream the weights) and splits; a very wide layer (the
+    // vocabulary) has tiles enough, and wide ones keep more of the weights on their way (50,257 columns,
+    // us at 64, 128, 192 and 256 wide: 32 x 1,024 37, 29, 26, 30; 17 x 1,600 65, 48, 36, 37; 64 x 768 28, 22,
+    // 21, 27)
+    bn = ((N + 63) / 64 >= 2 * sms) ? 192 : 64;
+  }
   if (pl.pair) {
     // 256 x BN tiles over sms / 2 pairs; a CTA loads 128 + BN/2 rows per k-block
     const int pairs = sms / 2 > 0 ? sms / 2 : 1;
-    const int mt2 = (M + 2 * TC_BM - 1) / (2 * TC_BM);
-    int bn = tile_n;
-    if (bn == 0) {
-      long best = -1;
-      for (int cand : {256, 128}) {
-        if (cand / 2 >= N && cand > 128) continue;
-        const long tiles = (long)mt2 * ((N + cand - 1) / cand);
-        const long cost = ((tiles + pairs - 1) / pairs) * (cand / 2 + 128 + 64);
-        if (best < 0 || cost < best) {
-          best = cost;
-          bn = cand;
-        }
-      }
-    }
     if (bn != 128 && bn != 256) return false;
     pl.bn = bn;
-    pl.tiles_m = mt2;
+    pl.tiles_m = (M + 2 * TC_BM - 1) / (2 * TC_BM);
     pl.tiles_n = (N + bn - 1) / bn;
     pl.splits = 1;
     pl.kb_per_split = num_kb;
     const int tiles = pl.tiles_m * pl.tiles_n;
     pl.grid = 2 * (tiles < pairs ? tiles : pairs);
     return true;
-  }
-  int bn = tile_n;
-  if (bn == 0) {
-    // A tile's time grows with the bytes it loads per k-block (128 + width rows) plus a fixed
-    // part; pick the width for which rounds over the SMs x that is smallest.
-    long best = -1;
-    for (int cand : {256, 192, 128, 64}) {
-      if (cand > 64 && cand / 2 >= N) continue;
-      const long tiles = (long)mt * ((N + cand - 1) / cand);
-      const long cost = ((tiles + sms - 1) / sms) * (cand + 128 + 64);
-      if (best < 0 || cost < best) {
-        best = cost;
-        bn = cand;
-      }
-    }
-    // few rows: narrow tiles (more CTAs stream the weights) and splits; a very wide layer (the
-    // vocabulary) has tiles enough, and wide ones keep more of the weights on their way (50,257 columns,
-    // us at 64, 128, 192 and 256 wide: 32 x 1,024 37, 29, 26, 30; 17 x 1,600 65, 48, 36, 37; 64 x 768 28, 22,
-    // 21, 27)
-    if (mt == 1) bn = ((N + 63) / 64 >= 2 * sms) ? 192 : 64;
   }
   if (bn != 64 && bn != 128 && bn != 192 && bn != 256) return false;
   pl.bn = bn;
@@ -1328,16 +1385,9 @@ static bool plan_tc(int M, int N, int K, int tile_n, int pair, TcPlan& pl) {
     if (splits < 1) splits = 1;
     if (splits > 16) splits = 16;
     // 64-column tiles split over k: the splits of a tile form a cluster, as many as the device
-    // holds at once for all tiles.  A cluster that has to wait for the next round costs more than
-    // its splits save: of this kernel 74 clusters of two fit, 45 of three, 33 of four, 22 of
-    // six, 15 of eight, so 48 tiles take two splits and 16 tiles six.  Measured in a decode
-    // step of GPT-2 medium at batch 32: 1.23 ms, against 1.53 ms with the shares going through
-    // scratch memory (3, 8, 2 and 8 splits).
+    // holds at once for all tiles
     if (g_split_clusters && bn == CL_BN) {
-      int pick = 0;
-      for (int cand = 2; cand <= splits && cand <= CL_MAX_SPLITS; ++cand)
-        if (cluster_capacity(cand) >= tiles) pick = cand;
-      if (pick) {
+      if (const int pick = cluster_splits(tiles, num_kb, sms)) {
         pl.cluster = true;
         splits = pick;
       }
