@@ -19,6 +19,8 @@
 // State of a slot: [heads x D x V | (taps-1) x channels] floats.
 #include "tcgen05.cuh"
 
+#include <type_traits>
+
 namespace hs {
 
 __device__ __forceinline__ float sigmoidf_(float z) { return 1.0f / (1.0f + expf(-z)); }
@@ -48,6 +50,8 @@ delta_prepare_kernel(float* __restrict__ qn, float* __restrict__ kn, float* __re
                      const int* __restrict__ req_slot, DeltaShape s,
                      const float* __restrict__ z_a) {
   extern __shared__ float s_c[];                 // [2 * kv_heads * D] q and k after conv and silu
+  pdl_trigger();
+  pdl_wait();
   const int t = blockIdx.x;
   const int r = tok_req[t];
   if (r < 0) return;
@@ -144,10 +148,146 @@ delta_prepare_kernel(float* __restrict__ qn, float* __restrict__ kn, float* __re
   }
 }
 
+// The same for prompts through four taps with heads of 32 to 128 key channels: a warp takes eight tokens of
+// one head's q or k, of 128 value channels or of 128 decays, lane l the channels l, l + 32, .. (the sums of the
+// kernel above, in its order: the same bits).  The eleven inputs of a channel are fetched once and slide
+// through registers, where a block a token reads every input four times.  Eight tokens that are not one
+// request's, or reach behind its portion, are taken one by one.  2,048 tokens of 3,072
+// channels and 1,024 decays: 39.6 us in blocks of a token, 29.8 so; exponentials and quotients issue for half of it.
+constexpr int DP_TOK = 8;
+
+__global__ void __launch_bounds__(128)
+delta_prepare_rows_kernel(float* __restrict__ qn, float* __restrict__ kn, float* __restrict__ vv,
+                          float* __restrict__ beta, float* __restrict__ decay,
+                          const float* __restrict__ proj, const float* __restrict__ conv_w,
+                          const float* __restrict__ a2, const float* __restrict__ dt_bias,
+                          const float* __restrict__ A_log, const float* __restrict__ state,
+                          const int* __restrict__ tok_req, const int* __restrict__ req_start,
+                          const int* __restrict__ req_slot, DeltaShape s,
+                          const float* __restrict__ z_a, int n_tokens) {
+  pdl_trigger();
+  pdl_wait();
+  const int lane = threadIdx.x & 31;
+  const int t0 = blockIdx.x * DP_TOK;
+  const int QK = s.kv_heads * s.D, HV = s.heads * s.V, HD = s.heads * s.D, C = channels(s);
+  const int v_groups = (HV + 127) / 128;
+  int g = blockIdx.y * 4 + (threadIdx.x >> 5);
+  const int mine = lane < DP_TOK && t0 + lane < n_tokens ? tok_req[t0 + lane] : -1;
+  const int here = min(DP_TOK, n_tokens - t0);
+  const unsigned live = __ballot_sync(0xffffffffu, mine >= 0);
+  if (g >= 2 * s.kv_heads + v_groups) {            // ---- decays
+    g -= 2 * s.kv_heads + v_groups;
+    for (int j = 0; j < 4; ++j) {
+      const int i = g * 128 + 32 * j + lane;
+      if (i >= HD) return;
+      const float bias = dt_bias[i], rate = -expf(A_log[i / s.D]);
+      float z[DP_TOK];
+#pragma unroll
+      for (int u = 0; u < DP_TOK; ++u) {
+        z[u] = 0.f;
+        if (u < here && z_a) z[u] = z_a[(size_t)(t0 + u) * HD + i];
+      }
+      if (!z_a)
+        for (int u = 0; u < here; ++u)
+#pragma unroll 8
+          for (int k = 0; k < s.ra; ++k)
+            z[u] = fmaf(a2[(size_t)k * HD + i], proj[(size_t)(t0 + u) * s.stride + s.a_off + k], z[u]);
+#pragma unroll
+      for (int u = 0; u < DP_TOK; ++u)
+        if (live >> u & 1)
+          decay[(size_t)(t0 + u) * HD + i] = expf(rate * softplusf_(z[u] + bias));
+    }
+    return;
+  }
+  const bool is_v = g >= 2 * s.kv_heads;
+  const int c0 = is_v ? 2 * QK + (g - 2 * s.kv_heads) * 128 : g * s.D;
+  const int nc = is_v ? min(128, 2 * QK + HV - c0) : s.D;
+  float w[4][4];                                   // [channel][tap]
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) w[j][k] = 32 * j + lane < nc ? conv_w[4 * (size_t)(c0 + 32 * j + lane) + k] : 0.f;
+  // what becomes of a token's convolved channels
+  auto finish = [&](int t, float (&x)[4]) {
+    if (is_v) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (32 * j + lane < nc) vv[(size_t)t * HV + c0 - 2 * QK + 32 * j + lane] = x[j];
+      return;
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (32 * j + lane < nc) ss = fmaf(x[j], x[j], ss);
+    ss = warp_sum(ss);
+    float inv = 1.0f / sqrtf(ss + 1e-6f);
+    const bool is_q = g < s.kv_heads;
+    if (is_q) inv *= 1.0f / sqrtf((float)s.D);
+    float* dst = (is_q ? qn : kn) + (size_t)t * QK + (size_t)(is_q ? g : g - s.kv_heads) * s.D;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (32 * j + lane < nc) dst[32 * j + lane] = x[j] * inv;
+  };
+  const int r0 = __shfl_sync(0xffffffffu, mine, 0);
+  const bool one = __all_sync(0xffffffffu, lane >= DP_TOK || mine == r0) && r0 >= 0;
+  if (one && t0 - req_start[r0] >= 3) {
+    float in[DP_TOK + 3][4];
+#pragma unroll
+    for (int m = 0; m < DP_TOK + 3; ++m)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        in[m][j] = 32 * j + lane < nc ? proj[(size_t)(t0 - 3 + m) * s.stride + c0 + 32 * j + lane] : 0.f;
+#pragma unroll
+    for (int u = 0; u < DP_TOK; ++u) {
+      float x[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float acc = fmaf(w[j][0], in[u][j], 0.f);
+#pragma unroll
+        for (int k = 1; k < 4; ++k) acc = fmaf(w[j][k], in[u + k][j], acc);
+        x[j] = acc * sigmoidf_(acc);
+      }
+      finish(t0 + u, x);
+    }
+  } else {
+    for (int u = 0; u < here; ++u) {
+      const int t = t0 + u, r = __shfl_sync(0xffffffffu, mine, u);
+      if (r < 0) continue;
+      const int first = req_start[r], l = t - first;
+      const float* cst = state + (size_t)req_slot[r] * s.state_stride + (size_t)s.heads * s.D * s.V;
+      float x[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int c = c0 + 32 * j + lane;
+        float acc = 0.f;
+        if (32 * j + lane < nc) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int local = l - (3 - k);
+            const float in = local >= 0 ? proj[(size_t)(first + local) * s.stride + c]
+                                        : cst[(size_t)(local + 3) * C + c];
+            acc = fmaf(w[j][k], in, acc);
+          }
+        }
+        x[j] = acc * sigmoidf_(acc);
+      }
+      finish(t, x);
+    }
+  }
+  if (g == 2 * s.kv_heads)
+    for (int i = lane; i < here * s.heads; i += 32) {
+      const int u = i / s.heads, h = i - u * s.heads;
+      if (tok_req[t0 + u] >= 0)
+        beta[(size_t)(t0 + u) * s.heads + h] = sigmoidf_(proj[(size_t)(t0 + u) * s.stride + s.b_off + h]);
+    }
+}
+
 __global__ void delta_conv_state_kernel(float* __restrict__ state, const float* __restrict__ proj,
                                         const int* __restrict__ req_start,
                                         const int* __restrict__ req_len,
                                         const int* __restrict__ req_slot, DeltaShape s) {
+  pdl_trigger();
+  pdl_wait();
   const int r = blockIdx.y;
   const int n = req_len[r];
   if (n <= 0) return;
@@ -403,6 +543,8 @@ delta_blocks_prepare_kernel(float* __restrict__ blocks, const float* __restrict_
                             const int* __restrict__ req_len, int n_requests, int cap_blocks,
                             DeltaShape s, int long_from) {
   __shared__ float red[4][16];
+  pdl_trigger();
+  pdl_wait();
   const int h = blockIdx.y;
   int before;                                      // the request this block of tokens belongs to
   const int r = db_request(req_len, n_requests, long_from, blockIdx.x, true, &before);
@@ -515,6 +657,8 @@ delta_blocks_kernel(float* __restrict__ o, float* __restrict__ state,
   extern __shared__ __align__(16) float sm[];                  // [stages][blocks of a stage][SZ]
   __shared__ float s_v[DB_STAGES][ST_TOK][CTA_COLS];
   __shared__ uint64_t full[DB_STAGES], empty[DB_STAGES];
+  pdl_trigger();
+  pdl_wait();
   const int h = blockIdx.y;
   int before;                                      // (there may be fewer long requests than blocks)
   const int r = db_request(req_len, n_requests, long_from, blockIdx.x, false, &before);
@@ -683,6 +827,39 @@ delta_blocks_kernel(float* __restrict__ o, float* __restrict__ state,
 
 // One block per token and head: the head's root mean square by a block reduction, then one
 // thread per output forms its gate (a sum over the rg inputs, several loads in flight).
+// The same where W_g2 g was formed as a matrix product and a head has 32 to 256 values, a multiple of 32: a
+// warp a token and head, its sums those of the four warps of a block below (the same bits).  2,048 tokens, 8
+// heads of 128: 21 us in blocks a token and head, 9.7 so.
+template <typename TO>
+__global__ void __launch_bounds__(256)
+delta_finish_rows_kernel(TO* __restrict__ out, const float* __restrict__ o,
+                         const float* __restrict__ norm_w, const int* __restrict__ tok_req, float eps,
+                         DeltaShape s, const float* __restrict__ z_g, int n_tokens) {
+  pdl_trigger();
+  pdl_wait();
+  const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int t = i / s.heads, h = i - t * s.heads;
+  if (t >= n_tokens || tok_req[t] < 0) return;
+  const size_t at = ((size_t)t * s.heads + h) * s.V;
+  constexpr int N = 8;
+  float x[N], z[N];
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    const int e = 32 * j + lane;
+    x[j] = e < s.V ? o[at + e] : 0.f;
+    z[j] = e < s.V ? z_g[at + e] : 0.f;
+  }
+  float tot = 0.f;
+#pragma unroll
+  for (int w = 0; w < 4; ++w) tot += warp_sum(fmaf(x[w + 4], x[w + 4], fmaf(x[w], x[w], 0.f)));
+  const float inv = 1.0f / sqrtf(tot / (float)s.V + eps);
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    const int e = 32 * j + lane;
+    if (e < s.V) out[at + e] = from_f<TO>(x[j] * inv * norm_w[e] * sigmoidf_(z[j]));
+  }
+}
+
 template <typename TO>
 __global__ void __launch_bounds__(128)
 delta_finish_kernel(TO* __restrict__ out, const float* __restrict__ o,
@@ -691,6 +868,8 @@ delta_finish_kernel(TO* __restrict__ out, const float* __restrict__ o,
                     float eps, DeltaShape s, const float* __restrict__ z_g) {
   __shared__ float red[4];
   extern __shared__ float s_gin[];                  // [rg]
+  pdl_trigger();
+  pdl_wait();
   const int t = blockIdx.x, h = blockIdx.y;
   if (tok_req[t] < 0) return;
   const int HV = s.heads * s.V;
@@ -756,16 +935,26 @@ HS_EXPORT int hs_delta_prepare(float* qn, float* kn, float* vv, float* beta, flo
   cudaStream_t st = (cudaStream_t)stream;
   const int widest = 2 * kv_heads * D > heads * V ? 2 * kv_heads * D : heads * V;
   const bool four = taps == 4 && widest > 512 && n_tokens >= 512 && n_tokens >= 8 * n_requests;
-  auto* prepare = four ? hs::delta_prepare_kernel<true> : hs::delta_prepare_kernel<false>;
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(prepare, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  prepare<<<dim3(n_tokens, 3), 256, smem, st>>>(qn, kn, vv, beta, decay, proj, conv_w, a2, dt_bias, A_log,
-                                                state, tok_req, req_start, req_slot, s, z_a);
-  HS_LAUNCH_CHECK();
+  const bool pdl = hs_pdl_enabled();
+  cudaError_t e;
+  if (four && D % 32 == 0 && D <= 128) {
+    const int groups = 2 * kv_heads + (heads * V + 127) / 128 + (heads * D + 127) / 128;
+    e = hs_launch(hs::delta_prepare_rows_kernel, dim3((n_tokens + hs::DP_TOK - 1) / hs::DP_TOK, (groups + 3) / 4),
+                  dim3(128), 0, st, pdl, qn, kn, vv, beta, decay, proj, conv_w, a2, dt_bias, A_log,
+                  (const float*)state, tok_req, req_start, req_slot, s, z_a, n_tokens);
+  } else {
+    auto* prepare = four ? hs::delta_prepare_kernel<true> : hs::delta_prepare_kernel<false>;
+    if (smem > 48 * 1024)
+      cudaFuncSetAttribute(prepare, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = hs_launch(prepare, dim3(n_tokens, 3), dim3(256), smem, st, pdl, qn, kn, vv, beta, decay, proj, conv_w, a2,
+                  dt_bias, A_log, (const float*)state, tok_req, req_start, req_slot, s, z_a);
+  }
+  if (e != cudaSuccess) return (int)e;
   if (taps > 1) {
     dim3 grid((C + 127) / 128, n_requests);
-    hs::delta_conv_state_kernel<<<grid, 128, 0, st>>>(state, proj, req_start, req_len, req_slot, s);
-    HS_LAUNCH_CHECK();
+    e = hs_launch(hs::delta_conv_state_kernel, grid, dim3(128), 0, st, pdl, state, proj, req_start, req_len,
+                  req_slot, s);
+    if (e != cudaSuccess) return (int)e;
   }
   return HS_OK;
 }
@@ -832,10 +1021,10 @@ HS_EXPORT int hs_delta_recurrence(float* o, float* state, const float* qn, const
   if (!with_blocks) return HS_OK;
   const int most = delta_most_long(n_tokens, n_requests, long_from);
   const int cap = delta_blocks_cap(n_tokens, n_requests, long_from);
-  hs::delta_blocks_prepare_kernel<<<dim3(cap, heads), 128, 0, st>>>(
-      blocks, qn, kn, beta, decay, req_start, req_len, n_requests, cap, s, long_from);
-  HS_LAUNCH_CHECK();
-  cudaError_t e = cudaSuccess;
+  cudaError_t e = hs_launch(hs::delta_blocks_prepare_kernel, dim3(cap, heads), dim3(128), 0, st,
+                            hs_pdl_enabled(), blocks, qn, kn, beta, decay, req_start, req_len, n_requests, cap,
+                            s, long_from);
+  if (e != cudaSuccess) return (int)e;
   const size_t block_smem =
       (size_t)hs::DB_STAGES * hs::DB_STAGE_BLOCKS * hs::db_floats(D) * sizeof(float);
 #define HS_DB(KS)                                                                                 \
@@ -844,10 +1033,11 @@ HS_EXPORT int hs_delta_recurrence(float* o, float* state, const float* qn, const
     e = cudaFuncSetAttribute(hs::delta_blocks_kernel<KS>,                                         \
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)block_smem);       \
     if (e == cudaSuccess)                                                                         \
-      hs::delta_blocks_kernel<KS><<<dim3(most, heads, (V + block_cols - 1) / block_cols),         \
-                                    hs::DB_WARPS * 32 + 32, block_smem, st>>>(                    \
-          o, state, blocks, vv, req_start, req_len, req_slot, n_requests, cap, s, long_from,      \
-          status);                                                                                \
+      e = hs_launch(hs::delta_blocks_kernel<KS>,                                                  \
+                    dim3(most, heads, (V + block_cols - 1) / block_cols),                         \
+                    dim3(hs::DB_WARPS * 32 + 32), block_smem, st, hs_pdl_enabled(), o, state,     \
+                    (const float*)blocks, vv, req_start, req_len, req_slot, n_requests, cap, s,   \
+                    long_from, status);                                                           \
   } while (0)
   if (D == 64) HS_DB(4);
   else if (D == 128) HS_DB(8);
@@ -868,14 +1058,20 @@ HS_EXPORT int hs_delta_finish(void* out, const float* o, const float* proj, cons
   if (rc) return rc;
   if (n_tokens <= 0) return HS_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  if (out_dtype == HS_DT_F32)
-    hs::delta_finish_kernel<float><<<dim3(n_tokens, heads), 128, rg * sizeof(float), st>>>(
-        (float*)out, o, proj, g2, norm_w, tok_req, eps, s, z_g);
-  else if (out_dtype == HS_DT_BF16)
-    hs::delta_finish_kernel<__nv_bfloat16><<<dim3(n_tokens, heads), 128, rg * sizeof(float), st>>>(
-        (__nv_bfloat16*)out, o, proj, g2, norm_w, tok_req, eps, s, z_g);
-  else
-    return HS_ERR_UNSUPPORTED;
-  HS_LAUNCH_CHECK();
-  return HS_OK;
+  const bool pdl = hs_pdl_enabled();
+  cudaError_t e;
+  auto go = [&](auto* dst) {
+    using TO = std::remove_pointer_t<decltype(dst)>;
+    if (z_g && V % 32 == 0 && V <= 256)
+      e = hs_launch(hs::delta_finish_rows_kernel<TO>, dim3(((long long)n_tokens * heads + 7) / 8), dim3(256), 0,
+                    st, pdl, dst, o, norm_w, tok_req, eps, s, z_g, n_tokens);
+    else
+      e = hs_launch(hs::delta_finish_kernel<TO>, dim3(n_tokens, heads), dim3(128), rg * sizeof(float), st, pdl,
+                    dst, o, proj, g2, norm_w, tok_req, eps, s, z_g);
+  };
+  if (out_dtype == HS_DT_F32) go((float*)out);
+  else if (out_dtype == HS_DT_BF16) go((__nv_bfloat16*)out);
+  else return HS_ERR_UNSUPPORTED;
+  return e == cudaSuccess ? HS_OK : (int)e;
 }
+
