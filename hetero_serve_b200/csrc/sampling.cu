@@ -543,6 +543,406 @@ sample_smem_kernel(int* __restrict__ out, const float* __restrict__ logits,
   }
 }
 
+// ---- a row over a cluster of eight blocks ------------------------------------------------------
+// The same rule, decision for decision and sum for sum, for long rows: block c of the cluster does the work
+// of threads 128 c .. 128 c + 127 of the kernel above and holds their positions.  Maxima, histograms and the
+// warps' sums meet in shared memory of the cluster; the sums of a thread, of a warp and over the warps are
+// formed in the order above, so the tokens are the same ones.  Of the maxima of each block's 64 groups of four
+// threads the (k/8)-th largest is found by counting; the smallest of these eight bounds the k largest entries
+// from below (there are k maxima, so k entries, from it up).  The entries from it up are listed, every block
+// gathers all lists and counts again; where they are too many, and for k above 256, the threshold is found a
+// digit of eight bits at a time with histograms that meet in the cluster.  One block a row leaves most SMs idle at the batches that
+// sample, and its 50,257 exponentials and quotients take one SM 20 us.  us, a block
+// a row against a cluster, without top-k, k = 40, k = 2,000 and greedy: 32 x 50,257 22.8 and 13.7, 29.1 and
+// 16.5, 45.6 and 27.1, 7.9 and 5.1; 64 x 32,000 16.6 and 13.6, 22.1 and 17.9, 32.8 and 27.8, 5.4 and 4.9.  Shorter
+// rows and larger batches gain nothing: 64 x 16,384 10.2 and 10.8, 128 x 32,000 16.6 and 20.3.
+constexpr int SC_BLOCKS = 8, SC_THREADS = 256, SC_OWN = 128;   // of a cluster; a block; positions' owners
+constexpr int SC_GROUPS = SC_THREADS / 4, SC_LIST_K = 256;      // maxima of a block; the largest k that lists
+constexpr int SC_LIST = 512, SC_CAND = 1024;                   // entries a block may list, a cluster
+constexpr int SC_VOCAB = 24576, SC_ROWS = 64;                  // the shortest row, the most rows
+
+__device__ __forceinline__ uint32_t sc_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void sc_sync() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t sc_addr(const void* p, int rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+               : "=r"(r) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ int sc_read(const int* p, int rank) {
+  int v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(sc_addr(p, rank)) : "memory");
+  return v;
+}
+__device__ __forceinline__ float sc_read(const float* p, int rank) {
+  return __int_as_float(sc_read((const int*)p, rank));
+}
+__device__ __forceinline__ void sc_write(int* p, int rank, int v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(sc_addr(p, rank)), "r"(v) : "memory");
+}
+
+// how many of n keys (a multiple of four) are larger than `key`, and how many equal to it
+__device__ __forceinline__ int2 sc_rank_of(uint32_t key, const uint32_t* keys, int n) {
+  int2 r = make_int2(0, 0);
+#pragma unroll 4
+  for (int i = 0; i < n; i += 4) {
+    const uint4 x = *(const uint4*)(keys + i);
+    r.x += (x.x > key) + (x.y > key) + (x.z > key) + (x.w > key);
+    r.y += (x.x == key) + (x.y == key) + (x.z == key) + (x.w == key);
+  }
+  return r;
+}
+
+__global__ void __launch_bounds__(SC_THREADS)
+sample_cluster_kernel(int* __restrict__ out, const float* __restrict__ logits,
+                      const float* __restrict__ temperature, const int* __restrict__ top_k,
+                      const int* __restrict__ seed_lo, const int* __restrict__ seed_hi,
+                      const int* __restrict__ position, int rows, int vocab, int* __restrict__ feedback,
+                      const int* __restrict__ feedback_slot, const int* __restrict__ status_word) {
+  extern __shared__ float s_row[];                  // [SC_OWN * C]: logits, then weights (-1: dropped)
+  __shared__ int hist[2][256], s_tot[256];
+  __shared__ __align__(16) uint32_t s_key[SC_GROUPS], s_list[SC_LIST], s_cand[SC_CAND];
+  __shared__ int s_digit, s_above, s_same, s_count, s_found, s_last, s_bound, s_n;
+  __shared__ float s_max[SC_THREADS / 32], s_own, s_sum[SC_OWN / 32], s_warps[32];
+  __shared__ int s_eq[SC_OWN / 32];
+  __shared__ int s_v[32], s_i[32];                  // block 0: what the others hand over
+  const int rank = (int)sc_rank(), rowi = blockIdx.x / SC_BLOCKS;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const float* row = logits + (size_t)rowi * vocab;
+  pdl_trigger();
+  const float temp = temperature[rowi];
+  const int fb = (feedback != nullptr && feedback_slot != nullptr) ? feedback_slot[rowi] : -1;
+  pdl_wait();                       // the logits are what the previous kernel wrote
+  if (status_word != nullptr && blockIdx.x == 0 && tid == 0) out[rows] = *status_word;
+  if (tid == 0) {
+    s_found = 0x7fffffff;
+    s_last = s_n = s_bound = 0;
+  }
+  if (!(temp > 0.f)) {              // (the same for the whole cluster) block_argmax over its 1,024 threads
+    ArgMax best{-INFINITY, 0x7fffffff};
+    if (tid < SC_OWN) {
+      constexpr int INFLIGHT = 16;
+      const int t = rank * SC_OWN + tid;
+      for (int base = t; base < vocab; base += INFLIGHT * SS_THREADS) {
+        float v[INFLIGHT];
+#pragma unroll
+        for (int j = 0; j < INFLIGHT; ++j) {
+          const int i = base + j * SS_THREADS;
+          v[j] = i < vocab ? row[i] : -INFINITY;
+        }
+#pragma unroll
+        for (int j = 0; j < INFLIGHT; ++j) {
+          const int i = base + j * SS_THREADS;
+          if (i < vocab && (v[j] > best.v || best.i == 0x7fffffff)) best = ArgMax{v[j], i};
+        }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        ArgMax other{__shfl_xor_sync(0xffffffffu, best.v, o), __shfl_xor_sync(0xffffffffu, best.i, o)};
+        best = better(best, other);
+      }
+    }
+    sc_sync();                      // block 0 has started: its memory may be written
+    if (tid < SC_OWN && lane == 0) {
+      sc_write(&s_v[rank * 4 + warp], 0, __float_as_int(best.v));
+      sc_write(&s_i[rank * 4 + warp], 0, best.i);
+    }
+    sc_sync();
+    if (rank == 0 && tid == 0) {
+      ArgMax b{__int_as_float(s_v[0]), s_i[0]};
+      for (int w = 1; w < 32; ++w) b = better(b, ArgMax{__int_as_float(s_v[w]), s_i[w]});
+      if (b.i == 0x7fffffff) b.i = 0;
+      out[rowi] = b.i;
+      if (fb >= 0) feedback[fb] = b.i;
+    }
+    return;
+  }
+
+  const int C = ((vocab + SS_THREADS - 1) / SS_THREADS) | 1;
+  const int from = min(vocab, rank * SC_OWN * C), size = min(vocab, (rank + 1) * SC_OWN * C) - from;
+  float m = -INFINITY;
+#pragma unroll 16
+  for (int i = tid; i < size; i += SC_THREADS) {
+    const float v = row[from + i];
+    s_row[i] = v;
+    m = fmaxf(m, v);
+  }
+  const int k = top_k[rowi];
+  const bool use_k = k > 0 && k < vocab;
+  {
+    uint32_t key = tid < size ? order_key(m) : 0u;
+    key = max(key, __shfl_xor_sync(0xffffffffu, key, 1));
+    key = max(key, __shfl_xor_sync(0xffffffffu, key, 2));
+    if ((tid & 3) == 0) s_key[tid >> 2] = key;
+    const float w = warp_max(m);
+    if (lane == 0) s_max[warp] = w;
+    __syncthreads();
+    if (tid == 0) {
+      float b = s_max[0];
+      for (int i = 1; i < SC_THREADS / 32; ++i) b = fmaxf(b, s_max[i]);
+      s_own = b;
+    }
+  }
+  const int share = (k + SC_BLOCKS - 1) / SC_BLOCKS;     // of the k maxima this block answers for
+  if (use_k && k <= SC_LIST_K && tid < SC_GROUPS) {
+    const int2 n = sc_rank_of(s_key[tid], s_key, SC_GROUPS);
+    if (n.x < share && share <= n.x + n.y) s_bound = (int)s_key[tid];
+  }
+  sc_sync();
+  float top = lane < SC_BLOCKS ? sc_read(&s_own, lane) : -INFINITY;
+  top = warp_max(top);
+  const float mx = top / temp;
+  uint32_t thr = 0;     // order key of the k-th largest logit; 0 keeps everything
+  int need_eq = 0;      // how many entries equal to the threshold are kept (lowest indices)
+  bool all_eq = true;   // ... which is all of them
+  uint32_t bound = 0;
+  bool listed = false;
+  if (use_k && k <= SC_LIST_K) {
+    {
+      uint32_t b = lane < SC_BLOCKS ? (uint32_t)sc_read(&s_bound, lane) : 0xffffffffu;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) b = min(b, __shfl_xor_sync(0xffffffffu, b, o));
+      bound = b;
+#pragma unroll 4
+      for (int i = tid; i < size; i += SC_THREADS) {
+        const uint32_t key = order_key(s_row[i]);
+        if (key >= bound) {
+          const int at = atomicAdd(&s_n, 1);
+          if (at < SC_LIST) s_list[at] = key;
+        }
+      }
+      sc_sync();
+      const int own = lane < SC_BLOCKS ? sc_read(&s_n, lane) : 0;      // of block `lane`
+      listed = __all_sync(0xffffffffu, own <= SC_LIST);
+      int incl = own;                                    // entries of the blocks up to it
+#pragma unroll
+      for (int o = 1; o < SC_BLOCKS; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += u;
+      }
+      const int n = __shfl_sync(0xffffffffu, incl, SC_BLOCKS - 1);
+      listed = listed && n >= k && n <= SC_CAND;
+      if (listed) {
+        for (int i0 = warp * 32; i0 < n; i0 += SC_THREADS) {
+          const int i = i0 + lane;
+          int c = 0, first = 0;
+#pragma unroll
+          for (int b = 0; b < SC_BLOCKS - 1; ++b) {
+            const int end = __shfl_sync(0xffffffffu, incl, b);
+            if (i >= end) { c = b + 1; first = end; }
+          }
+          if (i < n) s_cand[i] = (uint32_t)sc_read((const int*)&s_list[i - first], c);
+        }
+        for (int i = n + tid; i < ((n + 3) & ~3); i += SC_THREADS) s_cand[i] = 0;   // (no entry's key)
+        __syncthreads();
+        for (int i = tid; i < n; i += SC_THREADS) {
+          const int2 r = sc_rank_of(s_cand[i], s_cand, (n + 3) & ~3);
+          if (r.x < k && k <= r.x + r.y) {               // the same for all entries equal to it
+            s_tot[0] = (int)s_cand[i];
+            s_tot[1] = r.x;
+            s_tot[2] = r.y;
+          }
+        }
+        __syncthreads();
+        thr = (uint32_t)s_tot[0];
+        need_eq = k - s_tot[1];
+        all_eq = s_tot[2] == need_eq;
+      }
+    }
+  }
+  if (use_k && !listed) {
+    int turn = 0, remaining = 0;
+    // the want-th largest of the keys that the blocks' walks hand on; false where there are fewer
+    auto select = [&](int want, uint32_t& prefix, auto walk) {
+      prefix = 0;
+      remaining = want;
+      for (int shift = 24; shift >= 0; shift -= 8, turn ^= 1) {
+        int* h = hist[turn];
+        h[tid] = 0;
+        __syncthreads();
+        const uint32_t above_mask = shift == 24 ? 0u : (0xffffffffu << (shift + 8));
+        walk([&](uint32_t key) {
+          if ((key & above_mask) == prefix) atomicAdd(&h[(key >> shift) & 255u], 1);
+        });
+        sc_sync();
+        int sum = 0;
+#pragma unroll
+        for (int b = 0; b < SC_BLOCKS; ++b) sum += sc_read(&h[tid], b);
+        s_tot[tid] = sum;
+        __syncthreads();
+        if (tid < 32) {
+          // lane l owns digits 8l .. 8l+7; digits are taken from the largest down
+          int c[8], grp = 0;
+#pragma unroll
+          for (int b = 0; b < 8; ++b) {
+            c[b] = s_tot[8 * lane + b];
+            grp += c[b];
+          }
+          int incl = grp;             // inclusive sum over lanes lane .. 31
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_down_sync(0xffffffffu, incl, o);
+            if (lane + o < 32) incl += u;
+          }
+          if (lane == 0) s_count = incl;
+          int run = incl - grp;       // keys with a digit above this lane's
+          if (run < remaining && remaining <= incl) {
+#pragma unroll
+            for (int b = 7; b >= 0; --b) {
+              if (run < remaining && remaining <= run + c[b]) {
+                s_digit = 8 * lane + b;
+                s_above = run;
+                s_same = c[b];
+              }
+              run += c[b];
+            }
+          }
+        }
+        __syncthreads();
+        const bool few = s_count < remaining;     // (only with the first digit, and in every block)
+        const int digit = s_digit, above = s_above;
+        __syncthreads();              // they are read before the next digit takes their place
+        if (few) {
+          turn ^= 1;
+          return false;
+        }
+        prefix |= (uint32_t)digit << shift;
+        remaining -= above;
+      }
+      return true;
+    };
+    auto entries = [&](auto take) {
+      for (int i = tid; i < size; i += SC_THREADS) {
+        const uint32_t key = order_key(s_row[i]);
+        if (key >= bound) take(key);
+      }
+    };
+    if (!select(k, thr, entries)) {   // maxima that are no entries (of threads with NaNs alone)
+      bound = 0;
+      select(k, thr, entries);
+    }
+    need_eq = remaining;
+    all_eq = s_same == remaining;
+  }
+  const int lo = min(size, tid * C), hi = min(size, lo + C);   // (of the first SC_OWN threads)
+  int eq = 0;
+  if (use_k && !all_eq) {             // equal entries before each owner's positions
+    if (tid < SC_OWN) {
+      for (int i = lo; i < hi; ++i) eq += order_key(s_row[i]) == thr;
+      int incl = eq;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += u;
+      }
+      if (lane == 31) s_eq[warp] = incl;
+      eq = incl - eq;
+    }
+    sc_sync();
+    int before = 0;
+    for (int w = 0; w < rank * 4 + min(warp, 4); ++w) before += sc_read(&s_eq[w & 3], w >> 2);
+    eq += before;
+  }
+  __syncthreads();
+  // the weights: position by position, and where only some of the equal entries are kept owner by owner
+  const bool ordered = use_k && !all_eq;
+  if (!ordered) {
+#pragma unroll 4
+    for (int i = tid; i < size; i += SC_THREADS) {
+      const float v = s_row[i];
+      s_row[i] = !use_k || order_key(v) >= thr ? expf(v / temp - mx) : -1.f;
+    }
+    __syncthreads();
+  }
+  float sum = 0.f;
+  bool any = false;
+  if (tid < SC_OWN) {
+    for (int i = lo; i < hi; ++i) {
+      float e = s_row[i];
+      bool kept;
+      if (ordered) {
+        const uint32_t key = order_key(e);
+        kept = key > thr || (key == thr && eq++ < need_eq);
+        e = kept ? expf(e / temp - mx) : -1.f;
+        s_row[i] = e;
+      } else {
+        kept = !use_k || !(e == -1.f);
+      }
+      if (kept) {
+        sum += e;
+        any = true;
+      }
+    }
+  }
+  // weight of all kept entries below lo: within a warp, then over the 32 warps of the cluster
+  float before = 0.f, incl = sum;
+  if (tid < SC_OWN) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float u = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += u;
+    }
+    if (lane == 31) s_sum[warp] = incl;
+    before = __shfl_up_sync(0xffffffffu, incl, 1);
+    if (lane == 0) before = 0.f;
+  }
+  sc_sync();
+  if (warp == 0) {
+    float a = sc_read(&s_sum[lane & 3], lane >> 2);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float u = __shfl_up_sync(0xffffffffu, a, o);
+      if (lane >= o) a += u;
+    }
+    s_warps[lane] = a;
+  }
+  __syncthreads();
+  if (tid < SC_OWN) {
+    const int w = rank * 4 + warp;
+    const float total = s_warps[31];
+    float run = (w > 0 ? s_warps[w - 1] : 0.f) + before;
+    const float u = philox_uniform((uint32_t)seed_lo[rowi], (uint32_t)seed_hi[rowi],
+                                   (uint32_t)position[rowi]);
+    const float target = u * total;
+    int cand = 0x7fffffff, last_kept = -1;
+    for (int i = any ? lo : hi; i < hi; ++i) {
+      const float e = s_row[i];
+      if (e >= 0.f) {
+        run += e;
+        if (cand == 0x7fffffff && run > target) cand = from + i;
+        last_kept = from + i;
+      }
+    }
+    if (cand != 0x7fffffff) atomicMin(&s_found, cand);
+    if (last_kept >= 0) atomicMax(&s_last, last_kept);
+  }
+  __syncthreads();
+  if (tid == 0) {
+    sc_write(&s_v[rank], 0, s_found);
+    sc_write(&s_i[rank], 0, s_last);
+  }
+  sc_sync();
+  if (rank == 0 && tid == 0) {
+    int found = 0x7fffffff, last = 0;
+    for (int b = 0; b < SC_BLOCKS; ++b) {
+      found = min(found, s_v[b]);
+      last = max(last, s_i[b]);
+    }
+    // u * total rounded up to the total itself: the last kept token
+    const int tok = found != 0x7fffffff ? found : last;
+    out[rowi] = tok;
+    if (fb >= 0) feedback[fb] = tok;
+  }
+}
+
 }  // namespace hs
 
 HS_EXPORT int hs_argmax(int* out, const float* logits, int rows, int vocab, void* stream) {
@@ -568,7 +968,24 @@ HS_EXPORT int hs_sample(int* out, const float* logits, const float* temperature,
   // a row that fits shared memory (beside the kernel's own few KB) is read once
   const size_t row_bytes = (size_t)vocab * sizeof(float);
   cudaError_t le;
-  if (row_bytes <= 220 * 1024) {
+  if (row_bytes <= 220 * 1024 && vocab >= hs::SC_VOCAB && rows <= hs::SC_ROWS) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(rows * hs::SC_BLOCKS);
+    cfg.blockDim = dim3(hs::SC_THREADS);
+    cfg.dynamicSmemBytes = (size_t)hs::SC_OWN * (((vocab + hs::SS_THREADS - 1) / hs::SS_THREADS) | 1) * 4;
+    cfg.stream = (cudaStream_t)stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = hs::SC_BLOCKS;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = hs_pdl_enabled() ? 2 : 1;
+    le = cudaLaunchKernelEx(&cfg, hs::sample_cluster_kernel, out, logits, temperature, top_k, seed_lo, seed_hi,
+                            position, rows, vocab, feedback, feedback_slot, status_word);
+  } else if (row_bytes <= 220 * 1024) {
     static cudaError_t state = cudaErrorUnknown;
     if (state != cudaSuccess)
       state = cudaFuncSetAttribute(hs::sample_smem_kernel,
