@@ -329,6 +329,9 @@ lightning_chunk_chain_kernel(float* __restrict__ dS, float* __restrict__ state,
   const size_t next = (size_t)s.H * size / 4;              // from a chunk to the next
   const float g = decay[h], whole = (float)lc_power(g, LC_LEN);
   const float end = (float)lc_power(g, req_len[r] - (chunks - 1) * LC_LEN);
+  // a power that is below the range of numbers is zero, but no factor of the recurrence was: an infinity goes on
+  auto beyond = [&](float w) { return w == 0.f && g != 0.f ? copysignf(1.f, w) : w; };
+  const float whole_inf = beyond(whole), end_inf = beyond(end);
   float4 S = *slot;
   constexpr int B = 8;                                     // contributions on their way together
   for (int c0 = 0; c0 < chunks; c0 += B) {
@@ -340,9 +343,11 @@ lightning_chunk_chain_kernel(float* __restrict__ dS, float* __restrict__ state,
     for (int k = 0; k < B; ++k)
       if (c0 + k < chunks) {
         x[(c0 + k) * next] = S;
-        const float w = c0 + k + 1 < chunks ? whole : end;
-        S.x = fmaf(w, S.x, d[k].x); S.y = fmaf(w, S.y, d[k].y);
-        S.z = fmaf(w, S.z, d[k].z); S.w = fmaf(w, S.w, d[k].w);
+        const bool more = c0 + k + 1 < chunks;
+        const float w = more ? whole : end, w_inf = more ? whole_inf : end_inf;
+        auto carry = [&](float x, float add) { return fmaf(fabsf(x) <= 3.402823466e38f ? w : w_inf, x, add); };
+        S.x = carry(S.x, d[k].x); S.y = carry(S.y, d[k].y);
+        S.z = carry(S.z, d[k].z); S.w = carry(S.w, d[k].w);
       }
   }
   *slot = S;

@@ -116,3 +116,24 @@ def test_decays_at_the_ends():
     o, S = run(ops, *args, chunks=True)
     assert float((o.double() - want_o).norm() / want_o.norm()) < 1e-6
     assert float((S.double() - want_S).norm() / want_S.norm()) < 1e-6
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), float("-inf")])
+@pytest.mark.parametrize("where", ["k", "v", "state"])
+def test_infinities_under_decays_whose_powers_vanish(bad, where):
+    """The 64th power of these decays is zero or nearly; an infinity of the state is what the walk makes of it:
+    itself as long as the decay is not zero."""
+    H, D, V, lens, t = 4, 128, 128, (700,), 100
+    ops, decay = CudaOps(DEV), torch.tensor([0.0, 1e-3, 0.1, 0.3], device=DEV)
+    proj, state, pos, freq = inputs(lens, H, D, V, 0, 11)
+    for h in range(H):
+        if where == "state":
+            state[1, h * D * V + 5 * V + 3] = bad
+        else:
+            proj[t, 2 + h * 128 + {"k": H * D, "v": 2 * H * D}[where] + 3] = bad
+    args = (lens, proj, state, pos, freq, decay, H, D, V, 0, "none", 1.0)
+    (o, S), (po, pS) = run(ops, *args, chunks=True), run(ops, *args, chunks=False)
+    for got, want in ((o, po), (S, pS)):
+        assert torch.equal(got.isnan(), want.isnan())
+        assert torch.equal(got.isinf(), want.isinf()) and torch.equal(got[got.isinf()], want[want.isinf()])
+    assert bool(S.view(2, H, D * V)[1, 1:].isinf().any()) == (bad == bad)   # (a NaN leaves no infinity)
