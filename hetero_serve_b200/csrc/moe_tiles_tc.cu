@@ -52,15 +52,57 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
       : "memory");
 }
 
-// expert_act without branches: the quotient by the hardware's reciprocal (2 ulp of float32; the value is
-// rounded to bfloat16 next)
+// 1 / d and n / d for 1 <= d <= 2^126: an approximate value and one correction by its remainder (Markstein's
+// theorem), without the branch of the division, which keeps sixteen chains from running side by side (2,048
+// tokens, 32 experts: 106 us with it, 94 so).  Checked over all floats g: silu and the clamped gate are those
+// of expert_act, but for the last bit of one.
+__device__ __forceinline__ float near_reciprocal(float d) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  return r;
+}
+__device__ __forceinline__ float reciprocal(float d) {
+  const float r = near_reciprocal(d);
+  return fmaf(fmaf(-r, d, 1.0f), r, r);
+}
+__device__ __forceinline__ float quotient(float n, float d) {
+  const float r = near_reciprocal(d), q = n * r;
+  return fabsf(q) <= 3.402823466e38f ? fmaf(fmaf(-q, d, n), r, q) : q;
+}
+// what the gate's exponential is formed of, and below which its sum with 1 may leave quotient's range
 template <int ACT>
-__device__ __forceinline__ float expert_act_tc(float g, float u, float limit) {
-  if (ACT == 2) { const float r = fmaxf(u, 0.f); return r * r; }
-  if (ACT == 1) return __fdividef(g, 1.0f + expf(-g)) * u;
-  g = fminf(g, limit);
-  u = fminf(fmaxf(u, -limit), limit);
-  return __fdividef(g, 1.0f + expf(-1.702f * g)) * (u + 1.0f);
+__device__ __forceinline__ float gate_argument(float g, float limit) { return ACT == 1 ? g : 1.702f * fminf(g, limit); }
+constexpr float GATE_LOW = -87.f;
+// expert_act for gate arguments from GATE_LOW up
+template <int ACT>
+__device__ __forceinline__ float expert_act_near(float g, float u, float limit) {
+  const float d = 1.0f + expf(-gate_argument<ACT>(g, limit));
+  if (ACT == 1) return quotient(g, d) * u;
+  return fminf(g, limit) * reciprocal(d) * (fminf(fmaxf(u, -limit), limit) + 1.0f);
+}
+template <int ACT>
+__device__ __noinline__ float expert_act_low(float g, float u, float limit) { return expert_act<ACT>(g, u, limit); }
+// sixteen features' activations; one branch for all of them
+template <int ACT, bool GATED>
+__device__ __forceinline__ void expert_acts(float (&v)[16], const uint32_t (&u)[16], float limit) {
+  float least[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) least[j] = fminf(v[j], v[j + 8]);
+#pragma unroll
+  for (int n = 4; n; n >>= 1)
+#pragma unroll
+    for (int j = 0; j < n; ++j) least[j] = fminf(least[j], least[j + n]);
+  const bool low = gate_argument<ACT>(least[0], limit) < GATE_LOW;
+  if (ACT == 2) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] = expert_act<ACT>(v[j], v[j], limit);
+  } else if (low) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] = expert_act_low<ACT>(v[j], GATED ? __uint_as_float(u[j]) : v[j], limit);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] = expert_act_near<ACT>(v[j], GATED ? __uint_as_float(u[j]) : v[j], limit);
+  }
 }
 
 // NB weight matrices against the same rows (2: gate and up).  ACT: rows leave activated in bfloat16,
@@ -223,18 +265,10 @@ moe_tiles_tc_kernel(const __grid_constant__ CUtensorMap map_w0,
         float v[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(g[j]);
-        // one branch a chunk, so that the sixteen chains of an activation run side by side
         if (ACT) {
-          if (p.act == 0) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = expert_act_tc<0>(v[j], NB == 2 ? __uint_as_float(u[j]) : v[j], p.limit);
-          } else if (p.act == 1) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = expert_act_tc<1>(v[j], NB == 2 ? __uint_as_float(u[j]) : v[j], p.limit);
-          } else {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = expert_act_tc<2>(v[j], NB == 2 ? __uint_as_float(u[j]) : v[j], p.limit);
-          }
+          if (p.act == 0) expert_acts<0, NB == 2>(v, u, p.limit);
+          else if (p.act == 1) expert_acts<1, NB == 2>(v, u, p.limit);
+          else expert_acts<2, NB == 2>(v, u, p.limit);
         }
         const int n = f < p.N ? rows - c0 : 0;
         const size_t at = (size_t)(row0 + c0) * p.N + f;

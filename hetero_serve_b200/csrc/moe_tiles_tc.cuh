@@ -8,12 +8,16 @@ constexpr int MT_PAIRS = 256;         // pairs of one expert a tile takes at mos
 
 // act 0: g = min(g, limit), u = clamp(u, -limit, limit), g * sigmoid(1.702 g) * (u + 1); act 1:
 // silu(g) * u; act 2: relu(u)^2 (an expert without a gate matrix)
-__device__ __forceinline__ float expert_act(float g, float u, float limit, int act) {
-  if (act == 1) return g / (1.0f + expf(-g)) * u;
-  if (act == 2) { const float r = fmaxf(u, 0.f); return r * r; }
+template <int ACT>
+__device__ __forceinline__ float expert_act(float g, float u, float limit) {
+  if (ACT == 1) return g / (1.0f + expf(-g)) * u;
+  if (ACT == 2) { const float r = fmaxf(u, 0.f); return r * r; }
   g = fminf(g, limit);
   u = fminf(fmaxf(u, -limit), limit);
   return g * (1.0f / (1.0f + expf(-1.702f * g))) * (u + 1.0f);
+}
+__device__ __forceinline__ float expert_act(float g, float u, float limit, int act) {
+  return act == 1 ? expert_act<1>(g, u, limit) : act == 2 ? expert_act<2>(g, u, limit) : expert_act<0>(g, u, limit);
 }
 
 // The pairs sorted by expert: act_rows = activated gate / up rows (bfloat16 [pairs, ff]), down_rows =

@@ -81,3 +81,30 @@ def test_more_experts_than_sorting_threads():
     assert ops.status.item() == 0
     want = reference(h, wg, wu, wd, idx, wts, req, 7.0, "silu")
     assert (x.double() - want).norm() / want.norm() < 2e-3
+
+
+@pytest.mark.parametrize("act", ["silu", "clamped"])
+def test_gates_whose_exponential_is_near_the_end_of_the_range(act):
+    """Tiles and single pairs form the same quotient, up to where the exponential leaves the range."""
+    T, width, ff = 300, 32, 64
+    gates = -(80.0 + 0.5 * torch.arange(ff, device=DEV)) / (1.0 if act == "silu" else 1.702)
+    h = torch.zeros(T, width, device=DEV, dtype=torch.bfloat16)
+    h[:, 0] = 1.0
+    wg, wu = (torch.zeros(1, ff, width, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    wg[0, :, 0], wu[0, :, 0] = gates.to(torch.bfloat16), 2.0 ** 60
+    wd = torch.zeros(1, width, ff, device=DEV, dtype=torch.bfloat16)
+    idx, req = (torch.zeros(s, dtype=torch.int32, device=DEV) for s in ((T, 1), (T,)))
+    for first in (0, 32):                         # a feature an output
+        wd[0, :, first:first + 32] = torch.eye(32, device=DEV)
+        outs = []
+        for tiles in (True, False):
+            ops = CudaOps(DEV)
+            ops.sorted_experts = tiles
+            x = torch.zeros(T, width, device=DEV)
+            ops.moe_experts(x, torch.zeros(T, ff, device=DEV), h, wg, wu, wd, idx, torch.ones(T, 1, device=DEV), req,
+                            limit=2.0 ** 60, act=act, fresh=True)
+            outs.append(x)
+        wd.zero_()
+        # the tiles' activated rows are rounded to bfloat16: half a step of 2^-7 at most
+        assert bool(((outs[0] - outs[1]).abs() <= 2.0 ** -8 * outs[1].abs()).all())
+        assert bool((outs[1] != 0).any()) or first == 32
