@@ -137,3 +137,38 @@ def test_infinities_under_decays_whose_powers_vanish(bad, where):
         assert torch.equal(got.isnan(), want.isnan())
         assert torch.equal(got.isinf(), want.isinf()) and torch.equal(got[got.isinf()], want[want.isinf()])
     assert bool(S.view(2, H, D * V)[1, 1:].isinf().any()) == (bad == bad)   # (a NaN leaves no infinity)
+
+
+@pytest.mark.parametrize("rot, act", [(128, "none"), (0, "silu"), (4, "silu")])
+def test_chunks_without_numbers_take_no_longer_than_the_recurrence(rot, act):
+    """A prompt of NaNs from its middle on (what a layer before makes of one) in chunks, against the same prompt
+    token by token: the same entries are finite, and the walk of such chunks is no slower than that."""
+    H, D, V, lens = 8, 128, 128, (1024, 1024)
+    ops, decay = CudaOps(DEV), torch.linspace(0.9, 0.99, H, device=DEV)
+    proj, state, pos, freq = inputs(lens, H, D, V, rot, 3)
+    proj[700:1024] = float("nan")
+    proj[1500:, 2 + H * D + 5] = float("nan")                  # one entry of k of every later token
+    args = (lens, proj, state, pos, freq, decay, H, D, V, rot, act, 0.1)
+    (o, S), (po, pS) = run(ops, *args, chunks=True), run(ops, *args, chunks=False)
+    assert torch.equal(o.isnan(), po.isnan()) and torch.equal(S.isnan(), pS.isnan())
+    fine = po.isfinite()
+    assert bool(((o - po).abs()[fine] <= 1e-4 * po.abs()[fine] + 1e-4 * po[fine].abs().mean()).all())
+
+    def best(chunks):
+        graph, times = torch.cuda.CUDAGraph(), []
+        more = dict(tok_pos=i32(pos), freq=freq, rot_dims=rot, k_scale=0.1) if rot else {}
+        o, S, a = torch.empty_like(po), state.clone(), (i32([0, 1024]), i32(lens), i32([2, 1]))
+        with torch.cuda.graph(graph):
+            for _ in range(4):
+                ops.lightning_recurrence(o, S, proj, decay, *a, q_off=2, k_off=2 + H * D, v_off=2 + 2 * H * D,
+                                         heads=H, dim=D, vdim=V, act=act, chunks=chunks, **more)
+        for _ in range(6):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            graph.replay()
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    assert best(True) <= 1.25 * best(False)
