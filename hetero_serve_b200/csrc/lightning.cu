@@ -486,14 +486,15 @@ HS_EXPORT int hs_lightning_chunk_scratch(int n_tokens, int n_requests, int H, in
 // (hs_lightning_scratch floats, or null): with it the activations are applied in a pass of their own
 // and the recurrence streams the activated rows; the results are the same bits.  `chunks`
 // (hs_lightning_chunk_scratch floats, or null): with it requests of hs::LC_MIN tokens and more go in chunks
-// on the tensor cores (lightning_chunk.cu: sums in another order), each by its own length.
+// on the tensor cores (lightning_chunk.cu: sums in another order), each by its own length; `walks` 0 says that
+// there are no others, so that nothing is launched for them.
 HS_EXPORT int hs_lightning_recurrence(float* o, float* state, const float* proj,
                                       const float* decay, const int* req_start,
                                       const int* req_len, const int* req_slot, int n_requests,
                                       int n_tokens, int stride, int q_off, int k_off, int v_off,
                                       int H, int D, int V, int act, float* scratch,
                                       const int* tok_pos, const float* freq, int rot_dims,
-                                      float k_scale, float* chunks, int* status, void* stream) {
+                                      float k_scale, float* chunks, int walks, int* status, void* stream) {
   if (!o || !state || !proj || !decay || !req_start || !req_len || !req_slot)
     return HS_ERR_ARGUMENT;
   if (rot_dims < 0 || rot_dims % 2 || rot_dims > D || (rot_dims > 0 && (!freq || !tok_pos)))
@@ -510,6 +511,7 @@ HS_EXPORT int hs_lightning_recurrence(float* o, float* state, const float* proj,
                                      stride, q_off, k_off, v_off, H, D, V, act, chunks, tok_pos, freq, rot_dims,
                                      k_scale, st))
       return e;
+    if (!walks) return HS_OK;
     most = hs::LC_MIN - 1;
   }
   if (scratch && status && lightning_streams(n_tokens, n_requests, D) && !((uintptr_t)scratch & 15)) {

@@ -247,7 +247,7 @@ def _declare(lib) -> None:
         "hs_biased_attention_prefill": [P, P, P, P, P, P, I, P, P, I, P, I, I, I, I, I, I, I, I,
                                         F, F, I, I, P, P],
         "hs_lightning_recurrence": [P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, P, P, P, I,
-                                    F, P, P, P],
+                                    F, P, I, P, P],
         "hs_lightning_scratch": [I, I, I, I, I, P],
         "hs_lightning_chunk_scratch": [I, I, I, I, I, I, P],
         "hs_token_shift_mix": [P, P, P, P, I, I, P, P, P, P, I, I, I, I, P],
@@ -837,7 +837,8 @@ class CudaOps:
                                                  page_size, False)
         return AttentionPlan(torch.from_numpy(view).to(self.device), n_rows, dec, tiles, single,
                              self.plan_prompt_rows(host_batch, False),
-                             self.plan_sides(host_batch, sorted(set(self.DELTA_LONG.values()))))
+                             self.plan_sides(host_batch, sorted({*self.DELTA_LONG.values(),
+                                                                 self.LIGHTNING_LONG})))
 
     def _scratch_buffer(self, name, numel, dtype):
         key = (name, dtype)
@@ -1921,17 +1922,21 @@ class CudaOps:
             f"biased_attention(head_dim={head_dim})")
 
     # -- linear attention with a decay per head ---------------------------------------------
+    LIGHTNING_LONG = 512          # tokens from which on a request may go in chunks (lightning.cuh)
+
     def lightning_recurrence(self, o, state, proj, decay, req_start, req_len, req_slot, *, q_off,
                              k_off, v_off, heads, dim, vdim, act="silu", tok_pos=None, freq=None,
-                             rot_dims=0, k_scale=1.0, chunks=False):
+                             rot_dims=0, k_scale=1.0, chunks=False, plan=None):
         """Per request and head, token after token on the float32 state S [dim, vdim] of the
         request's slot: S <- decay[h] S + k v^T; o = S^T q, with q, k, v = act(columns of the
         float32 projection rows ``proj``), laid out head by head from ``q_off``, ``k_off``,
         ``v_off``.  ``o`` is float32 [T, heads * vdim].  With ``freq`` (float32 [rot_dims / 2])
         q and k are turned by ``tok_pos`` on their first ``rot_dims`` numbers (number i pairs
         with i + rot_dims / 2) before they are used; k is multiplied by ``k_scale``.
-        ``chunks``: requests that bring many tokens may go in chunks on the tensor cores (float32 terms
-        and sums, in another order than token after token; each request by its own length)."""
+        ``chunks``: requests that bring ``LIGHTNING_LONG`` tokens or more may go in chunks on the tensor
+        cores (float32 terms and sums, in another order than token after token; each request by its own
+        length).  ``plan``, the step's attention plan, may know that the step has no request of one
+        kind, whose kernels are then not launched."""
         _want(o, "o", torch.float32, 2)
         _want(proj, "proj", torch.float32, 2)
         _want(state, "state", torch.float32)
@@ -1962,21 +1967,23 @@ class CudaOps:
                                           ctypes.byref(need))
             if need.value:
                 scratch = self._scratch_buffer("lightning_rows", need.value, torch.float32)
-        self.launches += 2 if scratch is not None else 1
         parts = None
-        if chunks:
+        above, below = (True, True) if plan is None else plan.side(self.LIGHTNING_LONG)
+        if chunks and above:
             need = ctypes.c_longlong(0)
             self.lib.hs_lightning_chunk_scratch(T, req_start.shape[0], heads, dim, vdim, int(rot_dims),
                                                 ctypes.byref(need))
             if need.value:
                 parts = self._scratch_buffer("lightning_chunks", need.value, torch.float32)
                 self.launches += 4 if rot_dims else 3
+        if parts is None or below:
+            self.launches += 2 if scratch is not None else 1
         _check(self.lib.hs_lightning_recurrence(
             _ptr(o), _ptr(state), _ptr(proj), _ptr(decay), _ptr(req_start), _ptr(req_len),
             _ptr(req_slot), req_start.shape[0], T, proj.shape[1], int(q_off), int(k_off),
             int(v_off), heads, dim, vdim, ACTIVATIONS[act], _ptr(scratch),
             _ptr(tok_pos) if rot_dims else None, _ptr(freq) if rot_dims else None, int(rot_dims),
-            float(k_scale), _ptr(parts), _ptr(self.status), self._stream()),
+            float(k_scale), _ptr(parts), int(below), _ptr(self.status), self._stream()),
             f"lightning_recurrence(dim={dim},vdim={vdim})")
 
     # -- norms behind a sublayer, a learned activation, capped logits -----------------------

@@ -17,6 +17,7 @@ from __future__ import annotations
 
 import torch
 
+from ..kernels.ops import CudaOps
 from .base import Mixer, TensorRequest, register_mixer
 
 
@@ -31,6 +32,7 @@ class LightningAttention(Mixer):
         self.width, self.H, self.D, self.V = width, n_heads, dim, vdim
         self.decay_values, self.eps, self.p = decay, float(eps), prefix
         self.n_in = 2 * self.H * self.D + 2 * self.H * self.V             # q | k | v | gate
+        self.portion_limits = (CudaOps.LIGHTNING_LONG,) if dim == vdim == 128 else ()
 
     def tensor_requests(self):
         p, W, hd, hv = self.p, self.width, self.H * self.D, self.H * self.V
@@ -59,7 +61,9 @@ class LightningAttention(Mixer):
         hd, hv = self.H * self.D, self.H * self.V
         o = ctx.buffer("lightning_o", (T, hv), torch.float32)
         # rows leave in bfloat16: long portions in chunks (float32 engines keep one order of the sums)
-        more = {"chunks": True} if ctx.dtype == torch.bfloat16 else {}
+        more = {}
+        if ctx.dtype == torch.bfloat16:
+            more = {"chunks": True, "plan": getattr(ctx, "plan", None)}
         ops.lightning_recurrence(o, ctx.state(), proj, self.decay, ctx.req_start, ctx.req_len,
                                  ctx.req_slot, q_off=offset, k_off=offset + hd,
                                  v_off=offset + 2 * hd, heads=self.H, dim=self.D, vdim=self.V,

@@ -19,6 +19,7 @@ from __future__ import annotations
 
 import torch
 
+from ..kernels.ops import CudaOps
 from .base import Mixer, TensorRequest, register_mixer
 from .pooled_attention import rotary_frequencies
 
@@ -40,6 +41,7 @@ class Retention(Mixer):
         self.k_scale = float(dim) ** -0.5 if k_scale is None else float(k_scale)
         self.gate_act = gate_act
         self.n_in = 2 * self.H * self.D + 2 * self.H * self.V             # q | k | v | gate
+        self.portion_limits = (CudaOps.LIGHTNING_LONG,) if dim == vdim == 128 else ()
 
     def tensor_requests(self):
         p, W, hd, hv = self.p, self.width, self.H * self.D, self.H * self.V
@@ -69,7 +71,9 @@ class Retention(Mixer):
         ops.linear(proj, h, self.w_in)
         o = ctx.buffer("retention_o", (T, hv), torch.float32)
         # rows leave in bfloat16: long portions in chunks (float32 engines keep one order of the sums)
-        more = {"chunks": True} if ctx.dtype == torch.bfloat16 else {}
+        more = {}
+        if ctx.dtype == torch.bfloat16:
+            more = {"chunks": True, "plan": getattr(ctx, "plan", None)}
         ops.lightning_recurrence(o, ctx.state(), proj, self.decay, ctx.req_start, ctx.req_len,
                                  ctx.req_slot, q_off=0, k_off=hd, v_off=2 * hd, heads=self.H,
                                  dim=self.D, vdim=self.V, act="none", tok_pos=ctx.tok_pos,

@@ -172,3 +172,36 @@ def test_chunks_without_numbers_take_no_longer_than_the_recurrence(rot, act):
         return min(times)
     i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
     assert best(True) <= 1.25 * best(False)
+
+
+@pytest.mark.parametrize("lens", [(8,) * 64, (600, 700), (511, 1, 512)])
+@pytest.mark.parametrize("rot", [0, 128])
+def test_only_the_forms_of_the_step_are_launched(lens, rot):
+    """A plan says which lengths there are: the same bits as without one, and no kernel that has no request."""
+    H, D, V = 2, 128, 128
+    proj, state, pos, freq = inputs(lens, H, D, V, rot, 5)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    ops, decay = CudaOps(DEV), torch.tensor([0.9, 0.99], device=DEV)
+    start = [sum(lens[:r]) for r in range(len(lens))]
+    plan = ops.make_plan([(r, r, 0, n) for r, n in enumerate(lens)], sum(lens), 16)
+    more = dict(tok_pos=i32(pos), freq=freq, rot_dims=rot) if rot else {}
+    got, graph = [], []
+    for p in (None, plan):
+        o, S = torch.full((sum(lens), H * V), float("nan"), device=DEV), state.clone()
+        call = lambda: ops.lightning_recurrence(  # noqa: E731
+            o, S, proj, decay, i32(start), i32(lens), i32(list(range(len(lens)))), q_off=2, k_off=2 + H * D,
+            v_off=2 + 2 * H * D, heads=H, dim=D, vdim=V, act="silu", chunks=True, plan=p, **more)
+        before = ops.launches
+        call()
+        got.append((o.clone(), S.clone(), ops.launches - before))
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+            call()
+            torch.cuda.synchronize()
+        graph.append([e.key for e in prof.key_averages() if "lightning" in e.key])
+    (a, sa, _), (b, sb, launches) = got
+    assert torch.equal(a, b) and torch.equal(sa, sb)
+    chunked, walked = max(lens) >= 512, min(lens) < 512
+    assert launches == (3 + (rot > 0)) * chunked + 2 * walked
+    if graph[1]:                                             # (where the profiler can see kernels)
+        assert any("chunk" in k for k in graph[1]) == chunked
+        assert any("chunk" not in k and "turns" not in k for k in graph[1]) == walked
