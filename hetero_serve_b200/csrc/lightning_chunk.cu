@@ -370,17 +370,23 @@ lightning_chunk_state_kernel(float* __restrict__ dS, const float* __restrict__ p
 }
 
 // ---- the chain of states ------------------------------------------------------------------------
+// Blocks for as many requests as may go in chunks, not for all (600 tokens beside 60 single ones, 32 heads:
+// lightning attention 288 us with all, 258 so).  The outputs' blocks are let in late: when they come while the
+// contributions are being formed they share SMs and take longer (2 x 1,024 tokens of 4 heads 55 us, 50 so).
 __global__ void __launch_bounds__(LC_THREADS)
 lightning_chunk_chain_kernel(float* __restrict__ dS, float* __restrict__ state,
                              const float* __restrict__ decay, const int* __restrict__ req_len,
                              const int* __restrict__ req_slot, const LcShape s) {
-  pdl_trigger();
   pdl_wait();
-  const int r = blockIdx.z, h = blockIdx.y, chunks = lc_chunks(req_len[r]);
-  const int size = LC_D * LC_V, i = (blockIdx.x * LC_THREADS + threadIdx.x) * 4;
-  if (chunks == 0 || i >= size) return;
-  int first = 0;
-  for (int k = 0; k < r; ++k) first += lc_chunks(req_len[k]);
+  pdl_trigger();
+  const int h = blockIdx.y, size = LC_D * LC_V, i = (blockIdx.x * LC_THREADS + threadIdx.x) * 4;
+  int r = 0, chunks = 0, first = 0;                        // the blockIdx.z-th request in chunks, the chunks before
+  for (int nth = 0; r < s.n_requests; ++r) {
+    chunks = lc_chunks(req_len[r]);
+    if (chunks && nth++ == (int)blockIdx.z) break;
+    first += chunks;
+  }
+  if (r == s.n_requests || i >= size) return;
   float4* slot = (float4*)(state + ((size_t)req_slot[r] * s.H + h) * size + i);
   float4* x = (float4*)(dS + ((size_t)first * s.H + h) * size + i);
   const size_t next = (size_t)s.H * size / 4;              // from a chunk to the next
@@ -614,7 +620,8 @@ int lightning_chunks(float* o, float* state, const float* proj, const float* dec
   e = hs_launch(lightning_chunk_state_kernel, dim3(slots, H), dim3(LC_THREADS), (size_t)smem_a, st, pdl,
                 scratch, proj, decay, req_start, req_len, s);
   if (e != cudaSuccess) return (int)e;
-  e = hs_launch(lightning_chunk_chain_kernel, dim3((D * V / 4 + LC_THREADS - 1) / LC_THREADS, H, n_requests),
+  const int most = n_requests < n_tokens / LC_MIN ? n_requests : n_tokens / LC_MIN;
+  e = hs_launch(lightning_chunk_chain_kernel, dim3((D * V / 4 + LC_THREADS - 1) / LC_THREADS, H, most),
                 dim3(LC_THREADS), 0, st, pdl, scratch, state, decay, req_len, req_slot, s);
   if (e != cudaSuccess) return (int)e;
   e = hs_launch(lightning_chunk_out_kernel, dim3(slots, H), dim3(LC_THREADS), (size_t)smem_c, st, pdl, o,

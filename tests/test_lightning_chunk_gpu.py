@@ -205,3 +205,18 @@ def test_only_the_forms_of_the_step_are_launched(lens, rot):
     if graph[1]:                                             # (where the profiler can see kernels)
         assert any("chunk" in k for k in graph[1]) == chunked
         assert any("chunk" not in k and "turns" not in k for k in graph[1]) == walked
+
+
+def test_requests_in_chunks_among_many():
+    """More requests than can go in chunks, before, between and behind those that do: each has the bits it has
+    alone."""
+    H, D, V, lens = 2, 128, 128, (3,) * 40 + (600, 0, 0, 5, 700) + (1,) * 70 + (512,)
+    ops, decay = CudaOps(DEV), torch.tensor([0.9, 0.99], device=DEV)
+    proj, state, pos, freq = inputs(lens, H, D, V, 0, 13)
+    rest = (freq, decay, H, D, V, 0, "silu", 1.0)
+    o, S = run(ops, lens, proj, state, pos, *rest, chunks=True)
+    for r in (0, 40, 43, 44, 60, len(lens) - 1):
+        n, at, slot = lens[r], sum(lens[:r]), len(lens) - r
+        one, sone = run(ops, (n,), proj[at:at + n].clone(), state[[0, slot]].clone(), pos[at:at + n], *rest, chunks=True)
+        assert torch.equal(one, o[at:at + n]) and torch.equal(sone[1], S[slot])
+    assert torch.equal(S[0], state[0])
