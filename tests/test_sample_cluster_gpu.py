@@ -69,3 +69,48 @@ def test_feedback_and_status_word():
     t = out.tolist()
     assert t[0] == int(x[0].argmax()) and t[3] == 6
     assert back.tolist() == [t[2], -9, t[0], -9]
+
+
+@pytest.mark.parametrize("kind", ["normal", "rounded", "masked", "nan"])
+@pytest.mark.parametrize("vocab", [24576, 50257])
+def test_lists_of_every_length(vocab, kind):
+    """k around the lines between the ways its threshold is found: the tokens of a block a row."""
+    ops, ks = CudaOps(DEV), [1, 63, 64, 65, 66, 100, 129, 200, 255, 256, 257, 400, 511, 512, 513, 700]
+    g, n = torch.Generator(device=DEV).manual_seed(vocab + 1), len(ks)
+    x = rows_of(kind, n, vocab, g)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    times = MOST // n + 1
+    for draw in range(4):
+        args = (x, torch.full((n,), 1.3, device=DEV), i32(ks), i32([draw] * n), i32(list(range(n))), i32([3] * n))
+        got = torch.full((n,), -1, dtype=torch.int32, device=DEV)
+        ops.sample(got, *args)
+        want = torch.full((n * times,), -1, dtype=torch.int32, device=DEV)
+        ops.sample(want, *(t.repeat(times, *[1] * (t.dim() - 1)).contiguous() for t in args))
+        assert torch.equal(got, want[:n])
+
+
+@pytest.mark.parametrize("k", [40, 100, 256, 400])
+@pytest.mark.parametrize("vocab", [32000, 50257])
+def test_clusters_take_no_longer_than_a_block_a_row(vocab, k):
+    """Against one row more than clusters take, which goes a block a row, an SM each either way."""
+    ops, g = CudaOps(DEV), torch.Generator(device=DEV).manual_seed(k)
+    times = []
+    for n in (32, MOST + 1):
+        x = torch.randn(n, vocab, device=DEV, generator=g) * 3
+        zero = torch.zeros(n, dtype=torch.int32, device=DEV)
+        out, temp, graph = torch.empty(n, dtype=torch.int32, device=DEV), torch.full((n,), 0.8, device=DEV), None
+        ops.sample(out, x, temp, zero + k, zero, zero, zero)
+        kk, graph = zero + k, torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            for _ in range(10):
+                ops.sample(out, x, temp, kk, zero, zero, zero)
+        best = []
+        for _ in range(8):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            graph.replay()
+            b.record()
+            b.synchronize()
+            best.append(a.elapsed_time(b))
+        times.append(min(best))
+    assert times[0] <= 1.15 * times[1]
