@@ -142,15 +142,94 @@ __device__ __forceinline__ void lf_store_terms(uint32_t dst, uint32_t term_bytes
     asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(dst + t * term_bytes), "r"(lo), "r"(hi) : "memory");
   }
 }
-__device__ __noinline__ float lf_finish(const LfParams& p, float sum, int m, int n, float bias) {
-  if (!(fabsf(sum) <= 3.402823466e38f)) {             // an infinity or no number: the chain of FMAs
-    const float *x = p.a + (size_t)m * p.K, *y = p.w + (size_t)n * p.K;
-    sum = 0.f;
-    for (int k = 0; k < p.K; ++k) sum = fmaf(x[k], y[k], sum);
+// A result that is not finite is formed again as a chain of FMAs (the terms of an infinity are not numbers).
+// Where a row of `a` or a feature's weights hold no number, which a warp sees by a look along them, so does the
+// result; else the chain, its numbers eight pieces ahead, until it holds none.  (us for 8 x 1,024 x 4,096 with a row of
+// NaNs, 12 without: 294 as chains of single loads; 1,024 rows of NaNs, 83 without: 18,800.)
+__device__ __forceinline__ bool lf_finite(float x) { return fabsf(x) <= 3.402823466e38f; }
+// whether a row holds something that is no number; the whole warp asks for the same row
+__device__ __forceinline__ bool lf_row_nan(const float* __restrict__ row, int K) {
+  for (int k0 = 0; k0 < K; k0 += 512) {
+    bool nan = false;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int k = k0 + j * 128 + (threadIdx.x & 31) * 4;
+      const float4 x = k < K ? *(const float4*)(row + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+      nan = nan || x.x != x.x || x.y != x.y || x.z != x.z || x.w != x.w;
+    }
+    if (__any_sync(0xffffffffu, nan)) return true;
   }
-  float v = apply_act(sum + bias, p.act, p.act_ab);
-  if (p.residual) v += p.residual[(size_t)m * p.N + n];
-  return v;
+  return false;
+}
+// the chain of a row (the same for the whole warp) and the lane's weights; lanes that want none come along
+template <int AHEAD>
+__device__ __forceinline__ float lf_chain(const float* __restrict__ x, const float* __restrict__ y, int K, bool wanted) {
+  float sum = 0.f;
+  for (int k0 = 0; k0 < K; k0 += 4 * AHEAD) {
+    const int lane = threadIdx.x & 31;
+    const float mine = lane < 4 * AHEAD && k0 + lane < K ? x[k0 + lane] : 0.f;
+    float4 v[AHEAD];
+#pragma unroll
+    for (int j = 0; j < AHEAD; ++j)
+      if (k0 + 4 * j < K) v[j] = *(const float4*)(y + k0 + 4 * j);
+#pragma unroll
+    for (int j = 0; j < AHEAD; ++j)
+      if (k0 + 4 * j < K) {
+        sum = fmaf(__shfl_sync(0xffffffffu, mine, 4 * j), v[j].x, sum);
+        sum = fmaf(__shfl_sync(0xffffffffu, mine, 4 * j + 1), v[j].y, sum);
+        sum = fmaf(__shfl_sync(0xffffffffu, mine, 4 * j + 2), v[j].z, sum);
+        sum = fmaf(__shfl_sync(0xffffffffu, mine, 4 * j + 3), v[j].w, sum);
+      }
+    if (__all_sync(0xffffffffu, !wanted || sum != sum)) break;
+  }
+  return sum;
+}
+// The sums of a warp's lanes (feature n each, -1: none) with row m, those that are not finite formed again.  nans:
+// lanes whose weights are known to hold no number.
+template <int AHEAD>
+__device__ __forceinline__ float lf_again(const LfParams& p, float sum, int m, int n, unsigned& nans) {
+  const float nan = __int_as_float(0x7fffffff);
+  const int lane = threadIdx.x & 31;
+  unsigned odd = __ballot_sync(0xffffffffu, n >= 0 && !lf_finite(sum));
+  if (odd >> lane & 1 & nans >> lane) sum = nan;
+  odd &= ~nans;
+  if (odd == 0) return sum;
+  if (lf_row_nan(p.a + (size_t)m * p.K, p.K)) return odd >> lane & 1 ? nan : sum;
+  if (__popc(odd) <= 4) {
+    for (unsigned rest = odd; rest; rest &= rest - 1) {
+      const int l = __ffs(rest) - 1, f = __shfl_sync(0xffffffffu, n, l);
+      if (!lf_row_nan(p.w + (size_t)f * p.K, p.K)) continue;
+      nans |= 1u << l;
+      odd &= ~(1u << l);
+      if (lane == l) sum = nan;
+    }
+  }
+  const float chain = lf_chain<AHEAD>(p.a + (size_t)m * p.K, p.w + (size_t)max(n, 0) * p.K, p.K, odd >> lane & 1);
+  return odd >> lane & 1 ? chain : sum;
+}
+// Rows m0 .. m0 + n - 1 of a tile some of whose sums are not finite, finished (up to sixteen); the lane's feature is f.
+// (Few registers: what a called function needs the kernel keeps free, and its fetching warps have none to spare.)
+__device__ __noinline__ unsigned lf_odd_rows(const LfParams& p, uint32_t taddr, int m0, int n, int f, unsigned nans) {
+  // rows of NaNs are most often that from their first number on
+  float first = 0.f;
+  if ((threadIdx.x & 31) < min(n, 16)) first = p.a[(size_t)(m0 + (threadIdx.x & 31)) * p.K];
+  const unsigned gone = __ballot_sync(0xffffffffu, first != first);
+#pragma unroll 1
+  for (int j = 0; j < min(n, 16); ++j) {
+    uint32_t c;
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(c) : "r"(taddr + j) : "memory");
+    tmem_ld_wait();
+    float v = __uint_as_float(c);
+    if (!(gone >> j & 1)) v = lf_again<4>(p, v, m0 + j, f < p.N ? f : -1, nans);
+    if (f < p.N) {
+      v = apply_act(v + (p.bias ? p.bias[f] : 0.f), p.act, p.act_ab);
+      const size_t at = (size_t)(m0 + j) * p.N + f;
+      if (p.residual) v += p.residual[at];
+      p.out[at] = v;
+    }
+    __syncwarp();
+  }
+  return nans;
 }
 
 // where an item lies: tiles of rows run fastest (blocks that run together share the weights), then the
@@ -170,7 +249,7 @@ __device__ __forceinline__ LfItem lf_item(const LfParams& p, int w) {
 }
 
 template <int NR, bool SPLIT>
-__global__ void __launch_bounds__(LF_THREADS, 1) linear_f32_tc_kernel(const LfParams p) {
+__global__ void __launch_bounds__(LF_THREADS, 1) linear_f32_tc_kernel(const __grid_constant__ LfParams p) {
   using S = LfShape<NR>;
   extern __shared__ uint8_t lf_smem[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)lf_smem + 1023) & ~(uintptr_t)1023);
@@ -366,41 +445,41 @@ __global__ void __launch_bounds__(LF_THREADS, 1) linear_f32_tc_kernel(const LfPa
         const float bias = !SPLIT && p.bias && f < p.N ? p.bias[f] : 0.f;
         float* dst = SPLIT ? p.partial + ((size_t)(kb / LF_SEG) * p.M + it.m0) * p.N + f
                            : p.out + (size_t)it.m0 * p.N + f;
+        unsigned nans = 0;                       // lanes whose weights hold no number
 #pragma unroll 1
         for (int j0 = 0; j0 < n; j0 += 16) {
           uint32_t c[16];
           lf_tmem_ld16((SPLIT ? seg : total) + j0, c);
           tmem_ld_wait();
+          if (!SPLIT) {
+            bool finite = true;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) finite = finite && lf_finite(__uint_as_float(c[j]));
+            if (__any_sync(0xffffffffu, !finite && f < p.N)) {
+              nans = lf_odd_rows(p, total + j0, it.m0 + j0, n - j0, f, nans);
+              continue;
+            }
+          }
           if (f < p.N) {
             float v[16], res[16];
-            bool finite = true;
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
               v[j] = __uint_as_float(c[j]);
-              if (!SPLIT) {
-                finite = finite && fabsf(v[j]) <= 3.402823466e38f;
-                res[j] = (p.residual && j0 + j < n) ? p.residual[(size_t)(it.m0 + j0 + j) * p.N + f] : 0.f;
-              }
+              if (!SPLIT) res[j] = (p.residual && j0 + j < n) ? p.residual[(size_t)(it.m0 + j0 + j) * p.N + f] : 0.f;
             }
             if (!SPLIT) {
-              if (finite) {
 #pragma unroll
-                for (int j = 0; j < 16; ++j) v[j] += bias;
-                if (p.act == HS_ACT_GELU_TANH) {
+              for (int j = 0; j < 16; ++j) v[j] += bias;
+              if (p.act == HS_ACT_GELU_TANH) {
 #pragma unroll
-                  for (int j = 0; j < 16; ++j) v[j] = gelu_tanh(v[j]);
-                } else if (p.act != HS_ACT_NONE) {
+                for (int j = 0; j < 16; ++j) v[j] = gelu_tanh(v[j]);
+              } else if (p.act != HS_ACT_NONE) {
 #pragma unroll
-                  for (int j = 0; j < 16; ++j) v[j] = apply_act(v[j], p.act, p.act_ab);
-                }
-                if (p.residual) {
+                for (int j = 0; j < 16; ++j) v[j] = apply_act(v[j], p.act, p.act_ab);
+              }
+              if (p.residual) {
 #pragma unroll
-                  for (int j = 0; j < 16; ++j) v[j] += res[j];
-                }
-              } else {
-#pragma unroll
-                for (int j = 0; j < 16; ++j)
-                  if (j0 + j < n) v[j] = lf_finish(p, v[j], it.m0 + j0 + j, f, bias);
+                for (int j = 0; j < 16; ++j) v[j] += res[j];
               }
             }
 #pragma unroll
@@ -421,11 +500,11 @@ __global__ void __launch_bounds__(LF_THREADS, 1) linear_f32_tc_kernel(const LfPa
 }
 
 // the segments' sums added in order, bias, activation, residual
-__global__ void __launch_bounds__(128) linear_f32_tc_sum_kernel(const LfParams p) {
+__global__ void __launch_bounds__(128) linear_f32_tc_sum_kernel(const __grid_constant__ LfParams p) {
   pdl_trigger();
   pdl_wait();
-  const long long i = (long long)blockIdx.x * 128 + threadIdx.x, size = (long long)p.M * p.N;
-  if (i >= size) return;
+  const long long size = (long long)p.M * p.N, at = (long long)blockIdx.x * 128 + threadIdx.x;
+  const long long i = at < size ? at : size - 1;         // (whole warps come to the end)
   const float* src = p.partial + i;
   float sum = src[0];
   int c = 1;
@@ -444,7 +523,16 @@ __global__ void __launch_bounds__(128) linear_f32_tc_sum_kernel(const LfParams p
   for (int j = 0; j < 7; ++j)
     if (c + j < p.segs) sum += v[j];
   const int m = (int)(i / p.N), n = (int)(i - (long long)m * p.N);
-  p.out[i] = lf_finish(p, sum, m, n, p.bias ? p.bias[n] : 0.f);
+  if (__any_sync(0xffffffffu, !lf_finite(sum))) {
+    unsigned nans = 0;
+    const int last = __shfl_sync(0xffffffffu, m, 31);      // (a warp's outputs lie in one row, or in rows one by one)
+    for (int row = __shfl_sync(0xffffffffu, m, 0); row <= last; ++row)
+      sum = lf_again<8>(p, sum, row, m == row ? n : -1, nans);
+  }
+  if (at >= size) return;
+  float y = apply_act(sum + (p.bias ? p.bias[n] : 0.f), p.act, p.act_ab);
+  if (p.residual) y += p.residual[i];
+  p.out[i] = y;
 }
 
 struct LfPlan {

@@ -107,3 +107,43 @@ def test_shapes_it_refuses_go_to_the_cuda_cores():
     buf = torch.randn(50 * 64 + 1, device=DEV, generator=g)
     a, w = torch.randn(40, 64, device=DEV, generator=g), buf[1:].view(50, 64)
     assert torch.equal(run(ops, 0, a, w), chain(ops, a, w))              # weights off a 16-byte boundary
+
+
+def time_of(call):
+    graph, best = torch.cuda.CUDAGraph(), []
+    call()
+    with torch.cuda.graph(graph):
+        for _ in range(4):
+            call()
+    for _ in range(6):
+        a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        a.record()
+        graph.replay()
+        b.record()
+        b.synchronize()
+        best.append(a.elapsed_time(b))
+    return min(best)
+
+
+@pytest.mark.parametrize("what", ["row", "number", "rows", "weight"])
+@pytest.mark.parametrize("m, n, k", [(8, 1024, 4096), (1024, 1024, 4096), (1024, 4096, 1024)])
+def test_numbers_that_are_none_take_no_longer_than_chains(m, n, k, what):
+    """A row of NaNs, one NaN in a row, all rows, one NaN among the weights: as the CUDA cores answer and, since
+    those take as long as for other numbers, not slower than them by much."""
+    ops, g = CudaOps(DEV), torch.Generator(device=DEV).manual_seed(k)
+    a, w = torch.randn(m, k, device=DEV, generator=g), torch.randn(n, k, device=DEV, generator=g) * 0.03
+    if what == "row":
+        a[1] = float("nan")
+    elif what == "number":
+        a[1, k - 2] = float("nan")
+    elif what == "rows":
+        a[:] = float("nan")
+    else:
+        w[7, k // 2] = float("nan")
+    got, want = run(ops, 0, a, w), chain(ops, a, w)
+    assert torch.equal(got.isnan(), want.isnan()) and got.isfinite().equal(want.isfinite())
+    times = []
+    for ops.tensor_cores in (True, False):
+        out = torch.empty(m, n, device=DEV)
+        times.append(time_of(lambda: ops.linear(out, a, w)))
+    assert times[0] <= 2 * times[1]
