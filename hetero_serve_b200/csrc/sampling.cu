@@ -547,20 +547,20 @@ sample_smem_kernel(int* __restrict__ out, const float* __restrict__ logits,
 // The same rule, decision for decision and sum for sum, for long rows: block c of the cluster does the work
 // of threads 128 c .. 128 c + 127 of the kernel above and holds their positions.  Maxima, histograms and the
 // warps' sums meet in shared memory of the cluster; the sums of a thread, of a warp and over the warps are
-// formed in the order above, so the tokens are the same ones.  Of the maxima of each block's pairs of threads (for k
-// up to 64 its groups of four) the (k/8)-th largest is found by counting; the smallest of these eight bounds the k
-// largest entries from below (there are k maxima, so k entries, from it up).  The entries from it up are listed,
-// every block gathers all lists and counts again, more than a block has threads each for the entries it listed
-// itself (all of them in every block, of 64 groups: 64 x 32,000, k = 256, 101 us).  Where they are too many, and for
-// k above 200, the threshold is found a digit of eight bits at a time with histograms that meet in the cluster (us,
-// list against digits: 64 x 32,000 k = 112 27.2 and 27.2, k = 256 32.5 and 27.2; 32 x 50,257 k = 200 23.2 and 26.2,
-// k = 320 28.2 and 26.2).  One block a row leaves most SMs idle at the batches that sample, and its 50,257
-// exponentials and quotients take one SM 20 us.  us, a block a row against a cluster, without top-k, k = 40, k = 2,000
-// and greedy: 32 x 50,257 22.8 and 13.7, 29.1 and 16.5, 45.6 and 27.1, 7.9 and 5.1; 64 x 32,000 16.6 and 13.6, 22.1 and
-// 17.9, 32.8 and 27.8, 5.4 and 4.9 (k = 160 24.5 and 28.6: the one range that loses, with 24,576 columns 21.7 and 27.3).
-// Shorter rows and larger batches gain nothing: 64 x 16,384 10.2 and 10.8, 128 x 32,000 16.6 and 20.3.
+// formed in the order above, so the tokens are the same ones.  Of the maxima of each block's 64 groups of four
+// threads the (k/8)-th largest is found by counting; the smallest of these eight bounds the k largest entries
+// from below (there are k maxima, so k entries, from it up).  The entries from it up are listed, every block
+// gathers all lists and counts again, where there are more than a block has threads each for the entries it listed
+// itself (all of them in every block: 64 x 32,000, k = 200, 63 us against 27).  Where they are too many, and for k
+// above 200, the threshold is found a digit of eight bits at a time with histograms that meet in the cluster (us, k =
+// 200 and 256: 32 x 50,257 21.4 and 25.4, 64 x 32,000 27.0 and 26.6; as a list k = 256 took 47 and 101 in every block).
+// One block a row leaves most SMs idle at the batches that sample, and its 50,257 exponentials and quotients take one SM
+// 20 us.  us, a block a row against a cluster, without top-k, k = 40, k = 2,000 and greedy: 32 x 50,257 22.8 and 13.7,
+// 29.1 and 16.5, 45.6 and 27.1, 7.9 and 5.1; 64 x 32,000 16.6 and 13.6, 22.1 and 17.9, 32.8 and 27.8, 5.4 and 4.9 (k of
+// 80 to 400 is the range that loses there: 160 24.5 and 26.1; with 24,576 columns 21.7 and 25.8; 48 rows gain).  Shorter
+// rows and larger batches gain nothing: 64 x 16,384 10.2 and 10.8, 128 x 32,000 16.6 and 20.3.
 constexpr int SC_BLOCKS = 8, SC_THREADS = 256, SC_OWN = 128;   // of a cluster; a block; positions' owners
-constexpr int SC_GROUPS = SC_THREADS / 4, SC_GROUP_K = 64;      // of four threads; the largest k they serve
+constexpr int SC_GROUPS = SC_THREADS / 4;                       // of four threads: a block's maxima
 constexpr int SC_LIST_K = 200;                                  // the largest k that lists
 constexpr int SC_LIST = 512, SC_CAND = 1024;                   // entries a block may list, a cluster
 constexpr uint32_t SC_LOWEST = 0x007fffffu;                    // the key of minus infinity
@@ -614,7 +614,7 @@ sample_cluster_kernel(int* __restrict__ out, const float* __restrict__ logits,
                       const int* __restrict__ feedback_slot, const int* __restrict__ status_word) {
   extern __shared__ float s_row[];                  // [SC_OWN * C]: logits, then weights (-1: dropped)
   __shared__ int hist[2][256], s_tot[256];
-  __shared__ __align__(16) uint32_t s_key[2 * SC_GROUPS], s_list[SC_LIST], s_cand[SC_CAND];
+  __shared__ __align__(16) uint32_t s_key[SC_GROUPS], s_list[SC_LIST], s_cand[SC_CAND];
   __shared__ int s_digit, s_above, s_same, s_count, s_found, s_last, s_bound, s_n;
   __shared__ float s_max[SC_THREADS / 32], s_own, s_sum[SC_OWN / 32], s_warps[32];
   __shared__ int s_eq[SC_OWN / 32];
@@ -682,12 +682,11 @@ sample_cluster_kernel(int* __restrict__ out, const float* __restrict__ logits,
   }
   const int k = top_k[rowi];
   const bool use_k = k > 0 && k < vocab;
-  const bool coarse = k <= SC_GROUP_K;                   // maxima of four threads, else of two
   {
     uint32_t key = tid < size ? order_key(m) : 0u;
     key = max(key, __shfl_xor_sync(0xffffffffu, key, 1));
-    if (coarse) key = max(key, __shfl_xor_sync(0xffffffffu, key, 2));
-    if ((tid & (coarse ? 3 : 1)) == 0) s_key[coarse ? tid >> 2 : tid >> 1] = key;
+    key = max(key, __shfl_xor_sync(0xffffffffu, key, 2));
+    if ((tid & 3) == 0) s_key[tid >> 2] = key;
     const float w = warp_max(m);
     if (lane == 0) s_max[warp] = w;
     __syncthreads();
@@ -698,17 +697,9 @@ sample_cluster_kernel(int* __restrict__ out, const float* __restrict__ logits,
     }
   }
   const int share = (k + SC_BLOCKS - 1) / SC_BLOCKS;     // of the k maxima this block answers for
-  const int maxima = coarse ? SC_GROUPS : 2 * SC_GROUPS;
-  if (use_k && k <= SC_LIST_K && tid < maxima) {         // (whole warps) the largest with `share` from it up
-    const uint32_t key = s_key[tid];
-    int n = 0;
-#pragma unroll 4
-    for (int i = 0; i < maxima; i += 4) {
-      const uint4 x = *(const uint4*)(s_key + i);
-      n += (x.x >= key) + (x.y >= key) + (x.z >= key) + (x.w >= key);
-    }
-    const uint32_t most = __reduce_max_sync(0xffffffffu, n >= share ? key : 0u);
-    if (lane == 0) atomicMax((unsigned*)&s_bound, most);
+  if (use_k && k <= SC_LIST_K && tid < SC_GROUPS) {
+    const int2 n = sc_rank_of(s_key[tid], s_key, SC_GROUPS);
+    if (n.x < share && share <= n.x + n.y) s_bound = (int)s_key[tid];
   }
   sc_sync();
   float top = lane < SC_BLOCKS ? sc_read(&s_own, lane) : -INFINITY;
@@ -726,16 +717,11 @@ sample_cluster_kernel(int* __restrict__ out, const float* __restrict__ logits,
     bound = b;
     if (bound > SC_LOWEST) {                             // (from minus infinity up it would be the whole row)
 #pragma unroll 4
-      for (int i0 = warp * 32; i0 < size; i0 += SC_THREADS) {
-        const int i = i0 + lane;
-        const uint32_t key = i < size ? order_key(s_row[i]) : 0u;
-        const bool in = i < size && key >= bound;
-        const unsigned all = __ballot_sync(0xffffffffu, in);
-        if (all) {                                       // (one addition a warp: rows can be all of one number)
-          int at = 0;
-          if (lane == 0) at = atomicAdd(&s_n, __popc(all));
-          at = __shfl_sync(0xffffffffu, at, 0) + __popc(all & ((1u << lane) - 1u));
-          if (in && at < SC_LIST) s_list[at] = key;
+      for (int i = tid; i < size; i += SC_THREADS) {
+        const uint32_t key = order_key(s_row[i]);
+        if (key >= bound) {
+          const int at = atomicAdd(&s_n, 1);
+          if (at < SC_LIST) s_list[at] = key;
         }
       }
       sc_sync();
@@ -769,6 +755,7 @@ sample_cluster_kernel(int* __restrict__ out, const float* __restrict__ logits,
         for (int j = i; j < (shared ? end : n); j += SC_THREADS) {
           const int2 r = sc_rank_of(s_cand[j], s_cand, (n + 3) & ~3);
           if (r.x < k && k <= r.x + r.y)                 // the same for all entries equal to it
+#pragma unroll 1
             for (int b = shared ? 0 : rank; b <= (shared ? SC_BLOCKS - 1 : rank); ++b) {
               sc_write(&s_tot[0], b, (int)s_cand[j]);
               sc_write(&s_tot[1], b, r.x);
