@@ -825,9 +825,7 @@ delta_blocks_kernel(float* __restrict__ o, float* __restrict__ state,
   }
 }
 
-// One block per token and head: the head's root mean square by a block reduction, then one
-// thread per output forms its gate (a sum over the rg inputs, several loads in flight).
-// The same where W_g2 g was formed as a matrix product and a head has 32 to 256 values, a multiple of 32: a
+// The gated norm of a head's outputs where W_g2 g was formed as a matrix product and a head has 32 to 256 values, a multiple of 32: a
 // warp a token and head, its sums those of the four warps of a block below (the same bits).  2,048 tokens, 8
 // heads of 128: 21 us in blocks a token and head, 9.7 so.
 template <typename TO>
@@ -860,6 +858,8 @@ delta_finish_rows_kernel(TO* __restrict__ out, const float* __restrict__ o,
   }
 }
 
+// One block per token and head: the head's root mean square by a block reduction, then one
+// thread per output forms its gate (a sum over the rg inputs, several loads in flight).
 template <typename TO>
 __global__ void __launch_bounds__(128)
 delta_finish_kernel(TO* __restrict__ out, const float* __restrict__ o,
@@ -915,13 +915,14 @@ static int delta_shape(hs::DeltaShape* s, int heads, int kv_heads, int D, int V,
   return HS_OK;
 }
 
+// rows_form: a warp over several tokens or a head (1) or a block a token (0); -1: decided here.
 HS_EXPORT int hs_delta_prepare(float* qn, float* kn, float* vv, float* beta, float* decay,
                                const float* proj, const float* conv_w, const float* a2,
                                const float* dt_bias, const float* A_log, float* state,
                                const int* tok_req, const int* req_start, const int* req_len,
                                const int* req_slot, int n_tokens, int n_requests, int heads,
                                int kv_heads, int D, int V, int taps, int ra, int rg,
-                               const float* z_a, void* stream) {
+                               const float* z_a, int rows_form, void* stream) {
   if (!qn || !kn || !vv || !beta || !decay || !proj || !conv_w || !a2 || !dt_bias || !A_log ||
       !state || !tok_req || !req_start || !req_len || !req_slot)
     return HS_ERR_ARGUMENT;
@@ -937,7 +938,19 @@ HS_EXPORT int hs_delta_prepare(float* qn, float* kn, float* vv, float* beta, flo
   const bool four = taps == 4 && widest > 512 && n_tokens >= 512 && n_tokens >= 8 * n_requests;
   const bool pdl = hs_pdl_enabled();
   cudaError_t e;
-  if (four && D % 32 == 0 && D <= 128) {
+  // Eight tokens a warp where there is work for many warps and few of the eights straddle portions: us, a block a
+  // token against eight tokens a warp, 8 heads of 128 (W_a2 a handed in): 768 tokens 18.6 and 20.5, 1,536 30.1 and
+  // 26.2, in portions of 64 31.1 and 28.4, of 16 32.9 and 33.8; 4 heads, 1,536 20.2 and 20.7, 4,096 45.5 and 28.2;
+  // heads of 64 gain later (16 of them, 1,536 tokens 32.9 and 33.5, 4,096 91.7 and 71.8), heads of 32 not at all (64
+  // of them, 4,096 190 and 209).  Where the warps form W_a2 a themselves: 8 heads of 128, 2,048 tokens 104 and 108,
+  // 4,096 249 and 181; 16 heads, 512 tokens 66 and 97, 768 114 and 103, 1,536 236 and 158.
+  const long long size = (long long)n_tokens * heads * D;
+  bool rows = four && size >= (heads * D >= 2048 ? 3LL << 19 : 9LL << 18);
+  if (z_a)
+    rows = four && D >= 64 && n_tokens >= 32LL * n_requests &&
+           size * D >= (n_tokens >= 128LL * n_requests ? 128LL : 160LL) << 20;
+  if (rows_form >= 0) rows = rows_form && taps == 4;
+  if (rows && D % 32 == 0 && D <= 128) {
     const int groups = 2 * kv_heads + (heads * V + 127) / 128 + (heads * D + 127) / 128;
     e = hs_launch(hs::delta_prepare_rows_kernel, dim3((n_tokens + hs::DP_TOK - 1) / hs::DP_TOK, (groups + 3) / 4),
                   dim3(128), 0, st, pdl, qn, kn, vv, beta, decay, proj, conv_w, a2, dt_bias, A_log,
@@ -1048,10 +1061,11 @@ HS_EXPORT int hs_delta_recurrence(float* o, float* state, const float* qn, const
   return HS_OK;
 }
 
+// rows_form: a warp over several tokens or a head (1) or a block a token (0); -1: decided here.
 HS_EXPORT int hs_delta_finish(void* out, const float* o, const float* proj, const float* g2,
                               const float* norm_w, const int* tok_req, int n_tokens, float eps,
                               int heads, int kv_heads, int D, int V, int taps, int ra, int rg,
-                              int out_dtype, const float* z_g, void* stream) {
+                              int out_dtype, const float* z_g, int rows_form, void* stream) {
   if (!out || !o || !proj || !g2 || !norm_w || !tok_req) return HS_ERR_ARGUMENT;
   hs::DeltaShape s;
   int rc = delta_shape(&s, heads, kv_heads, D, V, taps, ra, rg);
@@ -1062,7 +1076,7 @@ HS_EXPORT int hs_delta_finish(void* out, const float* o, const float* proj, cons
   cudaError_t e;
   auto go = [&](auto* dst) {
     using TO = std::remove_pointer_t<decltype(dst)>;
-    if (z_g && V % 32 == 0 && V <= 256)
+    if (z_g && rows_form != 0 && V % 32 == 0 && V <= 256)
       e = hs_launch(hs::delta_finish_rows_kernel<TO>, dim3(((long long)n_tokens * heads + 7) / 8), dim3(256), 0,
                     st, pdl, dst, o, norm_w, tok_req, eps, s, z_g, n_tokens);
     else

@@ -229,10 +229,10 @@ def _declare(lib) -> None:
         "hs_latent_prefill_mma": [P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, I, I, I, P, P,
                                   I, I, P],
         "hs_latent_prefill_mma_takes": [I, I],
-        "hs_delta_prepare": [P] * 15 + [I] * 9 + [P, P],
+        "hs_delta_prepare": [P] * 15 + [I] * 9 + [P, I, P],
         "hs_delta_recurrence": [P] * 10 + [I] * 11 + [P, P, P],
         "hs_delta_blocks_scratch": [I, I, I, I, I, P],
-        "hs_delta_finish": [P, P, P, P, P, P, I, F, I, I, I, I, I, I, I, I, P, P],
+        "hs_delta_finish": [P, P, P, P, P, P, I, F, I, I, I, I, I, I, I, I, P, I, P],
         "hs_moe_route": [P, P, P, P, P, I, I, I, I, I, I, I, P, P],
         "hs_moe_experts": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, F, I, I, P, P, I, I, P, P],
         "hs_moe_route_softmax": [P, P, P, P, P, P, I, I, I, I, F, I, P, P],
@@ -394,6 +394,7 @@ class CudaOps:
         self.f32_tiles = True       # float32 prompt portions of heads of 64 as tiles of queries
         self.f32_single = True      # ... and their single tokens with chunks fetched ahead
         self.delta_blocks = True    # portions of the delta rule four tokens at a time
+        self.delta_rows = -1        # its pre-pass and finish by warps (1) or a block a token (0); -1: by size
         self.latent_splits = None   # blocks a token's keys are split over in latent attention
         #                             (None: chosen from the number of tokens in the step)
         self.sorted_experts = True  # many (token, expert) pairs in bfloat16: sorted by expert and
@@ -1486,7 +1487,7 @@ class CudaOps:
             _ptr(qn), _ptr(kn), _ptr(vv), _ptr(beta), _ptr(decay), _ptr(proj), _ptr(conv_w),
             _ptr(a2), _ptr(dt_bias), _ptr(a_log), _ptr(state), _ptr(tok_req), _ptr(req_start),
             _ptr(req_len), _ptr(req_slot), proj.shape[0], req_start.shape[0], H, HK, D, V, taps,
-            ra, rg, _ptr(z_a), self._stream()), "delta_prepare")
+            ra, rg, _ptr(z_a), int(self.delta_rows), self._stream()), "delta_prepare")
 
     # Tokens from which on a request goes four tokens at a time, by head size.  us, token after token
     # against blocks of four: 8 heads of 64, 16 portions of 32 tokens 18.5 and 19.5, 8 of 64 25.6 and
@@ -1534,8 +1535,8 @@ class CudaOps:
         self.launches += 1
         _check(self.lib.hs_delta_finish(
             _ptr(out), _ptr(o), _ptr(proj), _ptr(g2), _ptr(norm_w), _ptr(tok_req), out.shape[0],
-            float(eps), H, HK, D, V, taps, ra, rg, _DT[out.dtype], _ptr(z_g), self._stream()),
-            "delta_finish")
+            float(eps), H, HK, D, V, taps, ra, rg, _DT[out.dtype], _ptr(z_g), int(self.delta_rows),
+            self._stream()), "delta_finish")
 
     # -- routed feed-forward ---------------------------------------------------------------
     def moe_route(self, sel_idx, sel_w, h, w_router, tok_req, *, top, n_groups, keep, z=None):
