@@ -1338,6 +1338,24 @@ static TcShape pick_shape(int M, int N, int num_kb, int pair, int sms) {
   return best;
 }
 
+// The tile of a very wide layer of few rows: the width that leaves an SM the fewest columns, the wider of two that
+// leave it as many, since that keeps more of the weights on their way; 256 columns only of up to 64 rows, beyond
+// which its epilogue is what takes long.  us at 128, 192 and 256 wide, 1,024 summed: 32 x 18,944 12.4, 13.0, 21.7; 32 x
+// 28,160 17.9, 15.2, 16.8; 32 x 32,000 18.9, 17.7, 16.9; 32 x 50,257 30.4, 26.5, 31.0; 1,280 summed: 100 x 25,600 18.4, 16.4,
+// 18.0; 100 x 32,000 20.1, 24.3, 21.5; 100 x 40,000 27.5, 26.0, 31.2.
+static int wide_tile(int M, int N, int sms) {
+  int best = 0;
+  long least = 0;
+  for (int bn = 128; bn <= (M <= 64 ? 256 : 192); bn += 64) {
+    const long columns = (long)(((N + bn - 1) / bn + sms - 1) / sms) * bn;
+    if (!best || columns <= least) {
+      best = bn;
+      least = columns;
+    }
+  }
+  return best;
+}
+
 // pair: -1 = decide here, 0 = single CTAs, 1 = pairs of CTAs (256-row tiles)
 static bool plan_tc(int M, int N, int K, int tile_n, int pair, TcPlan& pl) {
   int sms = 148;
@@ -1353,10 +1371,8 @@ static bool plan_tc(int M, int N, int K, int tile_n, int pair, TcPlan& pl) {
     pl.pair = shape.pair;
   } else if (bn == 0) {
     // few rows: narrow tiles (more CTAs stream the weights) and splits; a very wide layer (the
-    // vocabulary) has tiles enough, and wide ones keep more of the weights on their way (50,257 columns,
-    // us at 64, 128, 192 and 256 wide: 32 x 1,024 37, 29, 26, 30; 17 x 1,600 65, 48, 36, 37; 64 x 768 28, 22,
-    // 21, 27)
-    bn = ((N + 63) / 64 >= 2 * sms) ? 192 : 64;
+    // vocabulary) has tiles enough
+    bn = ((N + 63) / 64 >= 2 * sms) ? wide_tile(M, N, sms) : 64;
   }
   if (pl.pair) {
     // 256 x BN tiles over sms / 2 pairs; a CTA loads 128 + BN/2 rows per k-block
