@@ -472,12 +472,15 @@ HS_EXPORT int hs_lightning_scratch(int n_tokens, int n_requests, int H, int D, i
   return HS_OK;
 }
 
-// Floats of scratch with which requests of many tokens go in chunks (0: none can).
+// Floats of scratch with which requests of many tokens go in chunks (0: none can), and how many groups of heads
+// take turns with it.
 HS_EXPORT int hs_lightning_chunk_scratch(int n_tokens, int n_requests, int H, int D, int V, int rot_dims,
-                                         long long* floats) {
-  if (!floats || n_tokens < 0 || n_requests < 0 || H <= 0 || D <= 0 || V <= 0) return HS_ERR_ARGUMENT;
+                                         long long* floats, int* groups) {
+  if (!floats || !groups || n_tokens < 0 || n_requests < 0 || H <= 0 || D <= 0 || V <= 0) return HS_ERR_ARGUMENT;
   *floats = hs::lightning_takes_chunks(D, V, rot_dims)
                 ? hs::lightning_chunk_floats(n_tokens, n_requests, H, D, V, rot_dims) : 0;
+  const int heads = hs::lightning_chunk_heads(n_tokens, n_requests, H, D, V);
+  *groups = (H + heads - 1) / heads;
   return HS_OK;
 }
 

@@ -36,10 +36,19 @@ __host__ __device__ constexpr int lightning_chunk_slots(int n_tokens, int n_requ
   return n_tokens < LC_MIN ? 0 : n_tokens / 64 + (n_requests < n_tokens / LC_MIN ? n_requests : n_tokens / LC_MIN);
 }
 
-// floats of scratch: a state of all heads a chunk, the tokens' cosines and sines (0: no chunks)
+// Heads that go together: a state a chunk and head is scratch, 64 KB, and a step's heads share 128 MB of it (8,192
+// tokens of 64 heads: 5 groups of 13, where all at once would keep 0.6 GB).
+constexpr long long LC_SCRATCH = 1LL << 25;
+constexpr int lightning_chunk_heads(int n_tokens, int n_requests, int H, int D, int V) {
+  const long long a_head = (long long)lightning_chunk_slots(n_tokens, n_requests) * D * V;
+  const long long most = a_head == 0 || LC_SCRATCH / a_head > H ? H : LC_SCRATCH / a_head < 1 ? 1 : LC_SCRATCH / a_head;
+  const long long groups = (H + most - 1) / most;
+  return (int)((H + groups - 1) / groups);
+}
+// floats of scratch: a state of these heads a chunk, the tokens' cosines and sines (0: no chunks)
 constexpr long long lightning_chunk_floats(int n_tokens, int n_requests, int H, int D, int V, int rot_dims) {
   const long long slots = lightning_chunk_slots(n_tokens, n_requests);
-  return slots ? slots * H * D * V + (long long)n_tokens * rot_dims : 0;
+  return slots ? slots * lightning_chunk_heads(n_tokens, n_requests, H, D, V) * D * V + (long long)n_tokens * rot_dims : 0;
 }
 
 bool lightning_takes_chunks(int D, int V, int rot_dims);

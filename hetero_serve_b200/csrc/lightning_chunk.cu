@@ -36,6 +36,7 @@ constexpr float LC_BIG = 1e38f;      // a number beyond this may have no first t
 
 struct LcShape {
   int H, stride, q_off, k_off, v_off, act, rot_dims, n_requests;
+  int h0, heads;                     // the group of heads of this launch: from which on, how many
   float k_scale;
   const float2* turns;               // [tokens][rot_dims / 2] cosine and sine of the tokens' angles
 };
@@ -293,7 +294,7 @@ lightning_chunk_state_kernel(float* __restrict__ dS, const float* __restrict__ p
   __shared__ float s_w[LC_LEN];
   pdl_trigger();
   pdl_wait();
-  const int slot = blockIdx.x, h = blockIdx.y;
+  const int slot = blockIdx.x, h = s.h0 + blockIdx.y;
   int r, c;
   if (!lc_find(req_len, s.n_requests, slot, r, c)) return;
   const int n = min(LC_LEN, req_len[r] - c * LC_LEN), t0 = req_start[r] + c * LC_LEN;
@@ -326,7 +327,7 @@ lightning_chunk_state_kernel(float* __restrict__ dS, const float* __restrict__ p
       lc_store(sV + i * VS + v, LC_LEN * VS, a[u]);
     }
   }
-  float* out = dS + ((size_t)slot * s.H + h) * LC_D * LC_V;
+  float* out = dS + ((size_t)slot * s.heads + blockIdx.y) * LC_D * LC_V;
   if (__syncthreads_or(odd)) {
     for (int i = threadIdx.x; i < LC_D * LC_V; i += LC_THREADS) out[i] = 0.f;
     __syncthreads();
@@ -379,7 +380,7 @@ lightning_chunk_chain_kernel(float* __restrict__ dS, float* __restrict__ state,
                              const int* __restrict__ req_slot, const LcShape s) {
   pdl_wait();
   pdl_trigger();
-  const int h = blockIdx.y, size = LC_D * LC_V, i = (blockIdx.x * LC_THREADS + threadIdx.x) * 4;
+  const int h = s.h0 + blockIdx.y, size = LC_D * LC_V, i = (blockIdx.x * LC_THREADS + threadIdx.x) * 4;
   int r = 0, chunks = 0, first = 0;                        // the blockIdx.z-th request in chunks, the chunks before
   for (int nth = 0; r < s.n_requests; ++r) {
     chunks = lc_chunks(req_len[r]);
@@ -388,8 +389,8 @@ lightning_chunk_chain_kernel(float* __restrict__ dS, float* __restrict__ state,
   }
   if (r == s.n_requests || i >= size) return;
   float4* slot = (float4*)(state + ((size_t)req_slot[r] * s.H + h) * size + i);
-  float4* x = (float4*)(dS + ((size_t)first * s.H + h) * size + i);
-  const size_t next = (size_t)s.H * size / 4;              // from a chunk to the next
+  float4* x = (float4*)(dS + ((size_t)first * s.heads + blockIdx.y) * size + i);
+  const size_t next = (size_t)s.heads * size / 4;              // from a chunk to the next
   const float g = decay[h], whole = (float)lc_power(g, LC_LEN);
   const float end = (float)lc_power(g, req_len[r] - (chunks - 1) * LC_LEN);
   // a power that is below the range of numbers is zero, but no factor of the recurrence was: an infinity goes on
@@ -426,7 +427,7 @@ lightning_chunk_out_kernel(float* __restrict__ o, float* __restrict__ states,
   __shared__ float s_p[LC_LEN + 1];                        // powers of the decay
   pdl_trigger();
   pdl_wait();
-  const int slot = blockIdx.x, h = blockIdx.y;
+  const int slot = blockIdx.x, h = s.h0 + blockIdx.y;
   int r, c;
   if (!lc_find(req_len, s.n_requests, slot, r, c)) return;
   const int n = min(LC_LEN, req_len[r] - c * LC_LEN), t0 = req_start[r] + c * LC_LEN;
@@ -435,7 +436,7 @@ lightning_chunk_out_kernel(float* __restrict__ o, float* __restrict__ states,
   __nv_bfloat16* sQ = (__nv_bfloat16*)lc_smem;             // [3][LC_LEN][DS]
   __nv_bfloat16* sK = sQ + 3 * LC_LEN * DS;                // the same; later the weights [3][LC_LEN][PS]
   if (threadIdx.x <= LC_LEN) s_p[threadIdx.x] = (float)lc_power(g, threadIdx.x);
-  float* S = states + ((size_t)slot * s.H + h) * LC_D * LC_V;
+  float* S = states + ((size_t)slot * s.heads + blockIdx.y) * LC_D * LC_V;
   bool odd = lc_rows<true>(sQ, sK, proj, s, h, t0, n, nullptr);
   if (__syncthreads_or(odd)) {                             // (nothing below would be of use)
     lc_walk<true>(S, o, proj, s, h, t0, n, g);
@@ -604,7 +605,8 @@ int lightning_chunks(float* o, float* state, const float* proj, const float* dec
   const int slots = lightning_chunk_slots(n_tokens, n_requests);
   const bool pdl = hs_pdl_enabled();
   const int smem_a = 3 * LC_LEN * (LC_DS + LC_VS) * 2, smem_c = 6 * LC_LEN * LC_DS * 2;
-  s.turns = (const float2*)(scratch + (size_t)slots * H * D * V);
+  const int group = lightning_chunk_heads(n_tokens, n_requests, H, D, V);
+  s.turns = (const float2*)(scratch + (size_t)slots * group * D * V);
   cudaError_t e = cudaSuccess;
   if (rot_dims) {
     const int size = n_tokens * (rot_dims / 2);
@@ -617,15 +619,19 @@ int lightning_chunks(float* o, float* state, const float* proj, const float* dec
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(lightning_chunk_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_c);
   if (e != cudaSuccess) return (int)e;
-  e = hs_launch(lightning_chunk_state_kernel, dim3(slots, H), dim3(LC_THREADS), (size_t)smem_a, st, pdl,
-                scratch, proj, decay, req_start, req_len, s);
-  if (e != cudaSuccess) return (int)e;
   const int most = n_requests < n_tokens / LC_MIN ? n_requests : n_tokens / LC_MIN;
-  e = hs_launch(lightning_chunk_chain_kernel, dim3((D * V / 4 + LC_THREADS - 1) / LC_THREADS, H, most),
-                dim3(LC_THREADS), 0, st, pdl, scratch, state, decay, req_len, req_slot, s);
-  if (e != cudaSuccess) return (int)e;
-  e = hs_launch(lightning_chunk_out_kernel, dim3(slots, H), dim3(LC_THREADS), (size_t)smem_c, st, pdl, o,
-                scratch, proj, decay, req_start, req_len, s);
+  for (s.h0 = 0; s.h0 < H; s.h0 += group) {
+    s.heads = H - s.h0 < group ? H - s.h0 : group;
+    e = hs_launch(lightning_chunk_state_kernel, dim3(slots, s.heads), dim3(LC_THREADS), (size_t)smem_a, st, pdl,
+                  scratch, proj, decay, req_start, req_len, s);
+    if (e != cudaSuccess) return (int)e;
+    e = hs_launch(lightning_chunk_chain_kernel, dim3((D * V / 4 + LC_THREADS - 1) / LC_THREADS, s.heads, most),
+                  dim3(LC_THREADS), 0, st, pdl, scratch, state, decay, req_len, req_slot, s);
+    if (e != cudaSuccess) return (int)e;
+    e = hs_launch(lightning_chunk_out_kernel, dim3(slots, s.heads), dim3(LC_THREADS), (size_t)smem_c, st, pdl, o,
+                  scratch, proj, decay, req_start, req_len, s);
+    if (e != cudaSuccess) return (int)e;
+  }
   return (int)e;
 }
 

@@ -249,7 +249,7 @@ def _declare(lib) -> None:
         "hs_lightning_recurrence": [P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, P, P, P, I,
                                     F, P, I, P, P],
         "hs_lightning_scratch": [I, I, I, I, I, P],
-        "hs_lightning_chunk_scratch": [I, I, I, I, I, I, P],
+        "hs_lightning_chunk_scratch": [I, I, I, I, I, I, P, P],
         "hs_token_shift_mix": [P, P, P, P, I, I, P, P, P, P, I, I, I, I, P],
         "hs_timemix_decay": [P, P, P, P, I, I, I, P],
         "hs_timemix_recurrence": [P, P, I, P, P, P, P, P, P, P, P, I, I, I, I, P],
@@ -1971,12 +1971,12 @@ class CudaOps:
         parts = None
         above, below = (True, True) if plan is None else plan.side(self.LIGHTNING_LONG)
         if chunks and above:
-            need = ctypes.c_longlong(0)
+            need, groups = ctypes.c_longlong(0), ctypes.c_int(0)
             self.lib.hs_lightning_chunk_scratch(T, req_start.shape[0], heads, dim, vdim, int(rot_dims),
-                                                ctypes.byref(need))
+                                                ctypes.byref(need), ctypes.byref(groups))
             if need.value:
                 parts = self._scratch_buffer("lightning_chunks", need.value, torch.float32)
-                self.launches += 4 if rot_dims else 3
+                self.launches += 3 * groups.value + (rot_dims > 0)
         if parts is None or below:
             self.launches += 2 if scratch is not None else 1
         _check(self.lib.hs_lightning_recurrence(

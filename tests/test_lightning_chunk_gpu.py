@@ -220,3 +220,22 @@ def test_requests_in_chunks_among_many():
         one, sone = run(ops, (n,), proj[at:at + n].clone(), state[[0, slot]].clone(), pos[at:at + n], *rest, chunks=True)
         assert torch.equal(one, o[at:at + n]) and torch.equal(sone[1], S[slot])
     assert torch.equal(S[0], state[0])
+
+
+@pytest.mark.parametrize("rot", [0, 128])
+def test_heads_that_take_turns_with_the_scratch(rot):
+    """More heads than the scratch holds states of: bounded, and each head has the bits it has in a part of them."""
+    H, D, V, lens = 40, 128, 128, (4096, 20, 513)
+    ops, decay = CudaOps(DEV), torch.linspace(0.5, 0.999, H, device=DEV)
+    proj, state, pos, freq = inputs(lens, H, D, V, rot, 17)
+    o, S = run(ops, lens, proj, state, pos, freq, decay, H, D, V, rot, "none", 0.5, chunks=True)
+    held = sum(t.numel() for (name, _), t in ops._scratch.items() if name == "lightning_chunks")
+    assert 0 < held <= 2 ** 25 + sum(lens) * rot
+    for h0 in (0, 15, 35):                                  # five heads at a time
+        cols = torch.cat([torch.arange(2 + b + h0 * 128, 2 + b + (h0 + 5) * 128) for b in (0, H * D, 2 * H * D)])
+        part = torch.cat([proj[:, :2], proj[:, cols.to(DEV)]], 1).contiguous()
+        st = state.view(-1, H, D * V)[:, h0:h0 + 5].reshape(-1, 5 * D * V).contiguous()
+        po, pS = run(CudaOps(DEV), lens, part, st, pos, freq, decay[h0:h0 + 5].contiguous(), 5, D, V, rot, "none", 0.5,
+                     chunks=True)
+        assert torch.equal(po, o[:, h0 * V:(h0 + 5) * V])
+        assert torch.equal(pS, S.view(-1, H, D * V)[:, h0:h0 + 5].reshape(-1, 5 * D * V))
