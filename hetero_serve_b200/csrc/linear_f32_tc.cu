@@ -280,6 +280,7 @@ __global__ void __launch_bounds__(LF_THREADS, 1) linear_f32_tc_kernel(const __gr
   if (warp == LF_CONV + LF_SUM) {
     constexpr uint32_t idesc = make_idesc(LF_BM, NR);
     constexpr uint64_t TA = LF_A_TERM >> 4, TB = S::B_TERM >> 4;
+    pdl_wait();                      // (the limit of the waits is not for the kernel before)
     uint32_t limit = HS_SPIN_LIMIT;
     int s = 0, round = 0, cc = 0;
     for (int w = blockIdx.x; w < p.items; w += gridDim.x) {
