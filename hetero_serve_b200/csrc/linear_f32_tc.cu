@@ -24,18 +24,25 @@
 //                 of shared memory) and finish the tile: a lane owns a feature, a column is a row of `a`,
 //                 so loads and stores are 128 contiguous bytes a warp;
 //   warp 12       issues the MMAs.
-// With few tiles the segments of a tile are shared out between blocks: each segment's sums go to scratch
-// and a second kernel adds them in order.
+// With few tiles the segments of a tile, or its single chunks, are shared out between blocks: their sums go to scratch
+// and a second kernel adds them in the same order.
 //
-// 1,024 x 4,096 x 1,024: 223 us as FMA chains (linear_simt.cu) -> 68; 1,024 x 1,024 x 4,096: 317 -> 85; 64 x
-// 4,096 x 1,024: 29 -> 18; 8 x 1,024 x 4,096: 19 -> 11.  A chunk of a 128 x 128 tile takes 1.8 us: 24 MMAs
-// that read 8 KB of shared memory each (1.5 us alone) beside the stores of terms.
+// Operands below 2^-109 have a third term below bfloat16's range: a product is off by 2^-134 of the other operand at
+// most, where a chain would keep their digits.
+//
+// Operands below 2^-109 have a third term below bfloat16's range: a product is off by 2^-134 of the other operand at
+// most, where a chain would keep their digits.
+//
+// 1,024 x 4,096 x 1,024: 223 us as FMA chains (linear_simt.cu) -> 68; 1,024 x 1,024 x 4,096: 317 -> 82; 64 x
+// 4,096 x 1,024: 29 -> 16; 8 x 1,024 x 4,096: 19 -> 11; 1 x 768 x 768 5.1 -> 5.6 (8.3 with whole segments a block).  A
+// chunk of a 128 x 128 tile takes 1.8 us: 24 MMAs that read 8 KB of shared memory each (1.5 us alone) beside the
+// stores of terms.
 #include "tcgen05.cuh"
 
 namespace hs {
 
 constexpr int LF_BM = 128, LF_BK = 64;
-constexpr int LF_SEG = 4;                 // chunks of 64 a segment holds
+constexpr int LF_SEG = 4;                 // chunks of 64 a segment holds (1 << 2)
 constexpr int LF_CONV = 8, LF_SUM = 4;    // warps
 constexpr int LF_THREADS = 32 * (LF_CONV + LF_SUM + 1);
 constexpr int LF_A_TERM = LF_BM * LF_BK * 2;
@@ -57,7 +64,7 @@ struct LfParams {
   int* status;
   int M, N, K, act;
   float2 act_ab;
-  int tiles_m, segs, splits, segs_per_split, items;
+  int tiles_m, parts, splits, kb_per_split, part_shift, items;   // a part: 1 << part_shift chunks summed up in scratch
 };
 
 __device__ __forceinline__ void lf_tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
@@ -243,8 +250,8 @@ __device__ __forceinline__ LfItem lf_item(const LfParams& p, int w) {
   const int s = w / p.tiles_m, f = s / p.splits;
   r.m0 = (w - s * p.tiles_m) * NR;
   r.f0 = f * LF_BM;
-  r.kb0 = (s - f * p.splits) * p.segs_per_split * LF_SEG;
-  r.kb1 = min(r.kb0 + p.segs_per_split * LF_SEG, (p.K + LF_BK - 1) / LF_BK);
+  r.kb0 = (s - f * p.splits) * p.kb_per_split;
+  r.kb1 = min(r.kb0 + p.kb_per_split, (p.K + LF_BK - 1) / LF_BK);
   return r;
 }
 
@@ -410,7 +417,8 @@ __global__ void __launch_bounds__(LF_THREADS, 1) linear_f32_tc_kernel(const __gr
       const int f = it.f0 + q * 32 + lane, n = min(NR, p.M - it.m0);
       for (int kb = it.kb0; kb < it.kb1; ++kb, ++cc) {
         const int b = cc & 1;
-        const bool opens = kb % LF_SEG == 0, last = kb + 1 == it.kb1, ends = last || (kb + 1) % LF_SEG == 0;
+        const int part = SPLIT ? (1 << p.part_shift) - 1 : LF_SEG - 1;
+        const bool opens = (kb & part) == 0, last = kb + 1 == it.kb1, ends = last || ((kb + 1) & part) == 0;
         ok = mbar_wait(&acc_full[b], (cc >> 1) & 1, p.status);
         if (!ok) break;
         tc_fence_after();
@@ -444,7 +452,7 @@ __global__ void __launch_bounds__(LF_THREADS, 1) linear_f32_tc_kernel(const __gr
         if (SPLIT ? !ends : !last) continue;
         // the sums of a segment (SPLIT) or of the tile, sixteen rows of `a` at a time
         const float bias = !SPLIT && p.bias && f < p.N ? p.bias[f] : 0.f;
-        float* dst = SPLIT ? p.partial + ((size_t)(kb / LF_SEG) * p.M + it.m0) * p.N + f
+        float* dst = SPLIT ? p.partial + ((size_t)(kb >> p.part_shift) * p.M + it.m0) * p.N + f
                            : p.out + (size_t)it.m0 * p.N + f;
         unsigned nans = 0;                       // lanes whose weights hold no number
 #pragma unroll 1
@@ -507,22 +515,33 @@ __global__ void __launch_bounds__(128) linear_f32_tc_sum_kernel(const __grid_con
   const long long size = (long long)p.M * p.N, at = (long long)blockIdx.x * 128 + threadIdx.x;
   const long long i = at < size ? at : size - 1;         // (whole warps come to the end)
   const float* src = p.partial + i;
-  float sum = src[0];
-  int c = 1;
-  for (; c + 8 <= p.segs; c += 8) {
-    float v[8];
+  float sum = 0.f;
+  if (p.part_shift) {                                    // segments
+    for (int c0 = 0; c0 < p.parts; c0 += 8) {
+      float v[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = src[(c + j) * size];
+      for (int j = 0; j < 8; ++j)
+        if (c0 + j < p.parts) v[j] = src[(c0 + j) * size];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) sum += v[j];
+      for (int j = 0; j < 8; ++j)
+        if (c0 + j < p.parts) sum = c0 + j ? sum + v[j] : v[j];
+    }
+  } else {                                               // chunks, four to a segment
+    for (int c0 = 0; c0 < p.parts; c0 += 16) {
+      float v[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        if (c0 + j < p.parts) v[j] = src[(c0 + j) * size];
+#pragma unroll
+      for (int j = 0; j < 16; j += LF_SEG) {
+        if (c0 + j >= p.parts) break;
+#pragma unroll
+        for (int k = 1; k < LF_SEG; ++k)
+          if (c0 + j + k < p.parts) v[j] += v[j + k];
+        sum = c0 + j ? sum + v[j] : v[j];
+      }
+    }
   }
-  float v[7];
-#pragma unroll
-  for (int j = 0; j < 7; ++j)
-    if (c + j < p.segs) v[j] = src[(c + j) * size];
-#pragma unroll
-  for (int j = 0; j < 7; ++j)
-    if (c + j < p.segs) sum += v[j];
   const int m = (int)(i / p.N), n = (int)(i - (long long)m * p.N);
   if (__any_sync(0xffffffffu, !lf_finite(sum))) {
     unsigned nans = 0;
@@ -537,15 +556,18 @@ __global__ void __launch_bounds__(128) linear_f32_tc_sum_kernel(const __grid_con
 }
 
 struct LfPlan {
-  int nr, splits, segs_per_split, tiles_m, segs, items;
+  int nr, splits, kb_per_split, part_shift, parts, tiles_m, items;
 };
 static bool plan_lf(int M, int N, int K, int force_nr, LfPlan& pl) {
-  if (K % 4 || M <= 0 || N <= 0 || K <= 0) return false;
+  // One chunk of 64 is a launch's beginning and end and little else: 4,096 x 1,024 x 16 22.9 us, 9.9 on the CUDA cores, x 64
+  // 22.9 and 21.9 (1,024 x 1,024 x 128: 10.9 and 13.6).  And a sum of up to eight products is no closer to float64 here.
+  if (K % 4 || M <= 0 || N <= 0 || K <= LF_BK) return false;
   const int sms = hs_sm_count(), ft = (N + LF_BM - 1) / LF_BM;
-  const int num_kb = (K + LF_BK - 1) / LF_BK, segs = (num_kb + LF_SEG - 1) / LF_SEG;
+  const int num_kb = (K + LF_BK - 1) / LF_BK;
   // us a chunk takes by rows of the tile, and a tile's beginning and end, measured (148 SMs, 1,024 rows: 16
   // rows a tile 268 us for 14 rounds of 16 chunks, 32 147 for 7, 64 76 for 3 and 84 for one of 64, 128 68
-  // for 2); segments through scratch cost the second launch and their way to the L2 and back
+  // for 2).  A tile's segments, or its single chunks, are shared out through scratch where tiles are few; that costs the second launch
+  // and their way to the L2 and back.
   const int sizes[4] = {16, 32, 64, 128};
   const double step[4] = {0.95, 1.06, 1.26, 1.8};
   double best = -1.0;
@@ -553,20 +575,23 @@ static bool plan_lf(int M, int N, int K, int force_nr, LfPlan& pl) {
     const int nr = sizes[i];
     if (force_nr ? nr != force_nr : (nr > 16 && nr / 2 >= M)) continue;
     const long long mt = (M + nr - 1) / nr, tiles = mt * ft;
-    if (tiles > (1 << 30)) continue;
-    for (int pass = 0; pass < 2; ++pass) {
-      int splits = pass == 0 ? 1 : (int)(sms / tiles < segs ? sms / tiles : segs);
-      if (pass == 1 && splits < 2) continue;
-      const int per = (segs + splits - 1) / splits;
-      splits = (segs + per - 1) / per;
+    if (tiles > (1 << 30) / num_kb) continue;
+    // whole tiles; segments and chunks that fill one round; single chunks, as many as there are
+    for (int form = 0; form < 4; ++form) {
+      const int unit = form == 1 ? LF_SEG : 1, parts = (num_kb + unit - 1) / unit;
+      int splits = form == 0 ? 1 : form == 3 ? parts : (int)(sms / tiles < parts ? sms / tiles : parts);
+      if (form && splits < 2) continue;
+      const int per = form ? (parts + splits - 1) / splits * unit : num_kb;
+      splits = (num_kb + per - 1) / per;
       const double rounds = (double)((tiles * splits + sms - 1) / sms);
-      const int steps = splits > 1 ? per * LF_SEG : num_kb;
-      double cost = rounds * (steps * step[i] + 4.0);
-      if (splits > 1) cost += 3.0 + 8.0 * segs * (double)M * N / 3e6;
+      double cost = form == 3 ? rounds * (step[i] + 0.4) + 4.0 : rounds * (per * step[i] + 4.0);
+      // (the adding kernel has eight segments or sixteen chunks on their way at a time)
+      if (form) cost += 3.0 + 8.0 * parts * (double)M * N / 3e6 + 1.5 * (unit == 1 ? (parts + 15) / 16 : (parts + 7) / 8);
       if (best < 0 || cost < best) {
         best = cost;
-        pl.nr = nr; pl.splits = splits; pl.segs_per_split = per;
-        pl.tiles_m = (int)mt; pl.segs = segs; pl.items = (int)(tiles * splits);
+        pl.nr = nr; pl.splits = form ? splits : 1; pl.kb_per_split = per;
+        pl.part_shift = unit == 1 ? 0 : 2; pl.parts = parts;
+        pl.tiles_m = (int)mt; pl.items = (int)(tiles * splits);
       }
     }
   }
@@ -597,7 +622,7 @@ static int launch_lf(const LfParams& p, cudaStream_t st) {
 HS_EXPORT int hs_linear_f32_tc_scratch(int M, int N, int K, int rows, long long* floats) {
   hs::LfPlan pl;
   if (!hs::plan_lf(M, N, K, rows, pl)) return HS_ERR_UNSUPPORTED;
-  *floats = pl.splits > 1 ? (long long)pl.segs * M * N : 0;
+  *floats = pl.splits > 1 ? (long long)pl.parts * M * N : 0;
   return HS_OK;
 }
 
@@ -617,8 +642,8 @@ HS_EXPORT int hs_linear_f32_tc(float* out, const float* a, const float* w, const
   LfParams p;
   p.out = out; p.a = a; p.w = w; p.bias = bias; p.residual = residual; p.partial = scratch; p.status = status;
   p.M = M; p.N = N; p.K = K; p.act = act; p.act_ab = make_float2(act_a, act_b);
-  p.tiles_m = pl.tiles_m; p.segs = pl.segs; p.splits = pl.splits;
-  p.segs_per_split = pl.segs_per_split; p.items = pl.items;
+  p.tiles_m = pl.tiles_m; p.parts = pl.parts; p.splits = pl.splits;
+  p.kb_per_split = pl.kb_per_split; p.part_shift = pl.part_shift; p.items = pl.items;
   cudaStream_t st = (cudaStream_t)stream;
 #define HS_LF(NR) (pl.splits > 1 ? launch_lf<NR, true>(p, st) : launch_lf<NR, false>(p, st))
   switch (pl.nr) {

@@ -1,5 +1,5 @@
-// A float32-accumulating linear layer on the CUDA cores (FFMA), for the true 32-bit path and
-// as the fallback for shapes the tensor-core kernel refuses.
+// A float32-accumulating linear layer on the CUDA cores (FFMA), for shapes and operands that the
+// tensor-core kernels refuse (linear_f32_tc.cu, linear_tcgen05.cu) and where they are switched off.
 //
 //   out[m, n] = act( sum_k a[m, k] * w[n, k] + bias[n] ) (+ residual[m, n])
 //

@@ -363,7 +363,7 @@ class CudaOps:
         self.device = dev
         self.lib = load_library()
         self.launches = 0          # kernels launched through this object (graph captures count once)
-        self.tensor_cores = True   # bfloat16 linears on tcgen05 (False: CUDA cores, for tests)
+        self.tensor_cores = True   # linears on tcgen05 (False: CUDA cores, float32 as chains of FMAs; for tests)
         self.fast_attention = True  # bfloat16 attention on the split-context / tensor-core kernels
         self.tc_attention = True    # head size 64: prompt portions on the tcgen05 attention kernel
         self.sm_count = torch.cuda.get_device_properties(dev).multi_processor_count
@@ -557,7 +557,8 @@ class CudaOps:
     def _linear(self, out, a, w, bias, act, residual, M, N, K):
         """``act`` is a code of ACTIVATIONS, or (code, a, b) with the two numbers of an
         activation that has some.  bfloat16 goes to the tcgen05 kernel when TMA can address the operands (K a multiple
-        of 8, 16-byte aligned pointers); everything else, and all of float32, to the CUDA cores."""
+        of 8, 16-byte aligned pointers), float32 with K above 64, a multiple of four, and 16-byte aligned
+        pointers to its products of bfloat16 terms; everything else to the CUDA cores."""
         self.launches += 1
         act, act_a, act_b = act if isinstance(act, tuple) else (act, 0.0, 0.0)
         if a.dtype == torch.bfloat16 and self._skinny_ok(M, N, K):

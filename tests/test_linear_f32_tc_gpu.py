@@ -147,3 +147,54 @@ def test_numbers_that_are_none_take_no_longer_than_chains(m, n, k, what):
         out = torch.empty(m, n, device=DEV)
         times.append(time_of(lambda: ops.linear(out, a, w)))
     assert times[0] <= 2 * times[1]
+
+
+@pytest.mark.parametrize("m", [1, 2, 8, 16, 17, 40])
+@pytest.mark.parametrize("n, k", [(768, 768), (64, 768), (1024, 1028), (6400, 1600), (130, 132), (200, 8192)])
+def test_chunks_and_segments_shared_out(m, n, k):
+    """Few rows: a tile's single chunks or its segments go to blocks, whichever fills the device; the bits of a
+    row do not show it."""
+    ops, g = CudaOps(DEV), torch.Generator(device=DEV).manual_seed(m * n + k)
+    ops.status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    a, w = torch.randn(300, k, device=DEV, generator=g), torch.randn(n, k, device=DEV, generator=g)
+    bias, res = torch.randn(n, device=DEV, generator=g), torch.randn(300, n, device=DEV, generator=g)
+    whole = run(ops, 128, a, w, bias, "silu", res)
+    assert torch.equal(run(ops, 0, a[:m].clone(), w, bias, "silu", res[:m].clone()), whole[:m])
+    assert torch.equal(run(ops, 16, a[:m].clone(), w, bias, "silu", res[:m].clone()), whole[:m])
+    assert ops.status.item() == 0
+
+
+@pytest.mark.parametrize("k", [4, 8, 12, 20, 36, 64, 68, 100, 128, 192])
+def test_short_sums_are_no_further_off_than_chains(k):
+    ops, g = CudaOps(DEV), torch.Generator(device=DEV).manual_seed(k)
+    for shape in (torch.randn, torch.rand):                # (sums that cancel and sums that do not)
+        a, w = shape(300, k, device=DEV, generator=g), shape(640, k, device=DEV, generator=g)
+        exact = a.double() @ w.double().T
+        err = lambda x: float((x.double() - exact).norm())  # noqa: E731
+        assert err(run(ops, 0, a, w)) <= err(chain(ops, a, w))
+
+
+@pytest.mark.parametrize("m, n, k", [(1, 768, 768), (1, 1024, 1024), (8, 768, 768), (1, 6400, 1600), (1024, 1024, 16),
+                                     (64, 1024, 64), (4096, 1024, 32)])
+def test_few_rows_and_short_sums_take_about_as_long_as_chains(m, n, k):
+    ops, g = CudaOps(DEV), torch.Generator(device=DEV).manual_seed(k)
+    a, w = torch.randn(m, k, device=DEV, generator=g), torch.randn(n, k, device=DEV, generator=g)
+    out, times = torch.empty(m, n, device=DEV), []
+    for ops.tensor_cores in (True, False):
+        times.append(time_of(lambda: ops.linear(out, a, w)))
+    assert times[0] <= 1.35 * times[1]
+
+
+@pytest.mark.parametrize("e", [-100, -108, -112, -120, -126])
+def test_numbers_near_the_end_of_the_range(e):
+    """A third term below bfloat16's range is lost: 2^-134 of the other operand a product, nothing above 2^-109."""
+    ops, g = CudaOps(DEV), torch.Generator(device=DEV).manual_seed(-e)
+    a, w = torch.randn(64, 256, device=DEV, generator=g) * 2.0 ** e, torch.randn(128, 256, device=DEV, generator=g)
+    exact = a.double() @ w.double().T
+    # the bound of the sums as above, half a step of bfloat16's smallest a product, float32's own last step
+    sums = (64 / 4 + 4 + 2) * 2.0 ** -23 * (a.abs().double() @ w.abs().double().T)
+    lost = 2.0 ** -134 * w.abs().double().sum(1) + 2.0 ** -149
+    assert bool(((run(ops, 0, a, w).double() - exact).abs() <= sums + lost).all())
+    if e >= -108:
+        err = lambda x: float((x.double() - exact).norm())  # noqa: E731
+        assert err(run(ops, 0, a, w)) <= err(chain(ops, a, w))
