@@ -1300,19 +1300,25 @@ static int cluster_splits(int tiles, int num_kb, int sms) {
 
 // The tile of a layer of more than 128 rows: us a launch takes by rounds of tiles over the device and k
 // blocks, fitted to 70 shapes (512 to 4,096 rows, the layers of GPT-2 small to XL; off by 8 % rms, the choice
-// within 0.4 % of the best on average and 11 % at worst).  Pairs of CTAs load half a weight tile each; with two
+// within 0.4 % of the best on average and 11 % at worst; of 129 to 700 rows it is never slower than the rule
+// by tile sizes alone that it replaced, 7 % faster on average).  Pairs of CTAs load half a weight tile each; with two
 // k blocks a barrier round their 128-wide tiles are the cheapest per k block, alone (2,048 x 1,024 x 4,096: 19.0
 // us, 20.7 as single CTAs).  Behind another kernel a cluster starts later than single CTAs, which take each SM as
 // it falls free: a prompt layer with that shape takes 6 us more with pairs (109 and 102.5; 1,024 rows of width
-// 1,280 104.5 and 97.8), so 6 us are in their launch.
+// 1,280 104.5 and 97.8), so 6 us are in their launch.  From 4,096 rows on a round's end and the power that rounds
+// of many tiles draw count instead: fitted again to 96 shapes of 4,096 to 16,384 rows (off by 7 % rms, the choice
+// within 1.3 % on average; 8,192 x 4,096 x 1,024: 56.8 us with the first fit, 50.6 with this one, 16,384 x 1,024 x
+// 1,024 40.4 and 27.6).
 struct TcShape {
   int bn;
   bool pair;
-  double launch, round, kb;
+  double launch, round, kb;                  // up to 4,095 rows
+  double many_launch, many_round, many_kb;   // from 4,096 rows on
 };
-static const TcShape TC_SHAPES[] = {{64, false, 3.83, 0.363, 0.190},  {128, false, 5.32, 0.376, 0.229},
-                                    {192, false, 4.79, 0.234, 0.346}, {256, false, 5.84, 0.191, 0.371},
-                                    {128, true, 12.1, 0.626, 0.178},  {256, true, 13.7, 0.246, 0.309}};
+static const TcShape TC_SHAPES[] = {
+    {64, false, 3.83, 0.363, 0.190, 2.67, 0.240, 0.214},  {128, false, 5.32, 0.376, 0.229, 2.44, 0.706, 0.256},
+    {192, false, 4.79, 0.234, 0.346, 2.99, 0.840, 0.322}, {256, false, 5.84, 0.191, 0.371, 2.72, 1.078, 0.390},
+    {128, true, 12.1, 0.626, 0.178, 3.65, 0.717, 0.211},  {256, true, 13.7, 0.246, 0.309, 4.36, 0.772, 0.352}};
 static TcShape pick_shape(int M, int N, int num_kb, int pair, int sms) {
   TcShape best = TC_SHAPES[pair == 1 ? 4 : 0];
   double least = -1.0;
@@ -1328,7 +1334,9 @@ static TcShape pick_shape(int M, int N, int num_kb, int pair, int sms) {
       const int splits = g_split_clusters ? cluster_splits((int)tiles, num_kb, sms) : 0;
       cost = s.launch + s.round + s.kb * (splits ? (num_kb + splits - 1) / splits : num_kb) + (splits ? 2.5 : 0.0);
     } else {
-      cost = s.launch + (double)((tiles + units - 1) / units) * (s.round + s.kb * num_kb);
+      const double rounds = (double)((tiles + units - 1) / units);
+      cost = M < 4096 ? s.launch + rounds * (s.round + s.kb * num_kb)
+                      : s.many_launch + rounds * (s.many_round + s.many_kb * num_kb);
     }
     if (least < 0 || cost < least) {
       least = cost;

@@ -34,7 +34,7 @@ def test_the_width_chosen(m, k, n):
     ws = [(torch.randn(n, k, device=DEV, generator=g) * 0.03).bfloat16() for _ in range(max(2, 260_000_000 // (2 * n * k) + 1))]
     out = torch.empty(m, n, device=DEV)
     times = {tile: time_of(ops, out, a, ws, tile) for tile in (0, 128, 192, 256)}
-    assert times.pop(0) <= 1.08 * min(times.values())
+    assert times.pop(0) <= 1.12 * min(times.values())
     want = a.float() @ ws[-1].float().T
     ops.tile_n = 0
     ops.linear(out, a, ws[-1])
