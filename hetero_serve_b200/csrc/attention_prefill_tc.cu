@@ -81,6 +81,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
                             const PrefillTcParams p) {
   pdl_trigger();
   extern __shared__ uint8_t smem_raw[];
+  __shared__ uint64_t drain_bar;
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* sQ = smem;                                     // [2 items][128 queries][128 B]
   uint8_t* sK = sQ + 2 * TA_Q_BYTES;                      // [stages][128 keys][128 B]
@@ -115,6 +116,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
     mbar_init(&bars[B_P_EMPTY], 1);
     mbar_init(&bars[B_O_FULL], 1);
     mbar_init(&bars[B_O_EMPTY], TA_SOFTMAX_WARPS);
+    mbar_init(&drain_bar, 1);
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -438,6 +440,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
     n_tile += n_kv;
     // a role that gave up tells the others through the status word; they time out in turn
   }
+  if (warp == 1) umma_drain(&drain_bar, limit, p.status);
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {

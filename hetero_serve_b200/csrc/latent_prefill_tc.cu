@@ -249,6 +249,7 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
                          const __grid_constant__ CUtensorMap map_kv,
                          const __grid_constant__ CUtensorMap map_rope, const LatentTcParams p) {
   extern __shared__ uint8_t smem_raw[];
+  __shared__ uint64_t drain_bar;
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* sQ = smem;                                    // [NK][128 queries][128 B]
   uint8_t* sK = sQ + NK * LP_CHUNK;                      // [2 stages][NK][128 keys][128 B]
@@ -280,6 +281,7 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
       const bool many = i == LB_S_EMPTY || i == LB_S_EMPTY + 1 || i == LB_P_FULL || i == LB_O_EMPTY;
       mbar_init(&bars[i], many ? LP_SOFTMAX_WARPS : 1);
     }
+    mbar_init(&drain_bar, 1);
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -373,6 +375,7 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
       }
       __syncwarp();
     }
+    umma_drain(&drain_bar, limit, p.status);
   } else {
     const int qtr = warp & 3;                              // TMEM lane quarter of this warp
     const int half = (warp - 2) >> 2;                      // keys 0..63 or 64..127 of a tile

@@ -30,9 +30,6 @@
 // Operands below 2^-109 have a third term below bfloat16's range: a product is off by 2^-134 of the other operand at
 // most, where a chain would keep their digits.
 //
-// Operands below 2^-109 have a third term below bfloat16's range: a product is off by 2^-134 of the other operand at
-// most, where a chain would keep their digits.
-//
 // 1,024 x 4,096 x 1,024: 223 us as FMA chains (linear_simt.cu) -> 68; 1,024 x 1,024 x 4,096: 317 -> 82; 64 x
 // 4,096 x 1,024: 29 -> 16; 8 x 1,024 x 4,096: 19 -> 11; 1 x 768 x 768 5.1 -> 5.6 (8.3 with whole segments a block).  A
 // chunk of a 128 x 128 tile takes 1.8 us: 24 MMAs that read 8 KB of shared memory each (1.5 us alone) beside the
@@ -260,7 +257,7 @@ __global__ void __launch_bounds__(LF_THREADS, 1) linear_f32_tc_kernel(const __gr
   using S = LfShape<NR>;
   extern __shared__ uint8_t lf_smem[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)lf_smem + 1023) & ~(uintptr_t)1023);
-  __shared__ uint64_t full_bar[S::STAGES], empty_bar[S::STAGES], acc_full[2], acc_empty[2];
+  __shared__ uint64_t full_bar[S::STAGES], empty_bar[S::STAGES], acc_full[2], acc_empty[2], drain_bar;
   __shared__ uint32_t tmem_slot;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   pdl_trigger();
@@ -273,6 +270,7 @@ __global__ void __launch_bounds__(LF_THREADS, 1) linear_f32_tc_kernel(const __gr
       mbar_init(&acc_full[b], 1);
       mbar_init(&acc_empty[b], LF_SUM);
     }
+    mbar_init(&drain_bar, 1);
     fence_barrier_init();
   }
   if (warp == LF_CONV + LF_SUM) {
@@ -317,6 +315,7 @@ __global__ void __launch_bounds__(LF_THREADS, 1) linear_f32_tc_kernel(const __gr
         if (++s == S::STAGES) { s = 0; ++round; }
       }
     }
+    umma_drain(&drain_bar, limit, p.status);
   } else if (warp < LF_CONV) {
     // ---- operands: four numbers a piece, 16 pieces a row of a step, 16 rows a pass
     constexpr int PA = LF_BM / 16, PB = NR / 16, AHEAD = S::AHEAD;

@@ -412,6 +412,7 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
   // their MMAs (325 ns for 256 columns) cover the round.
   constexpr int PER = BN <= 128 ? 2 : 1, RING = STAGES / PER;
   extern __shared__ uint8_t smem_raw[];
+  __shared__ uint64_t drain_bar;
   // 128-byte swizzled tiles need 1024-byte alignment
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* full_bar = (uint64_t*)(smem + S::BAR_OFFSET);
@@ -438,6 +439,7 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
       mbar_init(&acc_full[a], 1);
       mbar_init(&acc_empty[a], TC_EPI_WARPS);
     }
+    mbar_init(&drain_bar, 1);
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -542,6 +544,7 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
       if (elect_one()) umma_commit(&acc_full[acc]);      // this accumulator is complete (or the pipeline gave up)
       __syncwarp();
     }
+    umma_drain(&drain_bar, limit, p.status);
   } else if (warp >= 4) {
     // ---------------- epilogue: 8 warps; warp (w % 4) owns TMEM lanes 32*(w%4) .. +31, the two
     // groups of four take the two halves of the columns
@@ -715,6 +718,7 @@ linear_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a,
   using S = PairSmem<BN, STAGES>;
   constexpr int PER = 2, RING = STAGES / PER;           // k blocks a barrier round, as above
   extern __shared__ uint8_t smem_raw[];
+  __shared__ uint64_t drain_bar;
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* full_bar = (uint64_t*)(smem + S::BAR_OFFSET);
   uint64_t* empty_bar = full_bar + STAGES;
@@ -740,6 +744,7 @@ linear_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       mbar_init(&acc_full[a], 1);
       mbar_init(&acc_empty[a], 2 * TC_EPI_WARPS);
     }
+    mbar_init(&drain_bar, 1);
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -831,6 +836,10 @@ linear_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a,
         if (elect_one()) umma_commit_pair(&acc_full[acc], 3);      // both CTAs' epilogues may read
         __syncwarp();
       }
+      if (__any_sync(0xffffffffu, limit == 1)) {                   // as umma_drain
+        if (elect_one()) umma_commit_pair(&drain_bar, 1);
+        mbar_wait(&drain_bar, 0, p.status);
+      }
     }
   } else if (warp >= 4) {
     // ---------------- epilogue: this CTA's 128 rows of the tile
@@ -908,6 +917,7 @@ linear_tcgen05_cluster_kernel(const __grid_constant__ CUtensorMap map_a,
                               const __grid_constant__ CUtensorMap map_w, const TcParams p) {
   using S = ClSmem;
   extern __shared__ uint8_t smem_raw[];
+  __shared__ uint64_t drain_bar;
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   float* red = (float*)(smem + S::RED_OFFSET);
   uint64_t* full_bar = (uint64_t*)(smem + S::BAR_OFFSET);
@@ -932,6 +942,7 @@ linear_tcgen05_cluster_kernel(const __grid_constant__ CUtensorMap map_a,
       mbar_init(&empty_bar[s], 1);
     }
     mbar_init(acc_full, 1);
+    mbar_init(&drain_bar, 1);
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -997,6 +1008,7 @@ linear_tcgen05_cluster_kernel(const __grid_constant__ CUtensorMap map_a,
     }
     if (elect_one()) umma_commit(acc_full);   // the partial tile is complete (or the pipeline gave up)
     __syncwarp();
+    umma_drain(&drain_bar, limit, p.status);
   }
 
   // rows of the tile that exist, dealt to the CTAs of the cluster in blocks of `rpo`

@@ -18,7 +18,8 @@
 // and up 32 us, down 16, against 93 and 56 with 64 x 64 tiles on mma.sync; 64 tokens 30 us in all against
 // 67 (a kernel for few pairs a tile is not needed).  The floor is the weights: 15 us.
 //
-// Every wait is bounded (tcgen05.cuh); a wait that runs out sets the status bit and the block leaves.
+// Every wait is bounded (tcgen05.cuh); a wait that runs out sets the status bit, its warp leaves, and the issuing
+// warp goes on with waits that look once, then waits for the MMAs it has issued.
 #include "tcgen05.cuh"
 #include "moe_tiles_tc.cuh"
 
@@ -118,7 +119,7 @@ moe_tiles_tc_kernel(const __grid_constant__ CUtensorMap map_w0,
   constexpr int TMA_WARP = MT_EPI_WARPS + (GATHER ? MT_LOAD_WARPS : 0), MMA_WARP = TMA_WARP + 1;
   extern __shared__ uint8_t mt_smem[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)mt_smem + 1023) & ~(uintptr_t)1023);
-  __shared__ uint64_t full_bar[MT_MAX_STAGES], empty_bar[MT_MAX_STAGES], acc_full[2], acc_empty[2];
+  __shared__ uint64_t full_bar[MT_MAX_STAGES], empty_bar[MT_MAX_STAGES], acc_full[2], acc_empty[2], drain_bar;
   __shared__ uint32_t tmem_slot;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   pdl_trigger();
@@ -131,6 +132,7 @@ moe_tiles_tc_kernel(const __grid_constant__ CUtensorMap map_w0,
       mbar_init(&acc_full[a], 1);
       mbar_init(&acc_empty[a], MT_EPI_WARPS);
     }
+    mbar_init(&drain_bar, 1);
     fence_barrier_init();
   }
   if (warp == MMA_WARP) {
@@ -208,6 +210,7 @@ moe_tiles_tc_kernel(const __grid_constant__ CUtensorMap map_w0,
       if (elect_one()) umma_commit(&acc_full[acc]);
       __syncwarp();
     }
+    umma_drain(&drain_bar, limit, p.status);
   } else if (GATHER && warp >= MT_EPI_WARPS) {
     // a piece of 16 bytes is column c of its row, rows r0, r0 + 16, ..; a row beyond the segment, and
     // numbers beyond K, are zeros.  Each thread's copies arrive at the stage's barrier when they have

@@ -116,6 +116,14 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
                    smem_u32(bar))
                : "memory");
 }
+// Called by the whole issuing warp at its end.  After a wait that ran out it has gone on issuing MMAs nobody waits
+// for; the block must not give tensor and shared memory back under them, so they are waited for here, within a limit.
+// `bar`: for one arrival, used for nothing else.
+__device__ __forceinline__ void umma_drain(uint64_t* bar, uint32_t limit, int* status) {
+  if (!__any_sync(0xffffffffu, limit == 1)) return;
+  if (elect_one()) umma_commit(bar);
+  mbar_wait(bar, 0, status);
+}
 // ---- the same for a pair of CTAs (cta_group::2): a cluster of two CTAs on neighbouring SMs
 // works on one tile; the even CTA of the pair issues the MMAs, which read both CTAs' shared
 // memory (at the same offsets) and write both CTAs' tensor memory.
